@@ -21,7 +21,7 @@ namespace bsp {
 
 bsp_status csr2blocks(int32_t rows, int32_t nnz, const int32_t *rowPtr, const int32_t *colIdx, const double *values,
                       int32_t tm, int32_t tk, int32_t *blc_num_out, int32_t **blcPtr, int32_t **blcIdx,
-                      double **blcVal, uint16_t **map16, uint64_t **map64, cudaStream_t s);
+                      double **blcVal, uint16_t **map16, uint64_t **map64, int32_t *d_full, cudaStream_t s);
 
 __global__ void bcsr_mapping_kernel(int32_t nr, int32_t nc, const int32_t *__restrict__ rp,
                                     const int32_t *__restrict__ ci, int32_t *__restrict__ mapping) {
@@ -80,7 +80,7 @@ extern "C" bsp_status bsp_csr2bcsr(int32_t rows, int32_t cols, int32_t nnz, cons
   if (with_mapping && b.blockNum > ((int64_t)1 << 31))
     BSP_FAIL(BSP_ERR_UNSUPPORTED, "dense block mapping larger than 2^31 entries");
   BSP_TRY(csr2blocks(rows, nnz, rowPtr, colIdx, values, tile_m, tile_k, &b.nonzeroBlocks, &b.bcsrRowPtr,
-                     &b.bcsrcolIdx, &b.values, nullptr, nullptr, s));
+                     &b.bcsrcolIdx, &b.values, nullptr, nullptr, nullptr, s));
   b.elemCount = b.nonzeroBlocks * tile_m * tile_k;
   if (with_mapping) {
     BSP_TRY(dalloc(&b.relativeBlockIndexMapping, (size_t)b.blockNum, s));

@@ -112,6 +112,10 @@ __device__ __forceinline__ f64x4 ld_x4(const double *p) {
   asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
   return r;
 }
+// 256-bit store (32-byte aligned).
+__device__ __forceinline__ void st_f64x4(double *p, double x, double y, double z, double w) {
+  asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(p), "d"(x), "d"(y), "d"(z), "d"(w) : "memory");
+}
 __device__ __forceinline__ uint64_t evict_first_policy() {
   uint64_t pol;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));

@@ -138,6 +138,188 @@ __global__ void bsr_fill_kernel(int32_t rows, int32_t tm, int32_t tk, const int3
   }
 }
 
+// Square BS x BS blocks (4 or 8) of matrices without very long rows: the
+// block-row's BS sorted rows are merged directly, a lane per row, so a warp
+// walks 32 / BS block-rows at once.  Each trip takes the smallest block column
+// any of the BS lanes stands at; every lane then holds its own row of that
+// block (at most BS entries, loaded together) and in the fill pass stores it
+// whole -- values and zeros, 32 bytes per store, the BS lanes one contiguous
+// block -- so there are no searches, no per-nonzero position array, no zeroing
+// pass over the values and no atomics on the bitmaps.  The counting pass is
+// the same walk over the column indices alone.
+//
+// Bound by HBM: 27-point stencil 64^3 x 4 dof (110 M nonzeros), columns read
+// once to count (439 MB, 126 us), columns and values once to fill (1.3 GB) and
+// 906 MB written (496 us, 4.5 TB/s); the per-nonzero searches with their
+// position array took 4.4 ms for the same.  The value loads allocate in L1:
+// a lane returns to its line for the next blocks (without it every line was
+// fetched twice from DRAM, 829 us), which is also why more resident warps lose
+// (8 CTAs per SM: 804 us).  8x8 blocks, 61^3: 591 us at 5 CTAs per SM, 630 at 4.
+// A lane walks its row serially and a block takes a trip whatever it holds, so
+// scattered matrices and a few long rows keep the general path (merge_wins).
+// VEC: colIdx 16-byte and values 32-byte aligned; a lane at an aligned entry
+// then loads 4 columns (4 values) at once.
+template <int BS>
+struct MergeRun {
+  int32_t c[BS + 1];  // columns of entries j .. j + BS (-1 past the row's end)
+};
+
+template <int BS, bool VEC>
+__device__ __forceinline__ void merge_load(const int32_t *__restrict__ colIdx, int32_t j, int32_t e,
+                                           MergeRun<BS> &w) {
+#pragma unroll
+  for (int k = 0; k < BS; k += 4) {
+    if (VEC && (j & 3) == 0 && j + k + 4 <= e) {
+      const int4 t = __ldg(reinterpret_cast<const int4 *>(colIdx + j + k));
+      w.c[k] = t.x;
+      w.c[k + 1] = t.y;
+      w.c[k + 2] = t.z;
+      w.c[k + 3] = t.w;
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) w.c[k + u] = j + k + u < e ? __ldg(colIdx + j + k + u) : -1;
+    }
+  }
+  w.c[BS] = j + BS < e ? __ldg(colIdx + j + BS) : -1;
+}
+
+// What the choice between the two conversions rests on: the longest row, and
+// the entries per block in evenly spaced block-rows (the first warp of every
+// CTA merges 32 / BS of them, at most kSampleTrips blocks each).
+struct BlockProfile {
+  int64_t total;  // blocks of the whole matrix (the counting pass's scan)
+  int32_t longest, blocks, entries, pad;
+};
+constexpr int kSampleTrips = 16;
+
+template <int BS>
+__global__ void __launch_bounds__(256) bsr_profile_kernel(int32_t rows, int32_t blc_row,
+                                                          const int32_t *__restrict__ rowPtr,
+                                                          const int32_t *__restrict__ colIdx, BlockProfile *out) {
+  constexpr int32_t kNone = INT32_MAX;
+  const int lane = threadIdx.x & 31;
+  int32_t longest = 0;
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x)
+    longest = max(longest, rowPtr[r + 1] - rowPtr[r]);
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  if (lane == 0) atomicMax(&out->longest, longest);
+  if (threadIdx.x >= 32) return;
+  const int64_t r = (int64_t)blc_row * blockIdx.x / gridDim.x * BS + lane;
+  int32_t j = r < rows ? rowPtr[r] : 0, blocks = 0, entries = 0;
+  const int32_t e = r < rows ? rowPtr[r + 1] : 0;
+  int32_t cur = j < e ? colIdx[j] / BS : kNone;
+  for (int t = 0; t < kSampleTrips; ++t) {
+    int32_t m = cur;
+#pragma unroll
+    for (int o = 1; o < BS; o <<= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (__all_sync(0xffffffffu, m == kNone)) break;
+    blocks += m != kNone && lane % BS == 0;
+    while (cur == m && m != kNone) {
+      ++entries;
+      cur = ++j < e ? colIdx[j] / BS : kNone;
+    }
+  }
+  blocks = __reduce_add_sync(0xffffffffu, blocks);
+  entries = __reduce_add_sync(0xffffffffu, entries);
+  if (lane == 0) {
+    atomicAdd(&out->blocks, blocks);
+    atomicAdd(&out->entries, entries);
+  }
+}
+
+template <int BS, bool FILL, bool VEC, typename MapT>
+__global__ void __launch_bounds__(256, BS == 8 ? 5 : 1)
+    bsr_merge_kernel(int32_t rows, int32_t blc_row, const int32_t *__restrict__ rowPtr,
+                     const int32_t *__restrict__ colIdx, const double *__restrict__ val, int32_t *__restrict__ cnt,
+                     const int32_t *__restrict__ blcPtr,
+                     int32_t *__restrict__ blcIdx, double *__restrict__ blcVal, MapT *__restrict__ map,
+                     int32_t *__restrict__ full) {
+  constexpr int32_t kNone = INT32_MAX;
+  const int lane = threadIdx.x & 31, br_lane = lane % BS;
+  const int64_t nrow = (int64_t)blc_row * BS, stride = (int64_t)gridDim.x * blockDim.x;
+  int32_t nfull = 0;
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r - lane < nrow; r += stride) {
+    int32_t j = r < rows ? rowPtr[r] : 0;
+    const int32_t e = r < rows ? rowPtr[r + 1] : 0;
+    const int64_t br = r / BS;
+    int64_t blk = FILL && br < blc_row ? blcPtr[br] : 0;
+    const int64_t blk0 = blk;
+    MergeRun<BS> w;
+    merge_load<BS, VEC>(colIdx, j, e, w);
+    int32_t cur = w.c[0] >= 0 ? w.c[0] / BS : kNone;
+    for (;;) {
+      int32_t m = cur;
+#pragma unroll
+      for (int o = 1; o < BS; o <<= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if (__all_sync(0xffffffffu, m == kNone)) break;
+      // entries of my row in block column m: the first n of the window
+      int n = 0;
+      bool in = cur == m && m != kNone;
+      unsigned bits = 0;
+      bool take[BS];
+#pragma unroll
+      for (int k = 0; k < BS; ++k) {
+        in = in && w.c[k] >= 0 && w.c[k] / BS == m;
+        take[k] = in;
+        n += in;
+        if (in) bits |= 1u << (w.c[k] - m * BS);
+      }
+      if constexpr (FILL) {
+        double a[BS], out[BS];
+#pragma unroll
+        for (int k = 0; k < BS; k += 4) {
+          if (VEC && (j & 3) == 0 && take[k + 3]) {
+            const f64x4 t = ld_x4(val + j + k);
+            a[k] = t.x;
+            a[k + 1] = t.y;
+            a[k + 2] = t.z;
+            a[k + 3] = t.w;
+          } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) a[k + u] = take[k + u] ? __ldg(val + j + k + u) : 0.0;
+          }
+        }
+        if (n == BS) {  // a whole block row: columns m*BS .. m*BS + BS - 1 in order
+#pragma unroll
+          for (int q = 0; q < BS; ++q) out[q] = a[q];
+        } else {
+#pragma unroll
+          for (int q = 0; q < BS; ++q) {
+            out[q] = 0.0;
+#pragma unroll
+            for (int k = 0; k < BS; ++k)
+              if (take[k] && w.c[k] - m * BS == q) out[q] = a[k];
+          }
+        }
+        if (m != kNone) {
+          double *p = blcVal + (blk * BS + br_lane) * BS;
+#pragma unroll
+          for (int q = 0; q < BS; q += 4) st_f64x4(p + q, out[q], out[q + 1], out[q + 2], out[q + 3]);
+        }
+        uint64_t mb = (uint64_t)bits << (br_lane * BS);
+#pragma unroll
+        for (int o = 1; o < BS; o <<= 1) mb |= __shfl_xor_sync(0xffffffffu, mb, o);
+        if (m != kNone && br_lane == 0) {
+          blcIdx[blk] = m;
+          if (map) map[blk] = (MapT)mb;
+          nfull += mb == (BS == 4 ? 0xffffull : ~0ull);
+        }
+      }
+      if (m != kNone) ++blk;
+      if (n) {
+        j += n;
+        merge_load<BS, VEC>(colIdx, j, e, w);
+        cur = w.c[0] >= 0 ? w.c[0] / BS : kNone;
+      }
+    }
+    if (!FILL && br_lane == 0 && br < blc_row) cnt[br] = (int32_t)(blk - blk0);
+  }
+  if constexpr (FILL) {
+    nfull = __reduce_add_sync(0xffffffffu, nfull);
+    if (full && lane == 0 && nfull) atomicAdd(full, nfull);
+  }
+}
+
 __global__ void bsr_chunks_kernel(int32_t blc_row, const int32_t *__restrict__ blcPtr, int32_t *__restrict__ cnt,
                                   double avg_len, double *__restrict__ sq) {
   // cnt[br] = ceil(len/64) (get_rowPtrbyWarp, amgT.cu:523); sq[br] = (len-avg)^2.
@@ -157,19 +339,24 @@ __global__ void bsr_rowidx_kernel(int32_t blc_row, const int32_t *__restrict__ r
     for (int32_t w = rowPtrbyWarp[br]; w < rowPtrbyWarp[br + 1]; ++w) rowIdxbyWarp[w] = (int32_t)br;
 }
 
-// Deterministic sum of doubles (single CTA, fixed order per thread then a
-// fixed tree), for the block-length standard deviation.
-__global__ void sum_f64_kernel(const double *__restrict__ v, int64_t n, double *__restrict__ out) {
+// Deterministic sum of doubles for the block-length standard deviation: every
+// CTA sums its strided share (fixed tree), then one CTA the partials.  One CTA
+// over everything was a chain of n / 256 dependent additions (262,144
+// block-rows: 95 us; two stages 6 us).
+constexpr int kSumCtas = 148;
+
+__global__ void __launch_bounds__(256) sum_f64_kernel(const double *__restrict__ v, int64_t n,
+                                                      double *__restrict__ out) {
   __shared__ double part[256];
   double s = 0.0;
-  for (int64_t i = threadIdx.x; i < n; i += 256) s += v[i];
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) s += v[i];
   part[threadIdx.x] = s;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
     if (threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *out = part[0];
+  if (threadIdx.x == 0) out[blockIdx.x] = part[0];
 }
 
 __global__ void count_full_blocks_kernel(int64_t nb, int bs, const void *map, int32_t *out) {
@@ -198,49 +385,128 @@ static unsigned grid_for(int64_t n, int threads) {
   return (unsigned)b;
 }
 
-static unsigned grid_for(int64_t n, int threads);
+template <int BS, typename MapT>
+static bsp_status merge_fill(int32_t rows, int32_t blc_row, const int32_t *rowPtr, const int32_t *colIdx,
+                             const double *values, bool vec, const int32_t *blcPtr, int32_t *blcIdx, double *blcVal,
+                             MapT *map, int32_t *d_full, cudaStream_t s) {
+  const unsigned g = grid_for((int64_t)blc_row * BS, 256);
+  if (vec)
+    bsr_merge_kernel<BS, true, true, MapT><<<g, 256, 0, s>>>(rows, blc_row, rowPtr, colIdx, values, nullptr,
+                                                             blcPtr, blcIdx, blcVal, map, d_full);
+  else
+    bsr_merge_kernel<BS, true, false, MapT><<<g, 256, 0, s>>>(rows, blc_row, rowPtr, colIdx, values, nullptr,
+                                                              blcPtr, blcIdx, blcVal, map, d_full);
+  BSP_LAUNCH_CHECK();
+  return BSP_OK;
+}
+
+template <int BS>
+static bsp_status merge_count(int32_t rows, int32_t blc_row, const int32_t *rowPtr, const int32_t *colIdx, bool vec,
+                              int32_t *cnt, cudaStream_t s) {
+  const unsigned g = grid_for((int64_t)blc_row * BS, 256);
+  if (vec)
+    bsr_merge_kernel<BS, false, true, uint64_t><<<g, 256, 0, s>>>(rows, blc_row, rowPtr, colIdx, nullptr, cnt,
+                                                                  nullptr, nullptr, nullptr, nullptr, nullptr);
+  else
+    bsr_merge_kernel<BS, false, false, uint64_t><<<g, 256, 0, s>>>(rows, blc_row, rowPtr, colIdx, nullptr, cnt,
+                                                                   nullptr, nullptr, nullptr, nullptr, nullptr);
+  BSP_LAUNCH_CHECK();
+  return BSP_OK;
+}
+
+// Whether merging the rows beats searching per nonzero.  The merge takes one
+// trip per block: with fewer than 3 entries per block it moves mostly zeros
+// (400,000 random rows of 16, 8x8: 1470 us against 1306), and the block-row
+// with the most blocks sets a serial chain of about 1.2 us per block over the
+// two passes (4096 random rows of 64: 256 blocks, 311 us against 78).  The
+// search takes 41 ps (4x4) or 66 ps (8x8) per nonzero and no less than about
+// 100 us at row lengths where the chain could matter.
+static bool merge_wins(int bs, const BlockProfile &p, int32_t nnz) {
+  if (p.blocks == 0 || p.entries < 3 * (int64_t)p.blocks) return false;
+  const double blocks = (double)bs * p.longest * p.blocks / p.entries;
+  return blocks * 1.2e-6 <= std::max(100e-6, nnz * (bs == 4 ? 41e-12 : 66e-12));
+}
 
 // Canonical tm x tk blocking of a CSR matrix (block columns ascending per
 // block-row, row-major values).  map16 (tm*tk <= 16) or map64 (<= 64) get the
-// occupancy bitmaps when non-null.  Outputs are allocated here.
+// occupancy bitmaps when non-null; d_full (with a map, zeroed by the caller)
+// the number of full blocks.  Outputs are allocated here.
+//
+// 4x4 and 8x8 blocks merge the rows of a block-row (bsr_merge_kernel) where
+// merge_wins says so; other shapes and matrices search per nonzero
+// (bsr_canonical_kernel, bsr_fill_kernel).
 bsp_status csr2blocks(int32_t rows, int32_t nnz, const int32_t *rowPtr, const int32_t *colIdx, const double *values,
                       int32_t tm, int32_t tk, int32_t *blc_num_out, int32_t **blcPtr, int32_t **blcIdx,
-                      double **blcVal, uint16_t **map16, uint64_t **map64, cudaStream_t s) {
+                      double **blcVal, uint16_t **map16, uint64_t **map64, int32_t *d_full, cudaStream_t s) {
   const int32_t blc_row = (int32_t)ceil_div(rows, tm);
   int32_t *pos = nullptr;
-  int64_t *d_total = nullptr;
-  BSP_TRY(dalloc(&pos, (size_t)nnz + 1, s));
-  BSP_TRY(dalloc(&d_total, 2, s));
-  BSP_CUDA(cudaMemsetAsync(pos + nnz, 0, sizeof(int32_t), s));
-  if (nnz > 0) {
-    bsr_canonical_kernel<<<grid_for((int64_t)rows * 32, 256), 256, 0, s>>>(rows, tm, tk, rowPtr, colIdx, pos);
-    BSP_LAUNCH_CHECK();
-  }
-  BSP_TRY(exclusive_scan_i32(pos, pos, (int64_t)nnz + 1, d_total, s));
-  int64_t total = 0;
-  BSP_TRY(read_i64(d_total, &total, s));
-  dfree(d_total, s);
-  if (total > INT32_MAX / ((int64_t)tm * tk)) BSP_FAIL(BSP_ERR_UNSUPPORTED, "too many blocks for int32 indexing");
-  const int32_t nb = (int32_t)total;
-  *blc_num_out = nb;
+  BlockProfile h{}, *d_meta = nullptr;
+  BSP_TRY(dalloc(&d_meta, 1, s));
+  BSP_CUDA(cudaMemsetAsync(d_meta, 0, sizeof(BlockProfile), s));
   BSP_TRY(dalloc(blcPtr, (size_t)blc_row + 1, s));
-  bsr_ptr_kernel<<<grid_for((int64_t)blc_row + 1, 256), 256, 0, s>>>(rows, blc_row, tm, rowPtr, pos, *blcPtr);
-  BSP_LAUNCH_CHECK();
+  auto read_meta = [&]() -> bsp_status {
+    BSP_CUDA(cudaMemcpyAsync(&h, d_meta, sizeof(BlockProfile), cudaMemcpyDeviceToHost, s));
+    BSP_CUDA(cudaStreamSynchronize(s));
+    return BSP_OK;
+  };
+  const bool vec = ((uintptr_t)colIdx & 15) == 0 && ((uintptr_t)values & 31) == 0;
+  bool merge = tm == tk && (tm == 4 || tm == 8) && nnz > 0;
+  if (merge) {
+    const unsigned g = (unsigned)std::min<int64_t>(sm_count(), ceil_div(rows, 256));
+    if (tm == 4)
+      bsr_profile_kernel<4><<<g, 256, 0, s>>>(rows, blc_row, rowPtr, colIdx, d_meta);
+    else
+      bsr_profile_kernel<8><<<g, 256, 0, s>>>(rows, blc_row, rowPtr, colIdx, d_meta);
+    BSP_LAUNCH_CHECK();
+    BSP_TRY(read_meta());
+    merge = merge_wins(tm, h, nnz);
+  }
+  if (merge) {
+    BSP_CUDA(cudaMemsetAsync(*blcPtr + blc_row, 0, sizeof(int32_t), s));
+    BSP_TRY(tm == 4 ? merge_count<4>(rows, blc_row, rowPtr, colIdx, vec, *blcPtr, s)
+                    : merge_count<8>(rows, blc_row, rowPtr, colIdx, vec, *blcPtr, s));
+    BSP_TRY(exclusive_scan_i32(*blcPtr, *blcPtr, (int64_t)blc_row + 1, &d_meta->total, s));
+    BSP_TRY(read_meta());
+  } else {
+    BSP_TRY(dalloc(&pos, (size_t)nnz + 1, s));
+    BSP_CUDA(cudaMemsetAsync(pos + nnz, 0, sizeof(int32_t), s));
+    if (nnz > 0) {
+      bsr_canonical_kernel<<<grid_for((int64_t)rows * 32, 256), 256, 0, s>>>(rows, tm, tk, rowPtr, colIdx, pos);
+      BSP_LAUNCH_CHECK();
+    }
+    BSP_TRY(exclusive_scan_i32(pos, pos, (int64_t)nnz + 1, &d_meta->total, s));
+    BSP_TRY(read_meta());
+  }
+  dfree(d_meta, s);
+  if (h.total > INT32_MAX / ((int64_t)tm * tk)) BSP_FAIL(BSP_ERR_UNSUPPORTED, "too many blocks for int32 indexing");
+  const int32_t nb = (int32_t)h.total;
+  *blc_num_out = nb;
   BSP_TRY(dalloc(blcIdx, (size_t)nb, s));
   BSP_TRY(dalloc(blcVal, (size_t)nb * tm * tk, s));
+  // blc_num + 1 map entries as the reference allocates (amgT.cu:1162); the
+  // 16-bit map is rounded up to whole 32-bit words for the word-wide OR.
+  const size_t n16 = ((size_t)nb + 2) & ~size_t(1);
+  if (map16) BSP_TRY(dalloc(map16, n16, s));
+  if (map64) BSP_TRY(dalloc(map64, (size_t)nb + 1, s));
+  if (merge) {
+    if (map16) BSP_CUDA(cudaMemsetAsync(*map16 + nb, 0, sizeof(uint16_t) * (n16 - nb), s));
+    if (map64) BSP_CUDA(cudaMemsetAsync(*map64 + nb, 0, sizeof(uint64_t), s));
+    if (tm == 4)
+      return merge_fill<4, uint16_t>(rows, blc_row, rowPtr, colIdx, values, vec, *blcPtr, *blcIdx, *blcVal,
+                                     map16 ? *map16 : nullptr, d_full, s);
+    return merge_fill<8, uint64_t>(rows, blc_row, rowPtr, colIdx, values, vec, *blcPtr, *blcIdx, *blcVal,
+                                   map64 ? *map64 : nullptr, d_full, s);
+  }
+  bsr_ptr_kernel<<<grid_for((int64_t)blc_row + 1, 256), 256, 0, s>>>(rows, blc_row, tm, rowPtr, pos, *blcPtr);
+  BSP_LAUNCH_CHECK();
   BSP_CUDA(cudaMemsetAsync(*blcVal, 0, sizeof(double) * (size_t)nb * tm * tk, s));
   const unsigned g = grid_for((int64_t)rows * 32, 256);
   if (map16) {
-    // blc_num + 1 entries as the reference allocates (amgT.cu:1162), rounded
-    // up to whole 32-bit words for the word-wide OR.
-    const size_t n16 = ((size_t)nb + 2) & ~size_t(1);
-    BSP_TRY(dalloc(map16, n16, s));
     BSP_CUDA(cudaMemsetAsync(*map16, 0, sizeof(uint16_t) * n16, s));
     if (nnz > 0)
       bsr_fill_kernel<uint16_t><<<g, 256, 0, s>>>(rows, tm, tk, rowPtr, colIdx, values, pos, *blcPtr, *blcIdx,
                                                   *blcVal, *map16);
   } else if (map64) {
-    BSP_TRY(dalloc(map64, (size_t)nb + 1, s));
     BSP_CUDA(cudaMemsetAsync(*map64, 0, sizeof(uint64_t) * ((size_t)nb + 1), s));
     if (nnz > 0)
       bsr_fill_kernel<uint64_t><<<g, 256, 0, s>>>(rows, tm, tk, rowPtr, colIdx, values, pos, *blcPtr, *blcIdx,
@@ -250,6 +516,11 @@ bsp_status csr2blocks(int32_t rows, int32_t nnz, const int32_t *rowPtr, const in
                                             nullptr);
   }
   BSP_LAUNCH_CHECK();
+  if (d_full && nb > 0) {
+    count_full_blocks_kernel<<<grid_for(nb, 256), 256, 0, s>>>(nb, tm, map16 ? (void *)*map16 : (void *)*map64,
+                                                              d_full);
+    BSP_LAUNCH_CHECK();
+  }
   dfree(pos, s);
   return BSP_OK;
 }
@@ -265,8 +536,11 @@ bsp_status csr2bsr_impl(int32_t rows, int32_t cols, int32_t nnz, const int32_t *
   m.true_nnz = nnz;
   uint16_t *m16 = nullptr;
   uint64_t *m64 = nullptr;
+  int32_t *d_full = nullptr;
+  BSP_TRY(dalloc(&d_full, 1, s));
+  BSP_CUDA(cudaMemsetAsync(d_full, 0, sizeof(int32_t), s));
   BSP_TRY(csr2blocks(rows, nnz, rowPtr, colIdx, values, bs, bs, &m.blc_num, &m.blcPtr, &m.blcIdx, &m.blcVal,
-                     bs == 4 ? &m16 : nullptr, bs == 4 ? nullptr : &m64, s));
+                     bs == 4 ? &m16 : nullptr, bs == 4 ? nullptr : &m64, d_full, s));
   m.blcMap = bs == 4 ? (void *)m16 : (void *)m64;
   m.nnz = m.blc_num * bs * bs;
   m.avg_nnz = m.blc_num > 0 ? (double)nnz / (double)m.blc_num : 0.0;
@@ -277,7 +551,7 @@ bsp_status csr2bsr_impl(int32_t rows, int32_t cols, int32_t nnz, const int32_t *
   double *sq = nullptr, *d_sum = nullptr;
   BSP_TRY(dalloc(&m.rowPtrbyWarp, (size_t)m.blc_row + 1, s));
   BSP_TRY(dalloc(&sq, (size_t)m.blc_row + 1, s));
-  BSP_TRY(dalloc(&d_sum, 1, s));
+  BSP_TRY(dalloc(&d_sum, kSumCtas + 1, s));
   const double avg_len = m.blc_row > 0 ? (double)m.blc_num / (double)m.blc_row : 0.0;
   BSP_CUDA(cudaMemsetAsync(m.rowPtrbyWarp, 0, sizeof(int32_t) * ((size_t)m.blc_row + 1), s));
   if (m.blc_row > 0) {
@@ -286,26 +560,22 @@ bsp_status csr2bsr_impl(int32_t rows, int32_t cols, int32_t nnz, const int32_t *
   }
   BSP_TRY(exclusive_scan_i32(m.rowPtrbyWarp, m.rowPtrbyWarp, (int64_t)m.blc_row + 1, d_total, s));
   int64_t warpnum = 0;
+  double ss = 0.0;
+  if (m.blc_row > 0) {
+    sum_f64_kernel<<<kSumCtas, 256, 0, s>>>(sq, m.blc_row, d_sum + 1);
+    BSP_LAUNCH_CHECK();
+    sum_f64_kernel<<<1, 256, 0, s>>>(d_sum + 1, kSumCtas, d_sum);
+    BSP_LAUNCH_CHECK();
+    BSP_CUDA(cudaMemcpyAsync(&ss, d_sum, sizeof(double), cudaMemcpyDeviceToHost, s));
+  }
   BSP_TRY(read_i64(d_total, &warpnum, s));
   m.warpnum = (int32_t)warpnum;
   BSP_TRY(dalloc(&m.rowIdxbyWarp, (size_t)m.warpnum, s));
   if (m.blc_row > 0) {
     bsr_rowidx_kernel<<<grid_for(m.blc_row, 256), 256, 0, s>>>(m.blc_row, m.rowPtrbyWarp, m.rowIdxbyWarp);
     BSP_LAUNCH_CHECK();
-    sum_f64_kernel<<<1, 256, 0, s>>>(sq, m.blc_row, d_sum);
-    BSP_LAUNCH_CHECK();
-    double ss = 0.0;
-    BSP_CUDA(cudaMemcpyAsync(&ss, d_sum, sizeof(double), cudaMemcpyDeviceToHost, s));
-    BSP_CUDA(cudaStreamSynchronize(s));
     // The reference takes a single-precision square root (amgT.cu:1155).
     m.stand = (double)sqrtf((float)(ss / m.blc_row));
-  }
-  int32_t *d_full = nullptr;
-  BSP_TRY(dalloc(&d_full, 1, s));
-  BSP_CUDA(cudaMemsetAsync(d_full, 0, sizeof(int32_t), s));
-  if (m.blc_num > 0) {
-    count_full_blocks_kernel<<<grid_for(m.blc_num, 256), 256, 0, s>>>(m.blc_num, bs, m.blcMap, d_full);
-    BSP_LAUNCH_CHECK();
   }
   BSP_TRY(read_i32(d_full, &m.dense_blocks, s));
   dfree(d_full, s);

@@ -158,3 +158,59 @@ def test_bsr_host_pipelined_matches_host_call(cuda, kind, chunks):
         P.set_ctas(-1)
     P.close()
     M.free()
+
+
+def _blocky(rows, cols, lens, bs, seed):
+    """CSR with about the given row lengths, columns ascending without repeats.
+    Rows of a block-row share their block columns (whole, or with every third
+    entry missing), so the conversion merges them."""
+    rng = np.random.default_rng(seed)
+    nbc = -(-cols // bs)
+    rp, ci = [0], []
+    for r, k in enumerate(lens):
+        if r % bs == 0:
+            order = rng.permutation(nbc)
+        c = (np.sort(order[:min(nbc, -(-k // bs))])[:, None] * bs + np.arange(bs)).ravel()
+        c = c[c < cols][:k]
+        if r % 3 == 1:
+            c = c[(np.arange(c.size) + r) % 3 > 0]
+        ci.append(c)
+        rp.append(rp[-1] + c.size)
+    return np.array(rp, np.int32), np.concatenate(ci).astype(np.int32), rng.standard_normal(rp[-1])
+
+
+# rows and columns around multiples of the block, empty block-rows, one long
+# row, rows past a warp's and a CTA's share, and input arrays off their 16- and
+# 32-byte boundaries; `scattered` rows share no blocks and take the search
+@pytest.mark.parametrize("rows,cols,longest,shift,scattered", [
+    (1, 1, 1, 0, False), (3, 5, 5, 0, False), (4, 4, 4, 0, False), (5, 9, 9, 1, False), (33, 70, 40, 0, False),
+    (127, 260, 100, 3, False), (256, 1031, 31, 0, False), (1025, 4099, 64, 2, False), (64, 1500, 300, 0, False),
+    (4097, 6000, 20, 0, True), (65, 1500, 1400, 2, True)])
+@pytest.mark.parametrize("bs", [4, 8])
+def test_csr2bsr_both_conversions_at_the_edges(cuda, rows, cols, longest, shift, scattered, bs):
+    import torch
+    rng = np.random.default_rng(rows * 7 + longest)
+    lens = rng.integers(0, min(longest, 30) + 1, rows)
+    lens[rng.integers(rows)] = longest
+    if rows > 40:
+        lens[16:32] = 0
+        lens[rows - 1] = longest
+    if scattered:
+        rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+        ci = np.concatenate([np.sort(rng.choice(cols, k, replace=False)) for k in lens]).astype(np.int32)
+        va = rng.standard_normal(rp[-1])
+    else:
+        rp, ci, va = _blocky(rows, cols, lens, bs, rows)
+    drp = torch.from_numpy(rp).to(cuda)
+    dci = torch.empty(ci.size + shift, dtype=torch.int32, device=cuda)[shift:]
+    dva = torch.empty(va.size + shift, dtype=torch.float64, device=cuda)[shift:]
+    dci.copy_(torch.from_numpy(ci))
+    dva.copy_(torch.from_numpy(va))
+    M = bsp.csr2bsr(drp, dci, dva, rows=rows, cols=cols, bs=bs)
+    o = pyoracle.csr2bsr(rows, cols, rp, ci, va, bs)
+    _check_arrays(M, o)
+    full = 0xffff if bs == 4 else 0xffffffffffffffff
+    assert M.dense_blocks == int(np.sum(o["blcMap"][:o["blc_num"]].astype(np.uint64) == full))
+    a = bsp.csr2bcsr(drp, dci, dva, rows=rows, cols=cols, tile_m=bs, tile_k=bs).arrays()
+    assert np.array_equal(a["bcsrColIdx"], o["blcIdx"]) and np.array_equal(a["bcsrRowPtr"], o["blcPtr"])
+    assert np.array_equal(a["bcsrVal"], o["blcVal"])
