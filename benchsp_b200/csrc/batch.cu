@@ -966,14 +966,14 @@ static bsp_status batch_build(bsp_batch_plan P, cudaStream_t s) {
   dfree(P->d_items_sep, s);
   dfree(P->d_longs, s);
   dfree(P->d_arrive, s);
-  if (P->d_part) cudaFreeAsync(P->d_part, s);
+  if (P->d_part) pool_free(P->d_part, s);
   P->d_part = nullptr;
   BSP_TRY(dalloc(&P->d_items, all.size(), s));
   BSP_TRY(dalloc(&P->d_items_sep, sep.size(), s));
   BSP_TRY(dalloc(&P->d_longs, longs.size(), s));
   BSP_TRY(dalloc(&P->d_arrive, longs.size(), s));
   const size_t es = P->dtype == BSP_F64 ? 8 : 4;
-  BSP_CUDA(cudaMallocAsync(&P->d_part, (size_t)std::max<int64_t>(1, parts) * P->nrhs * es, s));
+  BSP_CUDA(pool_malloc(reinterpret_cast<void **>(&P->d_part), (size_t)std::max<int64_t>(1, parts) * P->nrhs * es, s));
   if (!all.empty())
     BSP_CUDA(cudaMemcpyAsync(P->d_items, all.data(), all.size() * sizeof(BatchItem), cudaMemcpyHostToDevice, s));
   if (!sep.empty())
@@ -1031,8 +1031,8 @@ extern "C" bsp_status bsp_batch_destroy(bsp_batch_plan P) {
   dfree(P->d_longs, s);
   dfree(P->d_arrive, s);
   dfree(P->d_next, s);
-  if (P->d_part) cudaFreeAsync(P->d_part, s);
-  if (P->d_sell_val) cudaFreeAsync(P->d_sell_val, s);
+  if (P->d_part) pool_free(P->d_part, s);
+  if (P->d_sell_val) pool_free(P->d_sell_val, s);
   dfree(P->d_sell_off, s);
   dfree(P->d_sell_ptr, s);
   dfree(P->d_sell_lo, s);
@@ -1087,7 +1087,7 @@ bsp_status build_sell(bsp_batch_plan P, cudaStream_t s) {
   }
   if (tot_ptr == 0) return BSP_OK;
   const size_t es = P->dtype == BSP_F64 ? 8 : 4;
-  BSP_CUDA(cudaMallocAsync(&P->d_sell_val, (size_t)std::max<int64_t>(tot_val, 1) * es, s));
+  BSP_CUDA(pool_malloc(reinterpret_cast<void **>(&P->d_sell_val), (size_t)std::max<int64_t>(tot_val, 1) * es, s));
   BSP_TRY(dalloc(&P->d_sell_off, (size_t)std::max<int64_t>(tot_narrow, 1), s));
   BSP_TRY(dalloc(&P->d_sell_col, (size_t)std::max<int64_t>(tot_wide, 1), s));
   BSP_TRY(dalloc(&P->d_sell_perm, (size_t)std::max<int64_t>(tot_perm, 1), s));

@@ -64,14 +64,18 @@ inline int sm_count() {
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-// Stream-ordered device allocation (cudaMallocAsync pool).
+// Stream-ordered device memory from the library's own pool (util.cu); same
+// contract as cudaMallocAsync / cudaFreeAsync.
+cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t s);
+cudaError_t pool_free(void *p, cudaStream_t s);
+
 template <typename T>
 bsp_status dalloc(T **p, size_t count, cudaStream_t s) {
   *p = nullptr;
   if (count == 0) count = 1;
-  cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(p), count * sizeof(T), s);
+  cudaError_t e = pool_malloc(reinterpret_cast<void **>(p), count * sizeof(T), s);
   if (e != cudaSuccess) {
-    set_error(std::string("cudaMallocAsync(") + std::to_string(count * sizeof(T)) +
+    set_error(std::string("device allocation (") + std::to_string(count * sizeof(T)) +
               " B) -> " + cudaGetErrorString(e));
     return BSP_ERR_ALLOC;
   }
@@ -80,7 +84,7 @@ bsp_status dalloc(T **p, size_t count, cudaStream_t s) {
 
 template <typename T>
 void dfree(T *&p, cudaStream_t s) {
-  if (p) cudaFreeAsync(p, s);
+  if (p) pool_free(p, s);
   p = nullptr;
 }
 

@@ -836,7 +836,7 @@ extern "C" bsp_status bsp_bsr_free(bsp_bsr *m) {
   dfree(m->blcPtr, s);
   dfree(m->blcIdx, s);
   dfree(m->blcVal, s);
-  if (m->blcMap) cudaFreeAsync(m->blcMap, s);
+  if (m->blcMap) pool_free(m->blcMap, s);
   m->blcMap = nullptr;
   dfree(m->rowPtrbyWarp, s);
   dfree(m->rowIdxbyWarp, s);

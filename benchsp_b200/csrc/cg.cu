@@ -1104,7 +1104,7 @@ template <typename VT>
 static bsp_status build_minv(bsp_cg_plan_s *P, cudaStream_t s) {
   const int bs = P->prec_bs;
   const int64_t nb = ((int64_t)P->n + bs - 1) / bs;
-  BSP_CUDA(cudaMallocAsync(&P->minv, sizeof(VT) * (size_t)(nb * bs * bs), s));
+  BSP_CUDA(pool_malloc(reinterpret_cast<void **>(&P->minv), sizeof(VT) * (size_t)(nb * bs * bs), s));
   int32_t *bad = nullptr;
   BSP_TRY(dalloc(&bad, 1, s));
   BSP_CUDA(cudaMemsetAsync(bad, 0, sizeof(int32_t), s));
@@ -1187,14 +1187,14 @@ extern "C" bsp_status bsp_cg_destroy(bsp_cg_plan P) {
   dfree(P->x64, s);
   dfree(P->r64, s);
   for (void *v : {P->x, P->r, P->p[0], P->p[1], P->q, P->lp_val, P->z, P->minv})
-    if (v) cudaFreeAsync(v, s);
+    if (v) pool_free(v, s);
   dfree(P->part_rz, s);
   dfree(P->p64, s);
   dfree(P->q64, s);
   dfree(P->z64, s);
   dfree(P->part_zq, s);
   dfree(P->part_pr, s);
-  if (P->lp_cols) cudaFreeAsync(P->lp_cols, s);
+  if (P->lp_cols) pool_free(P->lp_cols, s);
   dfree(P->exps, s);
   dfree(P->slice_len, s);
   dfree(P->slice_off, s);
@@ -1260,7 +1260,7 @@ extern "C" bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPt
   if (mixed) {
     P->x = nullptr;  // x32 allocated below
   }
-  for (void **v : {&P->x, &P->r, &P->p[0], &P->p[1], &P->q}) BSP_CG_CUDA(cudaMallocAsync(v, vt * (size_t)n, s));
+  for (void **v : {&P->x, &P->r, &P->p[0], &P->p[1], &P->q}) BSP_CG_CUDA(pool_malloc(reinterpret_cast<void **>(v), vt * (size_t)n, s));
   if (!mixed) {  // lanes per row from the mean row length
     const double mean = (double)nnz / n;
     P->lpr = mean <= 10.0 ? 1 : mean <= 20.0 ? 2 : mean <= 40.0 ? 4 : 8;
@@ -1276,12 +1276,12 @@ extern "C" bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPt
     BSP_CG_TRY(dalloc(&P->part_pr, (size_t)P->grid, s));
   }
   if (P->prec_bs) {
-    BSP_CG_CUDA(cudaMallocAsync(&P->z, vt * (size_t)n, s));
+    BSP_CG_CUDA(pool_malloc(reinterpret_cast<void **>(&P->z), vt * (size_t)n, s));
     BSP_CG_TRY(dalloc(&P->part_rz, (size_t)P->grid, s));
     BSP_CG_TRY(mixed ? build_minv<float>(P, s) : build_minv<double>(P, s));
   }
   if (!mixed) {  // FP64 mode iterates directly on x64
-    cudaFreeAsync(P->x, s);
+    pool_free(P->x, s);
     P->x = P->x64;
   }
   int64_t mat_bytes = (int64_t)nnz * 12;
@@ -1357,11 +1357,11 @@ extern "C" bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPt
     if (P->sell64) {
       // the FP64 copy is an optimisation: without room for it, stay on CSR
       const size_t ne = (size_t)(padded > 0 ? padded : 1);
-      if (cudaMallocAsync(&P->lp_val, 8 * ne, s) != cudaSuccess ||
-          cudaMallocAsync(&P->lp_cols, 2 * ne, s) != cudaSuccess) {
+      if (pool_malloc(reinterpret_cast<void **>(&P->lp_val), 8 * ne, s) != cudaSuccess ||
+          pool_malloc(reinterpret_cast<void **>(&P->lp_cols), 2 * ne, s) != cudaSuccess) {
         cudaGetLastError();
-        if (P->lp_val) cudaFreeAsync(P->lp_val, s);
-        if (P->lp_cols) cudaFreeAsync(P->lp_cols, s);
+        if (P->lp_val) pool_free(P->lp_val, s);
+        if (P->lp_cols) pool_free(P->lp_cols, s);
         P->lp_val = P->lp_cols = nullptr;
         dfree(P->slice_len, s);
         dfree(P->slice_off, s);
@@ -1371,9 +1371,9 @@ extern "C" bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPt
         P->sell64 = false;
       }
     } else {
-      BSP_CG_CUDA(cudaMallocAsync(&P->lp_val, (packed ? 4 : vsz) * (size_t)(padded > 0 ? padded : 1), s));
+      BSP_CG_CUDA(pool_malloc(reinterpret_cast<void **>(&P->lp_val), (packed ? 4 : vsz) * (size_t)(padded > 0 ? padded : 1), s));
       if (!packed)
-        BSP_CG_CUDA(cudaMallocAsync(&P->lp_cols, (P->delta16 ? 2 : 4) * (size_t)(padded > 0 ? padded : 1), s));
+        BSP_CG_CUDA(pool_malloc(reinterpret_cast<void **>(&P->lp_cols), (P->delta16 ? 2 : 4) * (size_t)(padded > 0 ? padded : 1), s));
     }
   }
   if (mixed || P->sell64) {

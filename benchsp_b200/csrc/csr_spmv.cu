@@ -458,10 +458,10 @@ extern "C" bsp_status bsp_csr_spmv(int32_t rows, int32_t cols, int32_t nnz, cons
     BSP_CHECK_ARG(dtype == BSP_F64, "merge-path is FP64 only");
     const size_t need = merge_workspace_bytes(rows, nnz);
     void *ws = nullptr;
-    BSP_CUDA(cudaMallocAsync(&ws, need, s));
+    BSP_CUDA(pool_malloc(reinterpret_cast<void **>(&ws), need, s));
     bsp_status st = bsp_csr_spmv_merge_f64(rows, cols, nnz, rowPtr, colIdx, (const double *)values,
                                            (const double *)x, (double *)y, alpha, beta, ws, need, stream);
-    cudaFreeAsync(ws, s);
+    pool_free(ws, s);
     return st;
   }
   if (algo == BSP_CSR_AUTO) {

@@ -1322,14 +1322,14 @@ extern "C" bsp_status bsp_spmm_csr(int32_t rows, int32_t cols, int32_t nnz, cons
       const size_t ws = bsp_spmm_plan_workspace(&plan, N);
       void *work = nullptr;
       bsp_status r2 = BSP_OK;
-      if (ws > 0 && cudaMallocAsync(&work, ws, s) != cudaSuccess) {
+      if (ws > 0 && pool_malloc(reinterpret_cast<void **>(&work), ws, s) != cudaSuccess) {
         set_error("bsp_spmm_csr: allocating the row-split workspace failed");
         r2 = BSP_ERR_ALLOC;
       }
       if (r2 == BSP_OK)
         r2 = bsp_spmm_csr_planned(&plan, cols, nnz, rowPtr, colIdx, values, dtype, B, N, ldb, C, ldc, alpha, beta,
                                   work, ws, stream);
-      if (work) cudaFreeAsync(work, s);
+      if (work) pool_free(work, s);
       bsp_spmm_plan_free(&plan);
       return r2;
     }
@@ -1385,7 +1385,7 @@ extern "C" bsp_status bsp_smat_free(bsp_smat *m) {
   clear_error();
   if (!m) return BSP_OK;
   cudaStream_t s = 0;
-  if (m->tile_val) cudaFreeAsync(m->tile_val, s);
+  if (m->tile_val) pool_free(m->tile_val, s);
   m->tile_val = nullptr;
   dfree(m->err, s);
   BSP_TRY(bsp_bcsr_free(&m->tiles));
@@ -2498,7 +2498,7 @@ extern "C" bsp_status bsp_gtile_free(bsp_gtile *g) {
   dfree(g->group_piece, s);
   dfree(g->split_groups, s);
   dfree(g->chunk_cols, s);
-  if (g->chunk_tiles) cudaFreeAsync(g->chunk_tiles, s);
+  if (g->chunk_tiles) pool_free(g->chunk_tiles, s);
   g->chunk_tiles = nullptr;
   dfree(g->err, s);
   BSP_CUDA(cudaStreamSynchronize(s));

@@ -249,7 +249,7 @@ static bsp_status materialize(bsp_spmv_plan P, const bsp_tune_result &c, cudaStr
     P->has_dasp = true;
   } else if (c.csr_algo == BSP_CSR_MERGE) {
     P->ws_bytes = bsp_csr_merge_workspace(P->rows, P->nnz);
-    BSP_CUDA(cudaMallocAsync(&P->ws, P->ws_bytes ? P->ws_bytes : 16, s));
+    BSP_CUDA(pool_malloc(reinterpret_cast<void **>(&P->ws), P->ws_bytes ? P->ws_bytes : 16, s));
   }
   P->choice = c;
   return BSP_OK;

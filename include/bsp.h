@@ -62,6 +62,10 @@ bsp_status bsp_device_sync(void);
  * cudaFree on the current device). */
 bsp_status bsp_device_alloc(void **ptr, size_t bytes);
 bsp_status bsp_device_free(void *ptr);
+/* The library allocates from a memory pool of its own per device, which keeps
+ * at most 1/64 of the device's memory idle between calls; this gives the
+ * current device's idle part back. */
+bsp_status bsp_pool_trim(void);
 /* Measurement utility (no reference counterpart): `count` gathers of `width`
  * bytes (8, or 16..256 read as width/16 lanes x 16 bytes) at pseudo-random
  * width-aligned offsets of the device buffer `buf` (`bytes` long), eight in
