@@ -9,8 +9,8 @@
 //   * scalar: one thread per row, left-to-right sum with separately rounded
 //     multiply and add -- bit-identical to ref_spmv_fp64 / ref_spmv_fp16
 //     (src/ref.cpp:3-37) on the same inputs;
-//   * vector: a power-of-two group of lanes per row, strided loads of
-//     values/columns, read-only cached gathers of x, shuffle reduction;
+//   * vector: a power-of-two group of lanes per row, 8 entries per lane loaded
+//     before their x gathers, shuffle reduction; long rows by a warp or the CTA;
 //   * merge-path: every warp takes an equal share of (rows + nnz) merge
 //     items, so power-law rows cost the same as short ones; warp-level
 //     segmented scan plus a carry fix-up kernel over a small workspace.
@@ -66,80 +66,150 @@ __global__ void __launch_bounds__(256) csr_scalar_kernel(int32_t rows, const int
   }
 }
 
-constexpr int kWarpRowFactor = 64;
+// Long rows are left out of the pass over a CTA's rows and summed after it by
+// more threads: a warp per row up to kCtaRow entries, the whole CTA above
+// (power-law rows: one 10,000-entry row was a chain of 78 dependent loads for
+// the warp that met it).  A row's summation order depends on its length alone.
+// CTAs without such rows pay one barrier.
+constexpr int kCsrThreads = 256;
+constexpr int kCsrWarps = kCsrThreads / 32;
+constexpr int kCtaRow = 512;
+constexpr int kLongList = 64;
 
-// LPR lanes per row (LPR in {1,2,4,8,16,32}); grid-stride over rows.
-template <typename V, int LPR>
-__global__ void __launch_bounds__(256) csr_vector_kernel(int32_t rows, const int32_t *__restrict__ rowPtr,
-                                                         const int32_t *__restrict__ colIdx,
-                                                         const V *__restrict__ val, const V *__restrict__ x,
-                                                         V *__restrict__ y, typename AccOf<V>::T alpha,
-                                                         typename AccOf<V>::T beta) {
+// Sum of entries j, j + STRIDE, ... < e (4 in flight), this thread's share of a row.
+template <typename V, int STRIDE>
+__device__ __forceinline__ typename AccOf<V>::T strided_sum(int32_t j, int32_t e, const int32_t *__restrict__ colIdx,
+                                                            const V *__restrict__ val, const V *__restrict__ x) {
   using A = typename AccOf<V>::T;
-  const int sub = threadIdx.x & (LPR - 1);
-  const int64_t groups = (int64_t)gridDim.x * (blockDim.x / LPR);
-  // The loop bound is uniform across the warp (base is the warp's first row)
-  // so the shuffle reduction always runs with every lane present.
-  const int64_t warp_first = ((int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / LPR;
-  for (int64_t base = warp_first; base < rows; base += groups) {
-    const int64_t r = base + (threadIdx.x & 31) / LPR;
-    const bool active = r < rows;
-    const int32_t s = active ? rowPtr[r] : 0, e0 = active ? rowPtr[r + 1] : 0;
-    // rows longer than kWarpRowFactor entries per lane are summed by the
-    // whole warp after the pass, so one long row does not hold its warp's
-    // other rows (power-law rows at one lane per row)
-    const bool big = LPR < 32 && e0 - s > kWarpRowFactor * LPR;
-    const int32_t e = big ? s : e0;
-    // The first kFirst entries of each lane are loaded together, then their x
-    // gathers together: the rowPtr -> column -> x chain is paid once per
-    // kFirst entries instead of once per entry.
-    constexpr int kFirst = LPR == 1 ? 8 : 4;
-    int32_t c[kFirst];
-    V a[kFirst];
+  A sum = A(0);
+  for (; j < e; j += 4 * STRIDE) {
+    int32_t c[4];
+    V a[4];
 #pragma unroll
-    for (int k = 0; k < kFirst; ++k) {
-      const int32_t j = s + sub + k * LPR;
-      c[k] = j < e ? colIdx[j] : -1;
-      a[k] = j < e ? val[j] : V(0);
+    for (int u = 0; u < 4; ++u) {
+      const bool in = j + u * STRIDE < e;
+      c[u] = in ? colIdx[j + u * STRIDE] : -1;
+      a[u] = in ? val[j + u * STRIDE] : V(0);
     }
-    A sum = A(0);
 #pragma unroll
-    for (int k = 0; k < kFirst; ++k)
-      if (c[k] >= 0) sum = fma(to_acc<V>(a[k]), to_acc<V>(__ldg(&x[c[k]])), sum);
-#pragma unroll 4
-    for (int32_t j = s + sub + kFirst * LPR; j < e; j += LPR)
-      sum = fma(to_acc<V>(val[j]), to_acc<V>(__ldg(&x[colIdx[j]])), sum);
+    for (int u = 0; u < 4; ++u)
+      if (c[u] >= 0) sum = fma(to_acc<V>(a[u]), to_acc<V>(__ldg(&x[c[u]])), sum);
+  }
+  return sum;
+}
+
+// Sums the CTA's long rows: `mine` says that this thread holds one, row `r`
+// with entries [s, e).  Every thread of the CTA calls it.
+template <typename V>
+__device__ __forceinline__ void sum_long_rows(bool mine, int64_t r, int32_t s, int32_t e,
+                                              const int32_t *__restrict__ rowPtr,
+                                              const int32_t *__restrict__ colIdx, const V *__restrict__ val,
+                                              const V *__restrict__ x, V *__restrict__ y,
+                                              typename AccOf<V>::T alpha, typename AccOf<V>::T beta) {
+  using A = typename AccOf<V>::T;
+  struct LongRow {
+    int32_t s, e, r;
+  };
+  __shared__ LongRow list[kLongList];
+  __shared__ int32_t count[kCsrWarps];
+  __shared__ A part[kCsrWarps];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (!__syncthreads_or(mine)) return;
+  const unsigned mask = __ballot_sync(0xffffffffu, mine);
+  if (lane == 0) count[w] = __popc(mask);
+  __syncthreads();
+  int32_t n = 0, base = 0;
 #pragma unroll
-    for (int o = LPR / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, LPR);
-    if (active && sub == 0 && !big) store_y<V, A>(y, r, sum, alpha, beta);
-    if constexpr (LPR < 32) {
-      unsigned todo = __ballot_sync(0xffffffffu, big && sub == 0);
-      const int lane = threadIdx.x & 31;
-      while (todo) {   // warp-uniform
-        const int b = __ffs(todo) - 1;
-        todo &= todo - 1;
-        const int64_t br = base + b / LPR;
-        const int32_t bs = rowPtr[br], be = rowPtr[br + 1];
-        A ws = A(0);
-        int32_t j = bs + lane;
-        for (; j + 96 < be; j += 128) {
-          int32_t c[4];
-          V a[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            c[u] = colIdx[j + 32 * u];
-            a[u] = val[j + 32 * u];
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) ws = fma(to_acc<V>(a[u]), to_acc<V>(__ldg(&x[c[u]])), ws);
-        }
-        for (; j < be; j += 32) ws = fma(to_acc<V>(val[j]), to_acc<V>(__ldg(&x[colIdx[j]])), ws);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
-        if (lane == 0) store_y<V, A>(y, br, ws, alpha, beta);
+  for (int q = 0; q < kCsrWarps; ++q) {
+    base += q < w ? count[q] : 0;
+    n += count[q];
+  }
+  base += __popc(mask & ((1u << lane) - 1));
+  if (sizeof(A) == 8 && mine) {
+    // read again rather than carried through the pass: with s and e alive the
+    // FP64 kernel takes 40 registers, and 6 instead of 8 CTAs fit an SM
+    asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(s) : "l"(rowPtr + r));
+    asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(e) : "l"(rowPtr + r + 1));
+  }
+  for (int32_t first = 0; first < n; first += kLongList) {  // CTA-uniform
+    const int32_t m = min(n - first, kLongList);
+    __syncthreads();
+    if (mine && base >= first && base < first + m) list[base - first] = {s, e, (int32_t)r};
+    __syncthreads();
+    for (int k = w; k < m; k += kCsrWarps) {
+      const LongRow L = list[k];
+      if (L.e - L.s > kCtaRow) continue;
+      const A sum = warp_sum(strided_sum<V, 32>(L.s + lane, L.e, colIdx, val, x));
+      if (lane == 0) store_y<V, A>(y, L.r, sum, alpha, beta);
+    }
+    for (int k = 0; k < m; ++k) {
+      const LongRow L = list[k];
+      if (L.e - L.s <= kCtaRow) continue;
+      const A sum = warp_sum(strided_sum<V, kCsrThreads>(L.s + threadIdx.x, L.e, colIdx, val, x));
+      if (lane == 0) part[w] = sum;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        A t = part[0];
+        for (int h = 1; h < kCsrWarps; ++h) t += part[h];
+        store_y<V, A>(y, L.r, t, alpha, beta);
       }
+      __syncthreads();
     }
   }
+}
+
+constexpr int kWarpRowFactor = 16;
+
+// LPR lanes per row (LPR in {1,2,4,8,16,32}), one pass: the grid covers the rows.
+//
+// A warp's life is one chain (row pointers -> entries -> x -> y), so the bytes a
+// lane has in flight set the rate: 8 entries per lane on half the lanes against
+// 4, 27-point stencil 128^3: FP16 112 -> 84 us (floor 54), FP32 124 -> 91 (72),
+// FP64 160 -> 132 (109); 16 per lane FP16 84, FP32 101, FP64 145.  No loop over
+// passes (the grid was capped at 64 CTAs per SM): FP64 160 -> 141 us at 4 per
+// lane.  Rows of more than kWarpRowFactor entries per lane are left to
+// sum_long_rows: power-law 2^20 (Zipf 2.0, cap 10k) FP64 134 -> 58 us, FP16 95
+// -> 47 us; 8 / 16 / 32 entries per lane 54 / 53 / 54 us, kCtaRow 256 / 512 /
+// 1024 54 / 53 / 52 us.  Resident CTAs: FP64 with several lanes needs 40
+// registers (6 CTAs; at 8 it spills, 138 us); FP64 with one lane is capped at 32
+// (at 40 the 1024 CTAs of a 512^2 grid take a second wave, 3.8 -> 4.5 us).
+template <typename V, int LPR>
+__global__ void __launch_bounds__(kCsrThreads, LPR > 1 && sizeof(V) == 8 ? 6 : LPR > 1 || sizeof(V) == 8 ? 8 : 0) csr_vector_kernel(int32_t rows, const int32_t *__restrict__ rowPtr,
+                                                                    const int32_t *__restrict__ colIdx,
+                                                                    const V *__restrict__ val,
+                                                                    const V *__restrict__ x, V *__restrict__ y,
+                                                                    typename AccOf<V>::T alpha,
+                                                                    typename AccOf<V>::T beta) {
+  using A = typename AccOf<V>::T;
+  const int sub = threadIdx.x & (LPR - 1);
+  const int64_t r = (int64_t)blockIdx.x * (kCsrThreads / LPR) + threadIdx.x / LPR;
+  const bool active = r < rows;
+  const int32_t s = active ? rowPtr[r] : 0, e0 = active ? rowPtr[r + 1] : 0;
+  const bool is_long = e0 - s > kWarpRowFactor * LPR;
+  const int32_t e = is_long ? s : e0;
+  // The first kFirst entries of each lane are loaded together, then their x
+  // gathers together: the rowPtr -> column -> x chain is paid once per
+  // kFirst entries instead of once per entry.
+  constexpr int kFirst = 8;
+  int32_t c[kFirst];
+  V a[kFirst];
+#pragma unroll
+  for (int k = 0; k < kFirst; ++k) {
+    const int32_t j = s + sub + k * LPR;
+    c[k] = j < e ? colIdx[j] : -1;
+    a[k] = j < e ? val[j] : V(0);
+  }
+  A sum = A(0);
+#pragma unroll
+  for (int k = 0; k < kFirst; ++k)
+    if (c[k] >= 0) sum = fma(to_acc<V>(a[k]), to_acc<V>(__ldg(&x[c[k]])), sum);
+#pragma unroll 4
+  for (int32_t j = s + sub + kFirst * LPR; j < e; j += LPR)
+    sum = fma(to_acc<V>(val[j]), to_acc<V>(__ldg(&x[colIdx[j]])), sum);
+#pragma unroll
+  for (int o = LPR / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, LPR);
+  if (active && sub == 0 && !is_long) store_y<V, A>(y, r, sum, alpha, beta);
+  sum_long_rows<V>(is_long && sub == 0, r, s, e0, rowPtr, colIdx, val, x, y, alpha, beta);
 }
 
 // Warp per 32 consecutive rows ("stream").  The warp's nonzero range
@@ -347,12 +417,8 @@ template <typename V>
 static bsp_status launch_vector(int lpr, int32_t rows, const int32_t *rp, const int32_t *ci, const V *v,
                                 const V *x, V *y, typename AccOf<V>::T a, typename AccOf<V>::T b,
                                 cudaStream_t s) {
-  const int threads = 256;
-  const int64_t rows_per_block = threads / lpr;
-  int64_t blocks = ceil_div(rows, rows_per_block);
-  const int64_t cap = (int64_t)sm_count() * 64;  // grid-stride beyond this
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
+  const int threads = kCsrThreads;
+  const int64_t blocks = ceil_div(rows, threads / lpr);  // rows > 0
   switch (lpr) {
 #define BSP_VEC_CASE(L)                                                                    \
   case L:                                                                                  \
@@ -392,14 +458,12 @@ static bsp_status launch_stream(int32_t rows, const int32_t *rp, const int32_t *
   return BSP_OK;
 }
 
-// Lanes per row from the mean row length: one lane per row up to 8 entries
-// (those are loaded together), then the smallest power of two >= mean/4,
-// up to 32.
+// Lanes per row from the mean row length: the smallest power of two whose lanes
+// hold the row in their 8 entries loaded together, up to 32.
 int auto_lanes(int32_t rows, int32_t nnz) {
   const double mean = rows > 0 ? (double)nnz / rows : 0.0;
-  if (mean <= 8.0) return 1;
-  int l = 2;
-  while (l < 32 && 4.0 * l < mean) l <<= 1;
+  int l = 1;
+  while (l < 32 && 8.0 * l < mean) l <<= 1;
   return l;
 }
 

@@ -215,3 +215,36 @@ def test_merge_workspace_too_small_is_rejected(cuda):
     ws = torch.empty(8, dtype=torch.uint8, device=cuda)
     with pytest.raises(bsp.BspError):
         bsp.csr_spmv_merge(*d, workspace=ws)
+
+
+# rows at the lengths where a row changes hands: 8 entries per lane, 16 per lane
+# (the lanes' own / a warp), 512 (a warp / the CTA), several rounds of the CTA,
+# more long rows in one CTA than its list holds, a ragged last CTA
+@pytest.mark.parametrize("rows,cols,lens", [
+    (1, 3000, [2500]), (300, 600, [16, 17, 8, 9, 0]), (257, 5000, [0, 1, 511, 512, 513, 3]), (520, 300, [33]),
+    (700, 9000, [2, 0, 4097, 1, 1, 1, 600, 129]), (64, 4000, [257, 256, 2049])])
+@pytest.mark.parametrize("lanes", [0, 1, 2, 8, 32])
+@pytest.mark.parametrize("dt", ["float64", "float32", "float16", "bfloat16"])
+def test_vector_long_rows(cuda, rows, cols, lens, lanes, dt):
+    import torch
+    rng = np.random.default_rng(rows + cols)
+    lens = np.resize(np.array(lens), rows)
+    rp = np.zeros(rows + 1, np.int32)
+    rp[1:] = np.cumsum(lens)
+    ci = np.concatenate([np.sort(rng.choice(cols, k, replace=False)) for k in lens]).astype(np.int32)
+    tdt = getattr(torch, dt)
+    v, x, y0 = (torch.from_numpy(a).to(tdt) for a in (rng.standard_normal(ci.size), rng.uniform(-1, 1, cols),
+                                                      rng.uniform(-1, 1, rows)))
+    vh, xh, yh = (t.double().numpy() for t in (v, x, y0))
+    ax = pyoracle.spmv_f64(rp, ci, vh, xh)
+    d_rp, d_ci = _dev(cuda, rp, ci)
+    y = y0.to(cuda)
+    bsp.csr_spmv(d_rp, d_ci, v.to(cuda), x.to(cuda), y, alpha=0.5, beta=-2.0, lanes=lanes)
+    got = y.double().cpu().numpy()
+    # the accumulation bound of A x, three roundings of alpha * (A x) + beta * y, one of the output
+    unit = 2.0 ** -53 if dt == "float64" else 2.0 ** -24
+    out = {"float64": 0.0, "float32": 0.0, "float16": 2.0 ** -11, "bfloat16": 2.0 ** -8}[dt]
+    ref = 0.5 * ax - 2.0 * yh
+    tol = 0.5 * pyoracle.spmv_tolerance(rp, ci, vh, xh, unit=unit) + \
+        3 * unit * (np.abs(0.5 * ax) + np.abs(2.0 * yh)) + 1.01 * out * np.abs(ref) + 2.0 ** -24 * (dt == "float16")
+    _within(got, ref, tol)
