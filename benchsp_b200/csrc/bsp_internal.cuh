@@ -69,6 +69,9 @@ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t s);
 cudaError_t pool_free(void *p, cudaStream_t s);
 
+// Id of the calling thread's context, never reused by the driver; 0 if unknown.
+unsigned long long context_id();
+
 template <typename T>
 bsp_status dalloc(T **p, size_t count, cudaStream_t s) {
   *p = nullptr;

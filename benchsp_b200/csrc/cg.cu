@@ -22,7 +22,8 @@
 // reliable updates), so the iteration count stays close to plain FP64 CG while
 // most bytes move at low precision.
 //
-// One CG iteration is two kernels:
+// One CG iteration is two kernels (matrices of few diagonals whose vectors fit
+// the SMs' shared memory run a fused form instead, cg_fused_kernel):
 //   A. beta = rr_k / rr_{k-1}; p_k = r_k + beta p_{k-1} formed on the fly for
 //      every gathered column (r and p_{k-1} are read, p_k written for the own
 //      row into the other p buffer); q = A p_k; partials of p_k.q;
@@ -36,6 +37,8 @@
 #include <string.h>
 
 #include <algorithm>
+#include <map>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -259,9 +262,14 @@ __global__ void __launch_bounds__(kCgThreads, (sizeof(V) == 8 || (sizeof(V) == 4
   }
 }
 
-// Kernel B: alpha = rr_k / p.q; x += alpha p; r -= alpha q; partials of r.r.
-// 16-byte vector accesses (4 floats or 2 doubles per load), two in flight
-// per thread; the scalar tail covers n not divisible by the vector width.
+template <typename V>
+__device__ __forceinline__ V from_float_lp(float f);
+template <> __device__ __forceinline__ float from_float_lp<float>(float f) { return f; }
+template <> __device__ __forceinline__ __half from_float_lp<__half>(float f) { return __float2half_rn(f); }
+template <> __device__ __forceinline__ __nv_bfloat16 from_float_lp<__nv_bfloat16>(float f) { return __float2bfloat16_rn(f); }
+
+// ---------------------------------------------------------------------------
+// 16-byte vectors of the iteration precision.
 template <typename VT> struct Vec16;
 template <> struct Vec16<float> { using T = float4; static constexpr int W = 4; };
 template <> struct Vec16<double> { using T = double2; static constexpr int W = 2; };
@@ -275,6 +283,431 @@ __device__ __forceinline__ void vset(double2 &v, int k, double a) {
   if (k == 0) v.x = a; else v.y = a;
 }
 
+// ---------------------------------------------------------------------------
+// Fused iteration: all iterations of a chunk in one cooperative launch, one CTA
+// per SM, for matrices of at most kFusedDiags distinct diagonals (grid stencils)
+// whose vectors fit in the SMs' shared memory: x, r, p and q of a CTA's rows, 16
+// bytes per row in FP32, 32 in FP64.
+//
+// The two-kernel iteration moves x, r, p and q through L2 several times, gathers
+// both r and p_{k-1} for every entry, and pays two launches with a reduction of
+// the previous kernel's partials at the head of each.  Here a CTA keeps its
+// consecutive slices' rows in shared memory and an iteration is
+//   p = r + beta p, published
+//   q = A p, p.q                        | grid sum
+//   x += alpha p, r -= alpha q, r.r     | grid sum
+// with the matrix stored by diagonals (values only, a row's eight in one place)
+// and p gathered from shared memory (a column among the CTA's own rows) or from
+// the published copy in global memory.  An element is published together with
+// the iteration's tag as one word, and a reader loads it again until the tag is
+// there: no barrier stands between publishing and gathering.  Every element sees
+// the same operations in the same order as in the two kernels (a diagonal that a
+// row lacks adds 0 * p); only the dot products' FP64 summation order differs.
+//
+// A grid sum: each CTA stores {partial, epoch} as one 16-byte word in its slot,
+// a thread of every CTA polls each slot until it carries the epoch, and the
+// partials are added in a fixed order.  Slots stand 128 bytes apart (side by
+// side, stores queue behind the polls of their line: 4.1 against 1.6 us per sum
+// with 148 CTAs) and alternate between two arrays: a slot is stored again two
+// sums later, when every CTA has read it.  What a CTA read before a sum went
+// into its partial, so the published elements need no fence either.
+//
+// Measured per iteration, Poisson 128^3 FP16 (FP32): two kernels 39 (42) us, here
+// 19.7 (20.9): p 2.1, q 11.3, sums 2.9 and 2.9, x and r 1.6.  Everything is in L2
+// and shared memory (no DRAM traffic); the product is bound by instruction issue
+// and by the 2 of 7 columns that come from another SM.  An earlier form on the
+// SELL copy with 16-bit offsets took 31 us (a decode, an address and a test per
+// entry).  FP64 100^3: 31 -> 24 us.  Below about 40^3 the two sums are most of an
+// iteration (24^3 FP16: 9.1 -> 6 us).
+//
+// The cooperative launch makes all CTAs resident; every wait is bounded all the
+// same (kFusedPolls, then *err is set and every CTA returns).
+constexpr int kFusedDiags = 8;
+constexpr int kFusedMaxCtas = 256;
+constexpr uint32_t kFusedPolls = 1u << 23;  // about 5 s
+struct __align__(128) CgSlot {
+  double v;
+  unsigned long long epoch;
+};
+
+// A published element: the value and a tag in one word.
+template <typename VT> struct FusedPub;
+template <> struct FusedPub<float> {
+  using T = unsigned long long;
+  static __device__ __forceinline__ T word(float v, uint32_t tag) {
+    return (T)tag << 32 | __float_as_uint(v);
+  }
+  // Column c (relative to the CTA's rows, `mine` of them): *near, or w = *far for a
+  // column of another CTA (row0 + c < n).
+  static __device__ __forceinline__ void gather(uint32_t c, uint32_t mine, uint32_t row, uint32_t n, uint32_t near,
+                                                const T *far, float &v, T &w) {
+    asm volatile(
+        "{.reg .pred o, f; setp.ge.u32 o, %2, %3; setp.lt.and.u32 f, %4, %5, o;"
+        " @!o ld.shared.f32 %0, [%6]; @f ld.relaxed.gpu.global.u64 %1, [%7];}"
+        : "+f"(v), "+l"(w)
+        : "r"(c), "r"(mine), "r"(row), "r"(n), "r"(near), "l"(far)
+        : "memory");
+  }
+  static __device__ __forceinline__ T get(const T *p) {
+    T t;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(t) : "l"(p) : "memory");
+    return t;
+  }
+  static __device__ __forceinline__ void put(T *p, float v, uint32_t tag) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(word(v, tag)) : "memory");
+  }
+  static __device__ __forceinline__ uint32_t tag(T t) { return (uint32_t)(t >> 32); }
+  static __device__ __forceinline__ float value(T t) { return __uint_as_float((uint32_t)t); }
+};
+struct FusedWord16 {
+  unsigned long long lo, hi;
+};
+__device__ __forceinline__ void st_word16(void *p, unsigned long long lo, unsigned long long hi) {
+  asm volatile("{.reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t;}" ::"l"(p), "l"(lo), "l"(hi)
+               : "memory");
+}
+__device__ __forceinline__ FusedWord16 ld_word16(const void *p) {
+  FusedWord16 t;
+  asm volatile("{.reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t;}"
+               : "=l"(t.lo), "=l"(t.hi)
+               : "l"(p)
+               : "memory");
+  return t;
+}
+template <> struct FusedPub<double> {
+  using T = FusedWord16;
+  static __device__ __forceinline__ T word(double v, uint32_t tag) {
+    return {(unsigned long long)__double_as_longlong(v), tag};
+  }
+  static __device__ __forceinline__ void gather(uint32_t c, uint32_t mine, uint32_t row, uint32_t n, uint32_t near,
+                                                const T *far, double &v, T &w) {
+    asm volatile(
+        "{.reg .pred o, f; .reg .b128 t; setp.ge.u32 o, %3, %4; setp.lt.and.u32 f, %5, %6, o;"
+        " mov.b128 t, {%1, %2}; @!o ld.shared.f64 %0, [%7]; @f ld.relaxed.gpu.global.b128 t, [%8];"
+        " mov.b128 {%1, %2}, t;}"
+        : "+d"(v), "+l"(w.lo), "+l"(w.hi)
+        : "r"(c), "r"(mine), "r"(row), "r"(n), "r"(near), "l"(far)
+        : "memory");
+  }
+  static __device__ __forceinline__ T get(const T *p) { return ld_word16(p); }
+  static __device__ __forceinline__ void put(T *p, double v, uint32_t tag) { st_word16(p, word(v, tag).lo, tag); }
+  static __device__ __forceinline__ uint32_t tag(T t) { return (uint32_t)t.hi; }
+  static __device__ __forceinline__ double value(T t) { return __longlong_as_double((long long)t.lo); }
+};
+
+// A CTA's slices of the ns, `ctas` in all.
+struct FusedSlices {
+  int32_t first, count;
+  __device__ FusedSlices(int64_t ns, int64_t cta, int64_t ctas)
+      : first((int32_t)(ns * cta / ctas)), count((int32_t)(ns * (cta + 1) / ctas) - first) {}
+};
+
+// The matrix's distinct diagonals (column - row): d[0] and d[ND - 1] the lowest
+// and the highest, the others between ascending and in [lo, hi].
+struct FusedDiags {
+  int32_t d[kFusedDiags], lo, hi;
+};
+
+// A row's values on the diagonals, kFusedDiags of them side by side.
+template <typename V> struct FusedRow {
+  static constexpr int kWords = kFusedDiags * (int)sizeof(V) / 16;
+  uint4 w[kWords];
+  __device__ __forceinline__ void load(const void *val, uint32_t row) {  // row * kWords < 2^32
+#pragma unroll
+    for (int k = 0; k < kWords; ++k) w[k] = __ldg(reinterpret_cast<const uint4 *>(val) + row * kWords + k);
+  }
+  template <int K>
+  __device__ __forceinline__ typename std::conditional<sizeof(V) == 8, double, float>::type value() const {
+    constexpr int kPer = 16 / (int)sizeof(V);
+    const uint4 t = w[K / kPer];
+    constexpr int e = K % kPer;
+    if constexpr (sizeof(V) == 8) {
+      return e ? __hiloint2double((int)t.w, (int)t.z) : __hiloint2double((int)t.y, (int)t.x);
+    } else if constexpr (sizeof(V) == 4) {
+      return __uint_as_float(e == 0 ? t.x : e == 1 ? t.y : e == 2 ? t.z : t.w);
+    } else {
+      const uint32_t u = e / 2 == 0 ? t.x : e / 2 == 1 ? t.y : e / 2 == 2 ? t.z : t.w;
+      if constexpr (std::is_same<V, __half>::value) {
+        const __half2 h = *reinterpret_cast<const __half2 *>(&u);
+        return e & 1 ? __high2float(h) : __low2float(h);
+      } else {
+        return __uint_as_float(e & 1 ? u & 0xffff0000u : u << 16);
+      }
+    }
+  }
+};
+
+// Distinct diagonals of the matrix into `set` (kFusedDiags values, kNoDiag when
+// free); *overflow when there are more.
+constexpr int32_t kNoDiag = INT32_MIN;
+__global__ void fused_diags_kernel(int32_t n, const int32_t *__restrict__ rowPtr, const int32_t *__restrict__ colIdx,
+                                   int32_t *set, int32_t *overflow) {
+  __shared__ int32_t seen[kFusedDiags];
+  if (threadIdx.x < kFusedDiags) seen[threadIdx.x] = kNoDiag;
+  __syncthreads();
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
+    if (*reinterpret_cast<volatile int32_t *>(overflow)) return;
+    for (int32_t j = rowPtr[t]; j < rowPtr[t + 1]; ++j) {
+      const int32_t d = (int32_t)(colIdx[j] - t);
+      bool known = false;
+#pragma unroll
+      for (int k = 0; k < kFusedDiags; ++k) known |= *reinterpret_cast<volatile int32_t *>(seen + k) == d;
+      if (known) continue;
+      int at = 0;  // into the grid's set (looked at before it is written), then the CTA's
+      for (; at < kFusedDiags; ++at) {
+        int32_t old = *reinterpret_cast<volatile int32_t *>(set + at);
+        if (old == kNoDiag) old = atomicCAS(set + at, kNoDiag, d);
+        if (old == kNoDiag || old == d) break;
+      }
+      if (at == kFusedDiags) {
+        *overflow = 1;
+        return;
+      }
+      seen[at] = d;
+    }
+  }
+}
+
+// Fills the copy by diagonals: thread per slice row; a diagonal that the row
+// lacks (and rows past n) gets 0.
+template <typename V, bool SCALED>
+__global__ void fused_fill_kernel(int32_t n, const int32_t *__restrict__ rowPtr, const int32_t *__restrict__ colIdx,
+                                  const double *__restrict__ val, const int8_t *__restrict__ exps, FusedDiags D,
+                                  V *__restrict__ out) {
+  const int64_t rows = ((int64_t)n + 31) / 32 * 32;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < rows; t += (int64_t)gridDim.x * blockDim.x) {
+    int32_t j = t < n ? rowPtr[t] : 0;
+    const int32_t e = t < n ? rowPtr[t + 1] : 0;
+#pragma unroll
+    for (int k = 0; k < kFusedDiags; ++k) {
+      double v = 0.0;
+      if (j < e && colIdx[j] - t == D.d[k]) {
+        v = val[j++];
+        if (SCALED) v = ldexp(v, -(int)exps[t]);
+      }
+      if constexpr (sizeof(V) == 8)
+        out[t * kFusedDiags + k] = v;
+      else
+        out[t * kFusedDiags + k] = from_float_lp<V>((float)v);
+    }
+  }
+}
+
+struct FusedGrid {
+  CgSlot *slots;  // [2][kFusedMaxCtas]
+  int32_t *err;
+  unsigned long long epoch;
+  double *part, *sum;  // shared: a partial per warp, a sum per polling warp
+  int *dead;           // shared, 0 at the start
+};
+
+__device__ __forceinline__ bool fused_give_up(FusedGrid &G, uint32_t polls) {
+  if ((polls & 1023u) != 0) return false;
+  if (polls < kFusedPolls && *reinterpret_cast<volatile int32_t *>(G.err) == 0) return false;
+  atomicExch(G.err, 1);
+  *reinterpret_cast<volatile int *>(G.dead) = 1;
+  return true;
+}
+
+// Sum over all threads of the grid (the same bits in every thread); the CTA's
+// threads are in step on both sides.
+template <int WARPS>
+__device__ __forceinline__ double fused_sum(FusedGrid &G, double v) {
+  constexpr int kPollWarps = kFusedMaxCtas / 32;
+  static_assert(WARPS >= kPollWarps && WARPS <= 32, "a slot per thread, a partial per lane");
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  ++G.epoch;
+  v = warp_sum(v);
+  if (lane == 0) G.part[w] = v;
+  __syncthreads();
+  if (w < kPollWarps) {
+    CgSlot *row = G.slots + (G.epoch & 1) * kFusedMaxCtas;
+    if (w == 0) {
+      const double t = warp_sum(lane < WARPS ? G.part[lane] : 0.0);
+      if (lane == 0) st_word16(row + blockIdx.x, (unsigned long long)__double_as_longlong(t), G.epoch);
+    }
+    double got = 0.0;
+    if (threadIdx.x < gridDim.x)
+      for (uint32_t polls = 1;; ++polls) {
+        const FusedWord16 t = ld_word16(row + threadIdx.x);
+        got = __longlong_as_double((long long)t.lo);
+        if (t.hi == G.epoch || fused_give_up(G, polls)) break;
+      }
+    got = warp_sum(got);
+    if (lane == 0) G.sum[w] = got;
+  }
+  __syncthreads();
+  double t = 0.0;
+#pragma unroll
+  for (int k = 0; k < kPollWarps; ++k) t += G.sum[k];
+  return t;
+}
+
+// acc += sum of a row's values times p, in the diagonals' order.
+template <int K, int ND, typename Row, typename VT>
+__device__ __forceinline__ void fused_dot(const Row &a, const VT (&p)[ND], VT &acc) {
+  if constexpr (K < ND) {
+    acc = fma((VT)a.template value<K>(), p[K], acc);
+    fused_dot<K + 1, ND>(a, p, acc);
+  }
+}
+
+// ND: the diagonals looked at (the rest of the kFusedDiags are unused).
+template <typename V, typename VT, int ND, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1)
+    cg_fused_kernel(int32_t n, const void *__restrict__ val, FusedDiags D, const int8_t *__restrict__ exps,
+                    VT *__restrict__ x, VT *__restrict__ r, VT *__restrict__ p_state, typename FusedPub<VT>::T *pub,
+                    double *rr_part, int npart, double *sc, int iters, CgSlot *slots, unsigned long long *epoch_mem,
+                    int32_t *err) {
+  using Pub = FusedPub<VT>;
+  using Vec = typename Vec16<VT>::T;
+  constexpr int W = Vec16<VT>::W;
+  constexpr bool kScaled = sizeof(V) == 2;
+  constexpr int kWarps = THREADS / 32;
+  extern __shared__ __align__(16) unsigned char fused_smem[];
+  __shared__ double part[kWarps], sum[kFusedMaxCtas / 32];
+  __shared__ int dead;
+  const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // uniform
+  const int64_t ns = ((int64_t)n + 31) / 32;
+  const FusedSlices T(ns, blockIdx.x, gridDim.x);
+  const int32_t S = T.count, s_lo = T.first, row0 = s_lo * 32;
+  const int32_t nloc = min(S * 32, n - row0);  // rows of the matrix; S * 32 with the padding
+  const int32_t cap = (int32_t)((ns + gridDim.x - 1) / gridDim.x) * 32;
+  VT *sx = reinterpret_cast<VT *>(fused_smem), *sr = sx + cap, *sp = sr + cap, *sq = sp + cap;
+  const uint32_t sp_base = (uint32_t)__cvta_generic_to_shared(sp);
+  typename Pub::T *pub0 = pub + row0;
+  FusedGrid G{slots, err, *epoch_mem, part, sum, &dead};
+  if (threadIdx.x == 0) dead = 0;
+  for (int32_t i = threadIdx.x; i < S * 32; i += THREADS) {  // padding rows stay 0
+    const bool in = i < nloc;
+    sx[i] = in ? x[row0 + i] : VT(0);
+    sr[i] = in ? r[row0 + i] : VT(0);
+    sp[i] = in ? p_state[row0 + i] : VT(0);
+    sq[i] = VT(0);
+  }
+  double rr = 0.0;
+  for (int i = threadIdx.x; i < npart; i += THREADS) rr += __ldcg(rr_part + i);
+  rr = warp_sum(rr);
+  if (lane == 0) part[w] = rr;
+  __syncthreads();
+  rr = warp_sum(lane < kWarps ? part[lane] : 0.0);
+  double rr_prev = sc[1];
+  __syncthreads();
+
+  for (int it = 0; it < iters; ++it) {
+    const double beta = (rr_prev != 0.0 && isfinite(rr)) ? rr / rr_prev : 0.0;
+    const VT bt = (VT)beta;
+    const uint32_t tag = (uint32_t)G.epoch + 1;
+    FusedRow<V> e;
+    int ex = 0;
+    auto fetch = [&](int32_t sl) {
+      e.load(val, row0 + sl * 32 + lane);
+      if (kScaled) ex = exps[row0 + min(sl * 32 + lane, nloc - 1)];
+    };
+    if (w < S) fetch(w);  // in flight while p is formed
+#pragma unroll 4
+    for (int32_t i = threadIdx.x; i < S * 32; i += THREADS) {
+      const VT pi = fma(bt, sp[i], sr[i]);
+      sp[i] = pi;
+      Pub::put(pub0 + i, pi, tag);
+    }
+    __syncthreads();
+    double dot = 0.0;
+    for (int32_t sl = w; sl < S; sl += kWarps) {
+      const int32_t i = sl * 32 + lane;
+      // p of the row's columns.  The inner diagonals of most slices lie among the
+      // CTA's rows: shared memory; the outer ones (and all of them otherwise) are
+      // told apart lane by lane.
+      const uint32_t own = sp_base + (uint32_t)i * (uint32_t)sizeof(VT);
+      VT near[ND];
+      typename Pub::T g[ND];
+      auto gather = [&](int k) {
+        near[k] = VT(0);
+        g[k] = Pub::word(VT(0), tag);
+        Pub::gather((uint32_t)(i + D.d[k]), (uint32_t)(S * 32), (uint32_t)(row0 + i + D.d[k]), (uint32_t)n,
+                    own + (uint32_t)D.d[k] * (uint32_t)sizeof(VT), pub0 + (i + D.d[k]), near[k], g[k]);
+      };
+      auto late = [&](int k) {
+        for (uint32_t polls = 1; Pub::tag(g[k]) != tag && !fused_give_up(G, polls); ++polls)
+          g[k] = Pub::get(pub0 + (i + D.d[k]));
+      };
+      auto take = [&](int k) {
+        if ((uint32_t)(i + D.d[k]) >= (uint32_t)(S * 32)) near[k] = Pub::value(g[k]);
+      };
+      const bool inner = sl * 32 + D.lo >= 0 && sl * 32 + 32 + D.hi <= S * 32;  // warp-uniform
+      gather(0);
+      gather(ND - 1);
+      if (inner) {
+        const char *own_p = reinterpret_cast<const char *>(sp + i);
+#pragma unroll
+        for (int k = 1; k < ND - 1; ++k) near[k] = *reinterpret_cast<const VT *>(own_p + D.d[k] * (int)sizeof(VT));
+      } else {
+#pragma unroll
+        for (int k = 1; k < ND - 1; ++k) gather(k);
+      }
+      const FusedRow<V> a = e;
+      const float scale = kScaled ? pow2f(ex) : 1.f;
+      if (sl + kWarps < S) fetch(sl + kWarps);  // in flight during this slice's gathers
+      // one test for the usual case: everything has arrived
+      if (Pub::tag(g[0]) != tag || Pub::tag(g[ND - 1]) != tag) {
+        late(0);
+        late(ND - 1);
+      }
+      take(0);
+      take(ND - 1);
+      if (!inner) {
+#pragma unroll
+        for (int k = 1; k < ND - 1; ++k) {
+          late(k);
+          take(k);
+        }
+      }
+      VT acc = VT(0);
+      fused_dot<0, ND>(a, near, acc);
+      if constexpr (kScaled) acc *= scale;
+      sq[i] = acc;  // 0 in a padding row
+      dot += (double)acc * (double)sp[i];
+    }
+    const double pq = fused_sum<kWarps>(G, dot);
+    if (dead) return;
+    const double alpha = (pq != 0.0 && rr != 0.0 && isfinite(pq)) ? rr / pq : 0.0;
+    const VT al = (VT)alpha;
+    double s = 0.0;
+    for (int32_t i = threadIdx.x * W; i < S * 32; i += THREADS * W) {
+      const Vec p = *reinterpret_cast<const Vec *>(sp + i), q = *reinterpret_cast<const Vec *>(sq + i);
+      Vec xv = *reinterpret_cast<Vec *>(sx + i), rv = *reinterpret_cast<Vec *>(sr + i);
+#pragma unroll
+      for (int k = 0; k < W; ++k) {
+        vset(xv, k, fma(al, vget(p, k), vget(xv, k)));
+        const VT ri = fma(-al, vget(q, k), vget(rv, k));
+        vset(rv, k, ri);
+        s += (double)ri * (double)ri;
+      }
+      *reinterpret_cast<Vec *>(sx + i) = xv;
+      *reinterpret_cast<Vec *>(sr + i) = rv;
+    }
+    rr_prev = rr;
+    rr = fused_sum<kWarps>(G, s);
+    if (dead) return;
+  }
+  for (int32_t i = threadIdx.x; i < nloc; i += THREADS) {
+    x[row0 + i] = sx[i];
+    r[row0 + i] = sr[i];
+    p_state[row0 + i] = sp[i];
+  }
+  if (blockIdx.x == 0) {
+    for (int i = threadIdx.x; i < npart; i += THREADS) rr_part[i] = i == 0 ? rr : 0.0;
+    if (threadIdx.x == 0) {
+      sc[1] = rr_prev;
+      sc[4] = rr;
+      *epoch_mem = G.epoch;
+    }
+  }
+}
+
+// Kernel B: alpha = rr_k / p.q; x += alpha p; r -= alpha q; partials of r.r.
+// 16-byte vector accesses (4 floats or 2 doubles per load), two in flight
+// per thread; the scalar tail covers n not divisible by the vector width.
 template <typename VT>
 __global__ void __launch_bounds__(kCgThreads) cg_update_kernel(int32_t n, const double *__restrict__ pq_part,
                                                                int npart, const double *__restrict__ rr_slot,
@@ -580,39 +1013,51 @@ __global__ void cg_minv_kernel(int32_t n, const int32_t *__restrict__ rowPtr, co
   }
 }
 
-// FP64 true residual r = b - A x, partials of ||r||^2; optionally also the
-// inner-precision copy r_lp = (VT) r and its partials (reliable update), and
-// the partials of ||r - r_lp_old||^2, the distance of the true residual from
-// the iterated one it replaces (part_dev, may be null).
-template <typename VT>
+// FP64 true residual r = b - A x, a row per thread and the grid over all rows:
+// the row's entries, then their x gathers, each loaded together.  (With the
+// norms below in the same kernel and one wave of CTAs, each thread's rows were a
+// serial chain of cold loads: Poisson 128^3 150 us, now 49 and 11.)
 __global__ void __launch_bounds__(kCgThreads) cg_residual_kernel(int32_t n, const int32_t *__restrict__ rowPtr,
                                                                  const int32_t *__restrict__ colIdx,
                                                                  const double *__restrict__ val,
                                                                  const double *__restrict__ b,
                                                                  const double *__restrict__ x,
-                                                                 double *__restrict__ r, VT *__restrict__ r_lp,
-                                                                 double *__restrict__ part,
-                                                                 double *__restrict__ part_lp,
-                                                                 double *__restrict__ part_dev = nullptr) {
+                                                                 double *__restrict__ r) {
+  const int64_t i = (int64_t)blockIdx.x * kCgThreads + threadIdx.x;
+  if (i >= n) return;
+  const int32_t s = rowPtr[i], e = rowPtr[i + 1];
+  int32_t c[kRowFirst];
+  double a[kRowFirst], xv[kRowFirst];
+#pragma unroll
+  for (int k = 0; k < kRowFirst; ++k) {
+    c[k] = s + k < e ? colIdx[s + k] : -1;
+    a[k] = s + k < e ? val[s + k] : 0.0;
+  }
+#pragma unroll
+  for (int k = 0; k < kRowFirst; ++k) xv[k] = c[k] >= 0 ? __ldg(x + c[k]) : 0.0;
+  double acc = 0.0;
+#pragma unroll
+  for (int k = 0; k < kRowFirst; ++k)
+    if (c[k] >= 0) acc = fma(a[k], xv[k], acc);
+  for (int32_t j = s + kRowFirst; j < e; ++j) acc = fma(val[j], __ldg(x + colIdx[j]), acc);
+  r[i] = b[i] - acc;
+}
+
+// Partials of ||r||^2; optionally also the inner-precision copy r_lp = (VT) r
+// and its partials (reliable update), and the partials of ||r - r_lp_old||^2,
+// the distance of the true residual from the iterated one it replaces
+// (part_dev, may be null).
+template <typename VT>
+__global__ void __launch_bounds__(kCgThreads) cg_norm_kernel(int32_t n, const double *__restrict__ r,
+                                                             VT *__restrict__ r_lp, double *__restrict__ part,
+                                                             double *__restrict__ part_lp,
+                                                             double *__restrict__ part_dev = nullptr) {
   __shared__ double smem[kCgThreads / 32];
   double nrm = 0.0, nrm_lp = 0.0, dev = 0.0;
   const int64_t stride = (int64_t)gridDim.x * kCgThreads;
+#pragma unroll 4
   for (int64_t i = (int64_t)blockIdx.x * kCgThreads + threadIdx.x; i < n; i += stride) {
-    const int32_t s = rowPtr[i], e = rowPtr[i + 1];
-    int32_t c[kRowFirst];
-    double a[kRowFirst];
-#pragma unroll
-    for (int k = 0; k < kRowFirst; ++k) {
-      c[k] = s + k < e ? colIdx[s + k] : -1;
-      a[k] = s + k < e ? val[s + k] : 0.0;
-    }
-    double acc = 0.0;
-#pragma unroll
-    for (int k = 0; k < kRowFirst; ++k)
-      if (c[k] >= 0) acc = fma(a[k], __ldg(x + c[k]), acc);
-    for (int32_t j = s + kRowFirst; j < e; ++j) acc = fma(val[j], __ldg(x + colIdx[j]), acc);
-    const double ri = b[i] - acc;
-    if (r) r[i] = ri;
+    const double ri = r[i];
     nrm += ri * ri;
     if (r_lp) {
       if (part_dev) {
@@ -783,12 +1228,6 @@ __global__ void row_exp_kernel(int32_t n, const int32_t *__restrict__ rowPtr, co
   }
 }
 
-template <typename V>
-__device__ __forceinline__ V from_float_lp(float f);
-template <> __device__ __forceinline__ float from_float_lp<float>(float f) { return f; }
-template <> __device__ __forceinline__ __half from_float_lp<__half>(float f) { return __float2half_rn(f); }
-template <> __device__ __forceinline__ __nv_bfloat16 from_float_lp<__nv_bfloat16>(float f) { return __float2bfloat16_rn(f); }
-
 // Thread per (slice row): its entries (scaled, converted) and columns (int16
 // offsets or int32) into the slice; padding = value 0, column = the row
 // itself (rows past n in the last slice: column 0, never gathered).
@@ -882,9 +1321,18 @@ struct bsp_cg_plan_s {
   double *p64 = nullptr, *q64 = nullptr, *z64 = nullptr;
   double *part_zq = nullptr, *part_pr = nullptr;
   int64_t bytes_outer = 0;
-  double *sc = nullptr, *h_sc = nullptr;  // [0],[1] rr slots, [2] ||b-Ax||^2, [3] ||b||^2, [4] rr after a chunk
+  double *sc = nullptr, *h_sc = nullptr;  // [0],[1] rr slots, [2] ||b-Ax||^2, [3] ||b||^2, [4] rr after a chunk,
+                                          // [8] error flag, [9] epoch of the fused iteration
   int grid = 0;    // update, residual and reduction kernels (writers of the rr partials)
   int grid_a = 0;  // direction/SpMV kernel (writer of the p.q partials)
+  // fused iteration (one cooperative launch per chunk): 0 CTAs = not used
+  int fused_ctas = 0;
+  size_t fused_smem = 0;
+  bsp::CgSlot *slots = nullptr;
+  void *pub = nullptr;  // published p with tags
+  void *fused_val = nullptr;  // the matrix by diagonals
+  bsp::FusedDiags fused_diags{};
+  int fused_nd = 0;
   cudaGraphExec_t graph = nullptr;
   cudaStream_t graph_stream = nullptr;
   int64_t bytes_iter = 0, bytes_residual = 0;
@@ -893,6 +1341,9 @@ struct bsp_cg_plan_s {
 namespace bsp {
 
 constexpr int kCgMaxCtasPerSm = 2048 / kCgThreads;
+constexpr int kCgScalars = 10;
+// 64 registers a thread in FP32; an FP64 thread holds twice the bytes in flight
+constexpr int kFusedThreads32 = 1024, kFusedThreads64 = 512;
 // Mixed modes: a replaced (true) residual whose distance from the iterated
 // one exceeds kCgDeviation x its norm, or an iterated residual above kCgGrowth
 // x the last true one, marks the low-precision matrix as too far from A for
@@ -1043,7 +1494,116 @@ static bsp_status cg_chunk(bsp_cg_plan_s *P, cudaStream_t s) {
   return BSP_OK;
 }
 
+struct FusedLaunch {
+  const void *kernel, *fill;
+  int threads;
+  size_t vsz;  // bytes of a stored value
+};
+template <typename V, typename VT, int THREADS>
+static FusedLaunch fused_for(int nd) {
+  const void *k = nd <= 5   ? (const void *)cg_fused_kernel<V, VT, 5, THREADS>
+                  : nd <= 7 ? (const void *)cg_fused_kernel<V, VT, 7, THREADS>
+                            : (const void *)cg_fused_kernel<V, VT, 8, THREADS>;
+  return {k, (const void *)fused_fill_kernel<V, sizeof(V) == 2>, THREADS, sizeof(V)};
+}
+
+static FusedLaunch fused_launch(const bsp_cg_plan_s *P) {
+  switch (P->opt.mode) {
+    case BSP_CG_FP64: return fused_for<double, double, kFusedThreads64>(P->fused_nd);
+    case BSP_CG_MIXED_F32: return fused_for<float, float, kFusedThreads32>(P->fused_nd);
+    case BSP_CG_MIXED_F16: return fused_for<__half, float, kFusedThreads32>(P->fused_nd);
+    default: return fused_for<__nv_bfloat16, float, kFusedThreads32>(P->fused_nd);
+  }
+}
+
+// Sets up the fused iteration where it applies: no preconditioner, one CTA per
+// SM whose share of the vectors fits in shared memory, and at most kFusedDiags
+// distinct diagonals that the rows fill by 3/4 or more.
+static bsp_status fused_setup(bsp_cg_plan_s *P, cudaStream_t s) {
+  if (P->prec_bs) return BSP_OK;
+  const size_t vt = cg_mixed(P) ? 4 : 8;
+  int dev = 0, coop = 0, optin = 0, sms = 0, occ = 0;
+  BSP_CUDA(cudaGetDevice(&dev));
+  BSP_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+  BSP_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  BSP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int64_t ns = ceil_div(P->n, 32);
+  const int threads = vt == 4 ? kFusedThreads32 : kFusedThreads64;
+  // a slice per warp before another CTA joins the sums
+  const int64_t ctas = std::min<int64_t>(ceil_div(ns, threads / 32), std::min(sms, kFusedMaxCtas));
+  const int64_t smem = ceil_div(ns, ctas) * 32 * 4 * (int64_t)vt;
+  if (!coop || smem > optin) return BSP_OK;
+  int32_t *d_set = nullptr, h_set[kFusedDiags + 1];
+  BSP_TRY(dalloc(&d_set, kFusedDiags + 1, s));
+  for (int k = 0; k < kFusedDiags; ++k) h_set[k] = kNoDiag;
+  h_set[kFusedDiags] = 0;
+  BSP_CUDA(cudaMemcpyAsync(d_set, h_set, sizeof(h_set), cudaMemcpyHostToDevice, s));
+  const unsigned gd = (unsigned)std::min<int64_t>(ceil_div(P->n, 256), (int64_t)sm_count() * 8);
+  fused_diags_kernel<<<gd, 256, 0, s>>>(P->n, P->rowPtr, P->colIdx, d_set, d_set + kFusedDiags);
+  BSP_LAUNCH_CHECK();
+  BSP_CUDA(cudaMemcpyAsync(h_set, d_set, sizeof(h_set), cudaMemcpyDeviceToHost, s));
+  BSP_CUDA(cudaStreamSynchronize(s));
+  dfree(d_set, s);
+  const int nd = (int)(std::find(h_set, h_set + kFusedDiags, kNoDiag) - h_set);
+  if (h_set[kFusedDiags] || nd == 0 || 4 * (int64_t)P->nnz < 3 * (int64_t)nd * P->n) return BSP_OK;
+  std::sort(h_set, h_set + nd);
+  // ascending, padded to the kernel's number with zero diagonals of its own row
+  // before the last one (their values are 0)
+  const int padded_nd = nd <= 5 ? 5 : nd <= 7 ? 7 : 8;
+  for (int k = 0; k < kFusedDiags; ++k) P->fused_diags.d[k] = 0;
+  for (int k = 0; k < nd; ++k) P->fused_diags.d[k + 1 == nd ? padded_nd - 1 : k] = h_set[k];
+  const auto range = std::minmax_element(P->fused_diags.d + 1, P->fused_diags.d + padded_nd - 1);
+  P->fused_diags.lo = *range.first;
+  P->fused_diags.hi = *range.second;
+  P->fused_nd = nd;
+  const FusedLaunch L = fused_launch(P);
+  cudaFuncAttributes fa{};
+  BSP_CUDA(cudaFuncGetAttributes(&fa, L.kernel));
+  if (smem + (int64_t)fa.sharedSizeBytes > optin) return BSP_OK;
+  BSP_CUDA(cudaFuncSetAttribute(L.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                optin - (int)fa.sharedSizeBytes));
+  BSP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L.kernel, threads, (size_t)smem));
+  if ((int64_t)occ * sms < ctas) return BSP_OK;
+  // an optimisation: without room for its buffers the two kernels run
+  if (pool_malloc(&P->fused_val, L.vsz * kFusedDiags * (size_t)ns * 32, s) != cudaSuccess ||
+      pool_malloc(&P->pub, 2 * vt * (size_t)ns * 32, s) != cudaSuccess ||
+      dalloc(&P->slots, 2 * kFusedMaxCtas, s) != BSP_OK) {
+    cudaGetLastError();
+    return BSP_OK;
+  }
+  BSP_CUDA(cudaMemsetAsync(P->slots, 0, 2 * kFusedMaxCtas * sizeof(CgSlot), s));
+  BSP_CUDA(cudaMemsetAsync(P->pub, 0, 2 * vt * (size_t)ns * 32, s));
+  const int64_t gf = std::min<int64_t>(ceil_div(P->n, 256), (int64_t)sm_count() * 32);
+  void *args[] = {&P->n, &P->rowPtr, &P->colIdx, &P->val, &P->exps, &P->fused_diags, &P->fused_val};
+  BSP_CUDA(cudaLaunchKernel(L.fill, dim3((unsigned)gf), dim3(256), args, 0, s));
+  P->fused_ctas = (int)ctas;
+  P->fused_smem = (size_t)smem;
+  return BSP_OK;
+}
+
+static bsp_status fused_chunk(bsp_cg_plan_s *P, cudaStream_t s) {
+  const FusedLaunch L = fused_launch(P);
+  int iters = P->opt.check_every, npart = P->grid;
+  double *epoch = P->sc + 9, *err = P->sc + 8;
+  void *args[] = {&P->n,   &P->fused_val, &P->fused_diags, &P->exps, &P->x,     &P->r,  &P->p[0], &P->pub,
+                  &P->part_rr, &npart,    &P->sc,          &iters,   &P->slots, &epoch, &err};
+  // One fused launch at a time on a device, whatever the streams and threads:
+  // two grids that wait for their own CTAs must not share the SMs by halves.
+  static std::mutex turn;
+  static std::map<unsigned long long, cudaEvent_t> last;  // by context
+  std::lock_guard<std::mutex> lock(turn);
+  cudaEvent_t &done = last[context_id()];
+  if (done)
+    BSP_CUDA(cudaStreamWaitEvent(s, done, 0));
+  else
+    BSP_CUDA(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+  BSP_CUDA(cudaLaunchCooperativeKernel(L.kernel, dim3(P->fused_ctas), dim3(L.threads), args, P->fused_smem, s));
+  BSP_CUDA(cudaEventRecord(done, s));
+  return BSP_OK;
+}
+
 static bsp_status cg_run_chunk(bsp_cg_plan_s *P, cudaStream_t s) {
+  if (P->fused_ctas) return fused_chunk(P, s);
   if (!P->opt.use_graphs) return cg_chunk(P, s);
   if (!P->graph) {
     if (!P->graph_stream) BSP_CUDA(cudaStreamCreateWithFlags(&P->graph_stream, cudaStreamNonBlocking));
@@ -1062,8 +1622,11 @@ static bsp_status cg_run_chunk(bsp_cg_plan_s *P, cudaStream_t s) {
 }
 
 static bsp_status read_scalars(bsp_cg_plan_s *P, cudaStream_t s) {
-  BSP_CUDA(cudaMemcpyAsync(P->h_sc, P->sc, 8 * sizeof(double), cudaMemcpyDeviceToHost, s));
+  BSP_CUDA(cudaMemcpyAsync(P->h_sc, P->sc, kCgScalars * sizeof(double), cudaMemcpyDeviceToHost, s));
   BSP_CUDA(cudaStreamSynchronize(s));
+  int32_t err = 0;
+  memcpy(&err, P->h_sc + 8, sizeof(err));
+  if (err) BSP_FAIL(BSP_ERR_TIMEOUT, "a bounded wait of the fused CG iteration gave up");
   return BSP_OK;
 }
 
@@ -1072,13 +1635,14 @@ static bsp_status read_scalars(bsp_cg_plan_s *P, cudaStream_t s) {
 // measure_dev (mixed modes): also ||r_true - r_iterated||^2 -> sc[7].
 static bsp_status cg_true_residual(bsp_cg_plan_s *P, const double *b, cudaStream_t s, bool measure_dev = false) {
   const int g = P->grid;
+  const unsigned gr = (unsigned)ceil_div(P->n, kCgThreads);
+  double *r = cg_mixed(P) ? P->r64 : (double *)P->r;
+  cg_residual_kernel<<<gr, kCgThreads, 0, s>>>(P->n, P->rowPtr, P->colIdx, P->val, b, P->x64, r);
   if (cg_mixed(P))
-    cg_residual_kernel<float><<<g, kCgThreads, 0, s>>>(P->n, P->rowPtr, P->colIdx, P->val, b, P->x64, P->r64,
-                                                        (float *)P->r, P->part_res, P->part_rr,
-                                                        measure_dev ? P->part_zq : nullptr);
+    cg_norm_kernel<float><<<g, kCgThreads, 0, s>>>(P->n, r, (float *)P->r, P->part_res, P->part_rr,
+                                                    measure_dev ? P->part_zq : nullptr);
   else
-    cg_residual_kernel<double><<<g, kCgThreads, 0, s>>>(P->n, P->rowPtr, P->colIdx, P->val, b, P->x64,
-                                                         (double *)P->r, nullptr, P->part_res, nullptr);
+    cg_norm_kernel<double><<<g, kCgThreads, 0, s>>>(P->n, r, nullptr, P->part_res, nullptr);
   BSP_LAUNCH_CHECK();
   if (!cg_mixed(P)) {  // the FP64 residual is the iterated one
     BSP_CUDA(cudaMemcpyAsync(P->part_rr, P->part_res, sizeof(double) * g, cudaMemcpyDeviceToDevice, s));
@@ -1194,6 +1758,9 @@ extern "C" bsp_status bsp_cg_destroy(bsp_cg_plan P) {
   dfree(P->z64, s);
   dfree(P->part_zq, s);
   dfree(P->part_pr, s);
+  dfree(P->slots, s);
+  if (P->pub) pool_free(P->pub, s);
+  if (P->fused_val) pool_free(P->fused_val, s);
   if (P->lp_cols) pool_free(P->lp_cols, s);
   dfree(P->exps, s);
   dfree(P->slice_len, s);
@@ -1255,8 +1822,9 @@ extern "C" bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPt
   BSP_CG_TRY(dalloc(&P->part_pq, (size_t)P->grid, s));
   BSP_CG_TRY(dalloc(&P->part_rr, (size_t)P->grid, s));
   BSP_CG_TRY(dalloc(&P->part_res, (size_t)P->grid, s));
-  BSP_CG_TRY(dalloc(&P->sc, 8, s));
-  BSP_CG_CUDA(cudaMallocHost(reinterpret_cast<void **>(&P->h_sc), 8 * sizeof(double)));
+  BSP_CG_TRY(dalloc(&P->sc, kCgScalars, s));
+  BSP_CG_CUDA(cudaMemsetAsync(P->sc, 0, kCgScalars * sizeof(double), s));
+  BSP_CG_CUDA(cudaMallocHost(reinterpret_cast<void **>(&P->h_sc), kCgScalars * sizeof(double)));
   if (mixed) {
     P->x = nullptr;  // x32 allocated below
   }
@@ -1291,7 +1859,19 @@ extern "C" bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPt
   const bool try64 = !mixed && P->lpr == 1;
   int64_t padded = 0;
   if (mixed || try64) {
-    const bool scaled = mixed && opt->mode != BSP_CG_MIXED_F32;
+    if (mixed && opt->mode != BSP_CG_MIXED_F32) {
+      BSP_CG_TRY(dalloc(&P->exps, (size_t)n, s));
+      const unsigned ge = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 16));
+      row_exp_kernel<<<ge, 256, 0, s>>>(n, rowPtr, values, P->exps);
+    }
+    BSP_CG_TRY(fused_setup(P, s));
+  }
+  if (P->fused_ctas) {  // the diagonals replace the SELL copy
+    const int64_t vsz = !mixed ? 8 : opt->mode == BSP_CG_MIXED_F32 ? 4 : 2;
+    mat_bytes = ceil_div(n, 32) * 32 * kFusedDiags * vsz + (P->exps ? (int64_t)n : 0);
+    const int32_t *d = P->fused_diags.d;
+    P->delta16 = std::all_of(d, d + kFusedDiags, [](int32_t v) { return v >= -32768 && v <= 32767; });
+  } else if (mixed || try64) {
     // SELL-32 slices: lengths on the device, offsets summed on the host
     const int64_t ns = ceil_div(n, 32);
     BSP_CG_TRY(dalloc(&P->slice_len, (size_t)ns, s));
@@ -1326,11 +1906,6 @@ extern "C" bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPt
       P->sell_uniform = 0;  // FP64 stays on the CSR arrays
     }
     BSP_CG_CUDA(cudaMemcpyAsync(P->slice_off, hoff.data(), sizeof(int64_t) * (ns + 1), cudaMemcpyHostToDevice, s));
-    if (scaled) {
-      BSP_CG_TRY(dalloc(&P->exps, (size_t)n, s));
-      const unsigned ge = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 16));
-      row_exp_kernel<<<ge, 256, 0, s>>>(n, rowPtr, values, P->exps);
-    }
     int32_t *bad = nullptr;
     BSP_CG_TRY(dalloc(&bad, 1, s));
     cudaMemsetAsync(bad, 0, sizeof(int32_t), s);
@@ -1350,7 +1925,8 @@ extern "C" bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPt
       P->sell_uniform = 0;
     }
   }
-  if (mixed || P->sell64) {
+  const bool sell = !P->fused_ctas && (mixed || P->sell64);
+  if (sell) {
     const bool scaled = mixed && opt->mode != BSP_CG_MIXED_F32;
     const size_t vsz = !mixed ? 8 : opt->mode == BSP_CG_MIXED_F32 ? 4 : 2;
     const bool packed = scaled && P->delta16;
@@ -1376,7 +1952,7 @@ extern "C" bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPt
         BSP_CG_CUDA(pool_malloc(reinterpret_cast<void **>(&P->lp_cols), (P->delta16 ? 2 : 4) * (size_t)(padded > 0 ? padded : 1), s));
     }
   }
-  if (mixed || P->sell64) {
+  if (sell && (mixed || P->sell64)) {
     const bool scaled = mixed && opt->mode != BSP_CG_MIXED_F32;
     const size_t vsz = !mixed ? 8 : opt->mode == BSP_CG_MIXED_F32 ? 4 : 2;
     const int64_t ns = ceil_div(n, 32);
@@ -1417,7 +1993,7 @@ extern "C" bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPt
   // gathers counted once) and writes p and q; kernel B reads p, q, x, r and
   // writes x, r.
   // Preconditioned: the update kernel also reads M^{-1} and writes z.
-  P->bytes_iter = mat_bytes + (mixed || P->sell64 ? 0 : 4 * ((int64_t)n + 1)) + 10 * (int64_t)vt * n;
+  P->bytes_iter = mat_bytes + (mixed || P->sell64 || P->fused_ctas ? 0 : 4 * ((int64_t)n + 1)) + 10 * (int64_t)vt * n;
   if (P->prec_bs)
     P->bytes_iter += (int64_t)vt * (ceil_div(n, P->prec_bs) * P->prec_bs * P->prec_bs + (int64_t)n);
   P->bytes_residual = (int64_t)nnz * 12 + 4 * ((int64_t)n + 1) + 3 * 8 * (int64_t)n;
@@ -1460,10 +2036,8 @@ extern "C" bsp_status bsp_cg_solve(bsp_cg_plan P, const double *b, double *x, bs
   BSP_CUDA(cudaEventCreate(&e0));
   BSP_CUDA(cudaEventCreate(&e1));
   BSP_CUDA(cudaEventRecord(e0, s));
-  // ||b||^2 via the residual of x = 0 (x64 zeroed), then x64 = x0
-  BSP_CUDA(cudaMemsetAsync(P->x64, 0, sizeof(double) * P->n, s));
-  cg_residual_kernel<double><<<g, kCgThreads, 0, s>>>(P->n, P->rowPtr, P->colIdx, P->val, b, P->x64, nullptr,
-                                                       nullptr, P->part_res, nullptr);
+  // ||b||^2, then x64 = x0
+  cg_norm_kernel<double><<<g, kCgThreads, 0, s>>>(P->n, b, nullptr, P->part_res, nullptr);
   sum_partials_kernel<<<1, kCgThreads, 0, s>>>(P->part_res, g, P->sc + 3);
   BSP_LAUNCH_CHECK();
   BSP_CUDA(cudaMemcpyAsync(P->x64, x, sizeof(double) * P->n, cudaMemcpyDeviceToDevice, s));

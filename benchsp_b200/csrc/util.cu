@@ -37,8 +37,8 @@ struct DevicePool {
 };
 std::mutex g_pool_mutex;
 DevicePool g_pools[kPoolDevices];
+}  // namespace
 
-// Id of the calling thread's context, never reused by the driver; 0 if unknown.
 unsigned long long context_id() {
   using IdFn = CUresult (*)(CUcontext, unsigned long long *);
   static const IdFn fn = [] {
@@ -53,6 +53,7 @@ unsigned long long context_id() {
   return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
 }
 
+namespace {
 // The pool of the stream's device, or an empty one where the default pool serves.
 DevicePool device_pool(cudaStream_t s) {
   int dev = 0, cur = 0;

@@ -118,3 +118,73 @@ def test_cg_without_graphs_matches(cuda):
     x2, r2 = bsp.CgSolver(rp, ci, va, mode="f16", use_graphs=False).solve(bb)
     assert r1["iterations"] == r2["iterations"]
     assert np.array_equal(x1.cpu().numpy(), x2.cpu().numpy())
+
+
+def _banded(n, diags, seed):
+    """SPD: symmetric bands at +-diags with varying negative values (every 50th
+    entry missing), diagonally dominant."""
+    import scipy.sparse as sp
+    rng = np.random.default_rng(seed)
+    M = sp.csr_matrix((n, n))
+    for d in diags:
+        if d < n:
+            v = -rng.uniform(0.5, 1.0, n - d)
+            v[::50] = 0.0
+            M = M + sp.diags([v, v], [d, -d], shape=(n, n), format="csr")
+    M.eliminate_zeros()
+    M = (M + sp.diags(np.asarray(abs(M).sum(1)).ravel() + 0.5, format="csr")).tocsr()
+    M.sort_indices()
+    return bsp.HostCSR(n, n, M.indptr.astype(np.int32), M.indices.astype(np.int32), M.data.astype(np.float64))
+
+
+# the fused iteration (at most 8 diagonals, vectors in shared memory): one row,
+# a part of a slice, one CTA and several, 1, 3, 5 and 7 diagonals, neighbours in
+# the next CTA and several CTAs away, a ragged last slice, the last size that
+# fits 148 SMs in FP32 and the first that does not; 9 diagonals take two kernels
+@pytest.mark.parametrize("n,diags", [
+    (1, []), (31, [1]), (33, [1]), (1000, []), (1025, [1, 7]), (5000, [1, 70]), (70001, [1, 33, 1024]),
+    (200003, [2, 450, 45000]), (20000, [1, 50, 700, 3000]), (2150144, [1, 1466]), (2160000, [1, 1466])])
+@pytest.mark.parametrize("mode", ["fp64", "f32", "f16", "bf16"])
+def test_cg_fused_edges(cuda, n, diags, mode):
+    A = _banded(n, diags, n)
+    b = bsp.gen_uniform(n, 15)
+    rp, ci, va, bb = _dev(cuda, A.rowptr, A.colidx, A.values, b)
+    S = bsp.CgSolver(rp, ci, va, mode=mode, tol=1e-10)
+    for start in (None, bb * 0.5):
+        x, res = S.solve(bb, None if start is None else start.clone())
+        assert res["converged"] == 1
+        assert pyoracle.rel_residual(A.rowptr, A.colidx, A.values, b, x.cpu().numpy()) <= 2e-10
+    S.close()
+
+
+def test_cg_fused_on_several_streams(cuda):
+    """Solves on streams of their own, all at once: the same bits as alone."""
+    import threading
+
+    import torch
+    A = bsp.gen_poisson3d(64)
+    rp, ci, va, bb = _dev(cuda, A.rowptr, A.colidx, A.values, bsp.gen_uniform(A.rows, 16))
+    modes = ["f16", "f32", "bf16", "f16"]
+    want = {}
+    for m in set(modes):
+        S = bsp.CgSolver(rp, ci, va, mode=m, tol=1e-10)
+        want[m] = S.solve(bb)[0]
+        S.close()
+    torch.cuda.synchronize()
+    same = [False] * len(modes)
+
+    def work(k):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            S = bsp.CgSolver(rp, ci, va, mode=modes[k], tol=1e-10)
+            xs = [S.solve(bb)[0] for _ in range(3)]
+            s.synchronize()
+            same[k] = all(torch.equal(x, want[modes[k]]) for x in xs)
+            S.close()
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(modes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert all(same)
