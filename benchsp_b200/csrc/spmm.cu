@@ -1759,6 +1759,29 @@ __global__ void spmm_long_chunk_kernel(int32_t rows, const int32_t *__restrict__
   }
 }
 
+// Sort keys of the long rows' chunks: the chunk's position in its row, in
+// 65536ths.  The slab engine takes the chunks in this order (rows in order
+// within a position), so the warps at work at one time read the same stretch
+// of every long row.  With sorted columns spread over the matrix that is the
+// same stretch of B, and a B row fetched from memory for one row is still in
+// L2 for the others; in row order the chunks of one row, which share no
+// column, run together and B is fetched again for each row.  Graph 2^20,
+// Zipf 1.8, FP16 (103,000 chunks hold 83% of the nonzeros): N = 128
+// 1.457 -> 1.119 ms, N = 64 0.796 -> 0.625, N = 32 0.408 -> 0.390, N = 256
+// 2.80 -> 2.31; DRAM reads at N = 128 2.6 GB for 8.1 GB gathered.  Rows whose
+// columns lie elsewhere lose nothing: a chunk's B rows are no longer read
+// beside those of the next chunk of its row, and the two share none.  The sums
+// are the same: every chunk still writes the partial row of its own slot.
+__global__ void spmm_long_key_kernel(int64_t nparts, const int32_t *__restrict__ long_chunk,
+                                     const int32_t *__restrict__ chunk_row, const int32_t *__restrict__ chunk_ptr,
+                                     int32_t *__restrict__ key, int32_t *__restrict__ slot) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nparts; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t w = long_chunk[i], r = chunk_row[w], c0 = chunk_ptr[r];
+    key[i] = (int32_t)(((int64_t)(w - c0) << 16) / (chunk_ptr[r + 1] - c0));
+    slot[i] = (int32_t)i;
+  }
+}
+
 // Sort keys for the short-row list: chunk - length for rows of at most
 // `chunk` nonzeros (so a stable ascending sort puts the longest first),
 // chunk + 1 for split rows (sorted past the end of the list).
@@ -1771,9 +1794,10 @@ __global__ void spmm_short_key_kernel(int32_t rows, const int32_t *__restrict__ 
   }
 }
 
-// Nonzero ranges for the slab engine: (start, end) of each partial-row
-// slot's chunk and of each listed short row.
+// Nonzero ranges for the slab engine: (start, end) of the chunk of each slot
+// in long_slot's order and of each listed short row.
 __global__ void spmm_range_kernel(int64_t nparts, const int32_t *__restrict__ long_chunk,
+                                  const int32_t *__restrict__ long_slot,
                                   const int32_t *__restrict__ chunk_row, const int32_t *__restrict__ chunk_ptr,
                                   int32_t chunk, int32_t nshort, const int32_t *__restrict__ short_rows,
                                   const int32_t *__restrict__ rowPtr, int2 *__restrict__ long_se,
@@ -1781,7 +1805,7 @@ __global__ void spmm_range_kernel(int64_t nparts, const int32_t *__restrict__ lo
   const int64_t n = nparts > nshort ? nparts : nshort;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     if (i < nparts) {
-      const int32_t w = long_chunk[i];
+      const int32_t w = long_chunk[long_slot[i]];
       const int32_t r = chunk_row[w];
       const int32_t st = rowPtr[r] + (w - chunk_ptr[r]) * chunk;
       long_se[i] = make_int2(st, min(st + chunk, rowPtr[r + 1]));
@@ -1866,15 +1890,23 @@ extern "C" bsp_status bsp_spmm_plan_create(int32_t rows, int32_t nnz, const int3
   }
   dfree(flag, s);
   dfree(tot, s);
-  // slab engine: the long chunks in partial-slot order, the short rows by length
+  // slab engine: the long chunks by position in their row, the short rows by length
   p.nshort = rows - p.nsplit;
-  BSP_TRY(dalloc(&p.long_chunk, (size_t)(p.nparts > 0 ? p.nparts : 1), s));
+  BSP_TRY(dalloc(&p.long_chunk, (size_t)2 * (p.nparts > 0 ? p.nparts : 1), s));
   BSP_TRY(dalloc(&p.short_rows, (size_t)(rows > 0 ? rows : 1), s));
   if (rows > 0) {
     spmm_long_chunk_kernel<<<g, 256, 0, s>>>(rows, p.chunk_ptr, p.part_ptr, p.long_chunk);
     BSP_LAUNCH_CHECK();
+    int32_t *const long_slot = p.long_chunk + p.nparts;
     int32_t *keys = nullptr;
-    BSP_TRY(dalloc(&keys, (size_t)rows, s));
+    BSP_TRY(dalloc(&keys, (size_t)std::max<int64_t>(rows, p.nparts), s));
+    if (p.nparts > 0) {
+      spmm_long_key_kernel<<<g, 256, 0, s>>>(p.nparts, p.long_chunk, p.chunk_row, p.chunk_ptr, keys, long_slot);
+      BSP_LAUNCH_CHECK();
+      const bsp_status st = radix_sort_pairs(keys, long_slot, p.nparts, 16, s);
+      if (st != BSP_OK) dfree(keys, s);
+      BSP_TRY(st);
+    }
     spmm_short_key_kernel<<<g, 256, 0, s>>>(rows, rowPtr, chunk, keys, p.short_rows);
     BSP_LAUNCH_CHECK();
     const bsp_status st = radix_sort_pairs(keys, p.short_rows, rows, bits_for(chunk + 1), s);
@@ -1886,8 +1918,8 @@ extern "C" bsp_status bsp_spmm_plan_create(int32_t rows, int32_t nnz, const int3
   if (p.nparts > 0 || p.nshort > 0) {
     const int64_t n = std::max<int64_t>(p.nparts, p.nshort);
     const unsigned gr = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 32));
-    spmm_range_kernel<<<gr, 256, 0, s>>>(p.nparts, p.long_chunk, p.chunk_row, p.chunk_ptr, chunk, p.nshort,
-                                         p.short_rows, rowPtr, reinterpret_cast<int2 *>(p.long_se),
+    spmm_range_kernel<<<gr, 256, 0, s>>>(p.nparts, p.long_chunk, p.long_chunk + p.nparts, p.chunk_row, p.chunk_ptr,
+                                         chunk, p.nshort, p.short_rows, rowPtr, reinterpret_cast<int2 *>(p.long_se),
                                          reinterpret_cast<int2 *>(p.short_se));
     BSP_LAUNCH_CHECK();
   }
@@ -2021,7 +2053,8 @@ static bsp_status chunked_typed(const bsp_spmm_plan *p, int32_t N, const int32_t
 // every gathered B row after the first touch is an L2 hit, at the price of
 // reading A once per slab.  Warp tasks [0, nlong) are the long rows' chunks,
 // a warp each (G groups of LPR lanes split the chunk's nonzeros, then a
-// fixed shuffle tree), written to their partial-row slot; the remaining tasks
+// fixed shuffle tree) in the plan's order, written to their partial-row slot
+// (long_slot[task]); the remaining tasks
 // take G consecutive rows of the length-sorted short-row list, one row per
 // group of LPR lanes, so a warp has G rows' load chains in flight at once
 // instead of one.  Every task reads its nonzero range from the plan in one
@@ -2082,8 +2115,9 @@ template <int LPR> struct SlabU {
 template <typename T, int LPR, int U, int UL>
 __global__ void __launch_bounds__(256, LPR >= 8 && LPR <= 16 ? (std::is_same<T, __nv_bfloat16>::value ? 4 : 5) : 0)
     spmm_slab_kernel(
-    int64_t nlong, const int2 *__restrict__ long_se, int32_t nshort, const int32_t *__restrict__ short_rows,
-    const int2 *__restrict__ short_se, const int32_t *__restrict__ colIdx, const T *__restrict__ val,
+    int64_t nlong, const int2 *__restrict__ long_se, const int32_t *__restrict__ long_slot, int32_t nshort,
+    const int32_t *__restrict__ short_rows, const int2 *__restrict__ short_se,
+    const int32_t *__restrict__ colIdx, const T *__restrict__ val,
     const T *__restrict__ B, int64_t ldb, int32_t col0, float *__restrict__ C, int64_t ldc,
     float *__restrict__ part, float alpha, float beta, int32_t hints) {
   constexpr int VEC = SpmmVec<T>::VEC;
@@ -2109,6 +2143,7 @@ __global__ void __launch_bounds__(256, LPR >= 8 && LPR <= 16 ? (std::is_same<T, 
       constexpr int BQ = 32 * Q;
       const int2 se = long_se[task];
       const int32_t e = se.y;
+      const int64_t slot = long_slot[task];
       int32_t cj[Q];
       float vj[Q];
 #pragma unroll
@@ -2159,7 +2194,7 @@ __global__ void __launch_bounds__(256, LPR >= 8 && LPR <= 16 ? (std::is_same<T, 
 #pragma unroll
         for (int k = 0; k < VEC; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
       if (lane < LPR) {
-        float *pp = part + task * NS + li * VEC;
+        float *pp = part + slot * NS + li * VEC;
 #pragma unroll
         for (int k = 0; k < VEC; ++k) pp[k] = acc[k];
       }
@@ -2225,12 +2260,16 @@ static bsp_status launch_slab(const bsp_spmm_plan *p, const int32_t *ci, const v
                               int32_t hints, cudaStream_t s) {
   constexpr int G = 32 / LPR;
   const int64_t ntasks = p->nparts + (p->nshort + G - 1) / G;
+  // 64 CTAs per SM, a few of them resident: their first tasks start in list
+  // order, which keeps the long chunks in step (graph 2^20, FP16, N = 128:
+  // 64 per SM 1.119 ms, 32 1.174, one task per warp 1.165, only the resident
+  // CTAs 1.37).
   int64_t blocks = ceil_div(ntasks, 8);
-  const int64_t cap = (int64_t)sm_count() * 32;
+  const int64_t cap = (int64_t)sm_count() * 64;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
   spmm_slab_kernel<T, LPR, SlabU<LPR>::U, SlabU<LPR>::UL><<<(unsigned)blocks, 256, 0, s>>>(
-      p->nparts, reinterpret_cast<const int2 *>(p->long_se), p->nshort, p->short_rows,
+      p->nparts, reinterpret_cast<const int2 *>(p->long_se), p->long_chunk + p->nparts, p->nshort, p->short_rows,
       reinterpret_cast<const int2 *>(p->short_se), ci, (const T *)val, (const T *)B, ldb, col0, C, ldc, part, a, b,
       hints);
   BSP_LAUNCH_CHECK();

@@ -460,8 +460,8 @@ typedef struct {
   int32_t *split_rows; /* [nsplit] */
   int32_t nshort;      /* rows of at most `chunk` nonzeros (empty rows included) */
   int32_t *short_rows; /* [nshort] those rows, longest first (stable) */
-  int32_t *long_chunk; /* [nparts] chunk index of each partial-row slot */
-  int32_t *long_se;    /* [2*nparts] (start, end) nonzero range of each slot's chunk */
+  int32_t *long_chunk; /* [2*nparts] chunk index of each partial-row slot, then the slots in the order the slab engine takes them */
+  int32_t *long_se;    /* [2*nparts] (start, end) nonzero range of each slot's chunk, in that order */
   int32_t *short_se;   /* [2*nshort] (start, end) nonzero range of each listed short row */
   int32_t slab_l2_hints; /* slab engine cache policy for slabs of B of at most 64 MiB
                             (cols x slab width; wider slabs use default caching), set to

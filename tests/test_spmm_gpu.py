@@ -304,6 +304,44 @@ def test_spmm_plan_ranges_match_row_pointers(cuda):
     P.free()
 
 
+@pytest.mark.parametrize("chunk,lens", [
+    (256, [1000, 257, 2900, 30, 0, 513]),
+    (256, [256] * 5),            # no long row
+    (32, [33, 64, 2900, 1, 65]),
+])
+def test_spmm_plan_orders_long_chunks(cuda, chunk, lens):
+    """The slab engine's order of the long rows' chunks: every partial-row
+    slot once, by the chunk's position in its row (ties in row order), with
+    its own nonzero range; the sums do not depend on it."""
+    import torch
+    from benchsp_b200.api import _d2h
+    rng = np.random.default_rng(4)
+    lens = np.asarray(lens)
+    n = 3000
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = np.concatenate([np.sort(rng.choice(n, l, replace=False)) for l in lens]).astype(np.int32)
+    rpd, cid = _dev(cuda, rp, ci)
+    v = torch.from_numpy(rng.integers(-3, 4, rp[-1]).astype(np.float16)).to(cuda)
+    P = bsp.SpmmPlan(rpd, cid, v, cols=n, chunk=chunk)
+    d = P._d
+    slots = [(r, k, -(-int(lens[r]) // chunk)) for r in np.flatnonzero(lens > chunk) for k in range(-(-int(lens[r]) // chunk))]
+    assert d.nparts == len(slots)
+    if slots:
+        slot = _d2h(d.long_chunk, 2 * d.nparts, np.int32)[d.nparts:]
+        se = _d2h(d.long_se, 2 * d.nparts, np.int32).reshape(-1, 2)
+        assert slot.tolist() == sorted(range(len(slots)), key=lambda i: (slots[i][1] << 16) // slots[i][2])
+        assert se.tolist() == [[int(rp[r]) + k * chunk, min(int(rp[r]) + (k + 1) * chunk, int(rp[r + 1]))]
+                               for r, k, _ in (slots[i] for i in slot)]
+    # small whole numbers: every sum is exact in FP32, whatever its order
+    B = torch.from_numpy(rng.integers(-3, 4, (n, 64)).astype(np.float16)).to(cuda)
+    want = np.zeros((len(lens), 64))
+    np.add.at(want, np.repeat(np.arange(len(lens)), lens),
+              v.cpu().numpy().astype(np.float64)[:, None] * B.cpu().numpy().astype(np.float64)[ci])
+    for slab in (0, 8, 32):
+        assert np.array_equal(P.spmm(B, engine="slab", slab_cols=slab).cpu().numpy().astype(np.float64), want)
+    P.free()
+
+
 def test_spmm_slab_engine_rejects_bad_widths(cuda):
     import torch
     A = bsp.gen_powerlaw(500, 1.8, 100, 3)
