@@ -2079,21 +2079,18 @@ __device__ __forceinline__ int32_t ld_hint_s32(const int32_t *p, uint64_t pol) {
   asm("ld.global.nc.L1::no_allocate.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(r) : "l"(p), "l"(pol));
   return r;
 }
-template <typename T> __device__ __forceinline__ float ld_hint_val(const T *p, uint64_t pol);
-template <> __device__ __forceinline__ float ld_hint_val<float>(const float *p, uint64_t pol) {
-  float r;
-  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(r) : "l"(p), "l"(pol));
-  return r;
-}
-template <> __device__ __forceinline__ float ld_hint_val<__half>(const __half *p, uint64_t pol) {
-  unsigned short r;
-  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(r) : "l"(p), "l"(pol));
-  return __half2float(__ushort_as_half(r));
-}
-template <> __device__ __forceinline__ float ld_hint_val<__nv_bfloat16>(const __nv_bfloat16 *p, uint64_t pol) {
-  unsigned short r;
-  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(r) : "l"(p), "l"(pol));
-  return __bfloat162float(__ushort_as_bfloat16(r));
+// An A value's bits (all types are carried as a 32-bit word until the FMA).
+template <typename T>
+__device__ __forceinline__ uint32_t ld_hint_val(const T *p, uint64_t pol) {
+  if constexpr (sizeof(T) == 4) {
+    uint32_t r;
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(r) : "l"(p), "l"(pol));
+    return r;
+  } else {
+    unsigned short r;
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(r) : "l"(p), "l"(pol));
+    return r;
+  }
 }
 __device__ __forceinline__ uint4 ld_hint_b16(const void *p, uint64_t pol) {
   uint4 r;
@@ -2103,17 +2100,67 @@ __device__ __forceinline__ uint4 ld_hint_b16(const void *p, uint64_t pol) {
   return r;
 }
 
+// acc[0 .. VEC) += v * the 16 bytes of a B row, each an FP32 fused multiply-add.
+// For 16-bit types it is the mixed form, which takes its factors as FP16 or
+// BF16 and accumulates in FP32: the product and the sum are those of fmaf on
+// the converted operands, bit for bit, without converting the 8 elements of
+// each gather.  The pass issues 71% of the time (N = 128), so instructions
+// are what it waits for: graph 2^20, FP16, N = 128 converted, with fmaf
+// 0.967 ms, with the two-wide FP32 form 0.986, mixed 0.915.
+__device__ __forceinline__ void fma16(float (&acc)[4], float v, const uint4 &u) {
+  acc[0] = fmaf(v, __uint_as_float(u.x), acc[0]);
+  acc[1] = fmaf(v, __uint_as_float(u.y), acc[1]);
+  acc[2] = fmaf(v, __uint_as_float(u.z), acc[2]);
+  acc[3] = fmaf(v, __uint_as_float(u.w), acc[3]);
+}
+__device__ __forceinline__ void fma16(float (&acc)[8], __half v, const uint4 &u) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    asm("{.reg .b16 l, h; mov.b32 {l, h}, %2; fma.rn.f32.f16 %0, l, %3, %0; fma.rn.f32.f16 %1, h, %3, %1;}"
+        : "+f"(acc[2 * k]), "+f"(acc[2 * k + 1])
+        : "r"(w[k]), "h"(__half_as_ushort(v)));
+}
+__device__ __forceinline__ void fma16(float (&acc)[8], __nv_bfloat16 v, const uint4 &u) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    asm("{.reg .b16 l, h; mov.b32 {l, h}, %2; fma.rn.f32.bf16 %0, l, %3, %0; fma.rn.f32.bf16 %1, h, %3, %1;}"
+        : "+f"(acc[2 * k]), "+f"(acc[2 * k + 1])
+        : "r"(w[k]), "h"(__bfloat16_as_ushort(v)));
+}
+
+// A value back from its bits.
+template <typename T> __device__ __forceinline__ T bits_val(uint32_t b);
+template <> __device__ __forceinline__ float bits_val<float>(uint32_t b) { return __uint_as_float(b); }
+template <> __device__ __forceinline__ __half bits_val<__half>(uint32_t b) { return __ushort_as_half((unsigned short)b); }
+template <> __device__ __forceinline__ __nv_bfloat16 bits_val<__nv_bfloat16>(uint32_t b) {
+  return __ushort_as_bfloat16((unsigned short)b);
+}
+
 // Gathers in flight per lane group: U for a short row, UL per warp step of a
-// long chunk.  8 at 4 lanes per B row (graph 2^20, FP16, N = 32) took 78
-// registers and 0.551 ms (UL alone 0.605 ms, UL capped at 64 registers
-// 0.507 ms) against 0.470 ms with 4.
+// long chunk.  8 per step of a long chunk at 8 and 16 lanes per B row measured
+// slower (graph 2^20, FP16: N = 128 0.929 ms against 0.903, N = 64 0.542
+// against 0.507), as at 4 lanes (N = 32, an earlier form: 0.551 ms against
+// 0.470): the registers cost more warps than the loads gain.
 template <int LPR> struct SlabU {
   static constexpr int U = 4;
   static constexpr int UL = 4;
 };
 
-template <typename T, int LPR, int U, int UL>
-__global__ void __launch_bounds__(256, LPR >= 8 && LPR <= 16 ? (std::is_same<T, __nv_bfloat16>::value ? 4 : 5) : 0)
+// Instructions bound this kernel, then warps in flight.  A whole batch of 32
+// nonzeros runs without masks (only a chunk's last batch is partial), A's
+// values stay in their own bits until the FMA, and a gather's address is one
+// 32 x 32 -> 64 bit multiply-add of the column and B's row pitch in bytes.
+// WIDE takes a 64-bit pitch, for rows of B 4 GiB apart or more.  Graph 2^20,
+// FP16, N = 128 1.119 -> 0.897 ms (843 M warp instructions before), N = 64
+// 0.625 -> 0.503, N = 32 0.390 -> 0.323, N = 256 2.31 -> 1.74; BF16 N = 64
+// 0.685 -> 0.503; graph 2^18, FP32, N = 128 0.474 -> 0.321.
+// Register bounds: 16-bit types 4 CTAs per SM (N = 128: 4 0.903 ms, 5 with
+// 48 bytes spilled 0.962, 6 1.041; N = 32: 4 0.323, 5 0.338; N = 256: 4 1.74,
+// none 1.93), FP32 5 (N = 128: 5 0.321, 6 0.343).
+template <typename T, int LPR, int U, int UL, bool WIDE>
+__global__ void __launch_bounds__(256, sizeof(T) == 2 ? (LPR >= 4 ? 4 : 0) : (LPR >= 8 ? 5 : 0))
     spmm_slab_kernel(
     int64_t nlong, const int2 *__restrict__ long_se, const int32_t *__restrict__ long_slot, int32_t nshort,
     const int32_t *__restrict__ short_rows, const int2 *__restrict__ short_se,
@@ -2127,6 +2174,9 @@ __global__ void __launch_bounds__(256, LPR >= 8 && LPR <= 16 ? (std::is_same<T, 
   const int li = lane % LPR;
   const int g = lane / LPR;
   const int32_t cl = col0 + li * VEC;
+  const char *const Bc = (const char *)(B + cl);
+  using pitch_t = typename std::conditional<WIDE, uint64_t, uint32_t>::type;
+  const pitch_t pitch = (pitch_t)(ldb * (int64_t)sizeof(T));
   const uint64_t pa = l2_policy(hints != 0, false), pb = l2_policy(hints == 1, true);
   const int64_t ntasks = nlong + (nshort + G - 1) / G;
   const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -2145,42 +2195,55 @@ __global__ void __launch_bounds__(256, LPR >= 8 && LPR <= 16 ? (std::is_same<T, 
       const int32_t e = se.y;
       const int64_t slot = long_slot[task];
       int32_t cj[Q];
-      float vj[Q];
+      uint32_t vj[Q];
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         const int32_t j = se.x + q * 32 + lane;
         cj[q] = j < e ? ld_hint_s32(colIdx + j, pa) : 0;
-        vj[q] = j < e ? ld_hint_val<T>(val + j, pa) : 0.f;
+        vj[q] = j < e ? ld_hint_val<T>(val + j, pa) : 0u;
       }
       for (int32_t j0 = se.x; j0 < e; j0 += BQ) {   // warp-uniform bounds
         int32_t cn[Q];
-        float vn[Q];
+        uint32_t vn[Q];
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
           const int32_t jn = j0 + BQ + q * 32 + lane;
           cn[q] = jn < e ? ld_hint_s32(colIdx + jn, pa) : 0;
-          vn[q] = jn < e ? ld_hint_val<T>(val + jn, pa) : 0.f;
+          vn[q] = jn < e ? ld_hint_val<T>(val + jn, pa) : 0u;
         }
         const int cnt = e - j0 < BQ ? e - j0 : BQ;
-        for (int t = 0; t < cnt; t += GU) {   // one trip when Q > 1
-          uint4 raw[UL];
-          float v[UL];
+        if (cnt == BQ) {   // a whole batch: nothing to mask
+#pragma unroll 1
+          for (int t = 0; t < BQ; t += GU) {
+            uint4 raw[UL];
+            uint32_t v[UL];
 #pragma unroll
-          for (int u = 0; u < UL; ++u) {
-            const int src = t + u * G + g;
-            const int q = Q > 1 ? (u * G) >> 5 : 0;   // t == 0 when Q > 1
-            const int32_t c = __shfl_sync(0xffffffffu, cj[q], src & 31);
-            const float vv = __shfl_sync(0xffffffffu, vj[q], src & 31);
-            const bool ok = src < cnt;
-            v[u] = ok ? vv : 0.f;
-            raw[u] = ok ? ld_hint_b16(B + (int64_t)c * ldb + cl, pb) : make_uint4(0, 0, 0, 0);
+            for (int u = 0; u < UL; ++u) {
+              const int src = t + u * G + g;
+              const int q = Q > 1 ? (u * G) >> 5 : 0;   // t == 0 when Q > 1
+              const int32_t c = __shfl_sync(0xffffffffu, cj[q], src & 31);
+              v[u] = __shfl_sync(0xffffffffu, vj[q], src & 31);
+              raw[u] = ld_hint_b16(Bc + (uint64_t)(uint32_t)c * pitch, pb);
+            }
+#pragma unroll
+            for (int u = 0; u < UL; ++u) fma16(acc, bits_val<T>(v[u]), raw[u]);
           }
+        } else {
+          for (int t = 0; t < cnt; t += GU) {   // one trip when Q > 1
+            uint4 raw[UL];
+            uint32_t v[UL];
 #pragma unroll
-          for (int u = 0; u < UL; ++u) {
-            float b[VEC];
-            unpack16<T>(raw[u], b);
+            for (int u = 0; u < UL; ++u) {
+              const int src = t + u * G + g;
+              const int q = Q > 1 ? (u * G) >> 5 : 0;   // t == 0 when Q > 1
+              const int32_t c = __shfl_sync(0xffffffffu, cj[q], src & 31);
+              const uint32_t vv = __shfl_sync(0xffffffffu, vj[q], src & 31);
+              const bool ok = src < cnt;
+              v[u] = ok ? vv : 0u;
+              raw[u] = ok ? ld_hint_b16(Bc + (uint64_t)(uint32_t)c * pitch, pb) : make_uint4(0, 0, 0, 0);
+            }
 #pragma unroll
-            for (int k = 0; k < VEC; ++k) acc[k] = fmaf(v[u], b[k], acc[k]);
+            for (int u = 0; u < UL; ++u) fma16(acc, bits_val<T>(v[u]), raw[u]);
           }
         }
 #pragma unroll
@@ -2206,35 +2269,30 @@ __global__ void __launch_bounds__(256, LPR >= 8 && LPR <= 16 ? (std::is_same<T, 
     const int2 se = short_se[i];
     const int32_t s = se.x, e = se.y;
     int32_t cn[U];
-    float vn[U];
+    uint32_t vn[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const bool ok = s + u < e;
       cn[u] = ok ? ld_hint_s32(colIdx + s + u, pa) : 0;
-      vn[u] = ok ? ld_hint_val<T>(val + s + u, pa) : 0.f;
+      vn[u] = ok ? ld_hint_val<T>(val + s + u, pa) : 0u;
     }
     for (int32_t j = s; j < e; j += U) {
       uint4 raw[U];
-      float v[U];
+      uint32_t v[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         v[u] = vn[u];
-        raw[u] = j + u < e ? ld_hint_b16(B + (int64_t)cn[u] * ldb + cl, pb) : make_uint4(0, 0, 0, 0);
+        raw[u] = j + u < e ? ld_hint_b16(Bc + (uint64_t)(uint32_t)cn[u] * pitch, pb) : make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int32_t jj = j + U + u;
         const bool ok = jj < e;
         cn[u] = ok ? ld_hint_s32(colIdx + jj, pa) : 0;
-        vn[u] = ok ? ld_hint_val<T>(val + jj, pa) : 0.f;
+        vn[u] = ok ? ld_hint_val<T>(val + jj, pa) : 0u;
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        float b[VEC];
-        unpack16<T>(raw[u], b);
-#pragma unroll
-        for (int k = 0; k < VEC; ++k) acc[k] = fmaf(v[u], b[k], acc[k]);
-      }
+      for (int u = 0; u < U; ++u) fma16(acc, bits_val<T>(v[u]), raw[u]);
     }
     float *cp = C + (int64_t)r * ldc + cl;
     if (beta != 0.f) {
@@ -2254,7 +2312,7 @@ __global__ void __launch_bounds__(256, LPR >= 8 && LPR <= 16 ? (std::is_same<T, 
   }
 }
 
-template <typename T, int LPR>
+template <typename T, int LPR, bool WIDE = false>
 static bsp_status launch_slab(const bsp_spmm_plan *p, const int32_t *ci, const void *val, const void *B,
                               int64_t ldb, int32_t col0, float *C, int64_t ldc, float *part, float a, float b,
                               int32_t hints, cudaStream_t s) {
@@ -2268,7 +2326,7 @@ static bsp_status launch_slab(const bsp_spmm_plan *p, const int32_t *ci, const v
   const int64_t cap = (int64_t)sm_count() * 64;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
-  spmm_slab_kernel<T, LPR, SlabU<LPR>::U, SlabU<LPR>::UL><<<(unsigned)blocks, 256, 0, s>>>(
+  spmm_slab_kernel<T, LPR, SlabU<LPR>::U, SlabU<LPR>::UL, WIDE><<<(unsigned)blocks, 256, 0, s>>>(
       p->nparts, reinterpret_cast<const int2 *>(p->long_se), p->long_chunk + p->nparts, p->nshort, p->short_rows,
       reinterpret_cast<const int2 *>(p->short_se), ci, (const T *)val, (const T *)B, ldb, col0, C, ldc, part, a, b,
       hints);
@@ -2311,6 +2369,9 @@ static bsp_status slab_typed(const bsp_spmm_plan *p, int32_t N, int32_t cols, in
                              const void *val, const void *B, int64_t ldb, float *C, int64_t ldc, float *part,
                              float a, float b, cudaStream_t s) {
   constexpr int VEC = SpmmVec<T>::VEC;
+  // rows of B 4 GiB apart or more: one kernel, 16 bytes of B row wide
+  const bool wide = (uint64_t)ldb * sizeof(T) > 0xffffffffull;
+  if (wide) ns = VEC;
   const int32_t hints = (double)cols * ns * sizeof(T) <= kHintSlabBytes ? p->slab_l2_hints : 0;
   for (int32_t col0 = 0; col0 < N; col0 += ns) {
     bsp_status st;
@@ -2320,7 +2381,10 @@ static bsp_status slab_typed(const bsp_spmm_plan *p, int32_t N, int32_t cols, in
       case 8: st = launch_slab<T, 8>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s); break;
       case 4: st = launch_slab<T, 4>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s); break;
       case 2: st = launch_slab<T, 2>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s); break;
-      case 1: st = launch_slab<T, 1>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s); break;
+      case 1:
+        st = wide ? launch_slab<T, 1, true>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s)
+                  : launch_slab<T, 1>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s);
+        break;
       default: BSP_FAIL(BSP_ERR_UNSUPPORTED, "slab width");
     }
     BSP_TRY(st);

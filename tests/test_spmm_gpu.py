@@ -342,6 +342,82 @@ def test_spmm_plan_orders_long_chunks(cuda, chunk, lens):
     P.free()
 
 
+@pytest.mark.parametrize("name", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("N", [8, 32, 64, 128, 256])
+def test_spmm_slab_products_are_fp32(cuda, name, N):
+    """Every entry of C is one FP32 product v*b plus zeros (each row has one
+    value that is not 0), so it equals the rounded product bit for bit: with
+    subnormals, the largest finite values, infinities and NaN, in a short row,
+    in a whole and a partial batch of a long row's chunk."""
+    import torch
+    dt = getattr(torch, name)
+    fi = torch.finfo(dt)
+    special = torch.tensor([1.0, -1.5, fi.max, -fi.max, fi.tiny, fi.smallest_normal / 4, -fi.smallest_normal / 2,
+                            fi.eps, 3.0, 0.0, float("inf"), float("nan")], dtype=torch.float64).to(dt)
+    lens = np.array([1, 5, 31, 256, 257, 300, 1024])
+    where = [0, 4, 30, 255, 256, 299, 500]          # the entry that is not 0
+    n = 1024
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = np.concatenate([np.arange(l) for l in lens]).astype(np.int32)
+    rpd, cid = _dev(cuda, rp, ci)
+    B = torch.ones(n, N, dtype=dt)
+    for k, w in enumerate(where):
+        B[w] = special[(torch.arange(N) + k) % len(special)]
+    Bd = B.to(cuda)
+    for v in special.tolist():
+        vals = torch.zeros(int(rp[-1]), dtype=dt)
+        for k, w in enumerate(where):
+            vals[rp[k] + w] = v
+        P = bsp.SpmmPlan(rpd, cid, vals.to(cuda), cols=n, chunk=256)
+        got = P.spmm(Bd, engine="slab").cpu()
+        for k, w in enumerate(where):
+            want = torch.tensor(v, dtype=dt).float() * B[w].float()
+            # 0 * (infinity or NaN) of another row's entry: NaN in this row too
+            bad = torch.zeros(N, dtype=torch.bool)
+            for w2 in where:
+                if w2 < lens[k] and w2 != w:
+                    bad |= ~torch.isfinite(B[w2])
+            assert torch.equal(got[k][bad].isnan(), torch.ones(int(bad.sum()), dtype=torch.bool))
+            g, t = got[k][~bad], want[~bad]
+            assert torch.equal(g.isnan(), t.isnan())
+            assert torch.equal(g[~t.isnan()], t[~t.isnan()])
+        P.free()
+
+
+def test_spmm_slab_rows_of_b_4gib_apart(cuda):
+    """A row pitch of B that does not fit 32 bits (the C call takes one)."""
+    import ctypes as C
+    import torch
+    from benchsp_b200._lib import check, lib
+    from benchsp_b200.api import _dtype_code
+    free, _ = torch.cuda.mem_get_info()
+    pitch = (1 << 31) + 8                 # FP16 elements: 4 GiB + 16 bytes
+    if free < 16 << 30:
+        pytest.skip("needs 16 GB of device memory")
+    rng = np.random.default_rng(6)
+    rp = np.array([0, 3, 4, 4, 304], np.int32)
+    ci = np.concatenate([[0, 1, 2], [2], rng.integers(0, 3, 300)]).astype(np.int32)
+    rpd, cid = _dev(cuda, rp, ci)
+    v = torch.from_numpy(rng.integers(-3, 4, 304).astype(np.float16)).to(cuda)
+    store = torch.empty(2 * pitch + 16, dtype=torch.float16, device=cuda)
+    Bd = torch.as_strided(store, (3, 16), (pitch, 1))
+    B = rng.integers(-3, 4, (3, 16)).astype(np.float16)
+    Bd.copy_(torch.from_numpy(B))
+    P = bsp.SpmmPlan(rpd, cid, v, cols=3)
+    want = np.zeros((4, 16))
+    np.add.at(want, np.repeat(np.arange(4), np.diff(rp)), v.cpu().numpy().astype(np.float64)[:, None] * B.astype(np.float64)[ci])
+    need = P.workspace_bytes(16)
+    ws = torch.empty(need, dtype=torch.uint8, device=cuda)
+    for slab in (0, 8, 16):
+        out = torch.full((4, 16), -1.0, device=cuda)
+        check(lib().bsp_spmm_csr_planned_variant(C.byref(P._d), 3, 304, rpd.data_ptr(), cid.data_ptr(), v.data_ptr(),
+                                                 _dtype_code(v), Bd.data_ptr(), 16, pitch, out.data_ptr(), 16, 1.0, 0.0,
+                                                 ws.data_ptr(), need, 2, slab, None))
+        torch.cuda.synchronize()
+        assert np.array_equal(out.cpu().numpy().astype(np.float64), want)
+    P.free()
+
+
 def test_spmm_slab_engine_rejects_bad_widths(cuda):
     import torch
     A = bsp.gen_powerlaw(500, 1.8, 100, 3)
