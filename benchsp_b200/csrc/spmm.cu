@@ -2048,13 +2048,10 @@ static bsp_status chunked_typed(const bsp_spmm_plan *p, int32_t N, const int32_t
 }
 
 // ---------------------------------------------------------------------------
-// Slab engine.  One pass per slab of NS = LPR*VEC columns [col0, col0 + NS):
-// B's slab (B rows x NS) is small enough to stay in L2 for the whole pass, so
-// every gathered B row after the first touch is an L2 hit, at the price of
-// reading A once per slab.  Warp tasks [0, nlong) are the long rows' chunks,
-// a warp each (G groups of LPR lanes split the chunk's nonzeros, then a
-// fixed shuffle tree) in the plan's order, written to their partial-row slot
-// (long_slot[task]); the remaining tasks
+// Slab engine.  One pass per slab of ns <= LPR*VEC columns [col0, col0 + ns).
+// Warp tasks [0, nlong) are the long rows' chunks, a warp each (G groups of
+// LPR lanes split the chunk's nonzeros, then a fixed shuffle tree) in the
+// plan's order, written to their partial-row slot (long_slot[task]); the rest
 // take G consecutive rows of the length-sorted short-row list, one row per
 // group of LPR lanes, so a warp has G rows' load chains in flight at once
 // instead of one.  Every task reads its nonzero range from the plan in one
@@ -2160,20 +2157,21 @@ template <int LPR> struct SlabU {
 // 48 bytes spilled 0.962, 6 1.041; N = 32: 4 0.323, 5 0.338; N = 256: 4 1.74,
 // none 1.93), FP32 5 (N = 128: 5 0.321, 6 0.343).
 template <typename T, int LPR, int U, int UL, bool WIDE>
-__global__ void __launch_bounds__(256, sizeof(T) == 2 ? (LPR >= 4 ? 4 : 0) : (LPR >= 8 ? 5 : 0))
+__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 4 : (LPR >= 8 ? 5 : 0))
     spmm_slab_kernel(
     int64_t nlong, const int2 *__restrict__ long_se, const int32_t *__restrict__ long_slot, int32_t nshort,
     const int32_t *__restrict__ short_rows, const int2 *__restrict__ short_se,
     const int32_t *__restrict__ colIdx, const T *__restrict__ val,
-    const T *__restrict__ B, int64_t ldb, int32_t col0, float *__restrict__ C, int64_t ldc,
+    const T *__restrict__ B, int64_t ldb, int32_t col0, int32_t ns, float *__restrict__ C, int64_t ldc,
     float *__restrict__ part, float alpha, float beta, int32_t hints) {
   constexpr int VEC = SpmmVec<T>::VEC;
-  constexpr int NS = LPR * VEC;
   constexpr int G = 32 / LPR;
   const int lane = threadIdx.x & 31;
   const int li = lane % LPR;
   const int g = lane / LPR;
-  const int32_t cl = col0 + li * VEC;
+  // a lane past the slab's last column reads that column again and stores nothing
+  const bool on = li * VEC < ns;
+  const int32_t cl = col0 + (on ? li * VEC : ns - VEC);
   const char *const Bc = (const char *)(B + cl);
   using pitch_t = typename std::conditional<WIDE, uint64_t, uint32_t>::type;
   const pitch_t pitch = (pitch_t)(ldb * (int64_t)sizeof(T));
@@ -2185,59 +2183,42 @@ __global__ void __launch_bounds__(256, sizeof(T) == 2 ? (LPR >= 4 ? 4 : 0) : (LP
 #pragma unroll
     for (int k = 0; k < VEC; ++k) acc[k] = 0.f;
     if (task < nlong) {   // warp-uniform
-      // Batches of BQ = 32*Q nonzeros: Q = 1 while a warp step's G*U gathers
-      // fit in 32 (LPR >= 4), else one step takes the whole batch, so narrow
-      // B rows still keep G*U gathers in flight per warp.
-      constexpr int GU = G * UL;
-      constexpr int Q = GU > 32 ? GU / 32 : 1;
-      constexpr int BQ = 32 * Q;
+      constexpr int GU = G * UL;   // nonzeros per step
+      static_assert(32 % GU == 0, "a step takes a part of a batch");
       const int2 se = long_se[task];
       const int32_t e = se.y;
       const int64_t slot = long_slot[task];
-      int32_t cj[Q];
-      uint32_t vj[Q];
-#pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        const int32_t j = se.x + q * 32 + lane;
-        cj[q] = j < e ? ld_hint_s32(colIdx + j, pa) : 0;
-        vj[q] = j < e ? ld_hint_val<T>(val + j, pa) : 0u;
-      }
-      for (int32_t j0 = se.x; j0 < e; j0 += BQ) {   // warp-uniform bounds
-        int32_t cn[Q];
-        uint32_t vn[Q];
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-          const int32_t jn = j0 + BQ + q * 32 + lane;
-          cn[q] = jn < e ? ld_hint_s32(colIdx + jn, pa) : 0;
-          vn[q] = jn < e ? ld_hint_val<T>(val + jn, pa) : 0u;
-        }
-        const int cnt = e - j0 < BQ ? e - j0 : BQ;
-        if (cnt == BQ) {   // a whole batch: nothing to mask
+      const int32_t jl = se.x + lane;
+      int32_t cj = jl < e ? ld_hint_s32(colIdx + jl, pa) : 0;
+      uint32_t vj = jl < e ? ld_hint_val<T>(val + jl, pa) : 0u;
+      for (int32_t j0 = se.x; j0 < e; j0 += 32) {   // warp-uniform bounds
+        const int32_t jn = j0 + 32 + lane;
+        const int32_t cn = jn < e ? ld_hint_s32(colIdx + jn, pa) : 0;
+        const uint32_t vn = jn < e ? ld_hint_val<T>(val + jn, pa) : 0u;
+        const int cnt = e - j0 < 32 ? e - j0 : 32;
+        if (cnt == 32) {   // a whole batch: nothing to mask
 #pragma unroll 1
-          for (int t = 0; t < BQ; t += GU) {
+          for (int t = 0; t < 32; t += GU) {
             uint4 raw[UL];
             uint32_t v[UL];
 #pragma unroll
             for (int u = 0; u < UL; ++u) {
-              const int src = t + u * G + g;
-              const int q = Q > 1 ? (u * G) >> 5 : 0;   // t == 0 when Q > 1
-              const int32_t c = __shfl_sync(0xffffffffu, cj[q], src & 31);
-              v[u] = __shfl_sync(0xffffffffu, vj[q], src & 31);
+              const int32_t c = __shfl_sync(0xffffffffu, cj, t + u * G + g);
+              v[u] = __shfl_sync(0xffffffffu, vj, t + u * G + g);
               raw[u] = ld_hint_b16(Bc + (uint64_t)(uint32_t)c * pitch, pb);
             }
 #pragma unroll
             for (int u = 0; u < UL; ++u) fma16(acc, bits_val<T>(v[u]), raw[u]);
           }
         } else {
-          for (int t = 0; t < cnt; t += GU) {   // one trip when Q > 1
+          for (int t = 0; t < cnt; t += GU) {
             uint4 raw[UL];
             uint32_t v[UL];
 #pragma unroll
             for (int u = 0; u < UL; ++u) {
               const int src = t + u * G + g;
-              const int q = Q > 1 ? (u * G) >> 5 : 0;   // t == 0 when Q > 1
-              const int32_t c = __shfl_sync(0xffffffffu, cj[q], src & 31);
-              const uint32_t vv = __shfl_sync(0xffffffffu, vj[q], src & 31);
+              const int32_t c = __shfl_sync(0xffffffffu, cj, src);
+              const uint32_t vv = __shfl_sync(0xffffffffu, vj, src);
               const bool ok = src < cnt;
               v[u] = ok ? vv : 0u;
               raw[u] = ok ? ld_hint_b16(Bc + (uint64_t)(uint32_t)c * pitch, pb) : make_uint4(0, 0, 0, 0);
@@ -2246,18 +2227,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == 2 ? (LPR >= 4 ? 4 : 0) : (LP
             for (int u = 0; u < UL; ++u) fma16(acc, bits_val<T>(v[u]), raw[u]);
           }
         }
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-          cj[q] = cn[q];
-          vj[q] = vn[q];
-        }
+        cj = cn;
+        vj = vn;
       }
 #pragma unroll
       for (int o = LPR; o < 32; o <<= 1)
 #pragma unroll
         for (int k = 0; k < VEC; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-      if (lane < LPR) {
-        float *pp = part + slot * NS + li * VEC;
+      if (lane < LPR && on) {
+        float *pp = part + slot * ns + li * VEC;
 #pragma unroll
         for (int k = 0; k < VEC; ++k) pp[k] = acc[k];
       }
@@ -2294,6 +2272,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 2 ? (LPR >= 4 ? 4 : 0) : (LP
 #pragma unroll
       for (int u = 0; u < U; ++u) fma16(acc, bits_val<T>(v[u]), raw[u]);
     }
+    if (!on) continue;
     float *cp = C + (int64_t)r * ldc + cl;
     if (beta != 0.f) {
 #pragma unroll
@@ -2314,8 +2293,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 2 ? (LPR >= 4 ? 4 : 0) : (LP
 
 template <typename T, int LPR, bool WIDE = false>
 static bsp_status launch_slab(const bsp_spmm_plan *p, const int32_t *ci, const void *val, const void *B,
-                              int64_t ldb, int32_t col0, float *C, int64_t ldc, float *part, float a, float b,
-                              int32_t hints, cudaStream_t s) {
+                              int64_t ldb, int32_t col0, int32_t ns, float *C, int64_t ldc, float *part, float a,
+                              float b, int32_t hints, cudaStream_t s) {
   constexpr int G = 32 / LPR;
   const int64_t ntasks = p->nparts + (p->nshort + G - 1) / G;
   // 64 CTAs per SM, a few of them resident: their first tasks start in list
@@ -2328,20 +2307,36 @@ static bsp_status launch_slab(const bsp_spmm_plan *p, const int32_t *ci, const v
   if (blocks < 1) blocks = 1;
   spmm_slab_kernel<T, LPR, SlabU<LPR>::U, SlabU<LPR>::UL, WIDE><<<(unsigned)blocks, 256, 0, s>>>(
       p->nparts, reinterpret_cast<const int2 *>(p->long_se), p->long_chunk + p->nparts, p->nshort, p->short_rows,
-      reinterpret_cast<const int2 *>(p->short_se), ci, (const T *)val, (const T *)B, ldb, col0, C, ldc, part, a, b,
-      hints);
+      reinterpret_cast<const int2 *>(p->short_se), ci, (const T *)val, (const T *)B, ldb, col0, ns, C, ldc, part, a,
+      b, hints);
   BSP_LAUNCH_CHECK();
   return BSP_OK;
 }
 
-// Slab width (columns per pass) for the slab engine; 0 when it cannot run
+// Lanes per B row of the next pass when `n` 16-byte pieces of the row are left:
+// the fewest of 4, 8, 16 and 32 that hold them all.  The lanes past the last
+// piece do the same work as its lane and store nothing, which costs less than
+// further passes (each reads A and runs the reduce again).  Graph 2^20, FP16:
+// N = 96 as 16 lanes 0.834 ms, as 8 + 4 0.932, as three times 4 1.091; N = 40
+// as 8 lanes 0.461, as 4 + 4 0.675; N = 136 as 32 lanes 1.44, as 16 + 4 1.38;
+// graph 100,000, FP16: N = 96 0.087 against 0.143 and 0.203, N = 136 0.142
+// against 0.177 (17 passes of one lane, the widest that divides it: 1.79).
+// One and two lanes per B row had kernels of their own: N = 8 / 16 0.240 /
+// 0.261 ms against 0.255 / 0.277 at 2^20, 0.042 against 0.027 for N = 8 at
+// 10,000.
+static int slab_lanes(int n) {
+  int l = 32;
+  while (l > 4 && n <= l / 2) l >>= 1;
+  return l;
+}
+
+// Slab width (most columns per pass) for the slab engine; 0 when it cannot run
 // (B rows not 16-byte aligned, N not a multiple of VEC).  With `want` == 0:
-// the widest slab of at most 32 lanes of 16 bytes that divides N (graph
-// 2^20, FP16, N = 256: 32 lanes 3.49 ms, 16 lanes in two passes 3.62).  Slabs
-// sized so that B's slab stays in L2 measured slower (power-law graph 2^20,
-// FP16, N = 128: four 32-column passes 2.42 ms against one 128-column pass
-// 1.81 ms): the gathers run at the same rate from L2 as from DRAM, and every
-// pass reads A again.
+// 32 lanes of 16 bytes, or N if that is narrower.  Slabs sized so that B's slab
+// stays in L2 measured slower (power-law graph 2^20, FP16, N = 128, before the
+// pass lost a third of its instructions: four 32-column passes 1.81 ms, two of
+// 64 1.30, one 1.16): every pass reads A again and B's rows are found in L2
+// without it.
 template <typename T>
 static int slab_width(int32_t N, int32_t cols, const void *B, int64_t ldb, int32_t want) {
   constexpr int VEC = SpmmVec<T>::VEC;
@@ -2353,9 +2348,7 @@ static int slab_width(int32_t N, int32_t cols, const void *B, int64_t ldb, int32
     return want;
   }
   (void)cols;
-  int l = 32;
-  while (l > 1 && N % (l * VEC) != 0) l >>= 1;
-  return l * VEC;
+  return std::min(32 * VEC, N);
 }
 
 // The plan's L2 hints apply to slabs of B of at most kHintSlabBytes
@@ -2365,27 +2358,26 @@ static int slab_width(int32_t N, int32_t cols, const void *B, int64_t ldb, int32
 constexpr double kHintSlabBytes = 64.0 * 1024 * 1024;
 
 template <typename T>
-static bsp_status slab_typed(const bsp_spmm_plan *p, int32_t N, int32_t cols, int32_t ns, const int32_t *ci,
+static bsp_status slab_typed(const bsp_spmm_plan *p, int32_t N, int32_t cols, int32_t width, const int32_t *ci,
                              const void *val, const void *B, int64_t ldb, float *C, int64_t ldc, float *part,
                              float a, float b, cudaStream_t s) {
   constexpr int VEC = SpmmVec<T>::VEC;
-  // rows of B 4 GiB apart or more: one kernel, 16 bytes of B row wide
+  // rows of B 4 GiB apart or more: one kernel, 4 lanes wide
   const bool wide = (uint64_t)ldb * sizeof(T) > 0xffffffffull;
-  if (wide) ns = VEC;
-  const int32_t hints = (double)cols * ns * sizeof(T) <= kHintSlabBytes ? p->slab_l2_hints : 0;
-  for (int32_t col0 = 0; col0 < N; col0 += ns) {
+  if (wide && width > 4 * VEC) width = 4 * VEC;
+  for (int32_t col0 = 0, ns; col0 < N; col0 += ns) {
+    const int l = slab_lanes(std::min(width, N - col0) / VEC);
+    ns = std::min(l * VEC, std::min(width, N - col0));
+    const int32_t hints = (double)cols * ns * sizeof(T) <= kHintSlabBytes ? p->slab_l2_hints : 0;
     bsp_status st;
-    switch (ns / VEC) {
-      case 32: st = launch_slab<T, 32>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s); break;
-      case 16: st = launch_slab<T, 16>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s); break;
-      case 8: st = launch_slab<T, 8>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s); break;
-      case 4: st = launch_slab<T, 4>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s); break;
-      case 2: st = launch_slab<T, 2>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s); break;
-      case 1:
-        st = wide ? launch_slab<T, 1, true>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s)
-                  : launch_slab<T, 1>(p, ci, val, B, ldb, col0, C, ldc, part, a, b, hints, s);
+    switch (l) {
+      case 32: st = launch_slab<T, 32>(p, ci, val, B, ldb, col0, ns, C, ldc, part, a, b, hints, s); break;
+      case 16: st = launch_slab<T, 16>(p, ci, val, B, ldb, col0, ns, C, ldc, part, a, b, hints, s); break;
+      case 8: st = launch_slab<T, 8>(p, ci, val, B, ldb, col0, ns, C, ldc, part, a, b, hints, s); break;
+      default:
+        st = wide ? launch_slab<T, 4, true>(p, ci, val, B, ldb, col0, ns, C, ldc, part, a, b, hints, s)
+                  : launch_slab<T, 4>(p, ci, val, B, ldb, col0, ns, C, ldc, part, a, b, hints, s);
         break;
-      default: BSP_FAIL(BSP_ERR_UNSUPPORTED, "slab width");
     }
     BSP_TRY(st);
     BSP_TRY(split_reduce(p, ns, part, part + (int64_t)p->nparts * N, C + col0, ldc, a, b, s));

@@ -343,6 +343,35 @@ def test_spmm_plan_orders_long_chunks(cuda, chunk, lens):
 
 
 @pytest.mark.parametrize("name", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("pieces", [1, 2, 3, 4, 5, 7, 8, 9, 12, 16, 17, 31, 32, 33, 69])
+def test_spmm_slab_any_number_of_pieces(cuda, name, pieces):
+    """N of any number of 16-byte pieces: one pass of the lanes that hold what
+    is left, the lanes past the last piece storing nothing.  Small whole
+    numbers, so every sum is exact in FP32; with beta too."""
+    import torch
+    dt = getattr(torch, name)
+    N = pieces * (16 // torch.empty(0, dtype=dt).element_size())
+    rng = np.random.default_rng(pieces)
+    lens = np.array([0, 1, 3, 40, 256, 257, 700, 2, 5, 0, 1030])
+    n = 1100
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = np.concatenate([np.sort(rng.choice(n, l, replace=False)) for l in lens]).astype(np.int32)
+    rpd, cid = _dev(cuda, rp, ci)
+    v = rng.integers(-3, 4, rp[-1]).astype(np.float64)
+    B = rng.integers(-3, 4, (n, N)).astype(np.float64)
+    P = bsp.SpmmPlan(rpd, cid, torch.from_numpy(v).to(dt).to(cuda), cols=n, chunk=256)
+    Bd = torch.from_numpy(B).to(dt).to(cuda)
+    want = np.zeros((len(lens), N))
+    np.add.at(want, np.repeat(np.arange(len(lens)), lens), v[:, None] * B[ci])
+    assert np.array_equal(P.spmm(Bd, engine="slab").cpu().numpy().astype(np.float64), want)
+    C0 = rng.integers(-5, 6, want.shape).astype(np.float32)
+    Cd = torch.from_numpy(C0.copy()).to(cuda)
+    P.spmm(Bd, Cd, alpha=2.0, beta=-3.0, engine="slab")
+    assert np.array_equal(Cd.cpu().numpy().astype(np.float64), 2.0 * want - 3.0 * C0)
+    P.free()
+
+
+@pytest.mark.parametrize("name", ["float16", "bfloat16", "float32"])
 @pytest.mark.parametrize("N", [8, 32, 64, 128, 256])
 def test_spmm_slab_products_are_fp32(cuda, name, N):
     """Every entry of C is one FP32 product v*b plus zeros (each row has one
