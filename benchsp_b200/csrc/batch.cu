@@ -238,72 +238,37 @@ __device__ __forceinline__ void rows_item(const BatchMatDev &M, int32_t r0, int3
   }
 }
 
-// SELL-32 slices [s0, s1): lane l owns slice row l and sums its entries
-// in stored order, U entries' loads issued before their gathers.  Value and
-// column loads of a warp are 32 consecutive entries (coalesced); for banded
-// matrices (narrow form) the gathered x rows are consecutive too.
-template <typename V, int NRHS, bool WIDE>
-__device__ __forceinline__ void sell_item(const BatchMatDev &M, int32_t s0, int32_t s1, int lane) {
-  constexpr int U = NRHS == 1 ? 4 : 2;
-  const V *sv = static_cast<const V *>(M.sell_val);
-  const V *x = static_cast<const V *>(M.x);
-  V *y = static_cast<V *>(M.y);
-  for (int32_t sl = s0; sl < s1; ++sl) {
-    const int32_t pos = sl * 32 + lane;
-    const bool live = pos < (WIDE ? M.sell_rows : M.rows);
-    const int32_t row = WIDE ? (live ? __ldg(M.sell_perm + pos) : 0) : pos;
-    const int32_t p0 = __ldg(M.sell_ptr + sl);
-    const int32_t w = live ? (__ldg(M.sell_ptr + sl + 1) - p0) >> 5 : 0;
-    const V *vp = sv + p0 + lane;
-    const int16_t *op = M.sell_off + p0 + lane;
-    const int32_t *cp = M.sell_col + p0 + lane;
-    V acc[NRHS];
-#pragma unroll
-    for (int k = 0; k < NRHS; ++k) acc[k] = V(0);
-    int32_t k = 0;
-    for (; k + U <= w; k += U) {
-      V a[U];
-      int32_t c[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        a[u] = __ldg(vp + 32 * (k + u));
-        c[u] = WIDE ? __ldg(cp + 32 * (k + u)) : row + (int32_t)__ldg(op + 32 * (k + u));
-      }
-      V xr[U][NRHS];
-#pragma unroll
-      for (int u = 0; u < U; ++u) load_xrow<V, NRHS>(x, c[u], xr[u]);
-#pragma unroll
-      for (int u = 0; u < U; ++u) fma_row<V, NRHS>(acc, a[u], xr[u]);
-    }
-    for (; k < w; ++k) {
-      V xr[NRHS];
-      load_xrow<V, NRHS>(x, WIDE ? __ldg(cp + 32 * k) : row + (int32_t)__ldg(op + 32 * k), xr);
-      fma_row<V, NRHS>(acc, __ldg(vp + 32 * k), xr);
-    }
-    if (live) {
-#pragma unroll
-      for (int j = 0; j < NRHS; ++j) y[(int64_t)row * NRHS + j] = acc[j];
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Several right-hand sides (x and y row-major, NRHS values per row): the
-// CPL = NRHS * sizeof(V) / 16 lanes of a row split its columns, one 16-byte
+// CPL = NRHS * sizeof(V) / 16 lanes of a row split its columns, one
 // piece each, so a gathered x row is one contiguous access of the row's
-// lanes and a lane keeps VW = 16 / sizeof(V) sums instead of NRHS (FP64, 8
-// vectors: 4 lanes of 2 columns).  L lanes per row split the nonzeros as in
+// lanes and a lane keeps VW sums instead of NRHS (FP64, 8
+// vectors: 2 lanes of 4 columns, or 4 of 2).  L lanes per row split the nonzeros as in
 // the one-vector items; each column is summed in the same order as there
 // (lane sub takes entries s+sub, s+sub+L, ... in order, then a fixed shuffle
 // tree over the L lanes).
-template <typename V> struct Piece { static constexpr int VW = 16 / (int)sizeof(V); };
-
-template <typename V>
-__device__ __forceinline__ void load_piece(const V *__restrict__ p, V (&o)[Piece<V>::VW]) {
-  if constexpr (sizeof(V) == 8) {
+//
+// A piece is VW values: 32 bytes (one 256-bit access) where every x and y is
+// 32-byte aligned, else 16.  The wider pieces take half the lanes per row, so a
+// pass has twice the rows (and loads) in flight and the entry loads, which all
+// lanes of a row repeat, are halved.  8 vectors, 512 matrices: FP32 354 ->
+// 345 us, FP64 648 -> 611; 100 matrices, FP32, 86.4 -> 81.4; 60, FP64, 104 -> 92.5.
+template <typename V, int VW>
+__device__ __forceinline__ void load_piece(const V *__restrict__ p, V (&o)[VW]) {
+  if constexpr (sizeof(V) == 8 && VW == 4) {
+    const f64x4 t = ld_x4(p);
+    o[0] = t.x;
+    o[1] = t.y;
+    o[2] = t.z;
+    o[3] = t.w;
+  } else if constexpr (sizeof(V) == 8) {
     const double2 t = __ldg(reinterpret_cast<const double2 *>(p));
     o[0] = t.x;
     o[1] = t.y;
+  } else if constexpr (VW == 8) {
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
+        : "l"(p));
   } else {
     const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
     o[0] = t.x;
@@ -313,23 +278,29 @@ __device__ __forceinline__ void load_piece(const V *__restrict__ p, V (&o)[Piece
   }
 }
 
-template <typename V>
-__device__ __forceinline__ void store_piece(V *p, const V (&v)[Piece<V>::VW]) {
-  if constexpr (sizeof(V) == 8)
-    *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
-  else
+// p: global, or (16-byte pieces and FP64) shared memory.
+template <typename V, int VW>
+__device__ __forceinline__ void store_piece(V *p, const V (&v)[VW]) {
+  if constexpr (sizeof(V) == 8) {
+#pragma unroll
+    for (int k = 0; k < VW; k += 2) *reinterpret_cast<double2 *>(p + k) = make_double2(v[k], v[k + 1]);
+  } else if constexpr (VW == 8) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+  } else {
     *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  }
 }
 
 // acc (columns [cp*VW, cp*VW + VW)) += sum over entries j, j + stride, ... < e
 // in order, in predicated groups of U: a group's entry loads go out together,
 // then its U gathers together, so a short row costs one entries -> x round
 // trip instead of one per entry.
-template <typename V, int NRHS>
+template <typename V, int NRHS, int VW>
 __device__ __forceinline__ void strided_piece_dot(const int32_t *__restrict__ ci, const V *__restrict__ val,
                                                   const V *__restrict__ x, int cp, int32_t j, int32_t e,
-                                                  int32_t stride, V (&acc)[Piece<V>::VW]) {
-  constexpr int VW = Piece<V>::VW;
+                                                  int32_t stride, V (&acc)[VW]) {
   constexpr int U = 4;
   for (; j < e; j += U * stride) {
     int32_t c[U];
@@ -344,7 +315,7 @@ __device__ __forceinline__ void strided_piece_dot(const int32_t *__restrict__ ci
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (c[u] >= 0) {
-        load_piece<V>(x + (int64_t)c[u] * NRHS + cp * VW, xr[u]);
+        load_piece<V, VW>(x + (int64_t)c[u] * NRHS + cp * VW, xr[u]);
       } else {
 #pragma unroll
         for (int k = 0; k < VW; ++k) xr[u][k] = V(0);
@@ -361,24 +332,22 @@ __device__ __forceinline__ void strided_piece_dot(const int32_t *__restrict__ ci
 
 // The whole warp on one row: 32 / CPL nonzero lanes; every lane returns the
 // sums of its column piece.
-template <typename V, int NRHS>
+template <typename V, int NRHS, int VW>
 __device__ __forceinline__ void warp_row_piece(const int32_t *ci, const V *val, const V *x, int32_t s, int32_t e,
-                                               int lane, V (&acc)[Piece<V>::VW]) {
-  constexpr int VW = Piece<V>::VW;
+                                               int lane, V (&acc)[VW]) {
   constexpr int CPL = NRHS / VW;
 #pragma unroll
   for (int k = 0; k < VW; ++k) acc[k] = V(0);
-  strided_piece_dot<V, NRHS>(ci, val, x, lane % CPL, s + lane / CPL, e, 32 / CPL, acc);
+  strided_piece_dot<V, NRHS, VW>(ci, val, x, lane % CPL, s + lane / CPL, e, 32 / CPL, acc);
 #pragma unroll
   for (int o = 16; o >= CPL; o >>= 1)
 #pragma unroll
     for (int k = 0; k < VW; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
 }
 
-template <typename V, int NRHS, int L>
+template <typename V, int NRHS, int VW, int L>
 __device__ __forceinline__ void rows_item_piece(const BatchMatDev &M, int32_t r0, int32_t r1, int32_t long_thr,
                                                 int lane) {
-  constexpr int VW = Piece<V>::VW;
   constexpr int CPL = NRHS / VW;
   constexpr int LT = CPL * L;   // lanes per row
   static_assert(LT <= 32, "lanes per row");
@@ -409,12 +378,12 @@ __device__ __forceinline__ void rows_item_piece(const BatchMatDev &M, int32_t r0
     V acc[VW];
 #pragma unroll
     for (int k = 0; k < VW; ++k) acc[k] = V(0);
-    strided_piece_dot<V, NRHS>(M.ci, val, x, cp, s + sub, e, L, acc);
+    strided_piece_dot<V, NRHS, VW>(M.ci, val, x, cp, s + sub, e, L, acc);
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1)
 #pragma unroll
       for (int k = 0; k < VW; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o * CPL);
-    if (active && sub == 0 && mine) store_piece<V>(y + (int64_t)row * NRHS + cp * VW, acc);
+    if (active && sub == 0 && mine) store_piece<V, VW>(y + (int64_t)row * NRHS + cp * VW, acc);
     unsigned med = __ballot_sync(0xffffffffu, medium && sub == 0 && cp == 0);
     while (med) {
       const int b = __ffs(med) - 1;
@@ -422,8 +391,72 @@ __device__ __forceinline__ void rows_item_piece(const BatchMatDev &M, int32_t r0
       const int32_t mrow = base + b / LT;
       const int32_t ms = __ldg(M.rp + mrow), me = __ldg(M.rp + mrow + 1);
       V w[VW];
-      warp_row_piece<V, NRHS>(M.ci, val, x, ms, me, lane, w);
-      if (lane < CPL) store_piece<V>(y + (int64_t)mrow * NRHS + lane * VW, w);
+      warp_row_piece<V, NRHS, VW>(M.ci, val, x, ms, me, lane, w);
+      if (lane < CPL) store_piece<V, VW>(y + (int64_t)mrow * NRHS + lane * VW, w);
+    }
+  }
+}
+
+// SELL-32 slices [s0, s1): lane l owns slice row l and sums its entries
+// in stored order, U entries' loads issued before their gathers.  Value and
+// column loads of a warp are 32 consecutive entries (coalesced); for banded
+// matrices (narrow form) the gathered x rows are consecutive too.
+// VW = NRHS (FP32, 8 vectors): x and y are 32-byte aligned, a row in one access;
+// a warp's 32 consecutive rows are then 8 whole lines, where two 16-byte halves at
+// a 32-byte stride were 16 wavefronts and eight scalar stores 64.
+template <typename V, int NRHS, int VW, bool WIDE>
+__device__ __forceinline__ void sell_item(const BatchMatDev &M, int32_t s0, int32_t s1, int lane) {
+  constexpr int U = NRHS == 1 ? 4 : 2;
+  constexpr bool kRow = NRHS > 1 && VW == NRHS;
+  const V *sv = static_cast<const V *>(M.sell_val);
+  const V *x = static_cast<const V *>(M.x);
+  V *y = static_cast<V *>(M.y);
+  for (int32_t sl = s0; sl < s1; ++sl) {
+    const int32_t pos = sl * 32 + lane;
+    const bool live = pos < (WIDE ? M.sell_rows : M.rows);
+    const int32_t row = WIDE ? (live ? __ldg(M.sell_perm + pos) : 0) : pos;
+    const int32_t p0 = __ldg(M.sell_ptr + sl);
+    const int32_t w = live ? (__ldg(M.sell_ptr + sl + 1) - p0) >> 5 : 0;
+    const V *vp = sv + p0 + lane;
+    const int16_t *op = M.sell_off + p0 + lane;
+    const int32_t *cp = M.sell_col + p0 + lane;
+    V acc[NRHS];
+#pragma unroll
+    for (int k = 0; k < NRHS; ++k) acc[k] = V(0);
+    int32_t k = 0;
+    for (; k + U <= w; k += U) {
+      V a[U];
+      int32_t c[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        a[u] = __ldg(vp + 32 * (k + u));
+        c[u] = WIDE ? __ldg(cp + 32 * (k + u)) : row + (int32_t)__ldg(op + 32 * (k + u));
+      }
+      V xr[U][NRHS];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if constexpr (kRow)
+          load_piece<V, VW>(x + (int64_t)c[u] * NRHS, xr[u]);
+        else
+          load_xrow<V, NRHS>(x, c[u], xr[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) fma_row<V, NRHS>(acc, a[u], xr[u]);
+    }
+    for (; k < w; ++k) {
+      V xr[NRHS];
+      const int32_t c = WIDE ? __ldg(cp + 32 * k) : row + (int32_t)__ldg(op + 32 * k);
+      if constexpr (kRow)
+        load_piece<V, VW>(x + (int64_t)c * NRHS, xr);
+      else
+        load_xrow<V, NRHS>(x, c, xr);
+      fma_row<V, NRHS>(acc, __ldg(vp + 32 * k), xr);
+    }
+    if constexpr (kRow) {
+      if (live) store_piece<V, VW>(y + (int64_t)row * NRHS, acc);
+    } else if (live) {
+#pragma unroll
+      for (int j = 0; j < NRHS; ++j) y[(int64_t)row * NRHS + j] = acc[j];
     }
   }
 }
@@ -437,31 +470,35 @@ __device__ __forceinline__ void rows_item_piece(const BatchMatDev &M, int32_t r0
 // 16-byte loads) and gathers from there: the 32 rows' overlapping x rows are
 // read once per slice instead of once per entry, and each entry's gather no
 // longer waits on L1/L2.  The arithmetic and its order are unchanged.
-template <typename V, int NRHS>
+template <typename V, int NRHS, int VW>
 __device__ __forceinline__ void fetch_piece(const V *__restrict__ x, const V *xw, int32_t lo, int32_t c, int cp,
-                                            V (&o)[Piece<V>::VW]) {
-  constexpr int VW = Piece<V>::VW;
+                                            V (&o)[VW]) {
   if (lo >= 0) {
     const V *p = xw + (c - lo) * NRHS + cp * VW;
-    if constexpr (VW == 2) {
-      const double2 t = *reinterpret_cast<const double2 *>(p);
-      o[0] = t.x;
-      o[1] = t.y;
+    if constexpr (sizeof(V) == 8) {
+#pragma unroll
+      for (int k = 0; k < VW; k += 2) {
+        const double2 t = *reinterpret_cast<const double2 *>(p + k);
+        o[k] = t.x;
+        o[k + 1] = t.y;
+      }
     } else {
-      const float4 t = *reinterpret_cast<const float4 *>(p);
-      o[0] = t.x;
-      o[1] = t.y;
-      o[2] = t.z;
-      o[3] = t.w;
+#pragma unroll
+      for (int k = 0; k < VW; k += 4) {
+        const float4 t = *reinterpret_cast<const float4 *>(p + k);
+        o[k] = t.x;
+        o[k + 1] = t.y;
+        o[k + 2] = t.z;
+        o[k + 3] = t.w;
+      }
     }
   } else {
-    load_piece<V>(x + (int64_t)c * NRHS + cp * VW, o);
+    load_piece<V, VW>(x + (int64_t)c * NRHS + cp * VW, o);
   }
 }
 
-template <typename V, int NRHS, bool WIDE>
+template <typename V, int NRHS, int VW, bool WIDE>
 __device__ __forceinline__ void sell_item_piece(const BatchMatDev &M, int32_t s0, int32_t s1, int lane, V *xw) {
-  constexpr int VW = Piece<V>::VW;
   constexpr int CPL = NRHS / VW;
   constexpr int RPP = 32 / CPL;
   constexpr int U = 4;
@@ -479,8 +516,8 @@ __device__ __forceinline__ void sell_item_piece(const BatchMatDev &M, int32_t s0
         const int32_t r = lo + t / CPL;
         if (r < M.cols) {
           V v[VW];
-          load_piece<V>(x + (int64_t)r * NRHS + (t % CPL) * VW, v);
-          store_piece<V>(xw + t * VW, v);
+          load_piece<V, VW>(x + (int64_t)r * NRHS + (t % CPL) * VW, v);
+          store_piece<V, VW>(xw + t * VW, v);
         }
       }
       __syncwarp();
@@ -510,7 +547,7 @@ __device__ __forceinline__ void sell_item_piece(const BatchMatDev &M, int32_t s0
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           if (c[u] >= 0) {
-            fetch_piece<V, NRHS>(x, xw, lo, c[u], cp, xr[u]);
+            fetch_piece<V, NRHS, VW>(x, xw, lo, c[u], cp, xr[u]);
           } else {
 #pragma unroll
             for (int t = 0; t < VW; ++t) xr[u][t] = V(0);
@@ -523,7 +560,7 @@ __device__ __forceinline__ void sell_item_piece(const BatchMatDev &M, int32_t s0
             for (int t = 0; t < VW; ++t) acc[t] = fma(a[u], xr[u][t], acc[t]);
           }
       }
-      if (live) store_piece<V>(y + (int64_t)row * NRHS + cp * VW, acc);
+      if (live) store_piece<V, VW>(y + (int64_t)row * NRHS + cp * VW, acc);
     }
   }
 }
@@ -594,7 +631,7 @@ __global__ void batch_sell_window_kernel(int32_t rows, int32_t cols, const int32
   }
 }
 
-template <typename V, int NRHS>
+template <typename V, int NRHS, int VW>
 __device__ __forceinline__ void segment_item(const BatchMatDev &M, int32_t row, int32_t seg, int32_t lid,
                                              int32_t seg_nnz, const LongRow *__restrict__ longs,
                                              V *__restrict__ part, int32_t *__restrict__ arrive, int lane) {
@@ -605,11 +642,10 @@ __device__ __forceinline__ void segment_item(const BatchMatDev &M, int32_t row, 
   const int32_t s = s0 + seg * seg_nnz;
   const int32_t e = min(s + seg_nnz, e0);
   if constexpr (NRHS > 1) {
-    constexpr int VW = Piece<V>::VW;
     V w[VW];
-    warp_row_piece<V, NRHS>(M.ci, val, x, s, e, lane, w);
+    warp_row_piece<V, NRHS, VW>(M.ci, val, x, s, e, lane, w);
     if (lane < NRHS / VW) {
-      store_piece<V>(part + (int64_t)(lr.part_base + seg) * NRHS + lane * VW, w);
+      store_piece<V, VW>(part + (int64_t)(lr.part_base + seg) * NRHS + lane * VW, w);
       __threadfence();
     }
   } else {
@@ -639,7 +675,8 @@ __device__ __forceinline__ void segment_item(const BatchMatDev &M, int32_t row, 
 // (222.5 -> 204.5 us) but now spills there, and 6 CTAs measured faster
 // (512-matrix batch, tuned: 190.7 -> 174.1 us).  FP64 and the 8-vector forms
 // keep the compiler's choice.
-template <typename V, int NRHS>
+// VW: values per column piece (NRHS > 1).
+template <typename V, int NRHS, int VW>
 __global__ void __launch_bounds__(kBatchThreads, (NRHS == 1 && sizeof(V) == 4) ? 6 : 0) batch_kernel(const BatchMatDev *__restrict__ mats,
                                                               const BatchItem *__restrict__ items, int32_t nitems,
                                                               int32_t *__restrict__ next,
@@ -663,32 +700,33 @@ __global__ void __launch_bounds__(kBatchThreads, (NRHS == 1 && sizeof(V) == 4) ?
     // against 224 us in pieces)
     if (I.info == kSellItem) {
       if constexpr (NRHS > 1 && sizeof(V) == 8)
-        sell_item_piece<V, NRHS, false>(M, I.a, I.b, lane, xw);
+        sell_item_piece<V, NRHS, VW, false>(M, I.a, I.b, lane, xw);
       else
-        sell_item<V, NRHS, false>(M, I.a, I.b, lane);
+        sell_item<V, NRHS, VW, false>(M, I.a, I.b, lane);
       continue;
     }
     if (I.info == kSellWideItem) {
       if constexpr (NRHS > 1 && sizeof(V) == 8)
-        sell_item_piece<V, NRHS, true>(M, I.a, I.b, lane, xw);
+        sell_item_piece<V, NRHS, VW, true>(M, I.a, I.b, lane, xw);
       else
-        sell_item<V, NRHS, true>(M, I.a, I.b, lane);
+        sell_item<V, NRHS, VW, true>(M, I.a, I.b, lane);
       continue;
     }
     if (I.info < 0) {
-      segment_item<V, NRHS>(M, I.a, I.b, -(I.info + 1), seg_nnz, longs, part, arrive, lane);
+      segment_item<V, NRHS, VW>(M, I.a, I.b, -(I.info + 1), seg_nnz, longs, part, arrive, lane);
       continue;
     }
     if constexpr (NRHS > 1) {
       // lanes per row split the nonzeros; at most 32 / CPL of them
-      constexpr int LMAX = 32 / (NRHS / Piece<V>::VW);
+      constexpr int LMAX = 32 / (NRHS / VW);
       const int32_t L = I.info < LMAX ? I.info : LMAX;
       switch (L) {
-        case 1: rows_item_piece<V, NRHS, 1>(M, I.a, I.b, long_thr, lane); break;
-        case 2: rows_item_piece<V, NRHS, 2>(M, I.a, I.b, long_thr, lane); break;
-        case 4: rows_item_piece<V, NRHS, 4>(M, I.a, I.b, long_thr, lane); break;
-        case 8: rows_item_piece<V, NRHS, (LMAX >= 8 ? 8 : LMAX)>(M, I.a, I.b, long_thr, lane); break;
-        default: rows_item_piece<V, NRHS, LMAX>(M, I.a, I.b, long_thr, lane); break;
+        case 1: rows_item_piece<V, NRHS, VW, 1>(M, I.a, I.b, long_thr, lane); break;
+        case 2: rows_item_piece<V, NRHS, VW, 2>(M, I.a, I.b, long_thr, lane); break;
+        case 4: rows_item_piece<V, NRHS, VW, 4>(M, I.a, I.b, long_thr, lane); break;
+        case 8: rows_item_piece<V, NRHS, VW, (LMAX >= 8 ? 8 : LMAX)>(M, I.a, I.b, long_thr, lane); break;
+        case 16: rows_item_piece<V, NRHS, VW, (LMAX >= 16 ? 16 : LMAX)>(M, I.a, I.b, long_thr, lane); break;
+        default: rows_item_piece<V, NRHS, VW, LMAX>(M, I.a, I.b, long_thr, lane); break;
       }
     } else {
       switch (I.info) {
@@ -736,11 +774,14 @@ struct bsp_batch_plan_s {
   int32_t *d_arrive = nullptr;
   int32_t *d_next = nullptr;  // [count + 1]: batched counter, then one per matrix
   int grid = 0;
+  bool row32 = false;  // 8 vectors: every x and y is 32-byte aligned
   cudaStream_t graph_stream = nullptr;
   cudaGraphExec_t graph = nullptr;
 };
 
 namespace {
+
+bool rows_aligned(const bsp_batch_mat &A) { return ((uintptr_t)A.x | (uintptr_t)A.y) % 32 == 0; }
 
 int model_lanes(const std::vector<int32_t> &len, int32_t long_thr, int nrhs) {
   double s = 0;
@@ -891,12 +932,12 @@ extern "C" bsp_status bsp_batch_default_options(bsp_batch_options *o) {
   return BSP_OK;
 }
 
-template <typename V, int NRHS>
+template <typename V, int NRHS, int VW>
 static bsp_status launch_batch(bsp_batch_plan P, const BatchItem *items, int64_t nitems, int32_t *next,
                                int grid, cudaStream_t s) {
-  batch_kernel<V, NRHS><<<grid, kBatchThreads, 0, s>>>(P->d_mats, items, (int32_t)nitems, next, P->d_longs,
-                                                       static_cast<V *>(P->d_part), P->d_arrive, P->opt.seg_nnz,
-                                                       P->opt.long_row_nnz);
+  batch_kernel<V, NRHS, VW><<<grid, kBatchThreads, 0, s>>>(P->d_mats, items, (int32_t)nitems, next, P->d_longs,
+                                                           static_cast<V *>(P->d_part), P->d_arrive, P->opt.seg_nnz,
+                                                           P->opt.long_row_nnz);
   BSP_LAUNCH_CHECK();
   return BSP_OK;
 }
@@ -904,17 +945,20 @@ static bsp_status launch_batch(bsp_batch_plan P, const BatchItem *items, int64_t
 static bsp_status dispatch(bsp_batch_plan P, const BatchItem *items, int64_t nitems, int32_t *next, int grid,
                            cudaStream_t s) {
   if (nitems == 0) return BSP_OK;
-  if (P->dtype == BSP_F64)
-    return P->nrhs == 8 ? launch_batch<double, 8>(P, items, nitems, next, grid, s)
-                        : launch_batch<double, 1>(P, items, nitems, next, grid, s);
-  return P->nrhs == 8 ? launch_batch<float, 8>(P, items, nitems, next, grid, s)
-                      : launch_batch<float, 1>(P, items, nitems, next, grid, s);
+  if (P->dtype == BSP_F64) {
+    if (P->nrhs == 1) return launch_batch<double, 1, 1>(P, items, nitems, next, grid, s);
+    return P->row32 ? launch_batch<double, 8, 4>(P, items, nitems, next, grid, s)
+                    : launch_batch<double, 8, 2>(P, items, nitems, next, grid, s);
+  }
+  if (P->nrhs == 1) return launch_batch<float, 1, 1>(P, items, nitems, next, grid, s);
+  return P->row32 ? launch_batch<float, 8, 8>(P, items, nitems, next, grid, s)
+                  : launch_batch<float, 8, 4>(P, items, nitems, next, grid, s);
 }
 
-template <typename V, int NRHS>
+template <typename V, int NRHS, int VW>
 static int occupancy() {
   int b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, batch_kernel<V, NRHS>, kBatchThreads, 0) != cudaSuccess ||
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, batch_kernel<V, NRHS, VW>, kBatchThreads, 0) != cudaSuccess ||
       b < 1)
     b = 1;
   return b;
@@ -929,9 +973,9 @@ static bsp_status batch_build(bsp_batch_plan P, cudaStream_t s) {
   const int warps_per_cta = kBatchThreads / 32;
   int occ = 1;
   if (P->dtype == BSP_F64)
-    occ = P->nrhs == 8 ? occupancy<double, 8>() : occupancy<double, 1>();
+    occ = P->nrhs == 1 ? occupancy<double, 1, 1>() : P->row32 ? occupancy<double, 8, 4>() : occupancy<double, 8, 2>();
   else
-    occ = P->nrhs == 8 ? occupancy<float, 8>() : occupancy<float, 1>();
+    occ = P->nrhs == 1 ? occupancy<float, 1, 1>() : P->row32 ? occupancy<float, 8, 8>() : occupancy<float, 8, 4>();
   P->grid = sm_count() * occ;
   if (item_nnz <= 0) {
     const int64_t warps = (int64_t)P->grid * warps_per_cta;
@@ -1200,6 +1244,7 @@ extern "C" bsp_status bsp_batch_create(int32_t count, const bsp_batch_mat *mats,
   P->host_mats.assign(mats, mats + count);
   P->lens.resize(count);
   P->lanes.assign(count, 1);
+  P->row32 = std::all_of(mats, mats + count, rows_aligned);
   auto fail = [&](bsp_status st) {
     bsp_batch_destroy(P);
     return st;
@@ -1327,6 +1372,10 @@ extern "C" bsp_status bsp_batch_set_vectors(bsp_batch_plan P, int32_t m, const v
   // the descriptor is read by the kernel: update it in stream order
   BSP_CUDA(cudaMemcpyAsync(P->d_mats + m, &d, sizeof(d), cudaMemcpyHostToDevice, s));
   BSP_CUDA(cudaStreamSynchronize(s));
+  if (P->nrhs == 8 && P->row32 && !rows_aligned(P->host_mats[m])) {  // 16-byte pieces from here on
+    P->row32 = false;
+    BSP_TRY(capture(P));
+  }
   return BSP_OK;
 }
 

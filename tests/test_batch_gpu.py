@@ -133,6 +133,49 @@ def test_batch_set_vectors_and_empty_matrix(cuda):
     P.close()
 
 
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("graph", [True, False])
+@pytest.mark.parametrize("sell", [True, False])
+def test_batch_8rhs_vectors_16_byte_aligned(cuda, dtype, graph, sell):
+    """8 right-hand sides: 32-byte accesses where every x and y is 32-byte
+    aligned, 16-byte ones when one vector is not, from the start or after
+    set_vectors."""
+    import torch
+    mats = _small_batch(37, count=9) + _sell_batch(71)[:3]
+    dev, host = _upload(cuda, mats, dtype, 8, 10)
+
+    def shifted(t):                         # a copy 16 bytes past a 32-byte boundary
+        k = 16 // t.element_size()
+        store = torch.empty(t.numel() + 2 * k, dtype=t.dtype, device=t.device)
+        v = store[k:k + t.numel()].view(t.shape)
+        assert v.data_ptr() % 32 == 16
+        return v.copy_(t)
+
+    P = bsp.BatchPlan(dev, nrhs=8, long_row_nnz=256, seg_nnz=64, use_graph=graph, sell=sell)
+    P.run()
+    torch.cuda.synchronize()
+    _check(mats, dev, host, dtype, 8)
+    for which in (4, 10):
+        x2, y2 = shifted(dev[which][3]), shifted(dev[which][4])
+        P.set_vectors(which, x2, y2)
+        dev[which] = (*dev[which][:3], x2, y2)
+        for d in dev:
+            d[4].fill_(float("nan"))
+        P.run()
+        torch.cuda.synchronize()
+        _check(mats, dev, host, dtype, 8)
+    first = [d[4].clone() for d in dev]
+    P.close()
+    Q = bsp.BatchPlan(dev, nrhs=8, long_row_nnz=256, seg_nnz=64, use_graph=graph, sell=sell)
+    for d in dev:
+        d[4].fill_(float("nan"))
+    Q.run_separate()
+    torch.cuda.synchronize()
+    for a, d in zip(first, dev):
+        assert torch.equal(a, d[4])
+    Q.close()
+
+
 def test_batch_rejects_bad_arguments(cuda):
     import torch
     mats = _small_batch(41, count=2)
