@@ -248,8 +248,8 @@ __device__ __forceinline__ void rows_item(const BatchMatDev &M, int32_t r0, int3
 // (lane sub takes entries s+sub, s+sub+L, ... in order, then a fixed shuffle
 // tree over the L lanes).
 //
-// A piece is VW values: 32 bytes (one 256-bit access) where every x and y is
-// 32-byte aligned, else 16.  The wider pieces take half the lanes per row, so a
+// A piece is VW values: 32 bytes (one 256-bit access) where the matrix's x and y
+// are 32-byte aligned, else 16.  The wider pieces take half the lanes per row, so a
 // pass has twice the rows (and loads) in flight and the entry loads, which all
 // lanes of a row repeat, are halved.  8 vectors, 512 matrices: FP32 354 ->
 // 345 us, FP64 648 -> 611; 100 matrices, FP32, 86.4 -> 81.4; 60, FP64, 104 -> 92.5.
@@ -670,13 +670,76 @@ __device__ __forceinline__ void segment_item(const BatchMatDev &M, int32_t row, 
   if (lane == 0) atomicExch(arrive + lid, 0);  // ready for the next launch
 }
 
+// One work item.  VW: values per column piece (NRHS > 1).
+template <typename V, int NRHS, int VW>
+__device__ __forceinline__ void run_item(const BatchMatDev &M, const BatchItem &I, const LongRow *__restrict__ longs,
+                                         V *__restrict__ part, int32_t *__restrict__ arrive, int32_t seg_nnz,
+                                         int32_t long_thr, int lane, V *xw) {
+  // SELL slices with several FP64 right-hand sides: column pieces and the
+  // shared-memory x window (512-matrix batch, banded half, 8 vectors: 517 ->
+  // 371 us); FP32 keeps a lane per row over all columns there (197 us
+  // against 224 us in pieces)
+  if (I.info == kSellItem) {
+    if constexpr (NRHS > 1 && sizeof(V) == 8)
+      sell_item_piece<V, NRHS, VW, false>(M, I.a, I.b, lane, xw);
+    else
+      sell_item<V, NRHS, VW, false>(M, I.a, I.b, lane);
+    return;
+  }
+  if (I.info == kSellWideItem) {
+    if constexpr (NRHS > 1 && sizeof(V) == 8)
+      sell_item_piece<V, NRHS, VW, true>(M, I.a, I.b, lane, xw);
+    else
+      sell_item<V, NRHS, VW, true>(M, I.a, I.b, lane);
+    return;
+  }
+  if (I.info < 0) {
+    segment_item<V, NRHS, VW>(M, I.a, I.b, -(I.info + 1), seg_nnz, longs, part, arrive, lane);
+    return;
+  }
+  if constexpr (NRHS > 1) {
+    // lanes per row split the nonzeros; at most 32 / CPL of them
+    constexpr int LMAX = 32 / (NRHS / VW);
+    const int32_t L = I.info < LMAX ? I.info : LMAX;
+    switch (L) {
+      case 1: rows_item_piece<V, NRHS, VW, 1>(M, I.a, I.b, long_thr, lane); break;
+      case 2: rows_item_piece<V, NRHS, VW, 2>(M, I.a, I.b, long_thr, lane); break;
+      case 4: rows_item_piece<V, NRHS, VW, 4>(M, I.a, I.b, long_thr, lane); break;
+      case 8: rows_item_piece<V, NRHS, VW, (LMAX >= 8 ? 8 : LMAX)>(M, I.a, I.b, long_thr, lane); break;
+      case 16: rows_item_piece<V, NRHS, VW, (LMAX >= 16 ? 16 : LMAX)>(M, I.a, I.b, long_thr, lane); break;
+      default: rows_item_piece<V, NRHS, VW, LMAX>(M, I.a, I.b, long_thr, lane); break;
+    }
+  } else {
+    switch (I.info) {
+      case 1: rows_item<V, NRHS, 1>(M, I.a, I.b, long_thr, lane); break;
+      case 2: rows_item<V, NRHS, 2>(M, I.a, I.b, long_thr, lane); break;
+      case 4: rows_item<V, NRHS, 4>(M, I.a, I.b, long_thr, lane); break;
+      case 8: rows_item<V, NRHS, 8>(M, I.a, I.b, long_thr, lane); break;
+      case 16: rows_item<V, NRHS, 16>(M, I.a, I.b, long_thr, lane); break;
+      default: rows_item<V, NRHS, 32>(M, I.a, I.b, long_thr, lane); break;
+    }
+  }
+}
+
+// 16-byte pieces, for a matrix whose x or y is not 32-byte aligned.  Not inlined:
+// in line with the 32-byte form it costs that form 2% (8 vectors, FP32 350 ->
+// 356 us, FP64 618 -> 625).
+template <typename V, int NRHS>
+__device__ __noinline__ void run_item_16(const BatchMatDev *__restrict__ mats, const BatchItem *__restrict__ item,
+                                         const LongRow *__restrict__ longs, V *__restrict__ part,
+                                         int32_t *__restrict__ arrive, int32_t seg_nnz, int32_t long_thr, int lane,
+                                         V *xw) {
+  const BatchItem I = *item;
+  const BatchMatDev M = mats[I.mat];
+  run_item<V, NRHS, 16 / (int)sizeof(V)>(M, I, longs, part, arrive, seg_nnz, long_thr, lane, xw);
+}
+
 // One FP32 vector: capped at 40 registers (6 resident CTAs per SM).  At 32
 // registers (8 CTAs) it was faster before the SELL items joined the kernel
 // (222.5 -> 204.5 us) but now spills there, and 6 CTAs measured faster
 // (512-matrix batch, tuned: 190.7 -> 174.1 us).  FP64 and the 8-vector forms
 // keep the compiler's choice.
-// VW: values per column piece (NRHS > 1).
-template <typename V, int NRHS, int VW>
+template <typename V, int NRHS>
 __global__ void __launch_bounds__(kBatchThreads, (NRHS == 1 && sizeof(V) == 4) ? 6 : 0) batch_kernel(const BatchMatDev *__restrict__ mats,
                                                               const BatchItem *__restrict__ items, int32_t nitems,
                                                               int32_t *__restrict__ next,
@@ -694,49 +757,14 @@ __global__ void __launch_bounds__(kBatchThreads, (NRHS == 1 && sizeof(V) == 4) ?
     if (it >= nitems) return;
     const BatchItem I = items[it];
     const BatchMatDev M = mats[I.mat];
-    // SELL slices with several FP64 right-hand sides: column pieces and the
-    // shared-memory x window (512-matrix batch, banded half, 8 vectors: 517 ->
-    // 371 us); FP32 keeps a lane per row over all columns there (197 us
-    // against 224 us in pieces)
-    if (I.info == kSellItem) {
-      if constexpr (NRHS > 1 && sizeof(V) == 8)
-        sell_item_piece<V, NRHS, VW, false>(M, I.a, I.b, lane, xw);
-      else
-        sell_item<V, NRHS, VW, false>(M, I.a, I.b, lane);
-      continue;
-    }
-    if (I.info == kSellWideItem) {
-      if constexpr (NRHS > 1 && sizeof(V) == 8)
-        sell_item_piece<V, NRHS, VW, true>(M, I.a, I.b, lane, xw);
-      else
-        sell_item<V, NRHS, VW, true>(M, I.a, I.b, lane);
-      continue;
-    }
-    if (I.info < 0) {
-      segment_item<V, NRHS, VW>(M, I.a, I.b, -(I.info + 1), seg_nnz, longs, part, arrive, lane);
-      continue;
-    }
-    if constexpr (NRHS > 1) {
-      // lanes per row split the nonzeros; at most 32 / CPL of them
-      constexpr int LMAX = 32 / (NRHS / VW);
-      const int32_t L = I.info < LMAX ? I.info : LMAX;
-      switch (L) {
-        case 1: rows_item_piece<V, NRHS, VW, 1>(M, I.a, I.b, long_thr, lane); break;
-        case 2: rows_item_piece<V, NRHS, VW, 2>(M, I.a, I.b, long_thr, lane); break;
-        case 4: rows_item_piece<V, NRHS, VW, 4>(M, I.a, I.b, long_thr, lane); break;
-        case 8: rows_item_piece<V, NRHS, VW, (LMAX >= 8 ? 8 : LMAX)>(M, I.a, I.b, long_thr, lane); break;
-        case 16: rows_item_piece<V, NRHS, VW, (LMAX >= 16 ? 16 : LMAX)>(M, I.a, I.b, long_thr, lane); break;
-        default: rows_item_piece<V, NRHS, VW, LMAX>(M, I.a, I.b, long_thr, lane); break;
-      }
+    if constexpr (NRHS == 1) {
+      run_item<V, 1, 1>(M, I, longs, part, arrive, seg_nnz, long_thr, lane, xw);
     } else {
-      switch (I.info) {
-        case 1: rows_item<V, NRHS, 1>(M, I.a, I.b, long_thr, lane); break;
-        case 2: rows_item<V, NRHS, 2>(M, I.a, I.b, long_thr, lane); break;
-        case 4: rows_item<V, NRHS, 4>(M, I.a, I.b, long_thr, lane); break;
-        case 8: rows_item<V, NRHS, 8>(M, I.a, I.b, long_thr, lane); break;
-        case 16: rows_item<V, NRHS, 16>(M, I.a, I.b, long_thr, lane); break;
-        default: rows_item<V, NRHS, 32>(M, I.a, I.b, long_thr, lane); break;
-      }
+      // by what the descriptor holds now: it may change between launches
+      if ((((uintptr_t)M.x | (uintptr_t)M.y) & 31) == 0)
+        run_item<V, NRHS, 32 / (int)sizeof(V)>(M, I, longs, part, arrive, seg_nnz, long_thr, lane, xw);
+      else
+        run_item_16<V, NRHS>(mats, items + it, longs, part, arrive, seg_nnz, long_thr, lane, xw);
     }
   }
 }
@@ -774,14 +802,11 @@ struct bsp_batch_plan_s {
   int32_t *d_arrive = nullptr;
   int32_t *d_next = nullptr;  // [count + 1]: batched counter, then one per matrix
   int grid = 0;
-  bool row32 = false;  // 8 vectors: every x and y is 32-byte aligned
   cudaStream_t graph_stream = nullptr;
   cudaGraphExec_t graph = nullptr;
 };
 
 namespace {
-
-bool rows_aligned(const bsp_batch_mat &A) { return ((uintptr_t)A.x | (uintptr_t)A.y) % 32 == 0; }
 
 int model_lanes(const std::vector<int32_t> &len, int32_t long_thr, int nrhs) {
   double s = 0;
@@ -932,10 +957,10 @@ extern "C" bsp_status bsp_batch_default_options(bsp_batch_options *o) {
   return BSP_OK;
 }
 
-template <typename V, int NRHS, int VW>
+template <typename V, int NRHS>
 static bsp_status launch_batch(bsp_batch_plan P, const BatchItem *items, int64_t nitems, int32_t *next,
                                int grid, cudaStream_t s) {
-  batch_kernel<V, NRHS, VW><<<grid, kBatchThreads, 0, s>>>(P->d_mats, items, (int32_t)nitems, next, P->d_longs,
+  batch_kernel<V, NRHS><<<grid, kBatchThreads, 0, s>>>(P->d_mats, items, (int32_t)nitems, next, P->d_longs,
                                                            static_cast<V *>(P->d_part), P->d_arrive, P->opt.seg_nnz,
                                                            P->opt.long_row_nnz);
   BSP_LAUNCH_CHECK();
@@ -945,20 +970,17 @@ static bsp_status launch_batch(bsp_batch_plan P, const BatchItem *items, int64_t
 static bsp_status dispatch(bsp_batch_plan P, const BatchItem *items, int64_t nitems, int32_t *next, int grid,
                            cudaStream_t s) {
   if (nitems == 0) return BSP_OK;
-  if (P->dtype == BSP_F64) {
-    if (P->nrhs == 1) return launch_batch<double, 1, 1>(P, items, nitems, next, grid, s);
-    return P->row32 ? launch_batch<double, 8, 4>(P, items, nitems, next, grid, s)
-                    : launch_batch<double, 8, 2>(P, items, nitems, next, grid, s);
-  }
-  if (P->nrhs == 1) return launch_batch<float, 1, 1>(P, items, nitems, next, grid, s);
-  return P->row32 ? launch_batch<float, 8, 8>(P, items, nitems, next, grid, s)
-                  : launch_batch<float, 8, 4>(P, items, nitems, next, grid, s);
+  if (P->dtype == BSP_F64)
+    return P->nrhs == 8 ? launch_batch<double, 8>(P, items, nitems, next, grid, s)
+                        : launch_batch<double, 1>(P, items, nitems, next, grid, s);
+  return P->nrhs == 8 ? launch_batch<float, 8>(P, items, nitems, next, grid, s)
+                      : launch_batch<float, 1>(P, items, nitems, next, grid, s);
 }
 
-template <typename V, int NRHS, int VW>
+template <typename V, int NRHS>
 static int occupancy() {
   int b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, batch_kernel<V, NRHS, VW>, kBatchThreads, 0) != cudaSuccess ||
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, batch_kernel<V, NRHS>, kBatchThreads, 0) != cudaSuccess ||
       b < 1)
     b = 1;
   return b;
@@ -973,9 +995,9 @@ static bsp_status batch_build(bsp_batch_plan P, cudaStream_t s) {
   const int warps_per_cta = kBatchThreads / 32;
   int occ = 1;
   if (P->dtype == BSP_F64)
-    occ = P->nrhs == 1 ? occupancy<double, 1, 1>() : P->row32 ? occupancy<double, 8, 4>() : occupancy<double, 8, 2>();
+    occ = P->nrhs == 8 ? occupancy<double, 8>() : occupancy<double, 1>();
   else
-    occ = P->nrhs == 1 ? occupancy<float, 1, 1>() : P->row32 ? occupancy<float, 8, 8>() : occupancy<float, 8, 4>();
+    occ = P->nrhs == 8 ? occupancy<float, 8>() : occupancy<float, 1>();
   P->grid = sm_count() * occ;
   if (item_nnz <= 0) {
     const int64_t warps = (int64_t)P->grid * warps_per_cta;
@@ -1244,7 +1266,6 @@ extern "C" bsp_status bsp_batch_create(int32_t count, const bsp_batch_mat *mats,
   P->host_mats.assign(mats, mats + count);
   P->lens.resize(count);
   P->lanes.assign(count, 1);
-  P->row32 = std::all_of(mats, mats + count, rows_aligned);
   auto fail = [&](bsp_status st) {
     bsp_batch_destroy(P);
     return st;
@@ -1372,10 +1393,6 @@ extern "C" bsp_status bsp_batch_set_vectors(bsp_batch_plan P, int32_t m, const v
   // the descriptor is read by the kernel: update it in stream order
   BSP_CUDA(cudaMemcpyAsync(P->d_mats + m, &d, sizeof(d), cudaMemcpyHostToDevice, s));
   BSP_CUDA(cudaStreamSynchronize(s));
-  if (P->nrhs == 8 && P->row32 && !rows_aligned(P->host_mats[m])) {  // 16-byte pieces from here on
-    P->row32 = false;
-    BSP_TRY(capture(P));
-  }
   return BSP_OK;
 }
 

@@ -137,9 +137,9 @@ def test_batch_set_vectors_and_empty_matrix(cuda):
 @pytest.mark.parametrize("graph", [True, False])
 @pytest.mark.parametrize("sell", [True, False])
 def test_batch_8rhs_vectors_16_byte_aligned(cuda, dtype, graph, sell):
-    """8 right-hand sides: 32-byte accesses where every x and y is 32-byte
-    aligned, 16-byte ones when one vector is not, from the start or after
-    set_vectors."""
+    """8 right-hand sides: 32-byte accesses where a matrix's x and y are
+    32-byte aligned, 16-byte ones where they are not, from the start or after
+    set_vectors, also when a graph captured before it is replayed."""
     import torch
     mats = _small_batch(37, count=9) + _sell_batch(71)[:3]
     dev, host = _upload(cuda, mats, dtype, 8, 10)
@@ -162,6 +162,18 @@ def test_batch_8rhs_vectors_16_byte_aligned(cuda, dtype, graph, sell):
         for d in dev:
             d[4].fill_(float("nan"))
         P.run()
+        torch.cuda.synchronize()
+        _check(mats, dev, host, dtype, 8)
+    if not graph:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            P.run()
+        x2, y2 = shifted(dev[2][3]), shifted(dev[2][4])
+        P.set_vectors(2, x2, y2)
+        dev[2] = (*dev[2][:3], x2, y2)
+        for d in dev:
+            d[4].fill_(float("nan"))
+        g.replay()
         torch.cuda.synchronize()
         _check(mats, dev, host, dtype, 8)
     first = [d[4].clone() for d in dev]
