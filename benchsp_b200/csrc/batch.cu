@@ -248,8 +248,8 @@ __device__ __forceinline__ void rows_item(const BatchMatDev &M, int32_t r0, int3
 // (lane sub takes entries s+sub, s+sub+L, ... in order, then a fixed shuffle
 // tree over the L lanes).
 //
-// A piece is VW values: 32 bytes (one 256-bit access) where the matrix's x and y
-// are 32-byte aligned, else 16.  The wider pieces take half the lanes per row, so a
+// A piece is VW values: 32 bytes (one 256-bit access) where every x and y of the
+// batch is 32-byte aligned, else 16.  The wider pieces take half the lanes per row, so a
 // pass has twice the rows (and loads) in flight and the entry loads, which all
 // lanes of a row repeat, are halved.  8 vectors, 512 matrices: FP32 354 ->
 // 345 us, FP64 648 -> 611; 100 matrices, FP32, 86.4 -> 81.4; 60, FP64, 104 -> 92.5.
@@ -721,9 +721,11 @@ __device__ __forceinline__ void run_item(const BatchMatDev &M, const BatchItem &
   }
 }
 
-// 16-byte pieces, for a matrix whose x or y is not 32-byte aligned.  Not inlined:
-// in line with the 32-byte form it costs that form 2% (8 vectors, FP32 350 ->
-// 356 us, FP64 618 -> 625).
+// 16-byte pieces in the kernel of the 32-byte ones, for a matrix whose x or y is
+// not 32-byte aligned.  Not inlined: in line it costs the 32-byte form 2% (8
+// vectors, FP32 350 -> 356 us, FP64 618 -> 625).  A call costs its own items 12%
+// (FP32) and 25% (FP64), so a plan with such vectors launches the kernel of
+// 16-byte pieces; this is for graphs captured before set_vectors gave them.
 template <typename V, int NRHS>
 __device__ __noinline__ void run_item_16(const BatchMatDev *__restrict__ mats, const BatchItem *__restrict__ item,
                                          const LongRow *__restrict__ longs, V *__restrict__ part,
@@ -739,7 +741,7 @@ __device__ __noinline__ void run_item_16(const BatchMatDev *__restrict__ mats, c
 // (222.5 -> 204.5 us) but now spills there, and 6 CTAs measured faster
 // (512-matrix batch, tuned: 190.7 -> 174.1 us).  FP64 and the 8-vector forms
 // keep the compiler's choice.
-template <typename V, int NRHS>
+template <typename V, int NRHS, int VW>
 __global__ void __launch_bounds__(kBatchThreads, (NRHS == 1 && sizeof(V) == 4) ? 6 : 0) batch_kernel(const BatchMatDev *__restrict__ mats,
                                                               const BatchItem *__restrict__ items, int32_t nitems,
                                                               int32_t *__restrict__ next,
@@ -757,15 +759,12 @@ __global__ void __launch_bounds__(kBatchThreads, (NRHS == 1 && sizeof(V) == 4) ?
     if (it >= nitems) return;
     const BatchItem I = items[it];
     const BatchMatDev M = mats[I.mat];
-    if constexpr (NRHS == 1) {
-      run_item<V, 1, 1>(M, I, longs, part, arrive, seg_nnz, long_thr, lane, xw);
-    } else {
-      // by what the descriptor holds now: it may change between launches
-      if ((((uintptr_t)M.x | (uintptr_t)M.y) & 31) == 0)
-        run_item<V, NRHS, 32 / (int)sizeof(V)>(M, I, longs, part, arrive, seg_nnz, long_thr, lane, xw);
-      else
-        run_item_16<V, NRHS>(mats, items + it, longs, part, arrive, seg_nnz, long_thr, lane, xw);
-    }
+    // by what the descriptor holds now: set_vectors may change it under a graph
+    // that was captured with this kernel
+    if (VW * sizeof(V) != 32 || (((uintptr_t)M.x | (uintptr_t)M.y) & 31) == 0)
+      run_item<V, NRHS, VW>(M, I, longs, part, arrive, seg_nnz, long_thr, lane, xw);
+    else
+      run_item_16<V, NRHS>(mats, items + it, longs, part, arrive, seg_nnz, long_thr, lane, xw);
   }
 }
 
@@ -794,6 +793,7 @@ struct bsp_batch_plan_s {
   BatchMatDev *d_mats = nullptr;
   // batched list (long segments first) and per-matrix lists
   BatchItem *d_items = nullptr, *d_items_sep = nullptr;
+  bool row32 = false;  // 8 vectors: every x and y is 32-byte aligned
   int64_t nitems = 0;
   std::vector<int64_t> sep_off;  // [count+1] offsets into d_items_sep
   LongRow *d_longs = nullptr;
@@ -805,6 +805,8 @@ struct bsp_batch_plan_s {
   cudaStream_t graph_stream = nullptr;
   cudaGraphExec_t graph = nullptr;
 };
+
+static bool rows_aligned(const bsp_batch_mat &A) { return ((uintptr_t)A.x | (uintptr_t)A.y) % 32 == 0; }
 
 namespace {
 
@@ -957,10 +959,10 @@ extern "C" bsp_status bsp_batch_default_options(bsp_batch_options *o) {
   return BSP_OK;
 }
 
-template <typename V, int NRHS>
+template <typename V, int NRHS, int VW>
 static bsp_status launch_batch(bsp_batch_plan P, const BatchItem *items, int64_t nitems, int32_t *next,
                                int grid, cudaStream_t s) {
-  batch_kernel<V, NRHS><<<grid, kBatchThreads, 0, s>>>(P->d_mats, items, (int32_t)nitems, next, P->d_longs,
+  batch_kernel<V, NRHS, VW><<<grid, kBatchThreads, 0, s>>>(P->d_mats, items, (int32_t)nitems, next, P->d_longs,
                                                            static_cast<V *>(P->d_part), P->d_arrive, P->opt.seg_nnz,
                                                            P->opt.long_row_nnz);
   BSP_LAUNCH_CHECK();
@@ -971,16 +973,18 @@ static bsp_status dispatch(bsp_batch_plan P, const BatchItem *items, int64_t nit
                            cudaStream_t s) {
   if (nitems == 0) return BSP_OK;
   if (P->dtype == BSP_F64)
-    return P->nrhs == 8 ? launch_batch<double, 8>(P, items, nitems, next, grid, s)
-                        : launch_batch<double, 1>(P, items, nitems, next, grid, s);
-  return P->nrhs == 8 ? launch_batch<float, 8>(P, items, nitems, next, grid, s)
-                      : launch_batch<float, 1>(P, items, nitems, next, grid, s);
+    return P->nrhs == 1 ? launch_batch<double, 1, 1>(P, items, nitems, next, grid, s)
+           : P->row32   ? launch_batch<double, 8, 4>(P, items, nitems, next, grid, s)
+                        : launch_batch<double, 8, 2>(P, items, nitems, next, grid, s);
+  return P->nrhs == 1 ? launch_batch<float, 1, 1>(P, items, nitems, next, grid, s)
+         : P->row32   ? launch_batch<float, 8, 8>(P, items, nitems, next, grid, s)
+                      : launch_batch<float, 8, 4>(P, items, nitems, next, grid, s);
 }
 
-template <typename V, int NRHS>
+template <typename V, int NRHS, int VW>
 static int occupancy() {
   int b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, batch_kernel<V, NRHS>, kBatchThreads, 0) != cudaSuccess ||
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, batch_kernel<V, NRHS, VW>, kBatchThreads, 0) != cudaSuccess ||
       b < 1)
     b = 1;
   return b;
@@ -995,9 +999,9 @@ static bsp_status batch_build(bsp_batch_plan P, cudaStream_t s) {
   const int warps_per_cta = kBatchThreads / 32;
   int occ = 1;
   if (P->dtype == BSP_F64)
-    occ = P->nrhs == 8 ? occupancy<double, 8>() : occupancy<double, 1>();
+    occ = P->nrhs == 1 ? occupancy<double, 1, 1>() : P->row32 ? occupancy<double, 8, 4>() : occupancy<double, 8, 2>();
   else
-    occ = P->nrhs == 8 ? occupancy<float, 8>() : occupancy<float, 1>();
+    occ = P->nrhs == 1 ? occupancy<float, 1, 1>() : P->row32 ? occupancy<float, 8, 8>() : occupancy<float, 8, 4>();
   P->grid = sm_count() * occ;
   if (item_nnz <= 0) {
     const int64_t warps = (int64_t)P->grid * warps_per_cta;
@@ -1291,6 +1295,7 @@ extern "C" bsp_status bsp_batch_create(int32_t count, const bsp_batch_mat *mats,
     P->total_nnz += A.nnz;
     P->lanes[m] = model_lanes(L, o.long_row_nnz, nrhs);
   }
+  P->row32 = std::all_of(mats, mats + count, rows_aligned);
   P->dm.resize(count);
   for (int32_t m = 0; m < count; ++m)
     P->dm[m] = {mats[m].rowPtr, mats[m].colIdx, mats[m].values, mats[m].x, mats[m].y, mats[m].rows, mats[m].cols,
@@ -1393,6 +1398,10 @@ extern "C" bsp_status bsp_batch_set_vectors(bsp_batch_plan P, int32_t m, const v
   // the descriptor is read by the kernel: update it in stream order
   BSP_CUDA(cudaMemcpyAsync(P->d_mats + m, &d, sizeof(d), cudaMemcpyHostToDevice, s));
   BSP_CUDA(cudaStreamSynchronize(s));
+  if (P->nrhs == 8 && P->row32 && !rows_aligned(P->host_mats[m])) {  // 16-byte pieces from here on
+    P->row32 = false;
+    BSP_TRY(capture(P));
+  }
   return BSP_OK;
 }
 
