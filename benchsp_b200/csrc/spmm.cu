@@ -2138,13 +2138,13 @@ template <> __device__ __forceinline__ __nv_bfloat16 bits_val<__nv_bfloat16>(uin
 }
 
 // Gathers in flight per lane group: U for a short row, UL per warp step of a
-// long chunk.  8 per step of a long chunk at 8 and 16 lanes per B row measured
+// long chunk (at most 32 per warp, a batch).  8 per step of a long chunk at 8 and 16 lanes per B row measured
 // slower (graph 2^20, FP16: N = 128 0.929 ms against 0.903, N = 64 0.542
 // against 0.507), as at 4 lanes (N = 32, an earlier form: 0.551 ms against
 // 0.470): the registers cost more warps than the loads gain.
 template <int LPR> struct SlabU {
   static constexpr int U = 4;
-  static constexpr int UL = 4;
+  static constexpr int UL = LPR >= 4 ? 4 : LPR;
 };
 
 // Instructions bound this kernel, then warps in flight.  A whole batch of 32
@@ -2159,13 +2159,13 @@ template <int LPR> struct SlabU {
 // 48 bytes spilled 0.962, 6 1.041; N = 32: 4 0.323, 5 0.338; N = 256: 4 1.74,
 // none 1.93), FP32 5 (N = 128: 5 0.321, 6 0.343).
 template <typename T, int LPR, int U, int UL, bool WIDE>
-__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 4 : (LPR >= 8 ? 5 : 0))
+__global__ void __launch_bounds__(256, LPR < 4 ? 0 : sizeof(T) == 2 ? 4 : (LPR >= 8 ? 5 : 0))
     spmm_slab_kernel(
     int64_t nlong, const int2 *__restrict__ long_se, const int32_t *__restrict__ long_slot, int32_t nshort,
     const int32_t *__restrict__ short_rows, const int2 *__restrict__ short_se,
     const int32_t *__restrict__ colIdx, const T *__restrict__ val,
     const T *__restrict__ B, int64_t ldb, int32_t col0, int32_t ns, float *__restrict__ C, int64_t ldc,
-    float *__restrict__ part, float alpha, float beta, int32_t hints) {
+    float *__restrict__ part, float alpha, float beta, int32_t hints, bool vec_c) {
   constexpr int VEC = SpmmVec<T>::VEC;
   constexpr int G = 32 / LPR;
   const int lane = threadIdx.x & 31;
@@ -2276,7 +2276,28 @@ __global__ void __launch_bounds__(256, sizeof(T) == 2 ? 4 : (LPR >= 8 ? 5 : 0))
     }
     if (!on) continue;
     float *cp = C + (int64_t)r * ldc + cl;
-    if (beta != 0.f) {
+    // C's rows in 16-byte stores where they are aligned for them: a lane's 4 or 8
+    // columns were as many 4-byte stores, each touching a sector per lane of the
+    // warp.  FP16, 500,000 rows of 5, N = 256 342 -> 259 us, N = 128 175 -> 138;
+    // 27-point stencil 64^3 N = 64 98 -> 82; graph 2^20 N = 128 0.868 -> 0.818 ms,
+    // N = 32 0.319 -> 0.291.
+    if (vec_c) {
+#pragma unroll
+      for (int k = 0; k < VEC; k += 4) {
+        float4 o = make_float4(alpha * acc[k], alpha * acc[k + 1], alpha * acc[k + 2], alpha * acc[k + 3]);
+        if (beta != 0.f) {
+          const float4 c = *reinterpret_cast<const float4 *>(cp + k);
+          o.x += beta * c.x;
+          o.y += beta * c.y;
+          o.z += beta * c.z;
+          o.w += beta * c.w;
+        }
+        if (hints && beta == 0.f)
+          __stcs(reinterpret_cast<float4 *>(cp + k), o);
+        else
+          *reinterpret_cast<float4 *>(cp + k) = o;
+      }
+    } else if (beta != 0.f) {
 #pragma unroll
       for (int k = 0; k < VEC; ++k) {
         float o = alpha * acc[k];
@@ -2300,9 +2321,12 @@ static bsp_status launch_slab(const bsp_spmm_plan *p, const int32_t *ci, const v
   constexpr int G = 32 / LPR;
   const int64_t ntasks = p->nparts + (p->nshort + G - 1) / G;
   // 64 CTAs per SM, a few of them resident: their first tasks start in list
-  // order, which keeps the long chunks in step (graph 2^20, FP16, N = 128:
-  // 64 per SM 1.119 ms, 32 1.174, one task per warp 1.165, only the resident
-  // CTAs 1.37).
+  // order, which keeps the long chunks in step, and a warp still takes several
+  // of many short rows (graph 2^20, FP16, N = 128: 64 per SM 0.818 ms, 256
+  // 0.836, one task per warp 0.888; before the steps below 32 per SM 1.174
+  // against 1.119, only the resident CTAs 1.37; 500,000 rows of 5, N = 256: 64
+  // per SM 258 us, 256 283, one task per warp 306).
+  const bool vec_c = (uintptr_t)C % 16 == 0 && ldc % 4 == 0 && col0 % 4 == 0;
   int64_t blocks = ceil_div(ntasks, 8);
   const int64_t cap = (int64_t)sm_count() * 64;
   if (blocks > cap) blocks = cap;
@@ -2310,25 +2334,26 @@ static bsp_status launch_slab(const bsp_spmm_plan *p, const int32_t *ci, const v
   spmm_slab_kernel<T, LPR, SlabU<LPR>::U, SlabU<LPR>::UL, WIDE><<<(unsigned)blocks, 256, 0, s>>>(
       p->nparts, reinterpret_cast<const int2 *>(p->long_se), p->long_chunk + p->nparts, p->nshort, p->short_rows,
       reinterpret_cast<const int2 *>(p->short_se), ci, (const T *)val, (const T *)B, ldb, col0, ns, C, ldc, part, a,
-      b, hints);
+      b, hints, vec_c);
   BSP_LAUNCH_CHECK();
   return BSP_OK;
 }
 
 // Lanes per B row of the next pass when `n` 16-byte pieces of the row are left:
-// the fewest of 4, 8, 16 and 32 that hold them all.  The lanes past the last
-// piece do the same work as its lane and store nothing, which costs less than
-// further passes (each reads A and runs the reduce again).  Graph 2^20, FP16:
-// N = 96 as 16 lanes 0.834 ms, as 8 + 4 0.932, as three times 4 1.091; N = 40
-// as 8 lanes 0.461, as 4 + 4 0.675; N = 136 as 32 lanes 1.44, as 16 + 4 1.38;
+// the fewest of 1, 2, 4, 8, 16 and 32 that hold them all.  The lanes past the
+// last piece do the same work as its lane and store nothing, which costs less
+// than further passes (each reads A and runs the reduce again).  Graph 2^20,
+// FP16: N = 96 as 16 lanes 0.834 ms, as 8 + 4 0.932, as three times 4 1.091; N =
+// 40 as 8 lanes 0.461, as 4 + 4 0.675; N = 136 as 32 lanes 1.44, as 16 + 4 1.38;
 // graph 100,000, FP16: N = 96 0.087 against 0.143 and 0.203, N = 136 0.142
 // against 0.177 (17 passes of one lane, the widest that divides it: 1.79).
-// One and two lanes per B row had kernels of their own: N = 8 / 16 0.240 /
-// 0.261 ms against 0.255 / 0.277 at 2^20, 0.042 against 0.027 for N = 8 at
-// 10,000.
-static int slab_lanes(int n) {
+// One and two lanes only where rows are short (a mean of 8 entries at most): a
+// warp then takes 32 or 16 rows at once, which pays until one of them is long.
+// N = 8 on 500,000 rows of 5: one lane 14 us, four 34; on a graph of 10,000 one
+// lane 47, four 26; N = 16: two lanes 20, four 34.
+static int slab_lanes(int n, bool short_rows) {
   int l = 32;
-  while (l > 4 && n <= l / 2) l >>= 1;
+  while (l > (short_rows ? 1 : 4) && n <= l / 2) l >>= 1;
   return l;
 }
 
@@ -2360,15 +2385,16 @@ static int slab_width(int32_t N, int32_t cols, const void *B, int64_t ldb, int32
 constexpr double kHintSlabBytes = 64.0 * 1024 * 1024;
 
 template <typename T>
-static bsp_status slab_typed(const bsp_spmm_plan *p, int32_t N, int32_t cols, int32_t width, const int32_t *ci,
+static bsp_status slab_typed(const bsp_spmm_plan *p, int32_t nnz, int32_t N, int32_t cols, int32_t width, const int32_t *ci,
                              const void *val, const void *B, int64_t ldb, float *C, int64_t ldc, float *part,
                              float a, float b, cudaStream_t s) {
   constexpr int VEC = SpmmVec<T>::VEC;
   // rows of B 4 GiB apart or more: one kernel, 4 lanes wide
   const bool wide = (uint64_t)ldb * sizeof(T) > 0xffffffffull;
   if (wide && width > 4 * VEC) width = 4 * VEC;
+  const bool short_rows = nnz <= 8ll * p->rows;
   for (int32_t col0 = 0, ns; col0 < N; col0 += ns) {
-    const int l = slab_lanes(std::min(width, N - col0) / VEC);
+    const int l = slab_lanes(std::min(width, N - col0) / VEC, !wide && short_rows);
     ns = std::min(l * VEC, std::min(width, N - col0));
     const int32_t hints = (double)cols * ns * sizeof(T) <= kHintSlabBytes ? p->slab_l2_hints : 0;
     bsp_status st;
@@ -2376,6 +2402,8 @@ static bsp_status slab_typed(const bsp_spmm_plan *p, int32_t N, int32_t cols, in
       case 32: st = launch_slab<T, 32>(p, ci, val, B, ldb, col0, ns, C, ldc, part, a, b, hints, s); break;
       case 16: st = launch_slab<T, 16>(p, ci, val, B, ldb, col0, ns, C, ldc, part, a, b, hints, s); break;
       case 8: st = launch_slab<T, 8>(p, ci, val, B, ldb, col0, ns, C, ldc, part, a, b, hints, s); break;
+      case 2: st = launch_slab<T, 2>(p, ci, val, B, ldb, col0, ns, C, ldc, part, a, b, hints, s); break;
+      case 1: st = launch_slab<T, 1>(p, ci, val, B, ldb, col0, ns, C, ldc, part, a, b, hints, s); break;
       default:
         st = wide ? launch_slab<T, 4, true>(p, ci, val, B, ldb, col0, ns, C, ldc, part, a, b, hints, s)
                   : launch_slab<T, 4>(p, ci, val, B, ldb, col0, ns, C, ldc, part, a, b, hints, s);
@@ -2458,10 +2486,10 @@ static bsp_status spmm_planned_impl(const bsp_spmm_plan *p, int32_t cols, int32_
   if (ns > 0) {
     if (nnz > 0 && !(colIdx && values && B)) BSP_FAIL(BSP_ERR_INVALID, "null pointer");
     switch (dtype) {
-      case BSP_F16: return slab_typed<__half>(p, N, cols, ns, colIdx, values, B, ldb, C, ldc, part, alpha, beta, s);
+      case BSP_F16: return slab_typed<__half>(p, nnz, N, cols, ns, colIdx, values, B, ldb, C, ldc, part, alpha, beta, s);
       case BSP_BF16:
-        return slab_typed<__nv_bfloat16>(p, N, cols, ns, colIdx, values, B, ldb, C, ldc, part, alpha, beta, s);
-      default: return slab_typed<float>(p, N, cols, ns, colIdx, values, B, ldb, C, ldc, part, alpha, beta, s);
+        return slab_typed<__nv_bfloat16>(p, nnz, N, cols, ns, colIdx, values, B, ldb, C, ldc, part, alpha, beta, s);
+      default: return slab_typed<float>(p, nnz, N, cols, ns, colIdx, values, B, ldb, C, ldc, part, alpha, beta, s);
     }
   }
   switch (dtype) {

@@ -371,6 +371,48 @@ def test_spmm_slab_any_number_of_pieces(cuda, name, pieces):
     P.free()
 
 
+@pytest.mark.parametrize("name", ["float16", "float32"])
+@pytest.mark.parametrize("pieces", [1, 2, 3, 5, 8, 20])
+@pytest.mark.parametrize("off,pad", [(0, 0), (0, 4), (1, 0), (0, 1)])
+def test_spmm_slab_c_stores(cuda, name, pieces, off, pad):
+    """C in 16-byte stores where its base and row pitch allow them, else in
+    4-byte ones, on short rows (mean below 8: one and two lanes per B row too)
+    and one long row; what lies between C's rows is left alone.  Small whole
+    numbers, so every sum is exact."""
+    import ctypes as C
+    import torch
+    from benchsp_b200._lib import check, lib
+    from benchsp_b200.api import _dtype_code
+    dt = getattr(torch, name)
+    N = pieces * (16 // torch.empty(0, dtype=dt).element_size())
+    rng = np.random.default_rng(pieces)
+    lens = rng.integers(0, 9, 700)
+    lens[13] = 300
+    n = 400
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = np.concatenate([np.sort(rng.choice(n, l, replace=False)) for l in lens]).astype(np.int32)
+    rpd, cid = _dev(cuda, rp, ci)
+    v = rng.integers(-3, 4, rp[-1]).astype(np.float64)
+    B = rng.integers(-3, 4, (n, N)).astype(np.float64)
+    vd, Bd = torch.from_numpy(v).to(dt).to(cuda), torch.from_numpy(B).to(dt).to(cuda)
+    want = np.zeros((len(lens), N))
+    np.add.at(want, np.repeat(np.arange(len(lens)), lens), v[:, None] * B[ci])
+    P = bsp.SpmmPlan(rpd, cid, vd, cols=n)
+    ws = torch.empty(max(16, P.workspace_bytes(N)), dtype=torch.uint8, device=cuda)
+    ldc = N + pad
+    for alpha, beta in ((1.0, 0.0), (2.0, -3.0)):
+        store = torch.full((len(lens) * ldc + 8,), 7.0, device=cuda)
+        check(lib().bsp_spmm_csr_planned(C.byref(P._d), n, int(rp[-1]), rpd.data_ptr(), cid.data_ptr(), vd.data_ptr(),
+                                         _dtype_code(vd), Bd.data_ptr(), N, N, store.data_ptr() + 4 * off, ldc, alpha,
+                                         beta, ws.data_ptr(), P.workspace_bytes(N), None))
+        torch.cuda.synchronize()
+        full = store.cpu().numpy().astype(np.float64)
+        got = full[off:off + len(lens) * ldc].reshape(len(lens), ldc)
+        assert np.array_equal(got[:, :N], alpha * want + (beta * 7.0 if beta else 0.0))
+        assert np.all(got[:, N:] == 7.0) and np.all(full[:off] == 7.0) and np.all(full[off + len(lens) * ldc:] == 7.0)
+    P.free()
+
+
 @pytest.mark.parametrize("name", ["float16", "bfloat16", "float32"])
 @pytest.mark.parametrize("N", [8, 32, 64, 128, 256])
 def test_spmm_slab_products_are_fp32(cuda, name, N):
