@@ -2380,8 +2380,9 @@ static int slab_width(int32_t N, int32_t cols, const void *B, int64_t ldb, int32
 
 // The plan's L2 hints apply to slabs of B of at most kHintSlabBytes
 // (cols x slab width), the size that stays in L2 during a pass; wider slabs
-// gather with default caching (graph 2^20, FP16: hints at N = 32 (64 MB)
-// 0.489 -> 0.473 ms, at N = 128 (one 268 MB slab) 1.822 -> 1.853 ms).
+// gather with default caching (graph 2^20, FP16, with the long chunks in row
+// order: hints at N = 32 (64 MB) 0.489 -> 0.473 ms, at N = 128 (one 268 MB slab)
+// 1.822 -> 1.853 ms).
 constexpr double kHintSlabBytes = 64.0 * 1024 * 1024;
 
 template <typename T>
