@@ -438,7 +438,9 @@ template <typename V> struct FusedRow {
 };
 
 // Distinct diagonals of the matrix into `set` (kFusedDiags values, kNoDiag when
-// free); *overflow when there are more.
+// free); *overflow when there are more, or when a row's columns are not strictly
+// ascending (a repeated column, unsorted rows): the copy by diagonals has one
+// place per diagonal and takes a row's entries in order.
 constexpr int32_t kNoDiag = INT32_MIN;
 __global__ void fused_diags_kernel(int32_t n, const int32_t *__restrict__ rowPtr, const int32_t *__restrict__ colIdx,
                                    int32_t *set, int32_t *overflow) {
@@ -447,8 +449,14 @@ __global__ void fused_diags_kernel(int32_t n, const int32_t *__restrict__ rowPtr
   __syncthreads();
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
     if (*reinterpret_cast<volatile int32_t *>(overflow)) return;
+    int32_t before = INT32_MIN;
     for (int32_t j = rowPtr[t]; j < rowPtr[t + 1]; ++j) {
-      const int32_t d = (int32_t)(colIdx[j] - t);
+      const int32_t c = colIdx[j], d = (int32_t)(c - t);
+      if (c <= before) {
+        *overflow = 1;
+        return;
+      }
+      before = c;
       bool known = false;
 #pragma unroll
       for (int k = 0; k < kFusedDiags; ++k) known |= *reinterpret_cast<volatile int32_t *>(seen + k) == d;
@@ -1517,8 +1525,9 @@ static FusedLaunch fused_launch(const bsp_cg_plan_s *P) {
 }
 
 // Sets up the fused iteration where it applies: no preconditioner, one CTA per
-// SM whose share of the vectors fits in shared memory, and at most kFusedDiags
-// distinct diagonals that the rows fill by 3/4 or more.
+// SM whose share of the vectors fits in shared memory, strictly ascending columns
+// in every row, and at most kFusedDiags distinct diagonals that the rows fill by
+// 3/4 or more.
 static bsp_status fused_setup(bsp_cg_plan_s *P, cudaStream_t s) {
   if (P->prec_bs) return BSP_OK;
   const size_t vt = cg_mixed(P) ? 4 : 8;

@@ -188,3 +188,38 @@ def test_cg_fused_on_several_streams(cuda):
     for t in threads:
         t.join()
     assert all(same)
+
+
+def _rewritten(A, kind):
+    """A's entries stored another way: "repeated" splits every diagonal entry in
+    two equal halves (as reading a symmetric file entry by entry gives it),
+    "descending" reverses each row."""
+    rp, ci, va = [0], [], []
+    for i in range(A.rows):
+        s = slice(A.rowptr[i], A.rowptr[i + 1])
+        c, v = A.colidx[s], A.values[s]
+        if kind == "repeated":
+            k = 1 + (c == i)
+            c, v = np.repeat(c, k), np.repeat(v / k, k)
+        else:
+            c, v = c[::-1], v[::-1]
+        ci.append(c)
+        va.append(v)
+        rp.append(rp[-1] + len(c))
+    return bsp.HostCSR(A.rows, A.rows, np.asarray(rp, np.int32), np.concatenate(ci), np.concatenate(va))
+
+
+# a copy by 5 or 7 diagonals has no free place for a repeated entry, by 3 it has
+@pytest.mark.parametrize("diags", [[1], [1, 70], [1, 33, 1024]])
+@pytest.mark.parametrize("kind", ["repeated", "descending"])
+@pytest.mark.parametrize("mode", ["fp64", "f16"])
+def test_cg_rows_with_repeated_or_unsorted_columns(cuda, diags, kind, mode):
+    A = _banded(3000, diags, 7)
+    R = _rewritten(A, kind)
+    b = bsp.gen_uniform(A.rows, 8)
+    rp, ci, va, bb = _dev(cuda, R.rowptr, R.colidx, R.values, b)
+    S = bsp.CgSolver(rp, ci, va, mode=mode, tol=1e-10)
+    x, res = S.solve(bb)
+    S.close()
+    assert res["converged"] == 1
+    assert pyoracle.rel_residual(A.rowptr, A.colidx, A.values, b, x.cpu().numpy()) <= 2e-10
