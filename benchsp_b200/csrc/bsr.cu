@@ -157,6 +157,10 @@ __global__ void bsr_fill_kernel(int32_t rows, int32_t tm, int32_t tk, const int3
 // (8 CTAs per SM: 804 us).  8x8 blocks, 61^3: 591 us at 5 CTAs per SM, 630 at 4.
 // A lane walks its row serially and a block takes a trip whatever it holds, so
 // scattered matrices and a few long rows keep the general path (merge_wins).
+// A repeated column would be taken for the next one (n == BS entries need not be
+// BS columns), so the counting pass also compares each row's neighbouring columns
+// and *note tells the caller to search instead; in the fill pass *note counts the
+// full blocks.
 // VEC: colIdx 16-byte and values 32-byte aligned; a lane at an aligned entry
 // then loads 4 columns (4 values) at once.
 template <int BS>
@@ -188,7 +192,8 @@ __device__ __forceinline__ void merge_load(const int32_t *__restrict__ colIdx, i
 // CTA merges 32 / BS of them, at most kSampleTrips blocks each).
 struct BlockProfile {
   int64_t total;  // blocks of the whole matrix (the counting pass's scan)
-  int32_t longest, blocks, entries, pad;
+  int32_t longest, blocks, entries;
+  int32_t unsorted;  // the counting pass: some row's columns are not strictly ascending
 };
 constexpr int kSampleTrips = 16;
 
@@ -233,11 +238,12 @@ __global__ void __launch_bounds__(256, BS == 8 ? 5 : 1)
                      const int32_t *__restrict__ colIdx, const double *__restrict__ val, int32_t *__restrict__ cnt,
                      const int32_t *__restrict__ blcPtr,
                      int32_t *__restrict__ blcIdx, double *__restrict__ blcVal, MapT *__restrict__ map,
-                     int32_t *__restrict__ full) {
+                     int32_t *__restrict__ note) {
   constexpr int32_t kNone = INT32_MAX;
   const int lane = threadIdx.x & 31, br_lane = lane % BS;
   const int64_t nrow = (int64_t)blc_row * BS, stride = (int64_t)gridDim.x * blockDim.x;
   int32_t nfull = 0;
+  bool unsorted = false;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r - lane < nrow; r += stride) {
     int32_t j = r < rows ? rowPtr[r] : 0;
     const int32_t e = r < rows ? rowPtr[r + 1] : 0;
@@ -245,7 +251,14 @@ __global__ void __launch_bounds__(256, BS == 8 ? 5 : 1)
     int64_t blk = FILL && br < blc_row ? blcPtr[br] : 0;
     const int64_t blk0 = blk;
     MergeRun<BS> w;
+    auto look = [&] {  // consecutive windows share an entry: every pair of neighbours is seen
+      if constexpr (!FILL) {
+#pragma unroll
+        for (int k = 0; k < BS; ++k) unsorted |= w.c[k + 1] >= 0 && w.c[k + 1] <= w.c[k];
+      }
+    };
     merge_load<BS, VEC>(colIdx, j, e, w);
+    look();
     int32_t cur = w.c[0] >= 0 ? w.c[0] / BS : kNone;
     for (;;) {
       int32_t m = cur;
@@ -309,6 +322,7 @@ __global__ void __launch_bounds__(256, BS == 8 ? 5 : 1)
       if (n) {
         j += n;
         merge_load<BS, VEC>(colIdx, j, e, w);
+        look();
         cur = w.c[0] >= 0 ? w.c[0] / BS : kNone;
       }
     }
@@ -316,7 +330,9 @@ __global__ void __launch_bounds__(256, BS == 8 ? 5 : 1)
   }
   if constexpr (FILL) {
     nfull = __reduce_add_sync(0xffffffffu, nfull);
-    if (full && lane == 0 && nfull) atomicAdd(full, nfull);
+    if (note && lane == 0 && nfull) atomicAdd(note, nfull);
+  } else {
+    if (__any_sync(0xffffffffu, unsorted) && lane == 0) *note = 1;
   }
 }
 
@@ -402,14 +418,14 @@ static bsp_status merge_fill(int32_t rows, int32_t blc_row, const int32_t *rowPt
 
 template <int BS>
 static bsp_status merge_count(int32_t rows, int32_t blc_row, const int32_t *rowPtr, const int32_t *colIdx, bool vec,
-                              int32_t *cnt, cudaStream_t s) {
+                              int32_t *cnt, int32_t *unsorted, cudaStream_t s) {
   const unsigned g = grid_for((int64_t)blc_row * BS, 256);
   if (vec)
     bsr_merge_kernel<BS, false, true, uint64_t><<<g, 256, 0, s>>>(rows, blc_row, rowPtr, colIdx, nullptr, cnt,
-                                                                  nullptr, nullptr, nullptr, nullptr, nullptr);
+                                                                  nullptr, nullptr, nullptr, nullptr, unsorted);
   else
     bsr_merge_kernel<BS, false, false, uint64_t><<<g, 256, 0, s>>>(rows, blc_row, rowPtr, colIdx, nullptr, cnt,
-                                                                   nullptr, nullptr, nullptr, nullptr, nullptr);
+                                                                   nullptr, nullptr, nullptr, nullptr, unsorted);
   BSP_LAUNCH_CHECK();
   return BSP_OK;
 }
@@ -433,7 +449,8 @@ static bool merge_wins(int bs, const BlockProfile &p, int32_t nnz) {
 // the number of full blocks.  Outputs are allocated here.
 //
 // 4x4 and 8x8 blocks merge the rows of a block-row (bsr_merge_kernel) where
-// merge_wins says so; other shapes and matrices search per nonzero
+// merge_wins says so and every row's columns are strictly ascending; other shapes
+// and matrices search per nonzero
 // (bsr_canonical_kernel, bsr_fill_kernel).
 bsp_status csr2blocks(int32_t rows, int32_t nnz, const int32_t *rowPtr, const int32_t *colIdx, const double *values,
                       int32_t tm, int32_t tk, int32_t *blc_num_out, int32_t **blcPtr, int32_t **blcIdx,
@@ -463,11 +480,13 @@ bsp_status csr2blocks(int32_t rows, int32_t nnz, const int32_t *rowPtr, const in
   }
   if (merge) {
     BSP_CUDA(cudaMemsetAsync(*blcPtr + blc_row, 0, sizeof(int32_t), s));
-    BSP_TRY(tm == 4 ? merge_count<4>(rows, blc_row, rowPtr, colIdx, vec, *blcPtr, s)
-                    : merge_count<8>(rows, blc_row, rowPtr, colIdx, vec, *blcPtr, s));
+    BSP_TRY(tm == 4 ? merge_count<4>(rows, blc_row, rowPtr, colIdx, vec, *blcPtr, &d_meta->unsorted, s)
+                    : merge_count<8>(rows, blc_row, rowPtr, colIdx, vec, *blcPtr, &d_meta->unsorted, s));
     BSP_TRY(exclusive_scan_i32(*blcPtr, *blcPtr, (int64_t)blc_row + 1, &d_meta->total, s));
     BSP_TRY(read_meta());
-  } else {
+    merge = !h.unsorted;
+  }
+  if (!merge) {
     BSP_TRY(dalloc(&pos, (size_t)nnz + 1, s));
     BSP_CUDA(cudaMemsetAsync(pos + nnz, 0, sizeof(int32_t), s));
     if (nnz > 0) {

@@ -214,3 +214,22 @@ def test_csr2bsr_both_conversions_at_the_edges(cuda, rows, cols, longest, shift,
     a = bsp.csr2bcsr(drp, dci, dva, rows=rows, cols=cols, tile_m=bs, tile_k=bs).arrays()
     assert np.array_equal(a["bcsrColIdx"], o["blcIdx"]) and np.array_equal(a["bcsrRowPtr"], o["blcPtr"])
     assert np.array_equal(a["bcsrVal"], o["blcVal"])
+
+
+@pytest.mark.parametrize("where", ["every row", "last row"])
+@pytest.mark.parametrize("bs", [4, 8])
+def test_csr2bsr_rows_with_a_repeated_column(cuda, bs, where):
+    """A column stored twice with the same value (a symmetric file's diagonal):
+    the blocks are those of the matrix that holds it once."""
+    A = bsp.gen_stencil27(7, 4, 11)                # 1372 rows, whole blocks: the rows are merged
+    k = np.ones(A.nnz, np.int64)
+    for r in range(A.rows) if where == "every row" else [A.rows - 1]:
+        k[A.rowptr[r] + r % 5] = 2                 # not only at the start of a block
+    rp = np.concatenate([[0], np.cumsum(np.add.reduceat(k, A.rowptr[:-1]))]).astype(np.int32)
+    ci, va = np.repeat(A.colidx, k), np.repeat(A.values, k)
+    import torch
+    drp, dci, dva = (torch.from_numpy(a).to(cuda) for a in (rp, ci, va))
+    M = bsp.csr2bsr(drp, dci, dva, rows=A.rows, cols=A.cols, bs=bs)
+    o = pyoracle.csr2bsr(A.rows, A.cols, A.rowptr, A.colidx, A.values, bs)
+    _check_arrays(M, dict(o, avg_nnz=ci.size / o["blc_num"]))
+    M.free()
