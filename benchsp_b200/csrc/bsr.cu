@@ -171,9 +171,10 @@ struct MergeRun {
 template <int BS, bool VEC>
 __device__ __forceinline__ void merge_load(const int32_t *__restrict__ colIdx, int32_t j, int32_t e,
                                            MergeRun<BS> &w) {
+  const int32_t left = e - j;  // j + BS may pass 2^31
 #pragma unroll
   for (int k = 0; k < BS; k += 4) {
-    if (VEC && (j & 3) == 0 && j + k + 4 <= e) {
+    if (VEC && (j & 3) == 0 && k + 4 <= left) {
       const int4 t = __ldg(reinterpret_cast<const int4 *>(colIdx + j + k));
       w.c[k] = t.x;
       w.c[k + 1] = t.y;
@@ -181,10 +182,10 @@ __device__ __forceinline__ void merge_load(const int32_t *__restrict__ colIdx, i
       w.c[k + 3] = t.w;
     } else {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) w.c[k + u] = j + k + u < e ? __ldg(colIdx + j + k + u) : -1;
+      for (int u = 0; u < 4; ++u) w.c[k + u] = k + u < left ? __ldg(colIdx + j + k + u) : -1;
     }
   }
-  w.c[BS] = j + BS < e ? __ldg(colIdx + j + BS) : -1;
+  w.c[BS] = BS < left ? __ldg(colIdx + j + BS) : -1;
 }
 
 // What the choice between the two conversions rests on: the longest row, and

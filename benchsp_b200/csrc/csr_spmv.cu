@@ -77,8 +77,9 @@ constexpr int kCtaRow = 512;
 constexpr int kLongList = 64;
 
 // Sum of entries j, j + STRIDE, ... < e (4 in flight), this thread's share of a row.
+// Unsigned: the steps past a row that ends near 2^31 stay above e.
 template <typename V, int STRIDE>
-__device__ __forceinline__ typename AccOf<V>::T strided_sum(int32_t j, int32_t e, const int32_t *__restrict__ colIdx,
+__device__ __forceinline__ typename AccOf<V>::T strided_sum(uint32_t j, uint32_t e, const int32_t *__restrict__ colIdx,
                                                             const V *__restrict__ val, const V *__restrict__ x) {
   using A = typename AccOf<V>::T;
   A sum = A(0);
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(kCsrThreads, LPR > 1 && sizeof(V) == 8 ? 6 : L
   const bool active = r < rows;
   const int32_t s = active ? rowPtr[r] : 0, e0 = active ? rowPtr[r + 1] : 0;
   const bool is_long = e0 - s > kWarpRowFactor * LPR;
-  const int32_t e = is_long ? s : e0;
+  const uint32_t e = is_long ? s : e0;  // unsigned like the positions, which may pass 2^31 behind the row
   // The first kFirst entries of each lane are loaded together, then their x
   // gathers together: the rowPtr -> column -> x chain is paid once per
   // kFirst entries instead of once per entry.
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(kCsrThreads, LPR > 1 && sizeof(V) == 8 ? 6 : L
   V a[kFirst];
 #pragma unroll
   for (int k = 0; k < kFirst; ++k) {
-    const int32_t j = s + sub + k * LPR;
+    const uint32_t j = (uint32_t)s + sub + k * LPR;
     c[k] = j < e ? colIdx[j] : -1;
     a[k] = j < e ? val[j] : V(0);
   }
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(kCsrThreads, LPR > 1 && sizeof(V) == 8 ? 6 : L
   for (int k = 0; k < kFirst; ++k)
     if (c[k] >= 0) sum = fma(to_acc<V>(a[k]), to_acc<V>(__ldg(&x[c[k]])), sum);
 #pragma unroll 4
-  for (int32_t j = s + sub + kFirst * LPR; j < e; j += LPR)
+  for (uint32_t j = (uint32_t)s + sub + kFirst * LPR; j < e; j += LPR)
     sum = fma(to_acc<V>(val[j]), to_acc<V>(__ldg(&x[colIdx[j]])), sum);
 #pragma unroll
   for (int o = LPR / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, LPR);

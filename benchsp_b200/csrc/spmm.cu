@@ -1810,7 +1810,7 @@ __global__ void spmm_range_kernel(int64_t nparts, const int32_t *__restrict__ lo
       const int32_t w = long_chunk[long_slot[i]];
       const int32_t r = chunk_row[w];
       const int32_t st = rowPtr[r] + (w - chunk_ptr[r]) * chunk;
-      long_se[i] = make_int2(st, min(st + chunk, rowPtr[r + 1]));
+      long_se[i] = make_int2(st, st + min(chunk, rowPtr[r + 1] - st));
     }
     if (i < nshort) {
       const int32_t r = short_rows[i];
@@ -2188,16 +2188,16 @@ __global__ void __launch_bounds__(256, LPR < 4 ? 0 : sizeof(T) == 2 ? 4 : (LPR >
       constexpr int GU = G * UL;   // nonzeros per step
       static_assert(32 % GU == 0, "a step takes a part of a batch");
       const int2 se = long_se[task];
-      const int32_t e = se.y;
+      const uint32_t e = se.y;  // unsigned: positions behind a chunk that ends near 2^31 stay above e
       const int64_t slot = long_slot[task];
-      const int32_t jl = se.x + lane;
+      const uint32_t jl = (uint32_t)se.x + lane;
       int32_t cj = jl < e ? ld_hint_s32(colIdx + jl, pa) : 0;
       uint32_t vj = jl < e ? ld_hint_val<T>(val + jl, pa) : 0u;
-      for (int32_t j0 = se.x; j0 < e; j0 += 32) {   // warp-uniform bounds
-        const int32_t jn = j0 + 32 + lane;
+      for (uint32_t j0 = se.x; j0 < e; j0 += 32) {   // warp-uniform bounds
+        const uint32_t jn = j0 + 32 + lane;
         const int32_t cn = jn < e ? ld_hint_s32(colIdx + jn, pa) : 0;
         const uint32_t vn = jn < e ? ld_hint_val<T>(val + jn, pa) : 0u;
-        const int cnt = e - j0 < 32 ? e - j0 : 32;
+        const int cnt = e - j0 < 32 ? (int)(e - j0) : 32;
         if (cnt == 32) {   // a whole batch: nothing to mask
 #pragma unroll 1
           for (int t = 0; t < 32; t += GU) {
@@ -2247,7 +2247,7 @@ __global__ void __launch_bounds__(256, LPR < 4 ? 0 : sizeof(T) == 2 ? 4 : (LPR >
     if (i >= nshort) continue;
     const int32_t r = short_rows[i];
     const int2 se = short_se[i];
-    const int32_t s = se.x, e = se.y;
+    const uint32_t s = se.x, e = se.y;
     int32_t cn[U];
     uint32_t vn[U];
 #pragma unroll
@@ -2256,7 +2256,7 @@ __global__ void __launch_bounds__(256, LPR < 4 ? 0 : sizeof(T) == 2 ? 4 : (LPR >
       cn[u] = ok ? ld_hint_s32(colIdx + s + u, pa) : 0;
       vn[u] = ok ? ld_hint_val<T>(val + s + u, pa) : 0u;
     }
-    for (int32_t j = s; j < e; j += U) {
+    for (uint32_t j = s; j < e; j += U) {
       uint4 raw[U];
       uint32_t v[U];
 #pragma unroll
@@ -2266,7 +2266,7 @@ __global__ void __launch_bounds__(256, LPR < 4 ? 0 : sizeof(T) == 2 ? 4 : (LPR >
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int32_t jj = j + U + u;
+        const uint32_t jj = j + U + u;
         const bool ok = jj < e;
         cn[u] = ok ? ld_hint_s32(colIdx + jj, pa) : 0;
         vn[u] = ok ? ld_hint_val<T>(val + jj, pa) : 0u;
