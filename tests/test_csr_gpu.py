@@ -248,3 +248,70 @@ def test_vector_long_rows(cuda, rows, cols, lens, lanes, dt):
     tol = 0.5 * pyoracle.spmv_tolerance(rp, ci, vh, xh, unit=unit) + \
         3 * unit * (np.abs(0.5 * ax) + np.abs(2.0 * yh)) + 1.01 * out * np.abs(ref) + 2.0 ** -24 * (dt == "float16")
     _within(got, ref, tol)
+
+
+# few long rows among rows of 0 to 3, so that the bound for a long row is 16
+# entries per lane: rows at it, at the CTA's bound (512, with 8 and 16 lanes 128 per
+# lane) and one past each, several rounds of the CTA, and more of them in one CTA
+# than its list holds
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("dt", ["float64", "float32", "float16"])
+def test_vector_few_long_rows(cuda, lanes, dt):
+    import torch
+    rng = np.random.default_rng(lanes)
+    bound, cta = 16 * lanes, 128 * max(lanes, 4)
+    lens = np.resize([0, 3, 1, 2], 8000)
+    lens[[0, 5, 9, 300, 301, 302, lens.size - 1]] = [bound, bound + 1, cta, cta + 1, 4097, 9000, cta + 1]
+    lens[512:512 + 70] = bound + 1
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    assert 4 * rp[-1] // lens.size <= bound
+    cols = 9500
+    ci = np.concatenate([np.sort(rng.choice(cols, k, replace=False)) for k in lens]).astype(np.int32)
+    v, x = (torch.from_numpy(a).to(getattr(torch, dt)) for a in (rng.standard_normal(ci.size), rng.uniform(-1, 1, cols)))
+    vh, xh = (t.double().numpy() for t in (v, x))
+    d_rp, d_ci = _dev(cuda, rp, ci)
+    got = bsp.csr_spmv(d_rp, d_ci, v.to(cuda), x.to(cuda), lanes=lanes).double().cpu().numpy()
+    ref = pyoracle.spmv_f64(rp, ci, vh, xh)
+    unit = 2.0 ** -53 if dt == "float64" else 2.0 ** -24
+    tol = pyoracle.spmv_tolerance(rp, ci, vh, xh, unit=unit) + \
+        (1.01 * 2.0 ** -11 * np.abs(ref) + 2.0 ** -24 if dt == "float16" else 0.0)
+    _within(got, ref, tol)
+
+
+def _us_per_million(cuda, rows, length, dt):
+    """Best time of csr_spmv per million nonzeros: `rows` rows of `length`
+    consecutive columns around the diagonal."""
+    import torch
+    rp = torch.arange(0, rows * length + 1, length, dtype=torch.int32, device=cuda)
+    start = torch.arange(rows, dtype=torch.int32, device=cuda).clamp(max=rows - length)
+    ci = (start[:, None] + torch.arange(length, dtype=torch.int32, device=cuda)).reshape(-1)
+    va = torch.ones(ci.numel(), dtype=dt, device=cuda)
+    x, y = (torch.ones(rows, dtype=dt, device=cuda) for _ in range(2))
+    best = float("inf")
+    for _ in range(5):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        torch.cuda.synchronize()
+        e[0].record()
+        for _ in range(10):
+            bsp.csr_spmv(rp, ci, va, x, y)
+        e[1].record()
+        torch.cuda.synchronize()
+        best = min(best, e[0].elapsed_time(e[1]))
+    return best * 100 / (ci.numel() / 1e6)
+
+
+@pytest.mark.parametrize("dt", ["float64", "float16"])
+def test_rows_all_long_cost_no_more_per_entry(cuda, dt):
+    """A nonzero of a matrix whose rows are all long takes no longer than one of
+    rows of 200 (with every row left to the CTA it took 1.5x to 1.9x)."""
+    import torch
+    dt = getattr(torch, dt)
+    assert _us_per_million(cuda, 60000, 600, dt) <= 1.25 * _us_per_million(cuda, 200000, 200, dt)
+
+
+def test_lanes_out_of_range_are_refused(cuda):
+    A = bsp.gen_laplace2d(8, 8)
+    d = _dev(cuda, A.rowptr, A.colidx, A.values, np.ones(A.cols))
+    for lanes in (3, 64, 512):
+        with pytest.raises(bsp.BspError):
+            bsp.csr_spmv(*d, lanes=lanes)
