@@ -1549,7 +1549,7 @@ __global__ void spmm_plan_count_kernel(int32_t rows, const int32_t *__restrict__
                                        int32_t *__restrict__ nch, int32_t *__restrict__ npart) {
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
     const int32_t len = rowPtr[r + 1] - rowPtr[r];
-    const int32_t c = len > chunk ? (len + chunk - 1) / chunk : 1;
+    const int32_t c = len > chunk ? (len - 1) / chunk + 1 : 1;
     nch[r] = c;
     npart[r] = c > 1 ? c : 0;
   }
@@ -2147,11 +2147,16 @@ template <int LPR> struct SlabU {
   static constexpr int UL = LPR >= 4 ? 4 : LPR;
 };
 
+constexpr int32_t kSlabOvershoot = 64;
+
 // Instructions bound this kernel, then warps in flight.  A whole batch of 32
 // nonzeros runs without masks (only a chunk's last batch is partial), A's
 // values stay in their own bits until the FMA, and a gather's address is one
 // 32 x 32 -> 64 bit multiply-add of the column and B's row pitch in bytes.
-// WIDE takes a 64-bit pitch, for rows of B 4 GiB apart or more.  Graph 2^20,
+// WIDE takes a 64-bit pitch, for rows of B 4 GiB apart or more, and unsigned
+// positions, for matrices whose last nonzeros lie within kSlabOvershoot of 2^31 (a
+// batch's loads are issued that far behind a chunk; unsigned in all kernels: graph
+// 2^20, FP32, N = 128 1.50 -> 1.68 ms, stencil 64^3, FP16, N = 256 270 -> 304 us).  Graph 2^20,
 // FP16, N = 128 1.119 -> 0.897 ms (843 M warp instructions before), N = 64
 // 0.625 -> 0.503, N = 32 0.390 -> 0.323, N = 256 2.31 -> 1.74; BF16 N = 64
 // 0.685 -> 0.503; graph 2^18, FP32, N = 128 0.474 -> 0.321.
@@ -2176,6 +2181,7 @@ __global__ void __launch_bounds__(256, LPR < 4 ? 0 : sizeof(T) == 2 ? 4 : (LPR >
   const int32_t cl = col0 + (on ? li * VEC : ns - VEC);
   const char *const Bc = (const char *)(B + cl);
   using pitch_t = typename std::conditional<WIDE, uint64_t, uint32_t>::type;
+  using pos_t = typename std::conditional<WIDE, uint32_t, int32_t>::type;
   const pitch_t pitch = (pitch_t)(ldb * (int64_t)sizeof(T));
   const uint64_t pa = l2_policy(hints != 0, false), pb = l2_policy(hints == 1, true);
   const int64_t ntasks = nlong + (nshort + G - 1) / G;
@@ -2188,13 +2194,13 @@ __global__ void __launch_bounds__(256, LPR < 4 ? 0 : sizeof(T) == 2 ? 4 : (LPR >
       constexpr int GU = G * UL;   // nonzeros per step
       static_assert(32 % GU == 0, "a step takes a part of a batch");
       const int2 se = long_se[task];
-      const uint32_t e = se.y;  // unsigned: positions behind a chunk that ends near 2^31 stay above e
+      const pos_t e = se.y;
       const int64_t slot = long_slot[task];
-      const uint32_t jl = (uint32_t)se.x + lane;
+      const pos_t jl = (pos_t)se.x + lane;
       int32_t cj = jl < e ? ld_hint_s32(colIdx + jl, pa) : 0;
       uint32_t vj = jl < e ? ld_hint_val<T>(val + jl, pa) : 0u;
-      for (uint32_t j0 = se.x; j0 < e; j0 += 32) {   // warp-uniform bounds
-        const uint32_t jn = j0 + 32 + lane;
+      for (pos_t j0 = se.x; j0 < e; j0 += 32) {   // warp-uniform bounds
+        const pos_t jn = j0 + 32 + lane;
         const int32_t cn = jn < e ? ld_hint_s32(colIdx + jn, pa) : 0;
         const uint32_t vn = jn < e ? ld_hint_val<T>(val + jn, pa) : 0u;
         const int cnt = e - j0 < 32 ? (int)(e - j0) : 32;
@@ -2247,7 +2253,7 @@ __global__ void __launch_bounds__(256, LPR < 4 ? 0 : sizeof(T) == 2 ? 4 : (LPR >
     if (i >= nshort) continue;
     const int32_t r = short_rows[i];
     const int2 se = short_se[i];
-    const uint32_t s = se.x, e = se.y;
+    const pos_t s = se.x, e = se.y;
     int32_t cn[U];
     uint32_t vn[U];
 #pragma unroll
@@ -2256,7 +2262,7 @@ __global__ void __launch_bounds__(256, LPR < 4 ? 0 : sizeof(T) == 2 ? 4 : (LPR >
       cn[u] = ok ? ld_hint_s32(colIdx + s + u, pa) : 0;
       vn[u] = ok ? ld_hint_val<T>(val + s + u, pa) : 0u;
     }
-    for (uint32_t j = s; j < e; j += U) {
+    for (pos_t j = s; j < e; j += U) {
       uint4 raw[U];
       uint32_t v[U];
 #pragma unroll
@@ -2266,7 +2272,7 @@ __global__ void __launch_bounds__(256, LPR < 4 ? 0 : sizeof(T) == 2 ? 4 : (LPR >
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const uint32_t jj = j + U + u;
+        const pos_t jj = j + U + u;
         const bool ok = jj < e;
         cn[u] = ok ? ld_hint_s32(colIdx + jj, pa) : 0;
         vn[u] = ok ? ld_hint_val<T>(val + jj, pa) : 0u;
@@ -2390,8 +2396,8 @@ static bsp_status slab_typed(const bsp_spmm_plan *p, int32_t nnz, int32_t N, int
                              const void *val, const void *B, int64_t ldb, float *C, int64_t ldc, float *part,
                              float a, float b, cudaStream_t s) {
   constexpr int VEC = SpmmVec<T>::VEC;
-  // rows of B 4 GiB apart or more: one kernel, 4 lanes wide
-  const bool wide = (uint64_t)ldb * sizeof(T) > 0xffffffffull;
+  // rows of B 4 GiB apart or more, or positions near 2^31: one kernel, 4 lanes wide
+  const bool wide = (uint64_t)ldb * sizeof(T) > 0xffffffffull || nnz > INT32_MAX - kSlabOvershoot;
   if (wide && width > 4 * VEC) width = 4 * VEC;
   const bool short_rows = nnz <= 8ll * p->rows;
   for (int32_t col0 = 0, ns; col0 < N; col0 += ns) {
