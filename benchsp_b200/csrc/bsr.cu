@@ -195,6 +195,7 @@ struct BlockProfile {
   int64_t total;  // blocks of the whole matrix (the counting pass's scan)
   int32_t longest, blocks, entries;
   int32_t unsorted;  // the counting pass: some row's columns are not strictly ascending
+  int32_t chain;     // most blocks of an outlying block-row (bsr_chain_kernel)
 };
 constexpr int kSampleTrips = 16;
 
@@ -230,6 +231,54 @@ __global__ void __launch_bounds__(256) bsr_profile_kernel(int32_t rows, int32_t 
   if (lane == 0) {
     atomicAdd(&out->blocks, blocks);
     atomicAdd(&out->entries, entries);
+  }
+}
+
+// Blocks of the outlying block-rows, counted exactly (the entries that are the first
+// of their block, as in bsr_canonical_kernel): the most of any into out->chain.
+// Outlying, with more than `limit` entries: more than `bound` of them, or one row with
+// twice its share.  Counting a block-row stops above `limit`.
+template <int BS>
+__global__ void __launch_bounds__(256) bsr_chain_kernel(int32_t rows, int32_t blc_row,
+                                                        const int32_t *__restrict__ rowPtr,
+                                                        const int32_t *__restrict__ colIdx, int64_t bound,
+                                                        int64_t limit, BlockProfile *out) {
+  __shared__ int32_t list[256], n;
+  for (int64_t first = (int64_t)blockIdx.x * 256; first < blc_row; first += (int64_t)gridDim.x * 256) {
+    if (threadIdx.x == 0) n = 0;
+    __syncthreads();
+    const int64_t br = first + threadIdx.x;
+    if (br < blc_row) {
+      const int32_t *p = rowPtr + br * BS;
+      const int m = (int)min((int64_t)BS, rows - br * BS);
+      const int64_t entries = (int64_t)p[m] - p[0];
+      int64_t longest = 0;
+      for (int q = 0; q < m; ++q) longest = max(longest, (int64_t)p[q + 1] - p[q]);
+      if (entries > limit && (entries > bound || BS * longest > 2 * entries)) list[atomicAdd(&n, 1)] = (int32_t)br;
+    }
+    __syncthreads();
+    for (int k = 0; k < n; ++k) {  // CTA-uniform
+      const int32_t r0 = list[k] * BS, r1 = min(r0 + BS, rows);
+      int64_t blocks = 0;
+      for (int32_t r = r0; r < r1; ++r) {
+        const int64_t e = rowPtr[r + 1];
+        for (int64_t j0 = rowPtr[r]; j0 < e && blocks <= limit; j0 += 256) {
+          const int64_t j = j0 + threadIdx.x;
+          bool canon = j < e;
+          if (canon) {
+            const int32_t b = colIdx[j] / BS;
+            canon = j == rowPtr[r] || colIdx[j - 1] / BS != b;
+            for (int32_t q = r0; q < r && canon; ++q) {
+              const int32_t qe = rowPtr[q + 1], p = lower_bound_i32(colIdx, rowPtr[q], qe, b * BS);
+              canon = !(p < qe && colIdx[p] / BS == b);
+            }
+          }
+          blocks += __syncthreads_count(canon);
+        }
+      }
+      if (threadIdx.x == 0) atomicMax(&out->chain, (int32_t)min(blocks, (int64_t)INT32_MAX));
+    }
+    __syncthreads();
   }
 }
 
@@ -434,14 +483,29 @@ static bsp_status merge_count(int32_t rows, int32_t blc_row, const int32_t *rowP
 // Whether merging the rows beats searching per nonzero.  The merge takes one
 // trip per block: with fewer than 3 entries per block it moves mostly zeros
 // (400,000 random rows of 16, 8x8: 1470 us against 1306), and the block-row
-// with the most blocks sets a serial chain of about 1.2 us per block over the
-// two passes (4096 random rows of 64: 256 blocks, 311 us against 78).  The
-// search takes 41 ps (4x4) or 66 ps (8x8) per nonzero and no less than about
-// 100 us at row lengths where the chain could matter.
-static bool merge_wins(int bs, const BlockProfile &p, int32_t nnz) {
+// with the most blocks sets a serial chain of about 0.65 us (4x4) or 1.2 us (8x8)
+// per block over the two passes.  The search takes 41 ps (4x4) or 66 ps (8x8) per
+// nonzero and no less than about 100 us at row lengths where the chain could matter.
+static int64_t merge_chain_limit(int bs, int32_t nnz) {
+  return (int64_t)(bs == 4 ? std::max(100e-6, nnz * 41e-12) / 0.65e-6 : std::max(100e-6, nnz * 66e-12) / 1.2e-6);
+}
+
+// The sample gives the entries per block of ordinary block-rows, not of a long
+// row whose columns are scattered (a constraint in a finite-element matrix: one
+// block per entry where the others have 16 or 64 entries in one).  So block-rows with
+// over twice the mean, or one row with over twice its share, are counted exactly
+// (bsr_chain_kernel) where some row is long enough for that.  Stencil 40^3 x 4 dof
+// (26.6 M nonzeros) with one row of 3,000 scattered entries: merged, as the sample had
+// it, 4x4 2.35 ms, 8x8 3.96; searched 1.32 and 2.13; without that row 0.35 and 0.46.
+static int64_t merge_chain_bound(int bs, int32_t nnz, int32_t blc_row) {
+  return std::max(merge_chain_limit(bs, nnz), 2 * (int64_t)nnz / blc_row);
+}
+
+static bool merge_wins(int bs, const BlockProfile &p, int32_t nnz, int32_t blc_row) {
   if (p.blocks == 0 || p.entries < 3 * (int64_t)p.blocks) return false;
-  const double blocks = (double)bs * p.longest * p.blocks / p.entries;
-  return blocks * 1.2e-6 <= std::max(100e-6, nnz * (bs == 4 ? 41e-12 : 66e-12));
+  const int64_t limit = merge_chain_limit(bs, nnz);
+  const double entries = (double)std::min((int64_t)bs * p.longest, merge_chain_bound(bs, nnz, blc_row));
+  return p.chain <= limit && entries * p.blocks / p.entries <= limit;
 }
 
 // Canonical tm x tk blocking of a CSR matrix (block columns ascending per
@@ -477,7 +541,18 @@ bsp_status csr2blocks(int32_t rows, int32_t nnz, const int32_t *rowPtr, const in
       bsr_profile_kernel<8><<<g, 256, 0, s>>>(rows, blc_row, rowPtr, colIdx, d_meta);
     BSP_LAUNCH_CHECK();
     BSP_TRY(read_meta());
-    merge = merge_wins(tm, h, nnz);
+    merge = merge_wins(tm, h, nnz, blc_row);
+    const int64_t bound = merge_chain_bound(tm, nnz, blc_row);
+    if (merge && (int64_t)tm * h.longest > bound) {
+      const unsigned gc = (unsigned)std::min<int64_t>((int64_t)sm_count() * 4, ceil_div(blc_row, 256));
+      if (tm == 4)
+        bsr_chain_kernel<4><<<gc, 256, 0, s>>>(rows, blc_row, rowPtr, colIdx, bound, merge_chain_limit(tm, nnz), d_meta);
+      else
+        bsr_chain_kernel<8><<<gc, 256, 0, s>>>(rows, blc_row, rowPtr, colIdx, bound, merge_chain_limit(tm, nnz), d_meta);
+      BSP_LAUNCH_CHECK();
+      BSP_TRY(read_meta());
+      merge = merge_wins(tm, h, nnz, blc_row);
+    }
   }
   if (merge) {
     BSP_CUDA(cudaMemsetAsync(*blcPtr + blc_row, 0, sizeof(int32_t), s));

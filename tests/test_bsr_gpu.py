@@ -233,3 +233,55 @@ def test_csr2bsr_rows_with_a_repeated_column(cuda, bs, where):
     o = pyoracle.csr2bsr(A.rows, A.cols, A.rowptr, A.colidx, A.values, bs)
     _check_arrays(M, dict(o, avg_nnz=ci.size / o["blc_num"]))
     M.free()
+
+
+def _with_scattered_row(A, r, count, bs, seed):
+    """A with row r replaced by `count` entries, each in a block column of its own."""
+    rng = np.random.default_rng(seed)
+    c = np.sort(rng.choice(A.cols // bs, count, replace=False)) * bs + rng.integers(0, bs, count)
+    a, b = A.rowptr[r], A.rowptr[r + 1]
+    rp = A.rowptr.astype(np.int64)
+    rp[r + 1:] += count - (b - a)
+    return bsp.HostCSR(A.rows, A.cols, rp.astype(np.int32), np.concatenate([A.colidx[:a], c, A.colidx[b:]]).astype(np.int32),
+                       np.concatenate([A.values[:a], rng.standard_normal(count), A.values[b:]]))
+
+
+# one scattered row among whole blocks: short enough to be merged, around twice the
+# mean of a block-row and the longest chain that the merge takes, most of the columns
+@pytest.mark.parametrize("bs,count", [(4, 40), (4, 153), (4, 154), (4, 400), (4, 1000), (8, 40), (8, 83), (8, 84),
+                                      (8, 500)])
+def test_csr2bsr_one_scattered_row(cuda, bs, count):
+    import torch
+    A = _with_scattered_row(bsp.gen_stencil27(10, 4, 2), 1999, count, bs, count)
+    d = [torch.from_numpy(a).to(cuda) for a in (A.rowptr, A.colidx, A.values)]
+    M = bsp.csr2bsr(*d, rows=A.rows, cols=A.cols, bs=bs)
+    _check_arrays(M, pyoracle.csr2bsr(A.rows, A.cols, A.rowptr, A.colidx, A.values, bs))
+    M.free()
+
+
+@pytest.mark.parametrize("bs", [4, 8])
+def test_a_scattered_row_is_not_merged(cuda, bs):
+    """Conversion of a stencil (26.6M nonzeros) with one row of 3000 scattered
+    entries.  Merged, that row alone is 3000 trips of 0.65 us (4x4) or 1.2 us (8x8);
+    the search, which half the block's width always takes, 41 or 66 ps per nonzero:
+    2.35 against 1.15 ms and 3.96 against 1.93."""
+    import torch
+    A = _with_scattered_row(bsp.gen_stencil27(40, 4, 2), 128000, 3000, bs, 1)
+    d = [torch.from_numpy(a).to(cuda) for a in (A.rowptr, A.colidx, A.values)]
+
+    def best(f):
+        t = []
+        for _ in range(4):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            torch.cuda.synchronize()
+            e[0].record()
+            M = f()
+            e[1].record()
+            torch.cuda.synchronize()
+            t.append(e[0].elapsed_time(e[1]))
+            M.free()
+        return min(t)
+
+    whole = best(lambda: bsp.csr2bsr(*d, rows=A.rows, cols=A.cols, bs=bs))
+    half = best(lambda: bsp.csr2bcsr(*d, rows=A.rows, cols=A.cols, tile_m=bs, tile_k=bs // 2))
+    assert whole <= 1.5 * half, (whole, half)
