@@ -206,6 +206,8 @@ _PROTOS.update({
     "bsp_cg_create": (C.c_int, [_I32, _I32, _P, _P, _P, C.POINTER(BspCgOptions), C.POINTER(C.c_void_p), _P]),
     "bsp_cg_solve": (C.c_int, [C.c_void_p, _P, _P, C.POINTER(BspCgResult), _P]),
     "bsp_cg_destroy": (C.c_int, [C.c_void_p]),
+    "bsp_cg_fused_ctas": (C.c_int, [C.c_void_p, C.POINTER(C.c_int32)]),
+    "bsp_cg_set_wait_limit": (C.c_int, [C.c_void_p, C.c_uint32]),
 })
 
 

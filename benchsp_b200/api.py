@@ -637,6 +637,17 @@ class CgSolver:
             check(st)
         return x, {k: getattr(r, k) for k, _ in _lib.BspCgResult._fields_}
 
+    @property
+    def fused_ctas(self) -> int:
+        """CTAs of the fused iteration's launch; 0: two kernels per iteration."""
+        n = C.c_int32()
+        check(lib().bsp_cg_fused_ctas(self._plan, C.byref(n)))
+        return n.value
+
+    def set_wait_limit(self, polls: int) -> None:
+        """Reads per wait of the fused iteration before a solve ends with BSP_ERR_TIMEOUT."""
+        check(lib().bsp_cg_set_wait_limit(self._plan, polls))
+
     def solve_multi(self, B, X=None, *, stream=None, raise_on_stall: bool = True) -> tuple:
         """A X = B for the k columns of B (n x k, FP64, row-major); FP64
         plans with no or Jacobi preconditioning.  Returns (X, per-column

@@ -321,7 +321,8 @@ __device__ __forceinline__ void vset(double2 &v, int k, double a) {
 // iteration (24^3 FP16: 9.1 -> 6 us).
 //
 // The cooperative launch makes all CTAs resident; every wait is bounded all the
-// same (kFusedPolls, then *err is set and every CTA returns).
+// same (the plan's limit, then *err is set and every CTA returns; fused_reset makes
+// the plan usable again).
 constexpr int kFusedDiags = 8;
 constexpr int kFusedMaxCtas = 256;
 constexpr uint32_t kFusedPolls = 1u << 23;  // about 5 s
@@ -506,12 +507,12 @@ struct FusedGrid {
   int32_t *err;
   unsigned long long epoch;
   double *part, *sum;  // shared: a partial per warp, a sum per polling warp
-  int *dead;           // shared, 0 at the start
+  int *dead;           // shared: 0 at the start, then the polls of one wait
 };
 
 __device__ __forceinline__ bool fused_give_up(FusedGrid &G, uint32_t polls) {
-  if ((polls & 1023u) != 0) return false;
-  if (polls < kFusedPolls && *reinterpret_cast<volatile int32_t *>(G.err) == 0) return false;
+  if (polls < (uint32_t)G.dead[1] && ((polls & 1023u) != 0 || *reinterpret_cast<volatile int32_t *>(G.err) == 0))
+    return false;
   atomicExch(G.err, 1);
   *reinterpret_cast<volatile int *>(G.dead) = 1;
   return true;
@@ -566,7 +567,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     cg_fused_kernel(int32_t n, const void *__restrict__ val, FusedDiags D, const int8_t *__restrict__ exps,
                     VT *__restrict__ x, VT *__restrict__ r, VT *__restrict__ p_state, typename FusedPub<VT>::T *pub,
                     double *rr_part, int npart, double *sc, int iters, CgSlot *slots, unsigned long long *epoch_mem,
-                    int32_t *err) {
+                    int32_t *err, uint32_t limit) {
   using Pub = FusedPub<VT>;
   using Vec = typename Vec16<VT>::T;
   constexpr int W = Vec16<VT>::W;
@@ -574,7 +575,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   constexpr int kWarps = THREADS / 32;
   extern __shared__ __align__(16) unsigned char fused_smem[];
   __shared__ double part[kWarps], sum[kFusedMaxCtas / 32];
-  __shared__ int dead;
+  __shared__ int dead[2];
   const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // uniform
   const int64_t ns = ((int64_t)n + 31) / 32;
   const FusedSlices T(ns, blockIdx.x, gridDim.x);
@@ -584,8 +585,11 @@ __global__ void __launch_bounds__(THREADS, 1)
   VT *sx = reinterpret_cast<VT *>(fused_smem), *sr = sx + cap, *sp = sr + cap, *sq = sp + cap;
   const uint32_t sp_base = (uint32_t)__cvta_generic_to_shared(sp);
   typename Pub::T *pub0 = pub + row0;
-  FusedGrid G{slots, err, *epoch_mem, part, sum, &dead};
-  if (threadIdx.x == 0) dead = 0;
+  FusedGrid G{slots, err, *epoch_mem, part, sum, dead};
+  if (threadIdx.x == 0) {
+    dead[0] = 0;
+    dead[1] = (int)limit;
+  }
   for (int32_t i = threadIdx.x; i < S * 32; i += THREADS) {  // padding rows stay 0
     const bool in = i < nloc;
     sx[i] = in ? x[row0 + i] : VT(0);
@@ -677,7 +681,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       dot += (double)acc * (double)sp[i];
     }
     const double pq = fused_sum<kWarps>(G, dot);
-    if (dead) return;
+    if (dead[0]) return;
     const double alpha = (pq != 0.0 && rr != 0.0 && isfinite(pq)) ? rr / pq : 0.0;
     const VT al = (VT)alpha;
     double s = 0.0;
@@ -696,7 +700,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     rr_prev = rr;
     rr = fused_sum<kWarps>(G, s);
-    if (dead) return;
+    if (dead[0]) return;
   }
   for (int32_t i = threadIdx.x; i < nloc; i += THREADS) {
     x[row0 + i] = sx[i];
@@ -1341,6 +1345,7 @@ struct bsp_cg_plan_s {
   void *fused_val = nullptr;  // the matrix by diagonals
   bsp::FusedDiags fused_diags{};
   int fused_nd = 0;
+  uint32_t fused_polls = bsp::kFusedPolls;
   cudaGraphExec_t graph = nullptr;
   cudaStream_t graph_stream = nullptr;
   int64_t bytes_iter = 0, bytes_residual = 0;
@@ -1524,6 +1529,20 @@ static FusedLaunch fused_launch(const bsp_cg_plan_s *P) {
   }
 }
 
+static size_t fused_pub_bytes(const bsp_cg_plan_s *P) {  // value and tag, rows of whole slices
+  return 2 * (cg_mixed(P) ? 4 : 8) * (size_t)ceil_div(P->n, 32) * 32;
+}
+
+// Slots and published elements without an epoch, epoch 0, no error: the state before
+// the first launch, and after one that gave up (its epoch is not stored, so the next
+// launch would take that run's slots and elements for its own).
+static bsp_status fused_reset(bsp_cg_plan_s *P, cudaStream_t s) {
+  BSP_CUDA(cudaMemsetAsync(P->slots, 0, 2 * kFusedMaxCtas * sizeof(CgSlot), s));
+  BSP_CUDA(cudaMemsetAsync(P->pub, 0, fused_pub_bytes(P), s));
+  BSP_CUDA(cudaMemsetAsync(P->sc + 8, 0, 2 * sizeof(double), s));
+  return BSP_OK;
+}
+
 // Sets up the fused iteration where it applies: no preconditioner, one CTA per
 // SM whose share of the vectors fits in shared memory, strictly ascending columns
 // in every row, and at most kFusedDiags distinct diagonals that the rows fill by
@@ -1575,13 +1594,16 @@ static bsp_status fused_setup(bsp_cg_plan_s *P, cudaStream_t s) {
   if ((int64_t)occ * sms < ctas) return BSP_OK;
   // an optimisation: without room for its buffers the two kernels run
   if (pool_malloc(&P->fused_val, L.vsz * kFusedDiags * (size_t)ns * 32, s) != cudaSuccess ||
-      pool_malloc(&P->pub, 2 * vt * (size_t)ns * 32, s) != cudaSuccess ||
+      pool_malloc(&P->pub, fused_pub_bytes(P), s) != cudaSuccess ||
       dalloc(&P->slots, 2 * kFusedMaxCtas, s) != BSP_OK) {
     cudaGetLastError();
+    clear_error();
+    if (P->fused_val) pool_free(P->fused_val, s);
+    if (P->pub) pool_free(P->pub, s);
+    P->fused_val = P->pub = nullptr;
     return BSP_OK;
   }
-  BSP_CUDA(cudaMemsetAsync(P->slots, 0, 2 * kFusedMaxCtas * sizeof(CgSlot), s));
-  BSP_CUDA(cudaMemsetAsync(P->pub, 0, 2 * vt * (size_t)ns * 32, s));
+  BSP_TRY(fused_reset(P, s));
   const int64_t gf = std::min<int64_t>(ceil_div(P->n, 256), (int64_t)sm_count() * 32);
   void *args[] = {&P->n, &P->rowPtr, &P->colIdx, &P->val, &P->exps, &P->fused_diags, &P->fused_val};
   BSP_CUDA(cudaLaunchKernel(L.fill, dim3((unsigned)gf), dim3(256), args, 0, s));
@@ -1595,7 +1617,7 @@ static bsp_status fused_chunk(bsp_cg_plan_s *P, cudaStream_t s) {
   int iters = P->opt.check_every, npart = P->grid;
   double *epoch = P->sc + 9, *err = P->sc + 8;
   void *args[] = {&P->n,   &P->fused_val, &P->fused_diags, &P->exps, &P->x,     &P->r,  &P->p[0], &P->pub,
-                  &P->part_rr, &npart,    &P->sc,          &iters,   &P->slots, &epoch, &err};
+                  &P->part_rr, &npart,    &P->sc,          &iters,   &P->slots, &epoch, &err, &P->fused_polls};
   // One fused launch at a time on a device, whatever the streams and threads:
   // two grids that wait for their own CTAs must not share the SMs by halves.
   static std::mutex turn;
@@ -1635,7 +1657,10 @@ static bsp_status read_scalars(bsp_cg_plan_s *P, cudaStream_t s) {
   BSP_CUDA(cudaStreamSynchronize(s));
   int32_t err = 0;
   memcpy(&err, P->h_sc + 8, sizeof(err));
-  if (err) BSP_FAIL(BSP_ERR_TIMEOUT, "a bounded wait of the fused CG iteration gave up");
+  if (err) {
+    BSP_TRY(fused_reset(P, s));
+    BSP_FAIL(BSP_ERR_TIMEOUT, "a bounded wait of the fused CG iteration gave up");
+  }
   return BSP_OK;
 }
 
@@ -2032,6 +2057,20 @@ void cg_plan_view(const bsp_cg_plan_s *P, CgPlanView *v) {
 }
 }  // namespace bsp
 
+extern "C" bsp_status bsp_cg_fused_ctas(bsp_cg_plan P, int32_t *ctas) {
+  clear_error();
+  BSP_CHECK_ARG(P && ctas, "null argument");
+  *ctas = P->fused_ctas;
+  return BSP_OK;
+}
+
+extern "C" bsp_status bsp_cg_set_wait_limit(bsp_cg_plan P, uint32_t polls) {
+  clear_error();
+  BSP_CHECK_ARG(P && polls > 0, "null plan or a limit of 0");
+  P->fused_polls = polls;
+  return BSP_OK;
+}
+
 extern "C" bsp_status bsp_cg_solve(bsp_cg_plan P, const double *b, double *x, bsp_cg_result *res,
                                    bsp_stream_t stream) {
   clear_error();
@@ -2041,7 +2080,14 @@ extern "C" bsp_status bsp_cg_solve(bsp_cg_plan P, const double *b, double *x, bs
   const int g = P->grid;
   const bool mixed = cg_mixed(P);
   const size_t vt = mixed ? 4 : 8;
-  cudaEvent_t e0, e1;
+  struct Events {  // destroyed on every way out
+    cudaEvent_t e[2] = {nullptr, nullptr};
+    ~Events() {
+      for (cudaEvent_t v : e)
+        if (v) cudaEventDestroy(v);
+    }
+  } ev;
+  cudaEvent_t &e0 = ev.e[0], &e1 = ev.e[1];
   BSP_CUDA(cudaEventCreate(&e0));
   BSP_CUDA(cudaEventCreate(&e1));
   BSP_CUDA(cudaEventRecord(e0, s));
@@ -2150,8 +2196,6 @@ extern "C" bsp_status bsp_cg_solve(bsp_cg_plan P, const double *b, double *x, bs
   BSP_TRY(read_scalars(P, s));
   float ms = 0;
   cudaEventElapsedTime(&ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   res->iterations = (int32_t)iters;
   res->reliable_updates = updates;
   res->outer_steps = outer;

@@ -627,9 +627,9 @@ typedef struct {
   int32_t mode;          /* bsp_cg_mode */
   double tol;            /* relative residual target (1e-10) */
   int32_t max_iters;     /* CG iteration budget */
-  int32_t check_every;   /* iterations per CUDA graph between host checks (rounded up to even) */
+  int32_t check_every;   /* iterations per graph or fused launch between host checks (rounded up to even) */
   double reliable_delta; /* mixed modes: residual drop that triggers an FP64 update (0.1) */
-  int32_t use_graphs;    /* 1: replay captured iteration chunks */
+  int32_t use_graphs;    /* 1: replay captured iteration chunks (the fused form, below, has none) */
   int32_t precond;       /* bsp_cg_precond */
   int32_t precond_block; /* BLOCK_JACOBI: rows per diagonal block, 4 or 8 */
   int32_t refine;        /* bsp_cg_refine (mixed modes) */
@@ -662,6 +662,16 @@ bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPtr,
 bsp_status bsp_cg_solve(bsp_cg_plan plan, const double *b, double *x,
                         bsp_cg_result *res, bsp_stream_t stream);
 bsp_status bsp_cg_destroy(bsp_cg_plan plan);
+/* Without a preconditioner, a matrix of at most 8 diagonals with ascending
+ * columns whose vectors fit the SMs' shared memory (16 bytes a row in the mixed
+ * modes, 32 in FP64) runs check_every iterations in one cooperative launch of
+ * *ctas CTAs; *ctas = 0: two kernels per iteration.  That launch needs its SMs all
+ * at once (it fails on a stream confined to fewer), so fused solves of a device
+ * take turns, whatever their streams.  Its CTAs wait for one another, `polls` reads
+ * at most per wait (the default takes seconds); a wait that runs out ends the solve
+ * with BSP_ERR_TIMEOUT, x as it was and the plan ready for another solve. */
+bsp_status bsp_cg_fused_ctas(bsp_cg_plan plan, int32_t *ctas);
+bsp_status bsp_cg_set_wait_limit(bsp_cg_plan plan, uint32_t polls);
 /* k right-hand sides at once: A X = B with B, X device arrays, row-major with
  * leading dimensions ldb, ldx >= k (row i, column j at B[i*ldb + j]); X holds
  * the initial guesses on entry.  Every column runs its own FP64 CG (same

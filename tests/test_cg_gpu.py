@@ -223,3 +223,43 @@ def test_cg_rows_with_repeated_or_unsorted_columns(cuda, diags, kind, mode):
     S.close()
     assert res["converged"] == 1
     assert pyoracle.rel_residual(A.rowptr, A.colidx, A.values, b, x.cpu().numpy()) <= 2e-10
+
+
+@pytest.mark.parametrize("mode", ["fp64", "f16"])
+def test_cg_fused_wait_that_runs_out(cuda, mode):
+    """With one read per wait the fused launch gives up: the solve returns the
+    status, leaves x alone, and the plan solves again to the same bits."""
+    import torch
+    A = bsp.gen_poisson3d(48)
+    rp, ci, va, b = _dev(cuda, A.rowptr, A.colidx, A.values, bsp.gen_uniform(A.rows, 17))
+    S = bsp.CgSolver(rp, ci, va, mode=mode, tol=1e-10)
+    assert S.fused_ctas > 1
+    want, _ = S.solve(b)
+    for _ in range(2):
+        S.set_wait_limit(1)
+        x = torch.full_like(b, 0.25)
+        with pytest.raises(bsp.BspError) as e:
+            S.solve(b, x)
+        assert e.value.status == bsp._lib.BSP_ERR_TIMEOUT
+        assert torch.all(x == 0.25)
+        S.set_wait_limit(1 << 23)
+        got, res = S.solve(b)
+        assert res["converged"] == 1 and torch.equal(got, want)
+    with pytest.raises(bsp.BspError):
+        S.set_wait_limit(0)
+    S.close()
+
+
+@pytest.mark.parametrize("mode", ["fp64", "f16"])
+def test_cg_two_kernels_without_graphs_match(cuda, mode):
+    """use_graphs changes nothing in the two-kernel iteration (9 diagonals)."""
+    A = _banded(20000, [1, 50, 700, 3000], 3)
+    rp, ci, va, b = _dev(cuda, A.rowptr, A.colidx, A.values, bsp.gen_uniform(A.rows, 18))
+    out = []
+    for graphs in (True, False):
+        S = bsp.CgSolver(rp, ci, va, mode=mode, use_graphs=graphs)
+        assert S.fused_ctas == 0
+        x, res = S.solve(b)
+        out.append((x.cpu().numpy(), res["iterations"]))
+        S.close()
+    assert out[0][1] == out[1][1] and np.array_equal(out[0][0], out[1][0])
