@@ -1348,7 +1348,7 @@ struct bsp_cg_plan_s {
   uint32_t fused_polls = bsp::kFusedPolls;
   cudaGraphExec_t graph = nullptr;
   cudaStream_t graph_stream = nullptr;
-  int64_t bytes_iter = 0, bytes_residual = 0;
+  int64_t bytes_iter = 0, bytes_chunk = 0, bytes_residual = 0;
 };
 
 namespace bsp {
@@ -2023,13 +2023,19 @@ extern "C" bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPt
   }
 #undef BSP_CG_TRY
 #undef BSP_CG_CUDA
-  // algorithmic bytes: kernel A reads the matrix, r and p_prev (own rows;
-  // gathers counted once) and writes p and q; kernel B reads p, q, x, r and
-  // writes x, r.
-  // Preconditioned: the update kernel also reads M^{-1} and writes z.
-  P->bytes_iter = mat_bytes + (mixed || P->sell64 || P->fused_ctas ? 0 : 4 * ((int64_t)n + 1)) + 10 * (int64_t)vt * n;
-  if (P->prec_bs)
-    P->bytes_iter += (int64_t)vt * (ceil_div(n, P->prec_bs) * P->prec_bs * P->prec_bs + (int64_t)n);
+  // algorithmic bytes.  Two kernels: A reads the matrix, r and p_prev (own rows;
+  // gathers counted once) and writes p and q; B reads p, q, x, r and writes x, r.
+  // Preconditioned: the update kernel also reads M^{-1} and writes z.  Fused: the
+  // diagonals and the published p (value and tag, written and read once) per
+  // iteration, x, r and p in and out once per chunk; the rest stays on the SMs.
+  if (P->fused_ctas) {
+    P->bytes_iter = mat_bytes + 2 * (int64_t)fused_pub_bytes(P);
+    P->bytes_chunk = 6 * (int64_t)vt * n;
+  } else {
+    P->bytes_iter = mat_bytes + (mixed || P->sell64 ? 0 : 4 * ((int64_t)n + 1)) + 10 * (int64_t)vt * n;
+    if (P->prec_bs)
+      P->bytes_iter += (int64_t)vt * (ceil_div(n, P->prec_bs) * P->prec_bs * P->prec_bs + (int64_t)n);
+  }
   P->bytes_residual = (int64_t)nnz * 12 + 4 * ((int64_t)n + 1) + 3 * 8 * (int64_t)n;
   // flexible outer step: F1 8n+8n+8n, F2 24n, F3 matrix + 4(n+1) + 32n, F4 52n
   P->bytes_outer = (int64_t)nnz * 12 + 4 * ((int64_t)n + 1) + 132 * (int64_t)n;
@@ -2202,7 +2208,8 @@ extern "C" bsp_status bsp_cg_solve(bsp_cg_plan P, const double *b, double *x, bs
   res->seconds = ms * 1e-3;
   res->rel_residual = bb > 0 ? sqrt(P->h_sc[2] / bb) : 0.0;
   res->converged = res->rel_residual <= P->opt.tol;
-  res->bytes_moved = residuals * P->bytes_residual + iters * P->bytes_iter + (int64_t)outer * P->bytes_outer;
+  res->bytes_moved = residuals * P->bytes_residual + iters * P->bytes_iter +
+                     iters / P->opt.check_every * P->bytes_chunk + (int64_t)outer * P->bytes_outer;
   res->delta16 = P->delta16 ? 1 : 0;
   if (!res->converged) {
     set_error("CG stopped at relative residual " + std::to_string(res->rel_residual) +

@@ -641,8 +641,10 @@ typedef struct {
   double rel_residual;      /* final ||b - A x|| / ||b|| in FP64 */
   double seconds;           /* device time of the solve (CUDA events) */
   int32_t converged;
-  int64_t bytes_moved;      /* algorithmic bytes of all kernels */
-  int32_t delta16;          /* int16 column offsets were used */
+  int64_t bytes_moved;      /* algorithmic bytes of all kernels (fused form: what reaches L2, on a
+                               small enough matrix all of it; not DRAM traffic) */
+  int32_t delta16;          /* every |col - row| fits int16: column offsets are (or, in the fused
+                               form, which stores none, would be) 16 bits wide */
   int32_t outer_steps;      /* mixed modes: outer flexible steps taken (0 when
                                residual replacement sufficed) */
 } bsp_cg_result;

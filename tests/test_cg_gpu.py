@@ -263,3 +263,21 @@ def test_cg_two_kernels_without_graphs_match(cuda, mode):
         out.append((x.cpu().numpy(), res["iterations"]))
         S.close()
     assert out[0][1] == out[1][1] and np.array_equal(out[0][0], out[1][0])
+
+
+@pytest.mark.parametrize("mode,value,vector", [("fp64", 8, 8), ("f32", 4, 4), ("f16", 2, 4)])
+def test_cg_fused_bytes_leave_out_what_stays_on_the_sms(cuda, mode, value, vector):
+    """bytes_moved of a fused solve: per iteration 8 diagonals, an exponent per row
+    in FP16, and p published with its tag, written and read; per chunk x, r and p in
+    and out; per FP64 residual the CSR matrix and three vectors."""
+    A = bsp.gen_poisson3d(16)
+    n = A.rows
+    rp, ci, va, b = _dev(cuda, A.rowptr, A.colidx, A.values, bsp.gen_uniform(n, 19))
+    S = bsp.CgSolver(rp, ci, va, mode=mode, check_every=8)
+    assert S.fused_ctas > 0
+    _, r = S.solve(b)
+    S.close()
+    per_iter = n * (8 * value + (value == 2) + 4 * vector)
+    residuals = r["reliable_updates"] + 2
+    assert r["bytes_moved"] == r["iterations"] * per_iter + r["iterations"] // 8 * 6 * vector * n + \
+        residuals * (12 * A.nnz + 4 * (n + 1) + 24 * n)
