@@ -281,3 +281,50 @@ def test_cg_fused_bytes_leave_out_what_stays_on_the_sms(cuda, mode, value, vecto
     residuals = r["reliable_updates"] + 2
     assert r["bytes_moved"] == r["iterations"] * per_iter + r["iterations"] // 8 * 6 * vector * n + \
         residuals * (12 * A.nnz + 4 * (n + 1) + 24 * n)
+
+
+# the last size whose vectors fit 148 SMs next to the kernel's own shared memory (453
+# slices of 512 bytes per CTA in the mixed modes, 226 of 1024 in FP64), with the last
+# slice ragged, and the first size past it; the iterates of both forms agree
+@pytest.mark.parametrize("mode,n", [("f32", 2145408), ("f16", 2145408), ("bf16", 2145395), ("f32", 2145409),
+                                    ("fp64", 1070336), ("fp64", 1070325), ("fp64", 1070337)])
+def test_cg_fused_up_to_the_last_size(cuda, mode, n):
+    import torch
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes of 148 SMs")
+    A = _banded(n, [1, 1466], n)
+    b = bsp.gen_uniform(n, 15)
+    rp, ci, va, bb = _dev(cuda, A.rowptr, A.colidx, A.values, b)
+    S = bsp.CgSolver(rp, ci, va, mode=mode, tol=1e-10)
+    assert S.fused_ctas == (0 if n in (2145409, 1070337) else 148)
+    x, res = S.solve(bb)
+    S.close()
+    assert res["converged"] == 1
+    assert pyoracle.rel_residual(A.rowptr, A.colidx, A.values, b, x.cpu().numpy()) <= 2e-10
+    if n not in (2145409, 1070337):            # the other form: 8192 rows more, uncoupled from the rest
+        R = bsp.HostCSR(n + 8192, n + 8192, np.append(A.rowptr, A.rowptr[-1] + np.arange(1, 8193)).astype(np.int32),
+                        np.append(A.colidx, np.arange(n, n + 8192)).astype(np.int32),
+                        np.append(A.values, np.ones(8192)))
+        rp, ci, va, b2 = _dev(cuda, R.rowptr, R.colidx, R.values, np.append(b, np.zeros(8192)))
+        S = bsp.CgSolver(rp, ci, va, mode=mode, tol=1e-10)
+        assert S.fused_ctas == 0
+        y, res2 = S.solve(b2)
+        S.close()
+        assert res2["iterations"] == res["iterations"] and torch.all(y[n:] == 0)
+        # two residuals of 1e-10, eigenvalues between 0.5 and 2 * 4 + 0.5
+        assert float((y[:n] - x).norm() / x.norm()) <= 2e-10 * 17
+
+
+@pytest.mark.parametrize("n,diags,fused", [(31, [1], True), (5000, [1, 70], True), (200003, [2, 450, 45000], True),
+                                           (20000, [1, 50, 700, 3000], False)])
+def test_cg_form_that_runs(cuda, n, diags, fused):
+    """Which matrices the fused iteration takes, and none with a preconditioner."""
+    A = _banded(n, diags, n)
+    rp, ci, va = _dev(cuda, A.rowptr, A.colidx, A.values)
+    for mode in ("fp64", "f32", "f16", "bf16"):
+        S = bsp.CgSolver(rp, ci, va, mode=mode)
+        assert (S.fused_ctas > 0) == fused
+        S.close()
+    S = bsp.CgSolver(rp, ci, va, mode="f16", precond="jacobi")
+    assert S.fused_ctas == 0
+    S.close()
