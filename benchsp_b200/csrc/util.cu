@@ -1,6 +1,7 @@
 // Error state, small C-ABI utilities and a device exclusive scan used by the
 // format conversions (the reference uses thrust::exclusive_scan for the same
 // steps: src/amgT.cu:1008,1043,1190 and src/csrspmv.cu:157).
+#include <map>
 #include <mutex>
 
 #include <cuda.h>
@@ -23,37 +24,49 @@ void clear_error() { g_last_error.clear(); }
 // 6.4 ms.  Here the release threshold follows the bytes in use plus
 // kPoolIdleShare of the device's memory (2.8 GB of 180), so that much idle
 // memory at most is kept, whatever was freed; bsp_pool_trim gives it back, and
-// so does an allocation that finds no room.  Pools of a context that has gone
-// are not used again.  Calls inside a stream capture keep the default pool.
+// so does an allocation that finds no room.  The bytes in use are read and the
+// threshold set under one lock, for the pool that a freed pointer came from.  Pools of
+// a context that has gone are not used again.  Calls inside a stream capture keep the
+// default pool.
 constexpr uint64_t kPoolIdleShare = 64;       // 1 / 64 of the device's memory
 constexpr size_t kPoolTrack = 1 << 20;        // allocations that move the threshold
-constexpr int kPoolDevices = 64;
 
 namespace {
 struct DevicePool {
   cudaMemPool_t pool = nullptr;
-  unsigned long long context = 0;
   uint64_t idle = 0;
 };
 std::mutex g_pool_mutex;
-DevicePool g_pools[kPoolDevices];
+std::map<unsigned long long, DevicePool> &g_pools = *new std::map<unsigned long long, DevicePool>;  // by context
+
+template <typename Fn>
+Fn driver_entry(const char *name) {
+  void *p = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+    p = nullptr;
+  return reinterpret_cast<Fn>(p);
+}
 }  // namespace
 
 unsigned long long context_id() {
   using IdFn = CUresult (*)(CUcontext, unsigned long long *);
-  static const IdFn fn = [] {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      p = nullptr;
-    return reinterpret_cast<IdFn>(p);
-  }();
+  static const IdFn fn = driver_entry<IdFn>("cuCtxGetId");
   unsigned long long id = 0;
   return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
 }
 
 namespace {
+// The memory pool that p was allocated from; null if it has none or is unknown.
+cudaMemPool_t pool_of(const void *p) {
+  using AttrFn = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+  static const AttrFn fn = driver_entry<AttrFn>("cuPointerGetAttribute");
+  cudaMemPool_t pool = nullptr;
+  return fn && fn(&pool, CU_POINTER_ATTRIBUTE_MEMPOOL_HANDLE, reinterpret_cast<CUdeviceptr>(p)) == CUDA_SUCCESS
+             ? pool
+             : nullptr;
+}
+
 // The pool of the stream's device, or an empty one where the default pool serves.
 DevicePool device_pool(cudaStream_t s) {
   int dev = 0, cur = 0;
@@ -65,38 +78,44 @@ DevicePool device_pool(cudaStream_t s) {
   }
   dev = cur;
   const bool named = s && s != cudaStreamLegacy && s != cudaStreamPerThread;
-  if ((named && cudaStreamGetDevice(s, &dev) != cudaSuccess) || dev != cur || dev >= kPoolDevices) {
+  if ((named && cudaStreamGetDevice(s, &dev) != cudaSuccess) || dev != cur) {
     cudaGetLastError();
     return {};
   }
   const unsigned long long ctx = context_id();
   if (!ctx) return {};
   std::lock_guard<std::mutex> lock(g_pool_mutex);
-  DevicePool &d = g_pools[dev];
-  if (d.context != ctx) {
-    d = {};
-    size_t free_b = 0, total = 0;
-    cudaMemPoolProps props{};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    if (cudaMemGetInfo(&free_b, &total) != cudaSuccess || cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) {
-      cudaGetLastError();
-      d.pool = nullptr;
-    }
-    d.idle = total / kPoolIdleShare;
-    d.context = ctx;
+  const auto found = g_pools.find(ctx);
+  if (found != g_pools.end()) return found->second;
+  DevicePool d;
+  size_t free_b = 0, total = 0;
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  if (cudaMemGetInfo(&free_b, &total) != cudaSuccess || cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) {
+    cudaGetLastError();
+    d.pool = nullptr;
   }
+  d.idle = total / kPoolIdleShare;
+  g_pools[ctx] = d;
   return d;
 }
 
-void move_threshold(const DevicePool &d) {
-  uint64_t used = 0;
-  if (cudaMemPoolGetAttribute(d.pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess) {
-    used += d.idle;
-    cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &used);
+// Release threshold of `pool`, if it is one of the library's: the bytes in use now
+// and the idle share.  Locked, or a thread that read them before another one's free
+// would set the threshold that it read last.
+void move_threshold(cudaMemPool_t pool) {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  for (const auto &e : g_pools) {
+    if (!pool || e.second.pool != pool) continue;
+    uint64_t used = 0;
+    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess) {
+      used += e.second.idle;
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &used);
+    }
+    cudaGetLastError();
   }
-  cudaGetLastError();
 }
 }  // namespace
 
@@ -109,16 +128,14 @@ cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t s) {
     cudaMemPoolTrimTo(d.pool, 0);
     e = cudaMallocFromPoolAsync(p, bytes, d.pool, s);
   }
-  if (e == cudaSuccess && bytes >= kPoolTrack) move_threshold(d);
+  if (e == cudaSuccess && bytes >= kPoolTrack) move_threshold(d.pool);
   return e;
 }
 
 cudaError_t pool_free(void *p, cudaStream_t s) {
+  const cudaMemPool_t pool = pool_of(p);
   const cudaError_t e = cudaFreeAsync(p, s);
-  if (e == cudaSuccess) {
-    const DevicePool d = device_pool(s);
-    if (d.pool) move_threshold(d);
-  }
+  if (e == cudaSuccess) move_threshold(pool);
   return e;
 }
 

@@ -62,3 +62,44 @@ def test_streams_and_threads_share_the_pool(cuda):
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_threads_leave_no_more_than_the_bound(cuda):
+    """Matrices made and freed by several threads, the frees on other streams than
+    the allocations: what the pool keeps at the end is bounded as for one thread."""
+    import torch
+    A = bsp.gen_stencil27(40, 4, 5)
+    rp, ci, va = A.to_device()
+    _lib.check(_lib.lib().bsp_pool_trim())
+    torch.cuda.synchronize()
+    base, total = torch.cuda.mem_get_info()
+    made, lock = [], threading.Lock()
+    start = threading.Barrier(4)
+
+    def work():
+        s = torch.cuda.Stream()
+        start.wait()
+        with torch.cuda.stream(s):
+            for k in range(24):
+                M = bsp.csr2bsr(rp, ci, va, rows=A.rows, cols=A.cols, bs=8 if k % 2 else 4)
+                s.synchronize()
+                with lock:
+                    made.append(M)
+                    M = made.pop(0) if len(made) > 12 else None
+                if M:
+                    M.free()
+
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    rest = [threading.Thread(target=M.free) for M in made]
+    for t in rest:
+        t.start()
+    for t in rest:
+        t.join()
+    assert _held(base) <= total // 64 + SLACK
+    _lib.check(_lib.lib().bsp_pool_trim())
+    assert _held(base) <= SLACK
