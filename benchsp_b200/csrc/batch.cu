@@ -794,6 +794,7 @@ struct bsp_batch_plan_s {
   // batched list (long segments first) and per-matrix lists
   BatchItem *d_items = nullptr, *d_items_sep = nullptr;
   bool row32 = false;  // 8 vectors: every x and y is 32-byte aligned
+  int32_t off32 = 0;   // matrices where one is not
   int64_t nitems = 0;
   std::vector<int64_t> sep_off;  // [count+1] offsets into d_items_sep
   LongRow *d_longs = nullptr;
@@ -1295,7 +1296,8 @@ extern "C" bsp_status bsp_batch_create(int32_t count, const bsp_batch_mat *mats,
     P->total_nnz += A.nnz;
     P->lanes[m] = model_lanes(L, o.long_row_nnz, nrhs);
   }
-  P->row32 = std::all_of(mats, mats + count, rows_aligned);
+  P->off32 = count - (int32_t)std::count_if(mats, mats + count, rows_aligned);
+  P->row32 = P->off32 == 0;
   P->dm.resize(count);
   for (int32_t m = 0; m < count; ++m)
     P->dm[m] = {mats[m].rowPtr, mats[m].colIdx, mats[m].values, mats[m].x, mats[m].y, mats[m].rows, mats[m].cols,
@@ -1390,16 +1392,18 @@ extern "C" bsp_status bsp_batch_set_vectors(bsp_batch_plan P, int32_t m, const v
   const bsp_batch_mat &A = P->host_mats[m];
   BSP_CHECK_ARG((A.cols == 0 || x) && (A.rows == 0 || y), "null vector");
   cudaStream_t s = as_stream(stream);
+  P->off32 += rows_aligned(A);
   P->host_mats[m].x = x;
   P->host_mats[m].y = y;
+  P->off32 -= rows_aligned(A);
   P->dm[m].x = x;
   P->dm[m].y = y;
   const BatchMatDev d = P->dm[m];
   // the descriptor is read by the kernel: update it in stream order
   BSP_CUDA(cudaMemcpyAsync(P->d_mats + m, &d, sizeof(d), cudaMemcpyHostToDevice, s));
   BSP_CUDA(cudaStreamSynchronize(s));
-  if (P->nrhs == 8 && P->row32 && !rows_aligned(P->host_mats[m])) {  // 16-byte pieces from here on
-    P->row32 = false;
+  if (P->nrhs == 8 && P->row32 != (P->off32 == 0)) {  // the other kernel from here on
+    P->row32 = P->off32 == 0;
     BSP_TRY(capture(P));
   }
   return BSP_OK;

@@ -326,3 +326,34 @@ def test_batch_sell_slices_with_and_without_x_window(cuda, dtype):
     for a, d in zip(first, dev):
         assert torch.equal(a, d[4])
     P.close()
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_batch_8rhs_returns_to_wide_accesses(cuda, graph):
+    """Once set_vectors has made every vector 32-byte aligned again the plan runs
+    the kernel it started with: the same bits (long rows are summed in another order
+    by the 16-byte one)."""
+    import torch
+    mats = _small_batch(37, count=9)
+    dev, _ = _upload(cuda, mats, "f32", 8, 10)
+    P = bsp.BatchPlan(dev, nrhs=8, use_graph=graph)
+
+    def run():
+        for d in dev:
+            d[4].fill_(float("nan"))
+        P.run()
+        torch.cuda.synchronize()
+        return [d[4].clone() for d in dev]
+
+    def off(t):
+        return torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)[4:4 + t.numel()].view(t.shape).copy_(t)
+
+    wide = run()
+    for m in (1, 6):
+        P.set_vectors(m, off(dev[m][3]), dev[m][4])
+    narrow = run()
+    assert not all(torch.equal(u, v) for u, v in zip(wide, narrow))
+    for m in (1, 6):
+        P.set_vectors(m, dev[m][3], dev[m][4])
+    assert all(torch.equal(u, v) for u, v in zip(wide, run()))
+    P.close()
