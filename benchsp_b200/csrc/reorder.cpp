@@ -346,16 +346,34 @@ int64_t count_tiles(int32_t n, const int32_t *rp, const int32_t *ci, const int32
 // measurements of the SMaT and CSR SpMM at N = 128 (dense-tile and
 // row-shuffled 524,288-row matrices, power-law graph): the persistent
 // tcgen05 kernel 163 us for 262,144 tiles at N = 128 (4.9e-12 s per
-// tile-column, 64-column slabs below N = 128), the grouped CSR kernel
-// 1.93 ms for 67.1M nonzeros (2.3e-13 s per nonzero-column).
+// tile-column, 64-column slabs below N = 128).
 constexpr double kTileColSecTc = 4.9e-12;
-constexpr double kNnzColSecCsr = 2.3e-13;
+// CSR: the planned product (bsp_spmm_csr_planned, slab engine), FP16 at N = 128:
+// 725 us for 45.8M nonzeros in 442,368 rows (column-permuted 27-point stencil 48^3 x
+// 4 dof), 588 for 33.6M in 262,144 (row-shuffled tiles), 146 for 5.0M in as many, 270
+// for 12M in 300,000 (random columns), 414 for 18M in 524,288 (power-law graph); the
+// model gives 788, 561, 141, 254 and 399.  A pass takes 4 to 32 lanes of 8 columns,
+// so N counts as the pieces' next power of two up to 256, and 32 columns take 0.75 to
+// 0.96 of the time of 64.  Without a plan bsp_spmm_csr takes 1.2 to 1.9 times as long.
+constexpr double kNnzColSecCsr = 1.15e-13;
+constexpr double kRowColSecCsr = 2.0e-12;
 // Gathered-tile tcgen05 kernel (bsp_gtile): 366,808 chunks of a
 // column-permuted 27-point stencil (48^3 x 4 dof) in 0.668 ms at N = 128 and
 // 1.33 ms at N = 256, 2.01M chunks of a power-law graph in 4.30 ms at N = 128:
 // 1.45e-11 s per chunk-column; below N = 128 the slab is 64 columns and a
 // chunk took 1.2-1.5 ns at N = 32 (counted as 96 columns).
 constexpr double kChunkColSecGt = 1.45e-11;
+
+// Columns that the slab engine's passes over N columns count as.
+double csr_columns(int32_t N) {
+  double cols = 256.0 * (N / 256);
+  if (const int32_t rest = N % 256) {
+    int32_t c = 64;
+    while (c < rest) c <<= 1;
+    cols += rest <= 32 && N < 256 ? 56 : c;
+  }
+  return cols;
+}
 
 // Chunks of the gathered-tile form with A's rows in the order `perm` (null:
 // as given): every 16-row group's distinct columns, in chunks of 16, summed.
@@ -550,7 +568,7 @@ extern "C" bsp_status bsp_spmm_choose_host(int32_t rows, int32_t cols, int32_t n
     similarity_order(rows, cols, rowPtr, colIdx, 16, 16, perm);
     c.tiles_reordered = count_tiles(rows, rowPtr, colIdx, perm);
   }
-  c.est_seconds_csr = kNnzColSecCsr * N * (double)nnz;
+  c.est_seconds_csr = csr_columns(N) * (kNnzColSecCsr * nnz + kRowColSecCsr * rows);
   c.est_seconds_smat_given = smat_ok ? per_tile * (double)c.tiles_given : -1.0;
   c.est_seconds_smat_reordered = smat_ok && c.tiles_reordered >= 0 ? per_tile * (double)c.tiles_reordered : -1.0;
   // the gathered-tile kernel: N % 8 == 0, slabs of 64 or 128 C columns

@@ -745,11 +745,13 @@ bsp_status bsp_reorder_similarity_host(int32_t rows, int32_t cols, int32_t nnz,
  * of its gathered-tile form (16 distinct columns of a 16-row group) as given
  * and, when `perm` (rows entries) is not NULL, after bsp_reorder_similarity
  * (written to perm), and estimates each engine from B200 measurements
- * (SMaT time per tile, gathered-tile time per chunk, grouped CSR time per
- * nonzero, all per column of B).  engine = BSP_SPMM_ENGINE_SMAT or
+ * (SMaT time per tile, gathered-tile time per chunk, planned CSR time per
+ * nonzero and row, all per column of B).  engine = BSP_SPMM_ENGINE_SMAT or
  * BSP_SPMM_ENGINE_GTILE (build that matrix from the rows in perm order when
  * reorder = 1, and read row i of C as original row perm[i]; smat_path says
- * which tile path) or BSP_SPMM_ENGINE_CSR (bsp_spmm_csr on A as given).
+ * which tile path) or BSP_SPMM_ENGINE_CSR (A as given: a plan from
+ * bsp_spmm_plan_create and bsp_spmm_csr_planned, which the estimate is for; a single
+ * product without a plan, bsp_spmm_csr, takes up to twice as long).
  * SMaT needs N % 32 == 0, the gathered tiles N % 8 == 0; the estimates are
  * -1 where an engine does not apply.  Host code, a one-time decision per
  * matrix. */

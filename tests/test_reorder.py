@@ -267,3 +267,38 @@ def test_device_similarity_matches_host_and_densifies_tiles(cuda):
     assert np.allclose(Y1, Y0[perm.cpu().numpy()], rtol=1e-4, atol=1e-4)
     before.free()
     after.free()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", [64, 128])
+def test_spmm_choice_is_the_faster_engine(cuda, N):
+    """A column-permuted stencil of 2 dof (77 nonzeros per gathered chunk): the
+    planned CSR product and the gathered tiles are timed, and the choice takes no
+    more than a tenth longer than the other."""
+    import torch
+    A = _permute_columns(bsp.gen_stencil27(40, 2, 3), 5)
+    d, _ = bsp.choose_spmm_host(A, N, reorder=False)
+    assert 63 < A.nnz / d["chunks_given"] < 100
+    rp, ci, va = A.to_device()
+    B = torch.rand(A.cols, N, device=cuda).half()
+    C = torch.empty(A.rows, N, device=cuda)
+    P = bsp.SpmmPlan(rp, ci, va.half(), cols=A.cols)
+    G = bsp.GatherTileMatrix(A, "f16")
+
+    def best(f):
+        t = []
+        for _ in range(5):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            torch.cuda.synchronize()
+            e[0].record()
+            for _ in range(5):
+                f()
+            e[1].record()
+            torch.cuda.synchronize()
+            t.append(e[0].elapsed_time(e[1]))
+        return min(t)
+
+    times = {"csr": best(lambda: P.spmm(B, C)), "gtile": best(lambda: G.spmm(B, C))}
+    P.free()
+    G.free()
+    assert times[d["engine"]] <= 1.1 * min(times.values()), (d["engine"], times)
