@@ -1205,8 +1205,15 @@ def run_profile(args) -> None:
         y = torch.empty(A.rows, dtype=torch.float64, device=dev)
         for _ in range(reps):
             S.spmv(x, y)
-    elif w == "csr":   # CSR FP64 vector kernel, 2-D Laplacian 512x512 (21 MB; ncu replays cold-cache)
-        A = bsp.gen_laplace2d(512, 512)
+    elif w == "convert":   # CSR -> BSR 4x4, stencil 40^3 x 4 dof (26.6M nonzeros, 320 MB of CSR)
+        A, _ = make_matrix(40)
+        rp, ci, va = up(A.rowptr, A.colidx, A.values)
+        for _ in range(reps):
+            bsp.csr2bsr(rp, ci, va, rows=A.rows, cols=A.cols, bs=4).free()
+    elif w in ("csr", "csr_powerlaw"):
+        # CSR FP64 vector kernel: 2-D Laplacian 512x512 (21 MB; ncu replays cold-cache), or power-law
+        # rows, Zipf 2.0 capped at 10k, n = 2^20 (95 MB)
+        A = bsp.gen_laplace2d(512, 512) if w == "csr" else bsp.gen_powerlaw(1 << 20, 2.0, 10000, SEED + 13)
         rp, ci, va, x = up(A.rowptr, A.colidx, A.values, bsp.gen_uniform(A.cols, SEED + 10))
         y = torch.empty(A.rows, dtype=torch.float64, device=dev)
         for _ in range(reps):
@@ -1264,7 +1271,8 @@ def main():
                     "smaller values only for profiling captures)")
     ap.add_argument("--profile", choices=["dasp", "cg_fp64", "cg_f16", "spmm", "batch", "smat_tc", "smat_mma", "csr",
                                           "pcg_bj", "spmm_grouped", "cg_multi", "smat_tc_w64", "smat_tc_w128",
-                                          "bsr_scaled", "smat_tcp", "smat_tcp_w64", "batch8"],
+                                          "bsr_scaled", "smat_tcp", "smat_tcp_w64", "batch8", "convert",
+                                          "csr_powerlaw"],
                     help="a few calls of one workload's kernels (for ncu captures)")
     ap.add_argument("--pn", type=int, default=0, help="columns of B for the SpMM profile workloads "
                     "(default 128 for spmm, 256 for the smat ones)")

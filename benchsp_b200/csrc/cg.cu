@@ -321,8 +321,9 @@ __device__ __forceinline__ void vset(double2 &v, int k, double a) {
 // iteration (24^3 FP16: 9.1 -> 6 us).
 //
 // The cooperative launch makes all CTAs resident; every wait is bounded all the
-// same (the plan's limit, then *err is set and every CTA returns; fused_reset makes
-// the plan usable again).
+// same: kFusedPolls, or in an instantiation of its own (LIMITED) the plan's limit, which
+// as an argument of every launch cost registers (FP16 12.34 -> 12.73 ms a solve).  Then
+// *err is set and every CTA returns; fused_reset makes the plan usable again.
 constexpr int kFusedDiags = 8;
 constexpr int kFusedMaxCtas = 256;
 constexpr uint32_t kFusedPolls = 1u << 23;  // about 5 s
@@ -507,12 +508,13 @@ struct FusedGrid {
   int32_t *err;
   unsigned long long epoch;
   double *part, *sum;  // shared: a partial per warp, a sum per polling warp
-  int *dead;           // shared: 0 at the start, then the polls of one wait
+  int *dead;           // shared, 0 at the start
+  uint32_t limit;      // LIMITED: polls of a grid sum
 };
 
 __device__ __forceinline__ bool fused_give_up(FusedGrid &G, uint32_t polls) {
-  if (polls < (uint32_t)G.dead[1] && ((polls & 1023u) != 0 || *reinterpret_cast<volatile int32_t *>(G.err) == 0))
-    return false;
+  if ((polls & 1023u) != 0) return false;
+  if (polls < kFusedPolls && *reinterpret_cast<volatile int32_t *>(G.err) == 0) return false;
   atomicExch(G.err, 1);
   *reinterpret_cast<volatile int *>(G.dead) = 1;
   return true;
@@ -520,7 +522,7 @@ __device__ __forceinline__ bool fused_give_up(FusedGrid &G, uint32_t polls) {
 
 // Sum over all threads of the grid (the same bits in every thread); the CTA's
 // threads are in step on both sides.
-template <int WARPS>
+template <int WARPS, bool LIMITED>
 __device__ __forceinline__ double fused_sum(FusedGrid &G, double v) {
   constexpr int kPollWarps = kFusedMaxCtas / 32;
   static_assert(WARPS >= kPollWarps && WARPS <= 32, "a slot per thread, a partial per lane");
@@ -540,7 +542,7 @@ __device__ __forceinline__ double fused_sum(FusedGrid &G, double v) {
       for (uint32_t polls = 1;; ++polls) {
         const FusedWord16 t = ld_word16(row + threadIdx.x);
         got = __longlong_as_double((long long)t.lo);
-        if (t.hi == G.epoch || fused_give_up(G, polls)) break;
+        if (t.hi == G.epoch || fused_give_up(G, LIMITED && polls >= G.limit ? kFusedPolls : polls)) break;
       }
     got = warp_sum(got);
     if (lane == 0) G.sum[w] = got;
@@ -562,7 +564,7 @@ __device__ __forceinline__ void fused_dot(const Row &a, const VT (&p)[ND], VT &a
 }
 
 // ND: the diagonals looked at (the rest of the kFusedDiags are unused).
-template <typename V, typename VT, int ND, int THREADS>
+template <typename V, typename VT, int ND, int THREADS, bool LIMITED>
 __global__ void __launch_bounds__(THREADS, 1)
     cg_fused_kernel(int32_t n, const void *__restrict__ val, FusedDiags D, const int8_t *__restrict__ exps,
                     VT *__restrict__ x, VT *__restrict__ r, VT *__restrict__ p_state, typename FusedPub<VT>::T *pub,
@@ -575,7 +577,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   constexpr int kWarps = THREADS / 32;
   extern __shared__ __align__(16) unsigned char fused_smem[];
   __shared__ double part[kWarps], sum[kFusedMaxCtas / 32];
-  __shared__ int dead[2];
+  __shared__ int dead;
   const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // uniform
   const int64_t ns = ((int64_t)n + 31) / 32;
   const FusedSlices T(ns, blockIdx.x, gridDim.x);
@@ -585,11 +587,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   VT *sx = reinterpret_cast<VT *>(fused_smem), *sr = sx + cap, *sp = sr + cap, *sq = sp + cap;
   const uint32_t sp_base = (uint32_t)__cvta_generic_to_shared(sp);
   typename Pub::T *pub0 = pub + row0;
-  FusedGrid G{slots, err, *epoch_mem, part, sum, dead};
-  if (threadIdx.x == 0) {
-    dead[0] = 0;
-    dead[1] = (int)limit;
-  }
+  FusedGrid G{slots, err, *epoch_mem, part, sum, &dead, limit};
+  if (threadIdx.x == 0) dead = 0;
   for (int32_t i = threadIdx.x; i < S * 32; i += THREADS) {  // padding rows stay 0
     const bool in = i < nloc;
     sx[i] = in ? x[row0 + i] : VT(0);
@@ -680,8 +679,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       sq[i] = acc;  // 0 in a padding row
       dot += (double)acc * (double)sp[i];
     }
-    const double pq = fused_sum<kWarps>(G, dot);
-    if (dead[0]) return;
+    const double pq = fused_sum<kWarps, LIMITED>(G, dot);
+    if (dead) return;
     const double alpha = (pq != 0.0 && rr != 0.0 && isfinite(pq)) ? rr / pq : 0.0;
     const VT al = (VT)alpha;
     double s = 0.0;
@@ -699,8 +698,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       *reinterpret_cast<Vec *>(sr + i) = rv;
     }
     rr_prev = rr;
-    rr = fused_sum<kWarps>(G, s);
-    if (dead[0]) return;
+    rr = fused_sum<kWarps, LIMITED>(G, s);
+    if (dead) return;
   }
   for (int32_t i = threadIdx.x; i < nloc; i += THREADS) {
     x[row0 + i] = sx[i];
@@ -1513,20 +1512,39 @@ struct FusedLaunch {
   size_t vsz;  // bytes of a stored value
 };
 template <typename V, typename VT, int THREADS>
-static FusedLaunch fused_for(int nd) {
-  const void *k = nd <= 5   ? (const void *)cg_fused_kernel<V, VT, 5, THREADS>
-                  : nd <= 7 ? (const void *)cg_fused_kernel<V, VT, 7, THREADS>
-                            : (const void *)cg_fused_kernel<V, VT, 8, THREADS>;
+static FusedLaunch fused_for(const bsp_cg_plan_s *P) {
+  const int nd = P->fused_nd;
+  const void *k;
+  if (P->fused_polls < kFusedPolls)
+    k = nd <= 5   ? (const void *)cg_fused_kernel<V, VT, 5, THREADS, true>
+        : nd <= 7 ? (const void *)cg_fused_kernel<V, VT, 7, THREADS, true>
+                  : (const void *)cg_fused_kernel<V, VT, 8, THREADS, true>;
+  else
+    k = nd <= 5   ? (const void *)cg_fused_kernel<V, VT, 5, THREADS, false>
+        : nd <= 7 ? (const void *)cg_fused_kernel<V, VT, 7, THREADS, false>
+                  : (const void *)cg_fused_kernel<V, VT, 8, THREADS, false>;
   return {k, (const void *)fused_fill_kernel<V, sizeof(V) == 2>, THREADS, sizeof(V)};
 }
 
 static FusedLaunch fused_launch(const bsp_cg_plan_s *P) {
   switch (P->opt.mode) {
-    case BSP_CG_FP64: return fused_for<double, double, kFusedThreads64>(P->fused_nd);
-    case BSP_CG_MIXED_F32: return fused_for<float, float, kFusedThreads32>(P->fused_nd);
-    case BSP_CG_MIXED_F16: return fused_for<__half, float, kFusedThreads32>(P->fused_nd);
-    default: return fused_for<__nv_bfloat16, float, kFusedThreads32>(P->fused_nd);
+    case BSP_CG_FP64: return fused_for<double, double, kFusedThreads64>(P);
+    case BSP_CG_MIXED_F32: return fused_for<float, float, kFusedThreads32>(P);
+    case BSP_CG_MIXED_F16: return fused_for<__half, float, kFusedThreads32>(P);
+    default: return fused_for<__nv_bfloat16, float, kFusedThreads32>(P);
   }
+}
+
+// Lets the kernel have all the dynamic shared memory that its own leaves (*most).
+static bsp_status fused_allow_smem(const void *kernel, int64_t *most) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes fa{};
+  BSP_CUDA(cudaGetDevice(&dev));
+  BSP_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  BSP_CUDA(cudaFuncGetAttributes(&fa, kernel));
+  *most = optin - (int64_t)fa.sharedSizeBytes;
+  BSP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*most));
+  return BSP_OK;
 }
 
 static size_t fused_pub_bytes(const bsp_cg_plan_s *P) {  // value and tag, rows of whole slices
@@ -1585,11 +1603,9 @@ static bsp_status fused_setup(bsp_cg_plan_s *P, cudaStream_t s) {
   P->fused_diags.hi = *range.second;
   P->fused_nd = nd;
   const FusedLaunch L = fused_launch(P);
-  cudaFuncAttributes fa{};
-  BSP_CUDA(cudaFuncGetAttributes(&fa, L.kernel));
-  if (smem + (int64_t)fa.sharedSizeBytes > optin) return BSP_OK;
-  BSP_CUDA(cudaFuncSetAttribute(L.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                optin - (int)fa.sharedSizeBytes));
+  int64_t most = 0;
+  BSP_TRY(fused_allow_smem(L.kernel, &most));
+  if (smem > most) return BSP_OK;
   BSP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L.kernel, threads, (size_t)smem));
   if ((int64_t)occ * sms < ctas) return BSP_OK;
   // an optimisation: without room for its buffers the two kernels run
@@ -2074,7 +2090,8 @@ extern "C" bsp_status bsp_cg_set_wait_limit(bsp_cg_plan P, uint32_t polls) {
   clear_error();
   BSP_CHECK_ARG(P && polls > 0, "null plan or a limit of 0");
   P->fused_polls = polls;
-  return BSP_OK;
+  int64_t most = 0;
+  return P->fused_ctas ? fused_allow_smem(fused_launch(P).kernel, &most) : BSP_OK;
 }
 
 extern "C" bsp_status bsp_cg_solve(bsp_cg_plan P, const double *b, double *x, bsp_cg_result *res,

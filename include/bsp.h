@@ -669,9 +669,10 @@ bsp_status bsp_cg_destroy(bsp_cg_plan plan);
  * modes, 32 in FP64) runs check_every iterations in one cooperative launch of
  * *ctas CTAs; *ctas = 0: two kernels per iteration.  That launch needs its SMs all
  * at once (it fails on a stream confined to fewer), so fused solves of a device
- * take turns, whatever their streams.  Its CTAs wait for one another, `polls` reads
- * at most per wait (the default takes seconds); a wait that runs out ends the solve
- * with BSP_ERR_TIMEOUT, x as it was and the plan ready for another solve. */
+ * take turns, whatever their streams.  Its CTAs wait for one another, at most `polls`
+ * reads per grid sum (the default, 2^23, takes seconds; more are not waited for).  A
+ * wait that runs out ends the solve with BSP_ERR_TIMEOUT, x as it was and the plan
+ * ready for another solve. */
 bsp_status bsp_cg_fused_ctas(bsp_cg_plan plan, int32_t *ctas);
 bsp_status bsp_cg_set_wait_limit(bsp_cg_plan plan, uint32_t polls);
 /* k right-hand sides at once: A X = B with B, X device arrays, row-major with
