@@ -56,6 +56,13 @@ __global__ void bcsr_spmv_kernel(int32_t row, int32_t col, int32_t nr, int32_t t
 
 using namespace bsp;
 
+static void bcsr_free_arrays(bsp_bcsr *b, cudaStream_t s) {
+  dfree(b->bcsrRowPtr, s);
+  dfree(b->bcsrcolIdx, s);
+  dfree(b->relativeBlockIndexMapping, s);
+  dfree(b->values, s);
+}
+
 extern "C" bsp_status bsp_csr2bcsr(int32_t rows, int32_t cols, int32_t nnz, const int32_t *rowPtr,
                                    const int32_t *colIdx, const double *values, int32_t tile_m, int32_t tile_k,
                                    int32_t with_mapping, bsp_bcsr *out, bsp_stream_t stream) {
@@ -65,7 +72,16 @@ extern "C" bsp_status bsp_csr2bcsr(int32_t rows, int32_t cols, int32_t nnz, cons
   BSP_CHECK_ARG(tile_m >= 1 && tile_k >= 1 && tile_m <= 64 && tile_k <= 64, "tile sizes must be in [1, 64]");
   BSP_CHECK_ARG(rowPtr && (nnz == 0 || (colIdx && values)), "null pointer");
   cudaStream_t s = as_stream(stream);
-  bsp_bcsr b{};
+  struct Owned {  // what has been made is freed unless it is handed out
+    bsp_bcsr b{};
+    bool done = false;
+    cudaStream_t s;
+    explicit Owned(cudaStream_t stream) : s(stream) {}
+    ~Owned() {
+      if (!done) bcsr_free_arrays(&b, s);
+    }
+  } owned(s);
+  bsp_bcsr &b = owned.b;
   b.row = rows;
   b.col = cols;
   b.nnz = nnz;
@@ -95,6 +111,7 @@ extern "C" bsp_status bsp_csr2bcsr(int32_t rows, int32_t cols, int32_t nnz, cons
   }
   BSP_CUDA(cudaStreamSynchronize(s));
   *out = b;
+  owned.done = true;
   return BSP_OK;
 }
 
@@ -102,10 +119,7 @@ extern "C" bsp_status bsp_bcsr_free(bsp_bcsr *b) {
   clear_error();
   if (!b) return BSP_OK;
   cudaStream_t s = 0;
-  dfree(b->bcsrRowPtr, s);
-  dfree(b->bcsrcolIdx, s);
-  dfree(b->relativeBlockIndexMapping, s);
-  dfree(b->values, s);
+  bcsr_free_arrays(b, s);
   BSP_CUDA(cudaStreamSynchronize(s));
   return BSP_OK;
 }

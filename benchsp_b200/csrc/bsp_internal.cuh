@@ -91,6 +91,16 @@ void dfree(T *&p, cudaStream_t s) {
   p = nullptr;
 }
 
+// Device memory of one call, given back in stream order on every way out.
+template <typename T>
+struct Scratch {
+  T *p = nullptr;
+  cudaStream_t s;
+  explicit Scratch(cudaStream_t stream) : s(stream) {}
+  Scratch(const Scratch &) = delete;
+  ~Scratch() { dfree(p, s); }
+};
+
 // ---------------------------------------------------------------------------
 // Device-side load helpers.  Streamed matrix data is read once: bypass L1 and
 // mark it evict-first in L2 so the gathered vector x stays resident.  sm_100

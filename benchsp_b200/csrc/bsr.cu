@@ -514,7 +514,8 @@ static bool merge_wins(int bs, const BlockProfile &p, int32_t nnz, int32_t blc_r
 // Canonical tm x tk blocking of a CSR matrix (block columns ascending per
 // block-row, row-major values).  map16 (tm*tk <= 16) or map64 (<= 64) get the
 // occupancy bitmaps when non-null; d_full (with a map, zeroed by the caller)
-// the number of full blocks.  Outputs are allocated here.
+// the number of full blocks.  Outputs (null on entry) are allocated here, and left to
+// the caller on failure too.
 //
 // 4x4 and 8x8 blocks merge the rows of a block-row (bsr_merge_kernel) where
 // merge_wins says so and every row's columns are strictly ascending; other shapes
@@ -524,9 +525,10 @@ bsp_status csr2blocks(int32_t rows, int32_t nnz, const int32_t *rowPtr, const in
                       int32_t tm, int32_t tk, int32_t *blc_num_out, int32_t **blcPtr, int32_t **blcIdx,
                       double **blcVal, uint16_t **map16, uint64_t **map64, int32_t *d_full, cudaStream_t s) {
   const int32_t blc_row = (int32_t)ceil_div(rows, tm);
-  int32_t *pos = nullptr;
-  BlockProfile h{}, *d_meta = nullptr;
-  BSP_TRY(dalloc(&d_meta, 1, s));
+  Scratch<int32_t> flags(s);
+  Scratch<BlockProfile> meta(s);
+  BSP_TRY(dalloc(&meta.p, 1, s));
+  BlockProfile h{}, *const d_meta = meta.p;
   BSP_CUDA(cudaMemsetAsync(d_meta, 0, sizeof(BlockProfile), s));
   BSP_TRY(dalloc(blcPtr, (size_t)blc_row + 1, s));
   auto read_meta = [&]() -> bsp_status {
@@ -566,7 +568,8 @@ bsp_status csr2blocks(int32_t rows, int32_t nnz, const int32_t *rowPtr, const in
     merge = !h.unsorted;
   }
   if (!merge) {
-    BSP_TRY(dalloc(&pos, (size_t)nnz + 1, s));
+    BSP_TRY(dalloc(&flags.p, (size_t)nnz + 1, s));
+    int32_t *const pos = flags.p;
     BSP_CUDA(cudaMemsetAsync(pos + nnz, 0, sizeof(int32_t), s));
     if (nnz > 0) {
       bsr_canonical_kernel<<<grid_for((int64_t)rows * 32, 256), 256, 0, s>>>(rows, tm, tk, rowPtr, colIdx, pos);
@@ -575,7 +578,6 @@ bsp_status csr2blocks(int32_t rows, int32_t nnz, const int32_t *rowPtr, const in
     BSP_TRY(exclusive_scan_i32(pos, pos, (int64_t)nnz + 1, &d_meta->total, s));
     BSP_TRY(read_meta());
   }
-  dfree(d_meta, s);
   if (h.total > INT32_MAX / ((int64_t)tm * tk)) BSP_FAIL(BSP_ERR_UNSUPPORTED, "too many blocks for int32 indexing");
   const int32_t nb = (int32_t)h.total;
   *blc_num_out = nb;
@@ -595,6 +597,7 @@ bsp_status csr2blocks(int32_t rows, int32_t nnz, const int32_t *rowPtr, const in
     return merge_fill<8, uint64_t>(rows, blc_row, rowPtr, colIdx, values, vec, *blcPtr, *blcIdx, *blcVal,
                                    map64 ? *map64 : nullptr, d_full, s);
   }
+  const int32_t *const pos = flags.p;
   bsr_ptr_kernel<<<grid_for((int64_t)blc_row + 1, 256), 256, 0, s>>>(rows, blc_row, tm, rowPtr, pos, *blcPtr);
   BSP_LAUNCH_CHECK();
   BSP_CUDA(cudaMemsetAsync(*blcVal, 0, sizeof(double) * (size_t)nb * tm * tk, s));
@@ -619,13 +622,31 @@ bsp_status csr2blocks(int32_t rows, int32_t nnz, const int32_t *rowPtr, const in
                                                               d_full);
     BSP_LAUNCH_CHECK();
   }
-  dfree(pos, s);
   return BSP_OK;
+}
+
+static void bsr_free_arrays(bsp_bsr *m, cudaStream_t s) {
+  dfree(m->blcPtr, s);
+  dfree(m->blcIdx, s);
+  dfree(m->blcVal, s);
+  if (m->blcMap) pool_free(m->blcMap, s);
+  m->blcMap = nullptr;
+  dfree(m->rowPtrbyWarp, s);
+  dfree(m->rowIdxbyWarp, s);
 }
 
 bsp_status csr2bsr_impl(int32_t rows, int32_t cols, int32_t nnz, const int32_t *rowPtr, const int32_t *colIdx,
                         const double *values, int32_t bs, bsp_bsr *out, cudaStream_t s) {
-  bsp_bsr m{};
+  struct Owned {  // what has been made is freed unless it is handed out
+    bsp_bsr m{};
+    bool done = false;
+    cudaStream_t s;
+    explicit Owned(cudaStream_t stream) : s(stream) {}
+    ~Owned() {
+      if (!done) bsr_free_arrays(&m, s);
+    }
+  } owned(s);
+  bsp_bsr &m = owned.m;
   m.row = rows;
   m.col = cols;
   m.bs = bs;
@@ -634,22 +655,26 @@ bsp_status csr2bsr_impl(int32_t rows, int32_t cols, int32_t nnz, const int32_t *
   m.true_nnz = nnz;
   uint16_t *m16 = nullptr;
   uint64_t *m64 = nullptr;
-  int32_t *d_full = nullptr;
-  BSP_TRY(dalloc(&d_full, 1, s));
+  Scratch<int32_t> full(s);
+  Scratch<int64_t> chunks(s);
+  Scratch<double> dev(s), sum(s);
+  BSP_TRY(dalloc(&full.p, 1, s));
+  int32_t *const d_full = full.p;
   BSP_CUDA(cudaMemsetAsync(d_full, 0, sizeof(int32_t), s));
-  BSP_TRY(csr2blocks(rows, nnz, rowPtr, colIdx, values, bs, bs, &m.blc_num, &m.blcPtr, &m.blcIdx, &m.blcVal,
-                     bs == 4 ? &m16 : nullptr, bs == 4 ? nullptr : &m64, d_full, s));
+  const bsp_status st = csr2blocks(rows, nnz, rowPtr, colIdx, values, bs, bs, &m.blc_num, &m.blcPtr, &m.blcIdx,
+                                   &m.blcVal, bs == 4 ? &m16 : nullptr, bs == 4 ? nullptr : &m64, d_full, s);
   m.blcMap = bs == 4 ? (void *)m16 : (void *)m64;
+  BSP_TRY(st);
   m.nnz = m.blc_num * bs * bs;
   m.avg_nnz = m.blc_num > 0 ? (double)nnz / (double)m.blc_num : 0.0;
-  int64_t *d_total = nullptr;
-  BSP_TRY(dalloc(&d_total, 1, s));
+  BSP_TRY(dalloc(&chunks.p, 1, s));
+  int64_t *const d_total = chunks.p;
 
   // Balanced chunks and block-length statistics.
-  double *sq = nullptr, *d_sum = nullptr;
   BSP_TRY(dalloc(&m.rowPtrbyWarp, (size_t)m.blc_row + 1, s));
-  BSP_TRY(dalloc(&sq, (size_t)m.blc_row + 1, s));
-  BSP_TRY(dalloc(&d_sum, kSumCtas + 1, s));
+  BSP_TRY(dalloc(&dev.p, (size_t)m.blc_row + 1, s));
+  BSP_TRY(dalloc(&sum.p, kSumCtas + 1, s));
+  double *const sq = dev.p, *const d_sum = sum.p;
   const double avg_len = m.blc_row > 0 ? (double)m.blc_num / (double)m.blc_row : 0.0;
   BSP_CUDA(cudaMemsetAsync(m.rowPtrbyWarp, 0, sizeof(int32_t) * ((size_t)m.blc_row + 1), s));
   if (m.blc_row > 0) {
@@ -676,11 +701,8 @@ bsp_status csr2bsr_impl(int32_t rows, int32_t cols, int32_t nnz, const int32_t *
     m.stand = (double)sqrtf((float)(ss / m.blc_row));
   }
   BSP_TRY(read_i32(d_full, &m.dense_blocks, s));
-  dfree(d_full, s);
-  dfree(sq, s);
-  dfree(d_sum, s);
-  dfree(d_total, s);
   *out = m;
+  owned.done = true;
   return BSP_OK;
 }
 
@@ -931,13 +953,7 @@ extern "C" bsp_status bsp_bsr_free(bsp_bsr *m) {
   clear_error();
   if (!m) return BSP_OK;
   cudaStream_t s = 0;
-  dfree(m->blcPtr, s);
-  dfree(m->blcIdx, s);
-  dfree(m->blcVal, s);
-  if (m->blcMap) pool_free(m->blcMap, s);
-  m->blcMap = nullptr;
-  dfree(m->rowPtrbyWarp, s);
-  dfree(m->rowIdxbyWarp, s);
+  bsr_free_arrays(m, s);
   BSP_CUDA(cudaStreamSynchronize(s));
   return BSP_OK;
 }

@@ -103,3 +103,28 @@ def test_threads_leave_no_more_than_the_bound(cuda):
     assert _held(base) <= total // 64 + SLACK
     _lib.check(_lib.lib().bsp_pool_trim())
     assert _held(base) <= SLACK
+
+
+@pytest.mark.parametrize("call", ["csr2bsr", "csr2bcsr"])
+def test_a_refused_conversion_keeps_no_memory(cuda, call):
+    """33,554,432 blocks of 8x8 (four entries each, in one of the block's rows) are one
+    more than int32 indexing holds: refused, and nothing of the attempt stays."""
+    import torch
+    k = torch.arange(4, dtype=torch.int32, device=cuda)
+    row = torch.arange(8, device=cuda, dtype=torch.int32)[:, None, None]
+    blk = torch.arange(8, device=cuda, dtype=torch.int32)[None, :, None] * 8
+    ci = ((blk + row) * 8 + k).reshape(-1).repeat(1 << 19)   # row r of a block-row: blocks r, 8 + r, ..., 56 + r
+    rp = torch.arange(0, ci.numel() + 1, 32, dtype=torch.int32, device=cuda)
+    va = torch.zeros(ci.numel(), dtype=torch.float64, device=cuda)
+    f = {"csr2bsr": lambda: bsp.csr2bsr(rp, ci, va, rows=1 << 22, cols=512, bs=8),
+         "csr2bcsr": lambda: bsp.csr2bcsr(rp, ci, va, rows=1 << 22, cols=512, tile_m=8, tile_k=8)}[call]
+    _lib.check(_lib.lib().bsp_pool_trim())
+    torch.cuda.synchronize()
+    base = torch.cuda.mem_get_info()[0]
+    for _ in range(40):                        # 2 MB of block pointers each
+        with pytest.raises(bsp.BspError) as e:
+            f()
+        assert e.value.status == bsp._lib.BSP_ERR_UNSUPPORTED
+    torch.cuda.synchronize()
+    _lib.check(_lib.lib().bsp_pool_trim())
+    assert _held(base) < 32 << 20
