@@ -317,8 +317,9 @@ __device__ __forceinline__ void vset(double2 &v, int k, double a) {
 // and shared memory (no DRAM traffic); the product is bound by instruction issue
 // and by the 2 of 7 columns that come from another SM.  An earlier form on the
 // SELL copy with 16-bit offsets took 31 us (a decode, an address and a test per
-// entry).  FP64 100^3: 31 -> 24 us.  Below about 40^3 the two sums are most of an
-// iteration (24^3 FP16: 9.1 -> 6 us).
+// entry).  Whole solves, checks and FP64 residuals included, per iteration: FP64 100^3
+// 31.0 -> 22.7 us, FP16 100^3 21.9 -> 15.5, 64^3 11.7 -> 10.3, 24^3 9.0 -> 7.9.  Below
+// about 40^3 the two sums are most of an iteration (two_kernels_faster).
 //
 // The cooperative launch makes all CTAs resident; every wait is bounded all the
 // same: kFusedPolls, or in an instantiation of its own (LIMITED) the plan's limit, which
@@ -1561,12 +1562,28 @@ static bsp_status fused_reset(bsp_cg_plan_s *P, cudaStream_t s) {
   return BSP_OK;
 }
 
+// Rows between which two kernels are the faster iteration.  Below them the fused one
+// is few CTAs, so its two grid sums are short; above them the vectors' traffic
+// decides.  In between the sums take most of an iteration of many CTAs, while two
+// kernels still run as fast as they can be launched.  7-point Poisson (5-point
+// Laplacian), us per iteration, fused / two kernels: FP64 24^3 7.4 / 7.6, 28^3 8.1 /
+// 7.5, 32^3 8.7 / 7.5 (200^2 7.9 / 7.0), 48^3 9.7 / 8.9, 56^3 10.5 / 10.4, 64^3 11.3 /
+// 11.9; FP32 32^3 8.5 / 8.7, 36^3 9.6 / 8.7, 48^3 9.9 / 9.5 (256^2 7.4 / 7.2), 52^3
+// 10.0 / 10.7.  FP16 differs by 3% either way there (40^3 7.8 / 8.9) and stays fused.
+static bool two_kernels_faster(int mode, int32_t n) {
+  switch (mode) {
+    case BSP_CG_FP64: return n > 18000 && n < 180000;
+    case BSP_CG_MIXED_F32: return n > 36000 && n < 120000;
+    default: return false;
+  }
+}
+
 // Sets up the fused iteration where it applies: no preconditioner, one CTA per
 // SM whose share of the vectors fits in shared memory, strictly ascending columns
 // in every row, and at most kFusedDiags distinct diagonals that the rows fill by
 // 3/4 or more.
 static bsp_status fused_setup(bsp_cg_plan_s *P, cudaStream_t s) {
-  if (P->prec_bs) return BSP_OK;
+  if (P->prec_bs || two_kernels_faster(P->opt.mode, P->n)) return BSP_OK;
   const size_t vt = cg_mixed(P) ? 4 : 8;
   int dev = 0, coop = 0, optin = 0, sms = 0, occ = 0;
   BSP_CUDA(cudaGetDevice(&dev));

@@ -667,7 +667,8 @@ bsp_status bsp_cg_destroy(bsp_cg_plan plan);
 /* Without a preconditioner, a matrix of at most 8 diagonals with ascending
  * columns whose vectors fit the SMs' shared memory (16 bytes a row in the mixed
  * modes, 32 in FP64) runs check_every iterations in one cooperative launch of
- * *ctas CTAs; *ctas = 0: two kernels per iteration.  That launch needs its SMs all
+ * *ctas CTAs, except where two kernels are the faster iteration (FP64 from 18,000 to
+ * 180,000 rows, FP32 from 36,000 to 120,000); *ctas = 0: two kernels per iteration.  That launch needs its SMs all
  * at once (it fails on a stream confined to fewer), so fused solves of a device
  * take turns, whatever their streams.  Its CTAs wait for one another, at most `polls`
  * reads per grid sum (the default, 2^23, takes seconds; more are not waited for).  A

@@ -230,7 +230,7 @@ def test_cg_fused_wait_that_runs_out(cuda, mode):
     """With one read per wait the fused launch gives up: the solve returns the
     status, leaves x alone, and the plan solves again to the same bits."""
     import torch
-    A = bsp.gen_poisson3d(48)
+    A = bsp.gen_poisson3d(64)
     rp, ci, va, b = _dev(cuda, A.rowptr, A.colidx, A.values, bsp.gen_uniform(A.rows, 17))
     S = bsp.CgSolver(rp, ci, va, mode=mode, tol=1e-10)
     assert S.fused_ctas > 1
@@ -328,3 +328,19 @@ def test_cg_form_that_runs(cuda, n, diags, fused):
     S = bsp.CgSolver(rp, ci, va, mode="f16", precond="jacobi")
     assert S.fused_ctas == 0
     S.close()
+
+
+@pytest.mark.parametrize("mode,n,fused", [("fp64", 18000, True), ("fp64", 18001, False), ("fp64", 179999, False),
+                                          ("fp64", 180000, True), ("f32", 36000, True), ("f32", 36001, False),
+                                          ("f32", 119999, False), ("f32", 120000, True), ("f16", 64000, True)])
+def test_cg_two_kernels_between_the_sizes(cuda, mode, n, fused):
+    """The middle sizes iterate with two kernels, and both forms solve."""
+    A = _banded(n, [1, 50], n)
+    b = bsp.gen_uniform(n, 15)
+    rp, ci, va, bb = _dev(cuda, A.rowptr, A.colidx, A.values, b)
+    S = bsp.CgSolver(rp, ci, va, mode=mode, tol=1e-10)
+    assert (S.fused_ctas > 0) == fused
+    x, res = S.solve(bb)
+    S.close()
+    assert res["converged"] == 1
+    assert pyoracle.rel_residual(A.rowptr, A.colidx, A.values, b, x.cpu().numpy()) <= 2e-10
