@@ -131,7 +131,8 @@ __device__ __forceinline__ typename AccOf<V>::T strided_sum(const int32_t *__res
 // Long rows are left out of the pass over a CTA's rows and summed after it by
 // more threads: a warp per row up to kCtaRow entries, the whole CTA above
 // (power-law rows: one 10,000-entry row was a chain of 78 dependent loads for
-// the warp that met it).  A row's summation order depends on its length alone.
+// the warp that met it).  A row's summation order depends on its length and on the
+// matrix's mean alone.
 // CTAs without such rows pay one barrier.
 //
 // Sums the CTA's long rows: `mine` says that this thread holds one, row `r`
@@ -145,11 +146,12 @@ __device__ __forceinline__ void sum_long_rows(bool mine, int64_t r, int32_t s, i
   using A = typename AccOf<V>::T;
   // A CTA takes its rows above kCtaRow one after another, so where rows are long on
   // average (and several such rows share a CTA) the bound is higher: 10% of the rows
-  // of 600 among rows of 40 (16 lanes), FP16 82 us at 512, 73 here.  With few lanes
-  // 512 is the faster one: power-law 2^17 FP64 16.9 us, 18.4 at 1024, 24 at 2048.
+  // of 600 among rows of 40 (16 lanes), FP16 87 us at 512, 65 here.  With few lanes
+  // 512 is the faster one: power-law 2^17 FP64 16.9 us, 18.4 at 1024; 2^14 11.4 at
+  // 1024, 14.5 at 2048, 24.7 at 4096.
   constexpr int kCtaRow = LPR <= 4 ? 512 : 128 * LPR;
-  // loads in flight: 8 where they fit the registers (FP32 with several lanes 64 in
-  // flight a warp more, stencil 128^3 89 -> 92 us)
+  // loads in flight: 8 where they leave the pass over the rows its registers (with 8
+  // in the other types it slows down: stencil 128^3 FP32 89 -> 91 us, FP64 130 -> 139)
   constexpr int U = (sizeof(V) == 8 && LPR == 1) || (sizeof(V) == 2 && LPR > 1) ? 8 : 4;
   struct LongRow {
     int32_t s, e, r;
@@ -219,11 +221,13 @@ __device__ __forceinline__ void sum_long_rows(bool mine, int64_t r, int32_t s, i
 // lane.
 //
 // Rows of more than long_len entries are left to sum_long_rows (power-law 2^20,
-// Zipf 2.0, cap 10k: FP64 105 -> 50 us, FP16 58 -> 38; 2^14 rows FP64 37 -> 10).
+// Zipf 2.0, cap 10k: FP64 119 -> 52 us, FP16 60 -> 39; 2^14 rows FP64 25 -> 9).
 // long_len is kWarpRowFactor entries per lane, but no less than 4 times the mean:
 // the barrier and the list only pay for rows far above the others.  2M rows of 7 on
 // average with 5% of 17 to 24 (an unstructured mesh), FP16: 37.8 us, at 16 entries
-// per lane alone 46.9 (FP32 44.2 against 51.8); power-law within 2% of it.
+// per lane alone 46.9 (FP32 44.2 against 51.8); power-law within 2% of it.  FP64 with
+// one lane keeps 78 us there (73 without the list, which takes the registers that its
+// later entries had).
 //
 // Resident CTAs: FP64 with several lanes needs 40 registers (6 CTAs; at 8 it
 // spills, 138 us); FP64 with one lane is capped at 32 (at 40 the 1024 CTAs of a

@@ -2103,8 +2103,8 @@ __device__ __forceinline__ uint4 ld_hint_b16(const void *p, uint64_t pol) {
 // For 16-bit types it is the mixed form, which takes its factors as FP16 or
 // BF16 and accumulates in FP32: the product and the sum are those of fmaf on
 // the converted operands, bit for bit, without converting the 8 elements of
-// each gather.  The pass issues 71% of the time (N = 128), so instructions
-// are what it waits for: graph 2^20, FP16, N = 128 converted, with fmaf
+// each gather.  The pass issued 71% of the time (N = 128), so instructions
+// were what it waited for: graph 2^20, FP16, N = 128 converted, with fmaf
 // 0.967 ms, with the two-wide FP32 form 0.986, mixed 0.915.
 __device__ __forceinline__ void fma16(float (&acc)[4], float v, const uint4 &u) {
   acc[0] = fmaf(v, __uint_as_float(u.x), acc[0]);
@@ -2162,7 +2162,10 @@ constexpr int32_t kSlabOvershoot = 64;
 // 0.685 -> 0.503; graph 2^18, FP32, N = 128 0.474 -> 0.321.
 // Register bounds: 16-bit types 4 CTAs per SM (N = 128: 4 0.903 ms, 5 with
 // 48 bytes spilled 0.962, 6 1.041; N = 32: 4 0.323, 5 0.338; N = 256: 4 1.74,
-// none 1.93), FP32 5 (N = 128: 5 0.321, 6 0.343).
+// none 1.93), FP32 5 with 8 lanes and more, which spill 12 to 24 bytes at its 48
+// registers (2^18, N = 128: 5 0.321, 6 0.343; 4, without spills, is faster where B
+// rows are shared and slower where they are not: stencil 832 -> 727 us, banded 635 ->
+// 551, but random rows 640 -> 682, short rows of 5 207 -> 225, graph 295 -> 308).
 template <typename T, int LPR, int U, int UL, bool WIDE>
 __global__ void __launch_bounds__(256, LPR < 4 ? 0 : sizeof(T) == 2 ? 4 : (LPR >= 8 ? 5 : 0))
     spmm_slab_kernel(
