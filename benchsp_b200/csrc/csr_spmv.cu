@@ -73,6 +73,7 @@ constexpr int kCsrThreads = 256;
 constexpr int kCsrWarps = kCsrThreads / 32;
 constexpr int kWarpRowFactor = 16;
 constexpr int kLongList = 64;
+constexpr int kWarpCtas = 64;  // of csr_warp_kernel per SM, at most
 
 // Positions among the nonzeros are of type J.  A step's loads lie up to kOvershoot
 // entries behind a row's end before they are masked.  Where nnz leaves that much
@@ -103,36 +104,23 @@ __device__ __forceinline__ typename AccOf<V>::T strided_sum(J j, J e, const int3
   return sum;
 }
 
-// The same with pointers to the first entry and the number of entries from there
-// on: with FP64 and one lane per row, 8 in flight take 32 registers this way and
-// spill 164 bytes as an index (power-law 2^20 50 us against 68; 4 in flight 52).
-template <typename V, int STRIDE, int U>
-__device__ __forceinline__ typename AccOf<V>::T strided_sum(const int32_t *__restrict__ ci,
-                                                            const V *__restrict__ va, int32_t left,
-                                                            const V *__restrict__ x) {
-  using A = typename AccOf<V>::T;
-  A sum = A(0);
-  for (; left > 0; left -= U * STRIDE, ci += U * STRIDE, va += U * STRIDE) {
-    int32_t c[U];
-    V a[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const bool in = u * STRIDE < left;
-      c[u] = in ? ci[u * STRIDE] : -1;
-      a[u] = in ? va[u * STRIDE] : V(0);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (c[u] >= 0) sum = fma(to_acc<V>(a[u]), to_acc<V>(__ldg(&x[c[u]])), sum);
-  }
-  return sum;
+// A long row by the lane that holds it.  Not inlined: in line, sum_long_rows slows down
+// (1M rows, Zipf 2.0, cap 1,000, FP32 44.8 -> 48.8 us).
+template <typename V, typename J>
+__device__ __noinline__ void sum_own_row(int64_t r, J s, J e, const int32_t *__restrict__ colIdx,
+                                         const V *__restrict__ val, const V *__restrict__ x, V *__restrict__ y,
+                                         typename AccOf<V>::T alpha, typename AccOf<V>::T beta) {
+  store_y<V, typename AccOf<V>::T>(y, r, strided_sum<V, 1, 4>(s, e, colIdx, val, x), alpha, beta);
 }
 
 // Long rows are left out of the pass over a CTA's rows and summed after it by
 // more threads: a warp per row up to kCtaRow entries, the whole CTA above
 // (power-law rows: one 10,000-entry row was a chain of 78 dependent loads for
-// the warp that met it).  A row's summation order depends on its length and on the
-// matrix's mean alone.
+// the warp that met it).  With one lane per row, and no row above kOwnRow in the CTA,
+// each lane sums its own: 2M rows, a tenth of them of 20 and the others empty, FP64
+// 71 -> 40 us, FP16 58 -> 39 (without any list 33 and 25, but the power-law matrices
+// below take 15 to 30% longer then).  A row's summation order depends on its length, on
+// the matrix's mean and, up to kOwnRow, on whether its CTA has a longer one.
 // CTAs without such rows pay one barrier.
 //
 // Sums the CTA's long rows: `mine` says that this thread holds one, row `r`
@@ -149,10 +137,11 @@ __device__ __forceinline__ void sum_long_rows(bool mine, int64_t r, int32_t s, i
   // of 600 among rows of 40 (16 lanes), FP16 87 us at 512, 65 here.  With few lanes
   // 512 is the faster one: power-law 2^17 FP64 16.9 us, 18.4 at 1024; 2^14 11.4 at
   // 1024, 14.5 at 2048, 24.7 at 4096.
-  constexpr int kCtaRow = LPR <= 4 ? 512 : 128 * LPR;
+  constexpr int kCtaRow = LPR <= 4 ? 512 : LPR == 32 ? 0 : 128 * LPR;
+  constexpr int kOwnRow = 64, kFar = 1 << 16;
   // loads in flight: 8 where they leave the pass over the rows its registers (with 8
   // in the other types it slows down: stencil 128^3 FP32 89 -> 91 us, FP64 130 -> 139)
-  constexpr int U = (sizeof(V) == 8 && LPR == 1) || (sizeof(V) == 2 && LPR > 1) ? 8 : 4;
+  constexpr int U = sizeof(V) == 2 && LPR > 1 && LPR < 32 ? 8 : 4;
   struct LongRow {
     int32_t s, e, r;
   };
@@ -161,8 +150,15 @@ __device__ __forceinline__ void sum_long_rows(bool mine, int64_t r, int32_t s, i
   __shared__ A part[kCsrWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (!__syncthreads_or(mine)) return;
+  if (sizeof(A) == 8 && mine) {
+    // read again rather than carried through the pass: with s and e alive the
+    // FP64 kernel takes 40 registers, and 6 instead of 8 CTAs fit an SM
+    asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(s) : "l"(rowPtr + r));
+    asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(e) : "l"(rowPtr + r + 1));
+  }
   const unsigned mask = __ballot_sync(0xffffffffu, mine);
-  if (lane == 0) count[w] = __popc(mask);
+  const bool far = LPR == 1 && __any_sync(0xffffffffu, mine && e - s > kOwnRow);
+  if (lane == 0) count[w] = __popc(mask) + (far ? kFar : 0);
   __syncthreads();
   int32_t n = 0, base = 0;
 #pragma unroll
@@ -170,35 +166,28 @@ __device__ __forceinline__ void sum_long_rows(bool mine, int64_t r, int32_t s, i
     base += q < w ? count[q] : 0;
     n += count[q];
   }
-  base += __popc(mask & ((1u << lane) - 1));
-  if (sizeof(A) == 8 && mine) {
-    // read again rather than carried through the pass: with s and e alive the
-    // FP64 kernel takes 40 registers, and 6 instead of 8 CTAs fit an SM
-    asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(s) : "l"(rowPtr + r));
-    asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(e) : "l"(rowPtr + r + 1));
+  if (LPR == 1 && n < kFar) {
+    if (mine) sum_own_row<V, J>(r, (J)s, (J)e, colIdx, val, x, y, alpha, beta);
+    return;
   }
-  auto share = [&](const LongRow &L, int32_t first, auto step) {
-    constexpr int stride = decltype(step)::value;
-    if constexpr (sizeof(V) == 8 && LPR == 1)
-      return warp_sum(strided_sum<V, stride, U>(colIdx + L.s + first, val + L.s + first, L.e - L.s - first, x));
-    else
-      return warp_sum(strided_sum<V, stride, U>((J)((J)L.s + first), (J)L.e, colIdx, val, x));
-  };
+  n %= kFar;
+  base %= kFar;
+  base += __popc(mask & ((1u << lane) - 1));
   for (int32_t first = 0; first < n; first += kLongList) {  // CTA-uniform
     const int32_t m = min(n - first, kLongList);
     __syncthreads();
     if (mine && base >= first && base < first + m) list[base - first] = {s, e, (int32_t)r};
     __syncthreads();
-    for (int k = w; k < m; k += kCsrWarps) {
+    for (int k = w; k < m && LPR < 32; k += kCsrWarps) {
       const LongRow L = list[k];
       if (L.e - L.s > kCtaRow) continue;
-      const A sum = share(L, lane, std::integral_constant<int, 32>());
+      const A sum = warp_sum(strided_sum<V, 32, U>((J)((J)L.s + lane), (J)L.e, colIdx, val, x));
       if (lane == 0) store_y<V, A>(y, L.r, sum, alpha, beta);
     }
     for (int k = 0; k < m; ++k) {
       const LongRow L = list[k];
       if (L.e - L.s <= kCtaRow) continue;
-      const A sum = share(L, threadIdx.x, std::integral_constant<int, kCsrThreads>());
+      const A sum = warp_sum(strided_sum<V, kCsrThreads, U>((J)((J)L.s + threadIdx.x), (J)L.e, colIdx, val, x));
       if (lane == 0) part[w] = sum;
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -227,7 +216,8 @@ __device__ __forceinline__ void sum_long_rows(bool mine, int64_t r, int32_t s, i
 // average with 5% of 17 to 24 (an unstructured mesh), FP16: 37.8 us, at 16 entries
 // per lane alone 46.9 (FP32 44.2 against 51.8); power-law within 2% of it.  FP64 with
 // one lane keeps 78 us there (73 without the list, which takes the registers that its
-// later entries had).
+// later entries had).  No more than 64 per lane where a caller asks for few lanes (rows
+// of 200, FP64, one lane: 152 -> 122 us).
 //
 // Resident CTAs: FP64 with several lanes needs 40 registers (6 CTAs; at 8 it
 // spills, 138 us); FP64 with one lane is capped at 32 (at 40 the 1024 CTAs of a
@@ -244,12 +234,13 @@ __global__ void __launch_bounds__(kCsrThreads, LPR > 1 && sizeof(V) == 8 ? 6 : L
   const int32_t s = active ? rowPtr[r] : 0, e0 = active ? rowPtr[r + 1] : 0;
   const bool is_long = e0 - s > long_len;
   // Several lanes count positions from their own first entry, which leaves the
-  // loads' offsets constant (rows of 30, FP16 53 -> 48 us); one lane counts from the
-  // arrays' start, which takes fewer registers.
+  // loads' offsets constant (rows of 30, FP16 53 -> 48 us; rows of 33, FP64 71 -> 66);
+  // one lane, and FP32 (rows of 64 33 -> 31 us), count from the arrays' start.
   const int32_t left = is_long ? 0 : max(e0 - s - sub, 0);
-  const J begin = LPR == 1 ? s : 0, end = begin + left;
-  const int32_t *ci = LPR == 1 ? colIdx : colIdx + s + sub;
-  const V *va = LPR == 1 ? val : val + s + sub;
+  constexpr bool kOwn = LPR > 1 && sizeof(V) != 4;
+  const J begin = kOwn ? 0 : (J)s + sub, end = begin + left;
+  const int32_t *ci = kOwn ? colIdx + s + sub : colIdx;
+  const V *va = kOwn ? val + s + sub : val;
   // The first kFirst entries of each lane are loaded together, then their x
   // gathers together: the rowPtr -> column -> x chain is paid once per
   // kFirst entries instead of once per entry.
@@ -275,23 +266,50 @@ __global__ void __launch_bounds__(kCsrThreads, LPR > 1 && sizeof(V) == 8 ? 6 : L
   sum_long_rows<V, LPR, J>(is_long && sub == 0, r, s, e0, rowPtr, colIdx, val, x, y, alpha, beta);
 }
 
-// A warp per row (32 lanes), whatever its length, a warp taking several rows: long
-// rows on average.  No list here: with all rows above its bound every row went
-// through the CTA one after another (60,000 rows of 600 near the diagonal, FP64
-// 138 us, FP16 112; here 69 and 44), and a grid that covers the rows in one pass
+// The long rows of a CTA of csr_warp_kernel: its rows once more, a row per thread.  Not
+// inlined, so that the pass over the rows keeps its registers.
+template <typename V>
+__device__ __noinline__ void sum_own_long_rows(int32_t rows, const int32_t *__restrict__ rowPtr,
+                                               const int32_t *__restrict__ colIdx, const V *__restrict__ val,
+                                               const V *__restrict__ x, V *__restrict__ y,
+                                               typename AccOf<V>::T alpha, typename AccOf<V>::T beta,
+                                               int32_t long_len) {
+  const int64_t nwarps = (int64_t)gridDim.x * kCsrWarps;
+  for (int64_t first = (int64_t)blockIdx.x * kCsrWarps; first < rows; first += 32 * nwarps) {  // CTA-uniform
+    const int64_t r = first + (threadIdx.x & (kCsrWarps - 1)) + (threadIdx.x / kCsrWarps) * nwarps;
+    const int32_t s = r < rows ? rowPtr[r] : 0, e = r < rows ? rowPtr[r + 1] : 0;
+    sum_long_rows<V, 32, uint32_t>(e - s > long_len, r, s, e, rowPtr, colIdx, val, x, y, alpha, beta);
+  }
+}
+
+// A warp per row (32 lanes), a warp taking several rows: long rows on average.  The list
+// of csr_vector_kernel would take most rows here (60,000 rows of 600 near the diagonal,
+// FP64 138 us, FP16 112; here 69 and 44), and a grid that covers the rows in one pass
 // leaves a warp one chain long (200,000 rows of 200, FP64 102 us; here 84, at 4
 // entries in flight 89).
-template <typename V>
+//
+// LIST: rows of more than long_len entries, 512 and 4 times the mean at least, are left
+// to the CTA.  Where warps take several rows, a longer one holds back all that its CTA
+// still has: 200,000 rows of 130 on average, the longest 20,000, FP64 391 -> 181 us.
+// With a row per warp the list only costs (20,000 rows of 275, the longest 5,000, FP32
+// 32 -> 37 us).
+template <typename V, bool LIST>
 __global__ void __launch_bounds__(kCsrThreads) csr_warp_kernel(int32_t rows, const int32_t *__restrict__ rowPtr,
                                                                const int32_t *__restrict__ colIdx,
                                                                const V *__restrict__ val, const V *__restrict__ x,
                                                                V *__restrict__ y, typename AccOf<V>::T alpha,
-                                                               typename AccOf<V>::T beta) {
+                                                               typename AccOf<V>::T beta, int32_t long_len) {
   using A = typename AccOf<V>::T;
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = (int64_t)gridDim.x * kCsrWarps;
+  bool any_long = false;
   for (int64_t r = (int64_t)blockIdx.x * kCsrWarps + (threadIdx.x >> 5); r < rows; r += nwarps) {
-    const uint32_t s = rowPtr[r] + lane, e = rowPtr[r + 1];  // unsigned: behind a row positions may pass 2^31
+    const int32_t s0 = rowPtr[r], e0 = rowPtr[r + 1];
+    if (LIST && e0 - s0 > long_len) {  // warp-uniform
+      any_long = true;
+      continue;
+    }
+    const uint32_t s = (uint32_t)s0 + lane, e = e0;
     constexpr int kFirst = 8;
     int32_t c[kFirst];
     V a[kFirst];
@@ -311,6 +329,8 @@ __global__ void __launch_bounds__(kCsrThreads) csr_warp_kernel(int32_t rows, con
     sum = warp_sum(sum);
     if (lane == 0) store_y<V, A>(y, r, sum, alpha, beta);
   }
+  if constexpr (LIST)
+    if (__syncthreads_or(any_long)) sum_own_long_rows<V>(rows, rowPtr, colIdx, val, x, y, alpha, beta, long_len);
 }
 
 // Warp per 32 consecutive rows ("stream").  The warp's nonzero range
@@ -519,12 +539,19 @@ static void launch_lanes(int lpr, int32_t rows, int32_t long_len, const int32_t 
                          const V *x, V *y, typename AccOf<V>::T a, typename AccOf<V>::T b, cudaStream_t s) {
   const unsigned blocks = (unsigned)ceil_div(rows, kCsrThreads / lpr);  // rows > 0
   switch (lpr) {
-#define BSP_VEC_CASE(L)                                                                                \
-  case L:                                                                                              \
+#define BSP_VEC_CASE(L)                                                                                   \
+  case L:                                                                                                 \
     csr_vector_kernel<V, L, J><<<blocks, kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b, long_len); \
     break;
-    BSP_VEC_CASE(1) BSP_VEC_CASE(2) BSP_VEC_CASE(4) BSP_VEC_CASE(8) BSP_VEC_CASE(16)
+    BSP_VEC_CASE(2) BSP_VEC_CASE(4) BSP_VEC_CASE(8) BSP_VEC_CASE(16)
 #undef BSP_VEC_CASE
+    case 1: csr_vector_kernel<V, 1, J><<<blocks, kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b, long_len); break;
+    case 32:
+      if (ceil_div(rows, kCsrWarps) > kWarpCtas * sm_count())
+        csr_warp_kernel<V, true><<<kWarpCtas * sm_count(), kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b, long_len);
+      else
+        csr_warp_kernel<V, false><<<blocks, kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b, 0);
+      break;
   }
 }
 
@@ -534,11 +561,11 @@ static bsp_status launch_vector(int lpr, int32_t rows, int32_t nnz, const int32_
                                 cudaStream_t s) {
   if (lpr < 1 || lpr > 32 || (lpr & (lpr - 1)) != 0)
     BSP_FAIL(BSP_ERR_INVALID, "lanes_per_row must be a power of two in [1,32]");
-  const int32_t long_len = (int32_t)std::max<int64_t>(kWarpRowFactor * lpr, 4 * (int64_t)nnz / rows);
-  if (lpr == 32)
-    csr_warp_kernel<V><<<(unsigned)std::min<int64_t>(ceil_div(rows, kCsrWarps), (int64_t)sm_count() * 64),
-                         kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b);
-  else if (nnz <= INT32_MAX - kOvershoot)
+  // fewer lanes than auto_lanes gives: the bound stays with the lanes
+  const int64_t mean4 = 4 * (int64_t)nnz / rows;
+  const int32_t long_len = (int32_t)std::min<int64_t>(
+      INT32_MAX, std::max<int64_t>(kWarpRowFactor * lpr, lpr == 32 ? mean4 : std::min<int64_t>(64 * lpr, mean4)));
+  if (nnz <= INT32_MAX - kOvershoot)
     launch_lanes<V, int32_t>(lpr, rows, long_len, rp, ci, v, x, y, a, b, s);
   else
     launch_lanes<V, uint32_t>(lpr, rows, long_len, rp, ci, v, x, y, a, b, s);

@@ -315,3 +315,110 @@ def test_lanes_out_of_range_are_refused(cuda):
     for lanes in (3, 64, 512):
         with pytest.raises(bsp.BspError):
             bsp.csr_spmv(*d, lanes=lanes)
+
+
+def _few_long(kind, lanes, sms):
+    """Row lengths: "own": rows above 16 entries in CTAs of 256 rows with none, one and
+    only rows above 64; "short": rows far below the lanes' 8 entries each, some at and
+    past 4 per lane; "queue": more rows than the warps of one launch, and rows past 512
+    among them, several of one CTA."""
+    if kind == "own":
+        n = np.resize([2, 0, 1, 3], 1100)
+        n[[3, 17, 255]] = [17, 64, 33]
+        n[[256, 300, 511]] = [17, 65, 64]
+        n[[600, 700]] = [600, 70]
+        n[1099] = 64
+    elif kind == "short":
+        n = np.resize([lanes, 0, 2 * lanes, 1], 3000)
+        n[[0, 7, 8, 2999]] = [4 * lanes, 4 * lanes + 1, 12 * lanes, 5 * lanes - 1]
+    else:
+        warps = sms * 64 * 8
+        n = np.resize([1, 0, 2], 2 * warps + 13)
+        n[[0, 1, 8, warps, warps + 1, 2 * warps, n.size - 1]] = [513, 512, 9000, 600, 3, 2000, 513]
+    return n
+
+
+@pytest.mark.parametrize("kind,lanes", [("own", 1), ("queue", 32)])
+@pytest.mark.parametrize("dt", ["float64", "float32", "float16"])
+def test_vector_rows_by_length(cuda, kind, lanes, dt):
+    import torch
+    rng = np.random.default_rng(lanes)
+    lens = _few_long(kind, lanes, torch.cuda.get_device_properties(0).multi_processor_count)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    cols = 9500
+    ci = rng.integers(0, cols, rp[-1]).astype(np.int32)
+    v, x = (torch.from_numpy(a).to(getattr(torch, dt)) for a in (rng.standard_normal(ci.size), rng.uniform(-1, 1, cols)))
+    vh, xh = (t.double().numpy() for t in (v, x))
+    d_rp, d_ci = _dev(cuda, rp, ci)
+    y = torch.full((lens.size,), float("nan"), dtype=v.dtype, device=cuda)
+    got = bsp.csr_spmv(d_rp, d_ci, v.to(cuda), x.to(cuda), y, lanes=lanes).double().cpu().numpy()
+    ref = pyoracle.spmv_f64(rp, ci, vh, xh)
+    unit = 2.0 ** -53 if dt == "float64" else 2.0 ** -24
+    tol = pyoracle.spmv_tolerance(rp, ci, vh, xh, unit=unit) + \
+        (1.01 * 2.0 ** -11 * np.abs(ref) + 2.0 ** -24 if dt == "float16" else 0.0)
+    _within(got, ref, tol)
+
+
+def _best_us(f):
+    import torch
+    best = float("inf")
+    for _ in range(6):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        torch.cuda.synchronize()
+        e[0].record()
+        for _ in range(10):
+            f()
+        e[1].record()
+        torch.cuda.synchronize()
+        best = min(best, e[0].elapsed_time(e[1]))
+    return best * 100
+
+
+def _rows_on_device(cuda, lens, cols, dt):
+    """Rows of the given lengths, their columns spread evenly."""
+    import torch
+    lens = lens.to(cuda)
+    rp = torch.zeros(lens.numel() + 1, dtype=torch.int64, device=cuda)
+    rp[1:] = lens.cumsum(0)
+    r = torch.repeat_interleave(torch.arange(lens.numel(), device=cuda), lens)
+    k = torch.arange(int(rp[-1]), device=cuda) - rp[r]
+    ci = (k * (cols // lens.clamp(min=1))[r] + r % 61).clamp(max=cols - 1)
+    va, x, y = (torch.ones(n, dtype=dt, device=cuda) for n in (ci.numel(), cols, lens.numel()))
+    return rp.int(), ci.int(), va, x, y
+
+
+@pytest.mark.parametrize("dt", ["float64", "float16"])
+def test_a_few_rows_above_16_do_not_go_to_the_list(cuda, dt):
+    """2M rows, a tenth of them of 20 entries and the others empty: a nonzero takes
+    no more than 1.6 times as long as one of rows of 16 (with the rows of 20 summed by a
+    warp each after the pass 1.7 to 2.2 times)."""
+    import torch
+    dt = getattr(torch, dt)
+
+    def per_nonzero(k):
+        lens = torch.zeros(2000000, dtype=torch.int64)
+        lens[::10] = k
+        a = _rows_on_device(cuda, lens, 2000000, dt)
+        return _best_us(lambda: bsp.csr_spmv(*a)) / a[1].numel()
+
+    assert per_nonzero(20) <= 1.6 * per_nonzero(16)
+
+
+def test_long_rows_among_long_rows_leave_their_warp(cuda):
+    """200,000 rows of 130 on average, the longest 20,000 (FP64): at most 1.25 times the
+    merge path, which splits such rows (with every row left to its warp 1.7 times)."""
+    import torch
+    g = torch.Generator().manual_seed(1)
+    u = torch.rand(200000, generator=g, dtype=torch.float64).clamp(min=1e-9)
+    a = _rows_on_device(cuda, (u ** (-1.0 / 0.6)).clamp(max=20000.0).long(), 200000, torch.float64)
+    assert a[1].numel() > 128 * 200000
+    assert _best_us(lambda: bsp.csr_spmv(*a)) <= 1.25 * _best_us(lambda: bsp.csr_spmv(*a, algo="merge"))
+
+
+def test_one_lane_on_long_rows_leaves_them_to_a_warp(cuda):
+    """100,000 rows of 200, FP64, by 1 lane: at most 1.85 times the time of 32 (with rows of
+    200 left to their lane 1.94 times)."""
+    import torch
+    a = _rows_on_device(cuda, torch.full((100000,), 200), 200000, torch.float64)
+    one, all32 = (_best_us(lambda: bsp.csr_spmv(*a, lanes=k)) for k in (1, 32))
+    assert one <= 1.85 * all32
