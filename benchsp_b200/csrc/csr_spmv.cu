@@ -222,7 +222,7 @@ __device__ __forceinline__ void sum_long_rows(bool mine, int64_t r, int32_t s, i
 // Resident CTAs: FP64 with several lanes needs 40 registers (6 CTAs; at 8 it
 // spills, 138 us); FP64 with one lane is capped at 32 (at 40 the 1024 CTAs of a
 // 512^2 grid take a second wave, 3.8 -> 4.5 us).
-template <typename V, int LPR, typename J>
+template <typename V, int LPR, int F, typename J>
 __global__ void __launch_bounds__(kCsrThreads, LPR > 1 && sizeof(V) == 8 ? 6 : LPR > 1 || sizeof(V) == 8 ? 8 : 0)
     csr_vector_kernel(int32_t rows, const int32_t *__restrict__ rowPtr, const int32_t *__restrict__ colIdx,
                       const V *__restrict__ val, const V *__restrict__ x, V *__restrict__ y,
@@ -241,24 +241,23 @@ __global__ void __launch_bounds__(kCsrThreads, LPR > 1 && sizeof(V) == 8 ? 6 : L
   const J begin = kOwn ? 0 : (J)s + sub, end = begin + left;
   const int32_t *ci = kOwn ? colIdx + s + sub : colIdx;
   const V *va = kOwn ? val + s + sub : val;
-  // The first kFirst entries of each lane are loaded together, then their x
+  // The first F entries of each lane are loaded together, then their x
   // gathers together: the rowPtr -> column -> x chain is paid once per
-  // kFirst entries instead of once per entry.
-  constexpr int kFirst = 8;
-  int32_t c[kFirst];
-  V a[kFirst];
+  // F entries instead of once per entry.
+  int32_t c[F];
+  V a[F];
 #pragma unroll
-  for (int k = 0; k < kFirst; ++k) {
+  for (int k = 0; k < F; ++k) {
     const J j = begin + k * LPR;
     c[k] = j < end ? ci[j] : -1;
     a[k] = j < end ? va[j] : V(0);
   }
   A sum = A(0);
 #pragma unroll
-  for (int k = 0; k < kFirst; ++k)
+  for (int k = 0; k < F; ++k)
     if (c[k] >= 0) sum = fma(to_acc<V>(a[k]), to_acc<V>(__ldg(&x[c[k]])), sum);
 #pragma unroll 4
-  for (J j = begin + kFirst * LPR; j < end; j += LPR)
+  for (J j = begin + F * LPR; j < end; j += LPR)
     sum = fma(to_acc<V>(va[j]), to_acc<V>(__ldg(&x[ci[j]])), sum);
 #pragma unroll
   for (int o = LPR / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, LPR);
@@ -293,7 +292,7 @@ __device__ __noinline__ void sum_own_long_rows(int32_t rows, const int32_t *__re
 // still has: 200,000 rows of 130 on average, the longest 20,000, FP64 391 -> 181 us.
 // With a row per warp the list only costs (20,000 rows of 275, the longest 5,000, FP32
 // 32 -> 37 us).
-template <typename V, bool LIST>
+template <typename V, int F, bool LIST>
 __global__ void __launch_bounds__(kCsrThreads) csr_warp_kernel(int32_t rows, const int32_t *__restrict__ rowPtr,
                                                                const int32_t *__restrict__ colIdx,
                                                                const V *__restrict__ val, const V *__restrict__ x,
@@ -310,21 +309,20 @@ __global__ void __launch_bounds__(kCsrThreads) csr_warp_kernel(int32_t rows, con
       continue;
     }
     const uint32_t s = (uint32_t)s0 + lane, e = e0;
-    constexpr int kFirst = 8;
-    int32_t c[kFirst];
-    V a[kFirst];
+    int32_t c[F];
+    V a[F];
 #pragma unroll
-    for (int k = 0; k < kFirst; ++k) {
+    for (int k = 0; k < F; ++k) {
       const uint32_t j = s + 32 * k;
       c[k] = j < e ? colIdx[j] : -1;
       a[k] = j < e ? val[j] : V(0);
     }
     A sum = A(0);
 #pragma unroll
-    for (int k = 0; k < kFirst; ++k)
+    for (int k = 0; k < F; ++k)
       if (c[k] >= 0) sum = fma(to_acc<V>(a[k]), to_acc<V>(__ldg(&x[c[k]])), sum);
 #pragma unroll 4
-    for (uint32_t j = s + 32 * kFirst; j < e; j += 32)
+    for (uint32_t j = s + 32 * F; j < e; j += 32)
       sum = fma(to_acc<V>(val[j]), to_acc<V>(__ldg(&x[colIdx[j]])), sum);
     sum = warp_sum(sum);
     if (lane == 0) store_y<V, A>(y, r, sum, alpha, beta);
@@ -534,23 +532,23 @@ size_t merge_workspace_bytes(int32_t rows, int32_t nnz) {
 }
 
 // ---------------------------------------------------------------------------
-template <typename V, typename J>
+template <typename V, int F, typename J>
 static void launch_lanes(int lpr, int32_t rows, int32_t long_len, const int32_t *rp, const int32_t *ci, const V *v,
                          const V *x, V *y, typename AccOf<V>::T a, typename AccOf<V>::T b, cudaStream_t s) {
   const unsigned blocks = (unsigned)ceil_div(rows, kCsrThreads / lpr);  // rows > 0
   switch (lpr) {
 #define BSP_VEC_CASE(L)                                                                                   \
   case L:                                                                                                 \
-    csr_vector_kernel<V, L, J><<<blocks, kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b, long_len); \
+    csr_vector_kernel<V, L, F, J><<<blocks, kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b, long_len); \
     break;
     BSP_VEC_CASE(2) BSP_VEC_CASE(4) BSP_VEC_CASE(8) BSP_VEC_CASE(16)
 #undef BSP_VEC_CASE
-    case 1: csr_vector_kernel<V, 1, J><<<blocks, kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b, long_len); break;
+    case 1: csr_vector_kernel<V, 1, 8, J><<<blocks, kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b, long_len); break;
     case 32:
       if (ceil_div(rows, kCsrWarps) > kWarpCtas * sm_count())
-        csr_warp_kernel<V, true><<<kWarpCtas * sm_count(), kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b, long_len);
+        csr_warp_kernel<V, F, true><<<kWarpCtas * sm_count(), kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b, long_len);
       else
-        csr_warp_kernel<V, false><<<blocks, kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b, 0);
+        csr_warp_kernel<V, 8, false><<<blocks, kCsrThreads, 0, s>>>(rows, rp, ci, v, x, y, a, b, 0);
       break;
   }
 }
@@ -565,10 +563,19 @@ static bsp_status launch_vector(int lpr, int32_t rows, int32_t nnz, const int32_
   const int64_t mean4 = 4 * (int64_t)nnz / rows;
   const int32_t long_len = (int32_t)std::min<int64_t>(
       INT32_MAX, std::max<int64_t>(kWarpRowFactor * lpr, lpr == 32 ? mean4 : std::min<int64_t>(64 * lpr, mean4)));
-  if (nnz <= INT32_MAX - kOvershoot)
-    launch_lanes<V, int32_t>(lpr, rows, long_len, rp, ci, v, x, y, a, b, s);
+  // 4 entries per lane loaded together instead of 8 where rows do not fill those: asked
+  // for more lanes than auto_lanes gives (rows of 5, FP64: 8 lanes 59 -> 53 us, 32 184
+  // -> 151), or a warp per row (rows of 90 160 -> 135 us, of 160 even)
+  const bool four = nnz <= 2ll * lpr * rows || nnz == 4ll * lpr * rows || (lpr == 32 && nnz <= 160ll * rows);
+  const bool room = nnz <= INT32_MAX - kOvershoot;
+  if (four && room)
+    launch_lanes<V, 4, int32_t>(lpr, rows, long_len, rp, ci, v, x, y, a, b, s);
+  else if (four)
+    launch_lanes<V, 4, uint32_t>(lpr, rows, long_len, rp, ci, v, x, y, a, b, s);
+  else if (room)
+    launch_lanes<V, 8, int32_t>(lpr, rows, long_len, rp, ci, v, x, y, a, b, s);
   else
-    launch_lanes<V, uint32_t>(lpr, rows, long_len, rp, ci, v, x, y, a, b, s);
+    launch_lanes<V, 8, uint32_t>(lpr, rows, long_len, rp, ci, v, x, y, a, b, s);
   BSP_LAUNCH_CHECK();
   return BSP_OK;
 }
@@ -599,12 +606,22 @@ static bsp_status launch_stream(int32_t rows, const int32_t *rp, const int32_t *
 }
 
 // Lanes per row from the mean row length: the smallest power of two whose lanes
-// hold the row in their 8 entries loaded together, up to 32 (rows of 100, FP32: 16
-// lanes 72 us, 32 lanes 100).
-int auto_lanes(int32_t rows, int32_t nnz) {
+// hold the row in their 8 entries loaded together, up to 64 entries; a few more by the
+// same lanes cost less than twice the lanes (rows of 70, 60M nonzeros, FP64: 8 lanes 131
+// us, 16 177; rows of 130, FP16: 16 lanes 78, 32 107), and above that FP64 has a warp per
+// row, 4 loaded together (rows of 90: 135 us, 16 lanes 146; of 160: 119 against 142).
+// A mean of 16 (32) exactly is almost always rows of one length, whose starts then lie
+// on the same banks of L1: twice the lanes with 4 entries each (rows of 16, 8M nonzeros:
+// FP32 20.6 -> 14.5 us, FP16 16.6 -> 12.5, FP64 31 -> 25; of 32: FP32 20.4 -> 14.5, FP16
+// 16.5 -> 12.5, FP64 24.7 and 23.2 but 144 and 160 at 60M).
+int auto_lanes(int32_t rows, int32_t nnz, size_t value_bytes) {
   const double mean = rows > 0 ? (double)nnz / rows : 0.0;
+  const bool wide = value_bytes == 8;
+  if (mean == 16.0) return 4;
+  if (mean == 32.0 && !wide) return 8;
+  if (mean > 64.0) return wide ? (mean <= 88.0 ? 8 : 32) : (mean <= 144.0 ? 16 : 32);
   int l = 1;
-  while (l < 32 && 8.0 * l < mean) l <<= 1;
+  while (8.0 * l < mean) l <<= 1;
   return l;
 }
 
@@ -615,7 +632,7 @@ static bsp_status csr_dispatch(int32_t rows, int32_t nnz, const int32_t *rp, con
   using A = typename AccOf<V>::T;
   if (algo == BSP_CSR_SCALAR) return launch_scalar<V>(rows, rp, ci, v, x, y, (A)alpha, (A)beta, s);
   if (algo == BSP_CSR_STREAM) return launch_stream<V>(rows, rp, ci, v, x, y, (A)alpha, (A)beta, s);
-  if (lpr <= 0) lpr = auto_lanes(rows, nnz);
+  if (lpr <= 0) lpr = auto_lanes(rows, nnz, sizeof(V));
   return launch_vector<V>(lpr, rows, nnz, rp, ci, v, x, y, (A)alpha, (A)beta, s);
 }
 

@@ -104,7 +104,7 @@ __global__ void key_kernel(int32_t rows, int32_t nnz, const int32_t *__restrict_
   if ((threadIdx.x & 31) == 0) atomicAdd(out, h);
 }
 
-int auto_lanes(int32_t rows, int32_t nnz);  // csr_spmv.cu
+int auto_lanes(int32_t rows, int32_t nnz, size_t value_bytes);  // csr_spmv.cu
 
 namespace {
 
@@ -205,7 +205,7 @@ static bsp_status stats(int32_t rows, int32_t nnz, const int32_t *rowPtr, const 
 static void model_choice(int32_t rows, int32_t nnz, bsp_tune_result &r) {
   r.format = BSP_FMT_CSR;
   r.csr_algo = BSP_CSR_VECTOR;
-  r.lanes = auto_lanes(rows, nnz);
+  r.lanes = auto_lanes(rows, nnz, sizeof(double));
   r.bs = 0;
   r.bsr_algo = BSP_BSR_FFMA;
   // modelled time per nonzero (bytes / relative efficiency)

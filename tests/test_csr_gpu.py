@@ -338,7 +338,8 @@ def _few_long(kind, lanes, sms):
     return n
 
 
-@pytest.mark.parametrize("kind,lanes", [("own", 1), ("queue", 32)])
+@pytest.mark.parametrize("kind,lanes", [("own", 1), ("short", 2), ("short", 4), ("short", 8), ("short", 16),
+                                        ("short", 32), ("queue", 32)])
 @pytest.mark.parametrize("dt", ["float64", "float32", "float16"])
 def test_vector_rows_by_length(cuda, kind, lanes, dt):
     import torch
@@ -413,6 +414,22 @@ def test_long_rows_among_long_rows_leave_their_warp(cuda):
     a = _rows_on_device(cuda, (u ** (-1.0 / 0.6)).clamp(max=20000.0).long(), 200000, torch.float64)
     assert a[1].numel() > 128 * 200000
     assert _best_us(lambda: bsp.csr_spmv(*a)) <= 1.25 * _best_us(lambda: bsp.csr_spmv(*a, algo="merge"))
+
+
+@pytest.mark.parametrize("dt,length", [("float32", 16), ("float32", 32), ("float32", 130), ("float16", 130)])
+def test_lanes_from_the_mean_are_near_the_best(cuda, dt, length):
+    """Rows of one length: no other number of lanes takes less than 0.87 of the time."""
+    import torch
+    dt = getattr(torch, dt)
+    rows = 8000000 // length
+    rp = torch.arange(0, rows * length + 1, length, dtype=torch.int32, device=cuda)
+    start = torch.arange(rows, dtype=torch.int32, device=cuda).clamp(max=rows - length)
+    ci = (start[:, None] + torch.arange(length, dtype=torch.int32, device=cuda)).reshape(-1)
+    va = torch.ones(ci.numel(), dtype=dt, device=cuda)
+    x, y = (torch.ones(rows, dtype=dt, device=cuda) for _ in range(2))
+    auto = _best_us(lambda: bsp.csr_spmv(rp, ci, va, x, y))
+    best = min(_best_us(lambda: bsp.csr_spmv(rp, ci, va, x, y, lanes=1 << k)) for k in range(6))
+    assert best >= 0.87 * auto
 
 
 def test_one_lane_on_long_rows_leaves_them_to_a_warp(cuda):
