@@ -1287,9 +1287,19 @@ __global__ void spmm_max_row_kernel(int32_t rows, const int32_t *__restrict__ ro
 constexpr int32_t kSpmmLongRow = 8192;
 constexpr int32_t kSpmmTempChunk = 256;
 
+// The plan's L2 hints apply to slabs of B of at most kHintSlabBytes
+// (cols x slab width), the size that stays in L2 during a pass; wider slabs
+// gather with default caching (graph 2^20, FP16, with the long chunks in row
+// order: hints at N = 32 (64 MB) 0.489 -> 0.473 ms, at N = 128 (one 268 MB slab)
+// 1.822 -> 1.853 ms).
+constexpr double kHintSlabBytes = 64.0 * 1024 * 1024;
+
 }  // namespace bsp
 
 using namespace bsp;
+
+static bsp_status spmm_plan_make(int32_t rows, int32_t nnz, const int32_t *rowPtr, int32_t chunk, int64_t unordered,
+                                 bsp_spmm_plan *out, cudaStream_t s);
 
 extern "C" bsp_status bsp_spmm_csr(int32_t rows, int32_t cols, int32_t nnz, const int32_t *rowPtr,
                                    const int32_t *colIdx, const void *values, bsp_dtype dtype, const void *B,
@@ -1318,7 +1328,12 @@ extern "C" bsp_status bsp_spmm_csr(int32_t rows, int32_t cols, int32_t nnz, cons
     BSP_TRY(st);
     if (h_max > kSpmmLongRow && (int64_t)h_max > 64 * ((int64_t)nnz / rows + 1)) {
       bsp_spmm_plan plan{};
-      BSP_TRY(bsp_spmm_plan_create(rows, nnz, rowPtr, kSpmmTempChunk, &plan, stream));
+      // the chunks' order only matters to the slab engine, where B does not stay in L2 and
+      // they do not all run at once: for one product the sort takes longer than it gains
+      // otherwise (200,000 rows, Zipf 1.8, FP16, N = 32 413 -> 356 us a call)
+      const int64_t es = dtype == BSP_F32 ? 4 : 2;
+      const bool order = N * es % 16 == 0 && (double)cols * std::min<int64_t>(N * es, 512) > kHintSlabBytes;
+      BSP_TRY(spmm_plan_make(rows, nnz, rowPtr, kSpmmTempChunk, order ? 32ll * sm_count() : INT64_MAX, &plan, s));
       const size_t ws = bsp_spmm_plan_workspace(&plan, N);
       void *work = nullptr;
       bsp_status r2 = BSP_OK;
@@ -1827,12 +1842,10 @@ __global__ void spmm_split_flag_kernel(int32_t rows, const int32_t *__restrict__
 
 }  // namespace bsp
 
-extern "C" bsp_status bsp_spmm_plan_create(int32_t rows, int32_t nnz, const int32_t *rowPtr, int32_t chunk,
-                                           bsp_spmm_plan *out, bsp_stream_t stream) {
-  clear_error();
-  BSP_CHECK_ARG(out && rowPtr && rows >= 0 && nnz >= 0, "bad argument");
-  BSP_CHECK_ARG(chunk >= 32, "chunk must be >= 32");
-  cudaStream_t s = as_stream(stream);
+// More than `unordered` chunks of long rows are put in the order of their position in
+// the row (spmm_long_key_kernel).
+static bsp_status spmm_plan_make(int32_t rows, int32_t nnz, const int32_t *rowPtr, int32_t chunk, int64_t unordered,
+                                 bsp_spmm_plan *out, cudaStream_t s) {
   bsp_spmm_plan p{};
   p.rows = rows;
   p.chunk = chunk;
@@ -1905,9 +1918,11 @@ extern "C" bsp_status bsp_spmm_plan_create(int32_t rows, int32_t nnz, const int3
     if (p.nparts > 0) {
       spmm_long_key_kernel<<<g, 256, 0, s>>>(p.nparts, p.long_chunk, p.chunk_row, p.chunk_ptr, keys, long_slot);
       BSP_LAUNCH_CHECK();
-      const bsp_status st = radix_sort_pairs(keys, long_slot, p.nparts, 16, s);
-      if (st != BSP_OK) dfree(keys, s);
-      BSP_TRY(st);
+      if (p.nparts > unordered) {
+        const bsp_status st = radix_sort_pairs(keys, long_slot, p.nparts, 16, s);
+        if (st != BSP_OK) dfree(keys, s);
+        BSP_TRY(st);
+      }
     }
     spmm_short_key_kernel<<<g, 256, 0, s>>>(rows, rowPtr, chunk, keys, p.short_rows);
     BSP_LAUNCH_CHECK();
@@ -1929,6 +1944,14 @@ extern "C" bsp_status bsp_spmm_plan_create(int32_t rows, int32_t nnz, const int3
   BSP_CUDA(cudaStreamSynchronize(s));
   *out = p;
   return BSP_OK;
+}
+
+extern "C" bsp_status bsp_spmm_plan_create(int32_t rows, int32_t nnz, const int32_t *rowPtr, int32_t chunk,
+                                           bsp_spmm_plan *out, bsp_stream_t stream) {
+  clear_error();
+  BSP_CHECK_ARG(out && rowPtr && rows >= 0 && nnz >= 0, "bad argument");
+  BSP_CHECK_ARG(chunk >= 32, "chunk must be >= 32");
+  return spmm_plan_make(rows, nnz, rowPtr, chunk, 0, out, as_stream(stream));
 }
 
 extern "C" bsp_status bsp_spmm_plan_free(bsp_spmm_plan *p) {
@@ -2386,13 +2409,6 @@ static int slab_width(int32_t N, int32_t cols, const void *B, int64_t ldb, int32
   (void)cols;
   return std::min(32 * VEC, N);
 }
-
-// The plan's L2 hints apply to slabs of B of at most kHintSlabBytes
-// (cols x slab width), the size that stays in L2 during a pass; wider slabs
-// gather with default caching (graph 2^20, FP16, with the long chunks in row
-// order: hints at N = 32 (64 MB) 0.489 -> 0.473 ms, at N = 128 (one 268 MB slab)
-// 1.822 -> 1.853 ms).
-constexpr double kHintSlabBytes = 64.0 * 1024 * 1024;
 
 template <typename T>
 static bsp_status slab_typed(const bsp_spmm_plan *p, int32_t nnz, int32_t N, int32_t cols, int32_t width, const int32_t *ci,

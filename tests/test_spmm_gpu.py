@@ -627,3 +627,29 @@ def test_spmm_split_rows_of_many_chunk_groups(cuda, engine, slab):
     want = -2.0 * Cref + 0.75 * Cin.astype(np.float64)
     assert np.all(np.abs(Cd.cpu().numpy().astype(np.float64) - want) <= _tol(A, absC, -2.0, Cin, 0.75))
     P.free()
+
+
+def _whole_numbers(cuda, lens, cols, N, dt, seed):
+    """A and B of small whole numbers (sums exact in FP32), and A B in FP64."""
+    import torch
+    g = torch.Generator(device=cuda).manual_seed(seed)
+    lens = torch.as_tensor(lens, device=cuda)
+    rp = torch.zeros(lens.numel() + 1, dtype=torch.int64, device=cuda)
+    rp[1:] = lens.cumsum(0)
+    nnz = int(rp[-1])
+    ci = torch.randint(0, cols, (nnz,), generator=g, device=cuda)
+    v, B = (torch.randint(-3, 4, s, generator=g, device=cuda).double() for s in ((nnz,), (cols, N)))
+    want = torch.sparse_csr_tensor(rp, ci, v, (lens.numel(), cols)) @ B
+    return rp.int(), ci.int(), v.to(dt), B.to(dt), want
+
+
+# a row of 9,000 and one of 300,000 entries: no order (N = 7, B within 64 MiB), few
+# chunks, and 4,883 chunks in order (B of 128 MiB)
+@pytest.mark.parametrize("cols,N,longest", [(4000, 7, 9000), (4000, 32, 300000), (262144, 128, 9000),
+                                            (262144, 128, 1250000)])
+def test_spmm_unplanned_long_rows(cuda, cols, N, longest):
+    import torch
+    lens = np.resize([0, 1, 5, 2], 4000)
+    lens[1234] = longest
+    rp, ci, v, B, want = _whole_numbers(cuda, lens, cols, N, torch.float32, 3)
+    assert torch.equal(bsp.spmm_csr(rp, ci, v, B).double(), want)
