@@ -2382,7 +2382,13 @@ static bsp_status launch_slab(const bsp_spmm_plan *p, const int32_t *ci, const v
 // One and two lanes only where rows are short (a mean of 8 entries at most): a
 // warp then takes 32 or 16 rows at once, which pays until one of them is long.
 // N = 8 on 500,000 rows of 5: one lane 14 us, four 34; on a graph of 10,000 one
-// lane 47, four 26; N = 16: two lanes 20, four 34.
+// lane 47, four 26; N = 16: two lanes 20, four 34.  And where every row is split into
+// chunks, a warp each: 5,000 rows of 2,000, N = 8, FP16 one lane 33 us, four 51.
+// FP32, 17 to 24 pieces: 16 lanes and a second pass instead of 32 lanes with a quarter or
+// more of them idle (100,000 rows of 100, N = 96 321 -> 254 us, N = 72 319 -> 242; random
+// rows of 5 134 -> 127 and 127 -> 101), where there is work for two passes (kTwoPassNnz)
+// and no mix of split and other rows (Zipf 1.8, N = 72 220 -> 234).
+constexpr int32_t kTwoPassNnz = 5 << 18;
 static int slab_lanes(int n, bool short_rows) {
   int l = 32;
   while (l > (short_rows ? 1 : 4) && n <= l / 2) l >>= 1;
@@ -2418,9 +2424,11 @@ static bsp_status slab_typed(const bsp_spmm_plan *p, int32_t nnz, int32_t N, int
   // rows of B 4 GiB apart or more, or positions near 2^31: one kernel, 4 lanes wide
   const bool wide = (uint64_t)ldb * sizeof(T) > 0xffffffffull || nnz > INT32_MAX - kSlabOvershoot;
   if (wide && width > 4 * VEC) width = 4 * VEC;
-  const bool short_rows = nnz <= 8ll * p->rows;
+  const bool short_rows = nnz <= 8ll * p->rows || p->nshort == 0;
+  const bool two_passes = nnz > kTwoPassNnz && (p->nsplit == 0 || p->nshort == 0);
   for (int32_t col0 = 0, ns; col0 < N; col0 += ns) {
-    const int l = slab_lanes(std::min(width, N - col0) / VEC, !wide && short_rows);
+    int l = slab_lanes(std::min(width, N - col0) / VEC, !wide && short_rows);
+    if (sizeof(T) == 4 && l == 32 && std::min(width, N - col0) <= 24 * VEC && two_passes) l = 16;
     ns = std::min(l * VEC, std::min(width, N - col0));
     const int32_t hints = (double)cols * ns * sizeof(T) <= kHintSlabBytes ? p->slab_l2_hints : 0;
     bsp_status st;

@@ -643,6 +643,25 @@ def _whole_numbers(cuda, lens, cols, N, dt, seed):
     return rp.int(), ci.int(), v.to(dt), B.to(dt), want
 
 
+# every row split into chunks (one and two lanes per B row), FP32 with 17, 20, 24 and 25
+# pieces where rows are whole or all split and there is work for two passes, and both not
+@pytest.mark.parametrize("lens,name,N", [([300] * 900, "float16", 8), ([257, 2000, 999] * 300, "float32", 4),
+                                         ([257, 2000, 999] * 300, "float16", 16),
+                                         ([70] * 20000, "float32", 68), ([70] * 20000, "float32", 80),
+                                         ([70] * 20000, "float32", 96), ([70] * 20000, "float32", 100),
+                                         ([70] * 20000, "float32", 224), ([300] * 5000, "float32", 72),
+                                         ([70] * 20000 + [300], "float32", 72), ([5] * 3000, "float32", 72)])
+def test_spmm_slab_passes_by_row_lengths(cuda, lens, name, N):
+    import torch
+    rp, ci, v, B, want = _whole_numbers(cuda, lens, 4000, N, getattr(torch, name), N)
+    P = bsp.SpmmPlan(rp, ci, v, cols=4000)
+    C = torch.full(want.shape, float("nan"), device=cuda)
+    assert torch.equal(P.spmm(B, C).double(), want)
+    C = torch.ones(want.shape, device=cuda)
+    assert torch.equal(P.spmm(B, C, alpha=2.0, beta=-3.0).double(), 2.0 * want - 3.0)
+    P.free()
+
+
 # a row of 9,000 and one of 300,000 entries: no order (N = 7, B within 64 MiB), few
 # chunks, and 4,883 chunks in order (B of 128 MiB)
 @pytest.mark.parametrize("cols,N,longest", [(4000, 7, 9000), (4000, 32, 300000), (262144, 128, 9000),
@@ -653,3 +672,31 @@ def test_spmm_unplanned_long_rows(cuda, cols, N, longest):
     lens[1234] = longest
     rp, ci, v, B, want = _whole_numbers(cuda, lens, cols, N, torch.float32, 3)
     assert torch.equal(bsp.spmm_csr(rp, ci, v, B).double(), want)
+
+
+@pytest.mark.parametrize("rows,length,name,N,other,share", [(5000, 2000, "float16", 8, 16, 0.9),
+                                                            (100000, 100, "float32", 72, 128, 0.85)])
+def test_spmm_slab_narrow_passes_pay(cuda, rows, length, name, N, other, share):
+    """5,000 split rows of 2,000, FP16, N = 8 against N = 16 (four lanes for either: 0.99);
+    100,000 rows of 100, FP32, N = 72 against N = 128 (32 lanes for either: 0.97)."""
+    import torch
+    dt = getattr(torch, name)
+    rp = torch.arange(0, rows * length + 1, length, dtype=torch.int32, device=cuda)
+    start = torch.arange(rows, dtype=torch.int32, device=cuda).clamp(max=rows - length)
+    ci = (start[:, None] + torch.arange(length, dtype=torch.int32, device=cuda)).reshape(-1)
+    P = bsp.SpmmPlan(rp, ci, torch.ones(ci.numel(), dtype=dt, device=cuda), cols=rows)
+    t = {}
+    for n in (N, other):
+        B, C = torch.ones(rows, n, dtype=dt, device=cuda), torch.empty(rows, n, device=cuda)
+        t[n] = float("inf")
+        for _ in range(6):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            torch.cuda.synchronize()
+            e[0].record()
+            for _ in range(5):
+                P.spmm(B, C)
+            e[1].record()
+            torch.cuda.synchronize()
+            t[n] = min(t[n], e[0].elapsed_time(e[1]))
+    P.free()
+    assert t[N] <= share * t[other]
