@@ -1507,6 +1507,161 @@ static bsp_status cg_chunk(bsp_cg_plan_s *P, cudaStream_t s) {
   return BSP_OK;
 }
 
+static size_t fused_pub_bytes(const bsp_cg_plan_s *P);
+
+// The two-kernel iteration's copy of the matrix: SELL-32 in the mixed modes and, where
+// its rows are short and uniform, in FP64 (else FP64 stays on the CSR arrays).
+#define BSP_CG_ALLOC(x)                                                                   \
+  do {                                                                                    \
+    cudaError_t e_ = (x);                                                                 \
+    if (e_ != cudaSuccess) {                                                              \
+      set_error(std::string("bsp_cg_create: ") + #x + " -> " + cudaGetErrorString(e_));   \
+      return BSP_ERR_ALLOC;                                                               \
+    }                                                                                     \
+  } while (0)
+static bsp_status two_kernel_setup(bsp_cg_plan_s *P, cudaStream_t s, int64_t *mat_bytes) {
+  const int32_t n = P->n;
+  const int32_t *rowPtr = P->rowPtr, *colIdx = P->colIdx;
+  const bool mixed = cg_mixed(P);
+  if (!mixed && P->lpr != 1) return BSP_OK;
+  int64_t padded = 0;
+  // SELL-32 slices: lengths on the device, offsets summed on the host
+  const int64_t ns = ceil_div(n, 32);
+  BSP_TRY(dalloc(&P->slice_len, (size_t)ns, s));
+  BSP_TRY(dalloc(&P->slice_off, (size_t)ns + 1, s));
+  const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(ns, 256), (int64_t)sm_count() * 16));
+  sell_len_kernel<<<gs, 256, 0, s>>>(n, rowPtr, P->slice_len);
+  std::vector<int32_t> hlen((size_t)ns);
+  std::vector<int64_t> hoff((size_t)ns + 1, 0);
+  BSP_CG_ALLOC(cudaMemcpyAsync(hlen.data(), P->slice_len, sizeof(int32_t) * ns, cudaMemcpyDeviceToHost, s));
+  BSP_CG_ALLOC(cudaStreamSynchronize(s));
+  // When padding every slice to the longest costs at most 1/32 more
+  // storage (stencils, banded matrices), the direction kernel computes a
+  // slice's offset instead of loading its length and offset.
+  int32_t lmax = 0;
+  int64_t natural = 0;
+  for (int64_t k = 0; k < ns; ++k) {
+    lmax = std::max(lmax, hlen[k]);
+    natural += 32 * (int64_t)hlen[k];
+  }
+  if (lmax > 0 && ns * 32 * (int64_t)lmax <= natural + natural / 32) {
+    std::fill(hlen.begin(), hlen.end(), lmax);
+    BSP_CG_ALLOC(cudaMemcpyAsync(P->slice_len, hlen.data(), sizeof(int32_t) * ns, cudaMemcpyHostToDevice, s));
+    P->sell_uniform = lmax;
+  }
+  for (int64_t k = 0; k < ns; ++k) hoff[k + 1] = hoff[k] + 32 * (int64_t)hlen[k];
+  padded = hoff[ns];
+  if (padded >= ((int64_t)1 << 31)) {
+    if (mixed) {
+      set_error("bsp_cg_create: the padded low-precision matrix needs >= 2^31 entries");
+      return BSP_ERR_UNSUPPORTED;
+    }
+    P->sell_uniform = 0;  // FP64 stays on the CSR arrays
+  }
+  BSP_CG_ALLOC(cudaMemcpyAsync(P->slice_off, hoff.data(), sizeof(int64_t) * (ns + 1), cudaMemcpyHostToDevice, s));
+  int32_t *bad = nullptr;
+  BSP_TRY(dalloc(&bad, 1, s));
+  cudaMemsetAsync(bad, 0, sizeof(int32_t), s);
+  int64_t gr = ceil_div(n, 256);
+  if (gr > (int64_t)sm_count() * 32) gr = (int64_t)sm_count() * 32;
+  cg_delta_check_kernel<<<(unsigned)gr, 256, 0, s>>>(n, rowPtr, colIdx, bad);
+  int32_t h_bad = 1;
+  BSP_TRY(read_i32(bad, &h_bad, s));
+  dfree(bad, s);
+  P->delta16 = !h_bad;
+  P->sell64 = !mixed && P->delta16 && P->sell_uniform > 0;
+  if (!mixed && !P->sell64) {  // FP64 stays on the CSR arrays
+    dfree(P->slice_len, s);
+    dfree(P->slice_off, s);
+    P->slice_len = nullptr;
+    P->slice_off = nullptr;
+    P->sell_uniform = 0;
+  }
+  if (!mixed && !P->sell64) return BSP_OK;
+  {
+    const bool scaled = mixed && P->opt.mode != BSP_CG_MIXED_F32;
+    const size_t vsz = !mixed ? 8 : P->opt.mode == BSP_CG_MIXED_F32 ? 4 : 2;
+    const bool packed = scaled && P->delta16;
+    if (P->sell64) {
+      // the FP64 copy is an optimisation: without room for it, stay on CSR
+      const size_t ne = (size_t)(padded > 0 ? padded : 1);
+      if (pool_malloc(reinterpret_cast<void **>(&P->lp_val), 8 * ne, s) != cudaSuccess ||
+          pool_malloc(reinterpret_cast<void **>(&P->lp_cols), 2 * ne, s) != cudaSuccess) {
+        cudaGetLastError();
+        if (P->lp_val) pool_free(P->lp_val, s);
+        if (P->lp_cols) pool_free(P->lp_cols, s);
+        P->lp_val = P->lp_cols = nullptr;
+        dfree(P->slice_len, s);
+        dfree(P->slice_off, s);
+        P->slice_len = nullptr;
+        P->slice_off = nullptr;
+        P->sell_uniform = 0;
+        P->sell64 = false;
+      }
+    } else {
+      BSP_CG_ALLOC(pool_malloc(reinterpret_cast<void **>(&P->lp_val), (packed ? 4 : vsz) * (size_t)(padded > 0 ? padded : 1), s));
+      if (!packed)
+        BSP_CG_ALLOC(pool_malloc(reinterpret_cast<void **>(&P->lp_cols), (P->delta16 ? 2 : 4) * (size_t)(padded > 0 ? padded : 1), s));
+    }
+  }
+  if (mixed || P->sell64) {
+    const bool scaled = mixed && P->opt.mode != BSP_CG_MIXED_F32;
+    const size_t vsz = !mixed ? 8 : P->opt.mode == BSP_CG_MIXED_F32 ? 4 : 2;
+    const int64_t ns = ceil_div(n, 32);
+    const bool packed = scaled && P->delta16;
+    int64_t gf = ceil_div(ns * 32, 256);
+    if (gf > (int64_t)sm_count() * 32) gf = (int64_t)sm_count() * 32;
+#define BSP_SELL_FILL(V, SC, D, PK)                                                                          \
+  sell_fill_kernel<V, SC, D, PK><<<(unsigned)gf, 256, 0, s>>>(n, rowPtr, colIdx, P->val, P->slice_len,           \
+                                                              P->slice_off, P->exps, (V *)P->lp_val, P->lp_cols)
+    if (!mixed) {
+      BSP_SELL_FILL(double, false, true, false);
+    } else if (P->opt.mode == BSP_CG_MIXED_F32) {
+      if (P->delta16) BSP_SELL_FILL(float, false, true, false); else BSP_SELL_FILL(float, false, false, false);
+    } else if (P->opt.mode == BSP_CG_MIXED_F16) {
+      if (P->delta16) BSP_SELL_FILL(__half, true, true, true); else BSP_SELL_FILL(__half, true, false, false);
+    } else {
+      if (P->delta16)
+        BSP_SELL_FILL(__nv_bfloat16, true, true, true);
+      else
+        BSP_SELL_FILL(__nv_bfloat16, true, false, false);
+    }
+#undef BSP_SELL_FILL
+    if (cudaGetLastError() != cudaSuccess) {
+      set_error("bsp_cg_create: building the low-precision matrix failed");
+      return BSP_ERR_CUDA;
+    }
+    *mat_bytes = padded * (packed ? 4 : (int64_t)vsz + (P->delta16 ? 2 : 4)) + (scaled ? (int64_t)n : 0) + 12 * ns;
+  }
+  return BSP_OK;
+}
+#undef BSP_CG_ALLOC
+
+// Launch grids of the two kernels and the bytes counted per iteration.
+static void plan_grids(bsp_cg_plan_s *P, int64_t mat_bytes) {
+  const int32_t n = P->n;
+  const bool mixed = cg_mixed(P);
+  const int64_t vt = mixed ? 4 : 8;
+  int oa = 4, ob = 4;  // partials were sized for the largest grid
+  cg_plan_occupancy(P, oa, ob);
+  P->grid_a = cg_grid(n, oa);
+  P->grid = cg_grid(n, ob);
+  // algorithmic bytes.  Two kernels: A reads the matrix, r and p_prev (own rows;
+  // gathers counted once) and writes p and q; B reads p, q, x, r and writes x, r.
+  // Preconditioned: the update kernel also reads M^{-1} and writes z.  Fused: the
+  // diagonals and the published p (value and tag, written and read once) per
+  // iteration, x, r and p in and out once per chunk; the rest stays on the SMs.
+  if (P->fused_ctas) {
+    P->bytes_iter = mat_bytes + 2 * (int64_t)fused_pub_bytes(P);
+    P->bytes_chunk = 6 * vt * n;
+  } else {
+    P->bytes_chunk = 0;
+    P->bytes_iter = mat_bytes + (mixed || P->sell64 ? 0 : 4 * ((int64_t)n + 1)) + 10 * vt * n;
+    if (P->prec_bs)
+      P->bytes_iter += vt * (ceil_div(n, P->prec_bs) * P->prec_bs * P->prec_bs + (int64_t)n);
+  }
+}
+
 struct FusedLaunch {
   const void *kernel, *fill;
   int threads;
@@ -1645,7 +1800,17 @@ static bsp_status fused_setup(bsp_cg_plan_s *P, cudaStream_t s) {
   return BSP_OK;
 }
 
-static bsp_status fused_chunk(bsp_cg_plan_s *P, cudaStream_t s) {
+static void fused_free(bsp_cg_plan_s *P, cudaStream_t s) {
+  dfree(P->slots, s);
+  if (P->pub) pool_free(P->pub, s);
+  if (P->fused_val) pool_free(P->fused_val, s);
+  P->pub = P->fused_val = nullptr;
+  P->fused_ctas = 0;
+}
+
+// *fits: whether the launch was taken; a stream confined to some of the SMs (a green
+// context's) has no room for all CTAs at once.
+static bsp_status fused_chunk(bsp_cg_plan_s *P, cudaStream_t s, bool *fits) {
   const FusedLaunch L = fused_launch(P);
   int iters = P->opt.check_every, npart = P->grid;
   double *epoch = P->sc + 9, *err = P->sc + 8;
@@ -1661,13 +1826,29 @@ static bsp_status fused_chunk(bsp_cg_plan_s *P, cudaStream_t s) {
     BSP_CUDA(cudaStreamWaitEvent(s, done, 0));
   else
     BSP_CUDA(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
-  BSP_CUDA(cudaLaunchCooperativeKernel(L.kernel, dim3(P->fused_ctas), dim3(L.threads), args, P->fused_smem, s));
+  const cudaError_t e =
+      cudaLaunchCooperativeKernel(L.kernel, dim3(P->fused_ctas), dim3(L.threads), args, P->fused_smem, s);
+  *fits = e != cudaErrorCooperativeLaunchTooLarge;
+  if (!*fits) {
+    cudaGetLastError();
+    return BSP_OK;
+  }
+  BSP_CUDA(e);
   BSP_CUDA(cudaEventRecord(done, s));
   return BSP_OK;
 }
 
 static bsp_status cg_run_chunk(bsp_cg_plan_s *P, cudaStream_t s) {
-  if (P->fused_ctas) return fused_chunk(P, s);
+  if (P->fused_ctas) {
+    bool fits = false;
+    BSP_TRY(fused_chunk(P, s, &fits));
+    if (fits) return BSP_OK;
+    // two kernels from here on: x, r, p and the scalars are where they start from
+    int64_t mat_bytes = (int64_t)P->nnz * 12;
+    fused_free(P, s);
+    BSP_TRY(two_kernel_setup(P, s, &mat_bytes));
+    plan_grids(P, mat_bytes);
+  }
   if (!P->opt.use_graphs) return cg_chunk(P, s);
   if (!P->graph) {
     if (!P->graph_stream) BSP_CUDA(cudaStreamCreateWithFlags(&P->graph_stream, cudaStreamNonBlocking));
@@ -1825,9 +2006,7 @@ extern "C" bsp_status bsp_cg_destroy(bsp_cg_plan P) {
   dfree(P->z64, s);
   dfree(P->part_zq, s);
   dfree(P->part_pr, s);
-  dfree(P->slots, s);
-  if (P->pub) pool_free(P->pub, s);
-  if (P->fused_val) pool_free(P->fused_val, s);
+  fused_free(P, s);
   if (P->lp_cols) pool_free(P->lp_cols, s);
   dfree(P->exps, s);
   dfree(P->slice_len, s);
@@ -1938,137 +2117,12 @@ extern "C" bsp_status bsp_cg_create(int32_t n, int32_t nnz, const int32_t *rowPt
     mat_bytes = ceil_div(n, 32) * 32 * kFusedDiags * vsz + (P->exps ? (int64_t)n : 0);
     const int32_t *d = P->fused_diags.d;
     P->delta16 = std::all_of(d, d + kFusedDiags, [](int32_t v) { return v >= -32768 && v <= 32767; });
-  } else if (mixed || try64) {
-    // SELL-32 slices: lengths on the device, offsets summed on the host
-    const int64_t ns = ceil_div(n, 32);
-    BSP_CG_TRY(dalloc(&P->slice_len, (size_t)ns, s));
-    BSP_CG_TRY(dalloc(&P->slice_off, (size_t)ns + 1, s));
-    const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(ns, 256), (int64_t)sm_count() * 16));
-    sell_len_kernel<<<gs, 256, 0, s>>>(n, rowPtr, P->slice_len);
-    std::vector<int32_t> hlen((size_t)ns);
-    std::vector<int64_t> hoff((size_t)ns + 1, 0);
-    BSP_CG_CUDA(cudaMemcpyAsync(hlen.data(), P->slice_len, sizeof(int32_t) * ns, cudaMemcpyDeviceToHost, s));
-    BSP_CG_CUDA(cudaStreamSynchronize(s));
-    // When padding every slice to the longest costs at most 1/32 more
-    // storage (stencils, banded matrices), the direction kernel computes a
-    // slice's offset instead of loading its length and offset.
-    int32_t lmax = 0;
-    int64_t natural = 0;
-    for (int64_t k = 0; k < ns; ++k) {
-      lmax = std::max(lmax, hlen[k]);
-      natural += 32 * (int64_t)hlen[k];
-    }
-    if (lmax > 0 && ns * 32 * (int64_t)lmax <= natural + natural / 32) {
-      std::fill(hlen.begin(), hlen.end(), lmax);
-      BSP_CG_CUDA(cudaMemcpyAsync(P->slice_len, hlen.data(), sizeof(int32_t) * ns, cudaMemcpyHostToDevice, s));
-      P->sell_uniform = lmax;
-    }
-    for (int64_t k = 0; k < ns; ++k) hoff[k + 1] = hoff[k] + 32 * (int64_t)hlen[k];
-    padded = hoff[ns];
-    if (padded >= ((int64_t)1 << 31)) {
-      if (mixed) {
-        set_error("bsp_cg_create: the padded low-precision matrix needs >= 2^31 entries");
-        return fail(BSP_ERR_UNSUPPORTED);
-      }
-      P->sell_uniform = 0;  // FP64 stays on the CSR arrays
-    }
-    BSP_CG_CUDA(cudaMemcpyAsync(P->slice_off, hoff.data(), sizeof(int64_t) * (ns + 1), cudaMemcpyHostToDevice, s));
-    int32_t *bad = nullptr;
-    BSP_CG_TRY(dalloc(&bad, 1, s));
-    cudaMemsetAsync(bad, 0, sizeof(int32_t), s);
-    int64_t gr = ceil_div(n, 256);
-    if (gr > (int64_t)sm_count() * 32) gr = (int64_t)sm_count() * 32;
-    cg_delta_check_kernel<<<(unsigned)gr, 256, 0, s>>>(n, rowPtr, colIdx, bad);
-    int32_t h_bad = 1;
-    BSP_CG_TRY(read_i32(bad, &h_bad, s));
-    dfree(bad, s);
-    P->delta16 = !h_bad;
-    P->sell64 = try64 && P->delta16 && P->sell_uniform > 0;
-    if (try64 && !P->sell64) {  // FP64 stays on the CSR arrays
-      dfree(P->slice_len, s);
-      dfree(P->slice_off, s);
-      P->slice_len = nullptr;
-      P->slice_off = nullptr;
-      P->sell_uniform = 0;
-    }
+  } else {
+    BSP_CG_TRY(two_kernel_setup(P, s, &mat_bytes));
   }
-  const bool sell = !P->fused_ctas && (mixed || P->sell64);
-  if (sell) {
-    const bool scaled = mixed && opt->mode != BSP_CG_MIXED_F32;
-    const size_t vsz = !mixed ? 8 : opt->mode == BSP_CG_MIXED_F32 ? 4 : 2;
-    const bool packed = scaled && P->delta16;
-    if (P->sell64) {
-      // the FP64 copy is an optimisation: without room for it, stay on CSR
-      const size_t ne = (size_t)(padded > 0 ? padded : 1);
-      if (pool_malloc(reinterpret_cast<void **>(&P->lp_val), 8 * ne, s) != cudaSuccess ||
-          pool_malloc(reinterpret_cast<void **>(&P->lp_cols), 2 * ne, s) != cudaSuccess) {
-        cudaGetLastError();
-        if (P->lp_val) pool_free(P->lp_val, s);
-        if (P->lp_cols) pool_free(P->lp_cols, s);
-        P->lp_val = P->lp_cols = nullptr;
-        dfree(P->slice_len, s);
-        dfree(P->slice_off, s);
-        P->slice_len = nullptr;
-        P->slice_off = nullptr;
-        P->sell_uniform = 0;
-        P->sell64 = false;
-      }
-    } else {
-      BSP_CG_CUDA(pool_malloc(reinterpret_cast<void **>(&P->lp_val), (packed ? 4 : vsz) * (size_t)(padded > 0 ? padded : 1), s));
-      if (!packed)
-        BSP_CG_CUDA(pool_malloc(reinterpret_cast<void **>(&P->lp_cols), (P->delta16 ? 2 : 4) * (size_t)(padded > 0 ? padded : 1), s));
-    }
-  }
-  if (sell && (mixed || P->sell64)) {
-    const bool scaled = mixed && opt->mode != BSP_CG_MIXED_F32;
-    const size_t vsz = !mixed ? 8 : opt->mode == BSP_CG_MIXED_F32 ? 4 : 2;
-    const int64_t ns = ceil_div(n, 32);
-    const bool packed = scaled && P->delta16;
-    int64_t gf = ceil_div(ns * 32, 256);
-    if (gf > (int64_t)sm_count() * 32) gf = (int64_t)sm_count() * 32;
-#define BSP_SELL_FILL(V, SC, D, PK)                                                                          \
-  sell_fill_kernel<V, SC, D, PK><<<(unsigned)gf, 256, 0, s>>>(n, rowPtr, colIdx, values, P->slice_len,           \
-                                                              P->slice_off, P->exps, (V *)P->lp_val, P->lp_cols)
-    if (!mixed) {
-      BSP_SELL_FILL(double, false, true, false);
-    } else if (opt->mode == BSP_CG_MIXED_F32) {
-      if (P->delta16) BSP_SELL_FILL(float, false, true, false); else BSP_SELL_FILL(float, false, false, false);
-    } else if (opt->mode == BSP_CG_MIXED_F16) {
-      if (P->delta16) BSP_SELL_FILL(__half, true, true, true); else BSP_SELL_FILL(__half, true, false, false);
-    } else {
-      if (P->delta16)
-        BSP_SELL_FILL(__nv_bfloat16, true, true, true);
-      else
-        BSP_SELL_FILL(__nv_bfloat16, true, false, false);
-    }
-#undef BSP_SELL_FILL
-    if (cudaGetLastError() != cudaSuccess) {
-      set_error("bsp_cg_create: building the low-precision matrix failed");
-      return fail(BSP_ERR_CUDA);
-    }
-    mat_bytes = padded * (packed ? 4 : (int64_t)vsz + (P->delta16 ? 2 : 4)) + (scaled ? (int64_t)n : 0) + 12 * ns;
-  }
-  {  // partials were sized for the largest grid
-    int oa = 4, ob = 4;
-    cg_plan_occupancy(P, oa, ob);
-    P->grid_a = cg_grid(n, oa);
-    P->grid = cg_grid(n, ob);
-  }
+  plan_grids(P, mat_bytes);
 #undef BSP_CG_TRY
 #undef BSP_CG_CUDA
-  // algorithmic bytes.  Two kernels: A reads the matrix, r and p_prev (own rows;
-  // gathers counted once) and writes p and q; B reads p, q, x, r and writes x, r.
-  // Preconditioned: the update kernel also reads M^{-1} and writes z.  Fused: the
-  // diagonals and the published p (value and tag, written and read once) per
-  // iteration, x, r and p in and out once per chunk; the rest stays on the SMs.
-  if (P->fused_ctas) {
-    P->bytes_iter = mat_bytes + 2 * (int64_t)fused_pub_bytes(P);
-    P->bytes_chunk = 6 * (int64_t)vt * n;
-  } else {
-    P->bytes_iter = mat_bytes + (mixed || P->sell64 ? 0 : 4 * ((int64_t)n + 1)) + 10 * (int64_t)vt * n;
-    if (P->prec_bs)
-      P->bytes_iter += (int64_t)vt * (ceil_div(n, P->prec_bs) * P->prec_bs * P->prec_bs + (int64_t)n);
-  }
   P->bytes_residual = (int64_t)nnz * 12 + 4 * ((int64_t)n + 1) + 3 * 8 * (int64_t)n;
   // flexible outer step: F1 8n+8n+8n, F2 24n, F3 matrix + 4(n+1) + 32n, F4 52n
   P->bytes_outer = (int64_t)nnz * 12 + 4 * ((int64_t)n + 1) + 132 * (int64_t)n;

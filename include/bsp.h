@@ -668,12 +668,13 @@ bsp_status bsp_cg_destroy(bsp_cg_plan plan);
  * columns whose vectors fit the SMs' shared memory (16 bytes a row in the mixed
  * modes, 32 in FP64) runs check_every iterations in one cooperative launch of
  * *ctas CTAs, except where two kernels are the faster iteration (FP64 from 18,000 to
- * 180,000 rows, FP32 from 36,000 to 120,000); *ctas = 0: two kernels per iteration.  That launch needs its SMs all
- * at once (it fails on a stream confined to fewer), so fused solves of a device
- * take turns, whatever their streams.  Its CTAs wait for one another, at most `polls`
- * reads per grid sum (the default, 2^23, takes seconds; more are not waited for).  A
- * wait that runs out ends the solve with BSP_ERR_TIMEOUT, x as it was and the plan
- * ready for another solve. */
+ * 180,000 rows, FP32 from 36,000 to 120,000); *ctas = 0: two kernels per iteration.
+ * That launch needs its SMs all at once, so fused solves of a device take turns,
+ * whatever their streams; on a stream confined to fewer SMs (a green context's) the
+ * plan goes over to two kernels for good.  Its CTAs wait for one another, at most
+ * `polls` reads per grid sum (the default, 2^23, takes seconds; more are not waited
+ * for).  A wait that runs out ends the solve with BSP_ERR_TIMEOUT, x as it was and the
+ * plan ready for another solve. */
 bsp_status bsp_cg_fused_ctas(bsp_cg_plan plan, int32_t *ctas);
 bsp_status bsp_cg_set_wait_limit(bsp_cg_plan plan, uint32_t polls);
 /* k right-hand sides at once: A X = B with B, X device arrays, row-major with

@@ -344,3 +344,39 @@ def test_cg_two_kernels_between_the_sizes(cuda, mode, n, fused):
     S.close()
     assert res["converged"] == 1
     assert pyoracle.rel_residual(A.rowptr, A.colidx, A.values, b, x.cpu().numpy()) <= 2e-10
+
+
+@pytest.mark.parametrize("mode", ["fp64", "f16"])
+def test_cg_on_a_stream_of_fewer_sms(cuda, mode):
+    """A stream confined to 16 SMs has no room for the fused launch: the plan goes over
+    to two kernels and solves."""
+    import torch
+    drv = pytest.importorskip("cuda.bindings.driver")
+
+    def ok(r):
+        assert int(r[0]) == 0, r[0]
+        return r[1] if len(r) == 2 else r[1:]
+
+    A = bsp.gen_poisson3d(64)
+    b = bsp.gen_uniform(A.rows, 21)
+    rp, ci, va, bb = _dev(cuda, A.rowptr, A.colidx, A.values, b)
+    S = bsp.CgSolver(rp, ci, va, mode=mode, tol=1e-10)
+    assert S.fused_ctas > 16
+    dev = ok(drv.cuDeviceGet(0))
+    sms = ok(drv.cuDeviceGetDevResource(dev, drv.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    part = ok(drv.cuDevSmResourceSplitByCount(1, sms, 0, 16))[0]
+    ctx = ok(drv.cuGreenCtxCreate(ok(drv.cuDevResourceGenerateDesc([part[0]], 1)), dev,
+                                  drv.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+    raw = ok(drv.cuGreenCtxStreamCreate(ctx, drv.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+    stream = torch.cuda.ExternalStream(int(raw))
+    torch.cuda.synchronize()
+    x, res = S.solve(bb, torch.zeros_like(bb), stream=stream)
+    stream.synchronize()
+    assert res["converged"] == 1 and S.fused_ctas == 0
+    assert pyoracle.rel_residual(A.rowptr, A.colidx, A.values, b, x.cpu().numpy()) <= 2e-10
+    _, again = S.solve(bb)                     # the whole device: two kernels too
+    assert again["converged"] == 1
+    S.close()
+    torch.cuda.synchronize()
+    ok(drv.cuStreamDestroy(raw) + (None,))
+    ok(drv.cuGreenCtxDestroy(ctx) + (None,))
