@@ -1725,7 +1725,11 @@ static bsp_status fused_reset(bsp_cg_plan_s *P, cudaStream_t s) {
 // 7.5, 32^3 8.7 / 7.5 (200^2 7.9 / 7.0), 48^3 9.7 / 8.9, 56^3 10.5 / 10.4, 64^3 11.3 /
 // 11.9; FP32 32^3 8.5 / 8.7, 36^3 9.6 / 8.7, 48^3 9.9 / 9.5 (256^2 7.4 / 7.2), 52^3
 // 10.0 / 10.7.  FP16 differs by 3% either way there (40^3 7.8 / 8.9) and stays fused.
-static bool two_kernels_faster(int mode, int32_t n) {
+// A launch of 2 iterations pays for loading and storing the vectors: FP16 16^3 17.4 / 17.0,
+// 48^3 18.6 / 16.2, 64^3 20.7 / 20.0, 700^2 20.5 / 19.8, 100^3 27.0 / 29.1; from 4 on the
+// two differ by 3%.
+static bool two_kernels_faster(int mode, int32_t n, int check_every) {
+  if (check_every < 4 && n < 600000) return true;
   switch (mode) {
     case BSP_CG_FP64: return n > 18000 && n < 180000;
     case BSP_CG_MIXED_F32: return n > 36000 && n < 120000;
@@ -1738,7 +1742,7 @@ static bool two_kernels_faster(int mode, int32_t n) {
 // in every row, and at most kFusedDiags distinct diagonals that the rows fill by
 // 3/4 or more.
 static bsp_status fused_setup(bsp_cg_plan_s *P, cudaStream_t s) {
-  if (P->prec_bs || two_kernels_faster(P->opt.mode, P->n)) return BSP_OK;
+  if (P->prec_bs || two_kernels_faster(P->opt.mode, P->n, P->opt.check_every)) return BSP_OK;
   const size_t vt = cg_mixed(P) ? 4 : 8;
   int dev = 0, coop = 0, optin = 0, sms = 0, occ = 0;
   BSP_CUDA(cudaGetDevice(&dev));

@@ -668,7 +668,8 @@ bsp_status bsp_cg_destroy(bsp_cg_plan plan);
  * columns whose vectors fit the SMs' shared memory (16 bytes a row in the mixed
  * modes, 32 in FP64) runs check_every iterations in one cooperative launch of
  * *ctas CTAs, except where two kernels are the faster iteration (FP64 from 18,000 to
- * 180,000 rows, FP32 from 36,000 to 120,000); *ctas = 0: two kernels per iteration.
+ * 180,000 rows, FP32 from 36,000 to 120,000, check_every = 2 below 600,000);
+ * *ctas = 0: two kernels per iteration.
  * That launch needs its SMs all at once, so fused solves of a device take turns,
  * whatever their streams; on a stream confined to fewer SMs (a green context's) the
  * plan goes over to two kernels for good.  Its CTAs wait for one another, at most

@@ -380,3 +380,13 @@ def test_cg_on_a_stream_of_fewer_sms(cuda, mode):
     torch.cuda.synchronize()
     ok(drv.cuStreamDestroy(raw) + (None,))
     ok(drv.cuGreenCtxDestroy(ctx) + (None,))
+
+
+@pytest.mark.parametrize("n,every,fused", [(599999, 1, False), (599999, 4, True), (600000, 2, True)])
+def test_cg_form_by_check_every(cuda, n, every, fused):
+    A = _banded(n, [1, 50], n)
+    rp, ci, va, b = _dev(cuda, A.rowptr, A.colidx, A.values, bsp.gen_uniform(n, 15))
+    S = bsp.CgSolver(rp, ci, va, mode="f16", check_every=every)
+    assert (S.fused_ctas > 0) == fused
+    assert S.solve(b)[1]["converged"] == 1
+    S.close()
