@@ -2357,10 +2357,12 @@ static bsp_status launch_slab(const bsp_spmm_plan *p, const int32_t *ci, const v
   // of many short rows (graph 2^20, FP16, N = 128: 64 per SM 0.818 ms, 256
   // 0.836, one task per warp 0.888; before the steps below 32 per SM 1.174
   // against 1.119, only the resident CTAs 1.37; 500,000 rows of 5, N = 256: 64
-  // per SM 258 us, 256 283, one task per warp 306).
+  // per SM 258 us, 256 283, one task per warp 306).  FP32 in 16 lanes or fewer, no split
+  // rows to keep in step: 32 (N = 32: 300,000 rows of 5 39.1 -> 35.9 us, 200,000 of 27 55.5
+  // -> 53.5; N = 64: 77.2 -> 74.0 and 105.1 -> 103.7; with split rows N = 32 89.7 -> 92.7).
   const bool vec_c = (uintptr_t)C % 16 == 0 && ldc % 4 == 0 && col0 % 4 == 0;
   int64_t blocks = ceil_div(ntasks, 8);
-  const int64_t cap = (int64_t)sm_count() * 64;
+  const int64_t cap = (int64_t)sm_count() * (sizeof(T) == 4 && LPR <= 16 && p->nsplit == 0 ? 32 : 64);
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
   spmm_slab_kernel<T, LPR, SlabU<LPR>::U, SlabU<LPR>::UL, WIDE><<<(unsigned)blocks, 256, 0, s>>>(
